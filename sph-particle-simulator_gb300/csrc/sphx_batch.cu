@@ -29,6 +29,7 @@ __global__ void k_batch_begin(SceneInfo* scenes, int nscenes, DevState* ds) {
         ds->n_tiles = 0;
         ds->work[0] = 0;
         ds->work[1] = 0;
+        ds->general = 0;
     }
     if (s >= nscenes) return;
     SceneInfo& sc = scenes[s];
@@ -106,7 +107,7 @@ int launch_batch_cfl(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, 
 // ---- grid ------------------------------------------------------------------------------
 
 __global__ void k_batch_bbox(const float4* __restrict__ pos4, const uint32_t* __restrict__ scene_of,
-                             int n, SceneInfo* scenes) {
+                             int n, SceneInfo* scenes, DevState* ds) {
     const int lane = threadIdx.x & 31;
     for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base < n;
          base += gridDim.x * blockDim.x) {
@@ -119,6 +120,7 @@ __global__ void k_batch_bbox(const float4* __restrict__ pos4, const uint32_t* __
             s = scene_of[i];
             const float4 p = pos4[i];
             fin = finite3(p.x, p.y, p.z);
+            if (tiny_coord(p.x) || tiny_coord(p.y) || tiny_coord(p.z)) ds->general = 1;
             if (fin) {
                 const float ic = scenes[s].c.inv_cell;
                 c[0] = d[0] = cell_coord(p.x, ic);
@@ -209,10 +211,10 @@ __global__ void k_batch_keys(const float4* __restrict__ pos4, const uint32_t* __
 int launch_batch_grid(const LaunchCtx& L, const Buffers& b, DevState* ds, int n,
                       uint32_t max_cells) {
     const int gb = blocks_for(L, n, 256);
-    k_batch_bbox<<<gb, 256, 0, L.stream>>>(b.pos4, b.scene_of, n, b.scenes);
+    k_batch_bbox<<<gb, 256, 0, L.stream>>>(b.pos4, b.scene_of, n, b.scenes, ds);
     k_batch_grid_setup<<<1, 32, 0, L.stream>>>(b.scenes, b.nscenes, max_cells, ds);
     k_batch_keys<<<gb, 256, 0, L.stream>>>(b.pos4, b.scene_of, n, b.scenes, ds, b.key[0]);
-    return 3 + launch_grid_sort(L, b, ds, n, 0.0f);
+    return 3 + launch_grid_sort(L, b, ds, n, StepConst{});  // (scenes carry their own)
 }
 
 // ---- FP64 diagnostics per scene (one block per scene, fixed order) ----------------------

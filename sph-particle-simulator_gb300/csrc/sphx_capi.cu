@@ -42,7 +42,7 @@ struct sphx_ctx {
     // or the stats are requested, so profiling adds no per-step host sync
     // batched scenes
     uint32_t nscenes = 0;
-    bool scenes_nz = false;  // every scene's divisors admit the untested divisions (div_nz)
+    bool scenes_div_nz = false, scenes_force_nz = false;  // StepConst's flags hold for every scene
     uint32_t scene_cap = 0;
     std::vector<sphx_params> scene_params;
     std::vector<uint64_t> scene_start;
@@ -203,10 +203,31 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
     s.div_nz = s.fast_div_h && s.fast_div_hsq && p.neighbor_search_radius > 0.0f &&
                        p.neighbor_search_radius <= 0x1p99f
                    ? 1 : 0;
+    // the force pass's divisions by |r| or |r| h through one reciprocal, and of the cubic
+    // spline's gradient components by h: with |x_t - x_j| per axis 0 or at least 2^-68, the
+    // smallest nonzero component is at least gmin 2^-68 / r, gmin the smallest nonzero
+    // gradient factor -- sigma 2^-47 for 2 - q >= 2^-23, 0.49 sigma q for q >= 1e-6 / h
+    s.force_nz = 0;
+    if (s.div_nz && p.neighbor_search_radius <= 0x1p20f) {
+        const double r = p.neighbor_search_radius, q1 = 0.49 * std::min(1e-6 / h, 1.0);
+        const double gmin = (double)s.sigma * std::min(0x1p-47, q1);
+        s.force_nz = kernel == SPHX_KERNEL_WENDLAND_C2 || gmin * 0x1p-68 / r >= 0x1p-99;
+    }
     s.precise = mode != SPHX_MODE_EXACT;
     s.fp16 = mode == SPHX_MODE_PRECISE_FP16;
     s.cs = p.neighbor_search_radius;
     s.cs_d = (double)p.neighbor_search_radius;
+    auto both = [](float x) {
+        uint32_t u;
+        std::memcpy(&u, &x, 4);
+        return (unsigned long long)u << 32 | u;
+    };
+    s.lit = PairLits{both(-0.0f), both(0.5f), both(1.0f), both(2.0f), both(-2.0f), both(3.0f),
+                     both(1.5f), both(-0x1p40f), both(0x1p-20f), both(-0x1p-20f), both(0x1p21f),
+                     both(kTwoThirds), both(kOneSixth), both(-5.0f), both(5.0f)};
+    s.pair = PairConst{both(-h), both(h), both(s.rcp_h), both(-s.h_sq), both(s.rcp_hsq),
+                       both(s.sigma), both(-s.sigma), both(s.gas), both(s.rest), both(s.wnorm),
+                       both(s.wl)};
     s.sw_cs = s.cs * s.rcp_h;  // 2 exactly for r_search = 2h
     s.sw_r2 = s.r2 * s.rcp_hsq;
     s.sw_r2m = s.sw_r2 * 1.0001f;
@@ -242,9 +263,9 @@ void free_all(sphx_ctx* c) {
     Buffers& b = c->b;
     void* ptrs[] = {b.pos4, b.vel4,   b.pos4_s, b.vel4_s,     b.aux4_s,    b.acc4_s,
                     b.key[0], b.key[1], b.val[0], b.val[1],   b.key_s,     b.id_s,
-                    b.off,  b.tile_start, b.hist, b.scan_part, b.diag_part, c->ds,
+                    b.off,  b.tiles, b.tgt, b.hist, b.scan_part, b.diag_part, c->ds,
                     c->stage, c->snap_pos, c->snap_vel, c->snap_cell, b.cell4, b.cell4_s,
-                    b.spread_tiles, b.runs,
+                    b.spread_tiles,
                     b.scene_of, b.scene_s, b.scenes, b.hitmask, b.tile_slot,
                     c->r_colors, c->r_inst, c->r_keys, c->r_rgba};
     for (void* p : ptrs)
@@ -330,7 +351,10 @@ int run_phases(sphx_ctx* c, float dt, bool integrate) {
         SPHX_CUDA(cudaEventRecord(slot->ev[0], c->stream));
     }
     const bool batch = c->b.nscenes > 0;
-    if (batch) c->sc.div_nz = c->scenes_nz ? 1 : 0;  // the passes' kernels serve all scenes
+    if (batch) {  // the passes' kernels serve all scenes
+        c->sc.div_nz = c->scenes_div_nz ? 1 : 0;
+        c->sc.force_nz = c->scenes_force_nz ? 1 : 0;
+    }
     int k = 0;
     if (batch) {
         k += launch_batch_begin(c->L, c->b, c->ds);
@@ -623,7 +647,7 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     if (c->tuning.tile_particles <= 0 || c->tuning.tile_particles > kTile)
         c->tuning.tile_particles = kTile;
     c->b.tile_n = c->tuning.tile_particles;
-    c->b.columns = c->tuning.mode != SPHX_MODE_EXACT ? 1 : 0;  // the precision-mode sweeps' tiles
+    c->b.columns = 1;
     c->tuning.bulk_copy = c->tuning.bulk_copy ? 1 : 0;
     int rc = SPHX_OK;
     auto fail = [&](int code) {
@@ -641,7 +665,6 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     c->L.num_sms = sms > 0 ? sms : 1;
     c->L.warps_per_block = c->tuning.warps_per_block;
     c->L.blocks_per_sm = c->tuning.blocks_per_sm;
-    c->L.bulk_copy = c->tuning.bulk_copy;
     c->L.stream = c->stream;
     c->capacity = capacity;
     int64_t max_cells = c->tuning.max_grid_cells;
@@ -666,16 +689,16 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
         (rc = dmalloc(&b.key[1], C)) || (rc = dmalloc(&b.val[0], C)) ||
         (rc = dmalloc(&b.val[1], C)) || (rc = dmalloc(&b.key_s, C)) ||
         (rc = dmalloc(&b.id_s, C)) || (rc = dmalloc(&b.off, (size_t)max_cells + 2)) ||
-        (rc = dmalloc(&b.tile_start, C)) || (rc = dmalloc(&b.hist, hist_n)) ||
+        (rc = dmalloc(&b.tiles, C)) || (rc = dmalloc(&b.hist, hist_n)) ||
         (rc = dmalloc(&b.scan_part, (size_t)b.scan_part_cap)) ||
         (rc = dmalloc(&b.diag_part, (size_t)b.diag_blocks * kDiagSums)) ||
         (rc = dmalloc(&c->ds, 1)) || (rc = dmalloc(&c->stage, 11 * C)))
         return fail(rc);
     if (c->tuning.mode != SPHX_MODE_EXACT &&
         ((rc = dmalloc(&b.cell4, C)) || (rc = dmalloc(&b.cell4_s, C)) ||
-         (rc = dmalloc(&b.spread_tiles, C)) ||
-         (rc = dmalloc(&b.runs, (size_t)max_cells + 1))))
+         (rc = dmalloc(&b.spread_tiles, C))))
         return fail(rc);
+    if (c->tuning.mode == SPHX_MODE_EXACT && (rc = dmalloc(&b.tgt, C))) return fail(rc);
     // Hit-mask pool (exact mode; the precision mode's sweeps keep no records): 4 records
     // (128 B each) per particle of capacity.  A dense state needs about 1.7-2.6 per particle
     // (32-particle tiles, 27-cell stencil); the rest is slack for the uneven split of tiles
@@ -777,8 +800,12 @@ int sphx_set_kernel(sphx_ctx* c, int kernel) {
             std::vector<SceneInfo> info(c->nscenes);
             SPHX_CUDA(cudaMemcpy(info.data(), c->b.scenes, c->nscenes * sizeof(SceneInfo),
                                  cudaMemcpyDeviceToHost));
-            for (uint32_t s = 0; s < c->nscenes; ++s)
+            c->scenes_div_nz = c->scenes_force_nz = true;
+            for (uint32_t s = 0; s < c->nscenes; ++s) {
                 fill_step_const_from(c, c->scene_params[s], info[s].count, info[s].c);
+                c->scenes_div_nz = c->scenes_div_nz && info[s].c.div_nz;
+                c->scenes_force_nz = c->scenes_force_nz && info[s].c.force_nz;
+            }
             SPHX_CUDA(cudaMemcpy(c->b.scenes, info.data(), c->nscenes * sizeof(SceneInfo),
                                  cudaMemcpyHostToDevice));
         }
@@ -933,15 +960,19 @@ int sphx_set_scenes(sphx_ctx* c, uint32_t nscenes, const uint64_t* scene_start,
         fill_step_const_from(c, params[s], si.count, si.c);
         for (uint64_t i = scene_start[s]; i < scene_start[s + 1]; ++i) owner[i] = s;
     }
-    bool all_nz = true;
-    for (const SceneInfo& si : info) all_nz = all_nz && si.c.div_nz;
+    bool div_nz = true, force_nz = true;
+    for (const SceneInfo& si : info) {
+        div_nz = div_nz && si.c.div_nz;
+        force_nz = force_nz && si.c.force_nz;
+    }
     SPHX_CUDA(cudaStreamSynchronize(c->stream));
     SPHX_CUDA(cudaMemcpy(b.scenes, info.data(), nscenes * sizeof(SceneInfo), cudaMemcpyHostToDevice));
     if (c->n) SPHX_CUDA(cudaMemcpy(b.scene_of, owner.data(), c->n * sizeof(uint32_t), cudaMemcpyHostToDevice));
     c->scene_params.assign(params, params + nscenes);
     c->scene_start.assign(scene_start, scene_start + nscenes + 1);
     c->nscenes = nscenes;
-    c->scenes_nz = all_nz;
+    c->scenes_div_nz = div_nz;
+    c->scenes_force_nz = force_nz;
     b.nscenes = (int)nscenes;
     if (!c->have_params) {  // the context-wide parameters default to the first scene's
         c->params = params[0];
@@ -1039,27 +1070,6 @@ int sphx_autotune(sphx_ctx* c, float dt, int* warps_per_block, int* blocks_per_s
     }
     c->b.tile_n = bt;
     c->tuning.tile_particles = bt;
-    // then the force pass's staging: bulk copies against the lanes' own loads
-    int bbulk = c->L.bulk_copy;
-    if (!rc && c->tuning.mode == SPHX_MODE_EXACT) {
-        c->L.bulk_copy = !bbulk;
-        if (!(rc = reset()) && !(rc = run_phases(c, dt, true)) && !(rc = reset())) {
-            SPHX_CUDA(cudaEventRecord(e0, c->stream));
-            if (!(rc = run_phases(c, dt, true)) && !(rc = reset()) &&
-                !(rc = run_phases(c, dt, true))) {
-                SPHX_CUDA(cudaEventRecord(e1, c->stream));
-                SPHX_CUDA(cudaEventSynchronize(e1));
-                float ms = 0.0f;
-                SPHX_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                if (ms < best) {
-                    best = ms;
-                    bbulk = c->L.bulk_copy;
-                }
-            }
-        }
-    }
-    c->L.bulk_copy = bbulk;
-    c->tuning.bulk_copy = bbulk;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     c->L.warps_per_block = bw;
@@ -1345,6 +1355,7 @@ int sphx_debug_pairs(sphx_ctx* c, int64_t* counts, int64_t* idx, size_t* total_i
     // the lists come in the reference's order: insertion order within each cell
     Buffers bq = c->b;
     bq.columns = 0;
+    bq.tgt = nullptr;
     launch_build_grid(c->L, c->sc, bq, c->ds);
     uint32_t* d_cnt = nullptr;
     if ((rc = dmalloc(&d_cnt, n))) return rc;
@@ -1407,6 +1418,7 @@ int sphx_debug_pairs_subset(sphx_ctx* c, size_t nsel, const int64_t* sel, int64_
     // the lists come in the reference's order: insertion order within each cell
     Buffers bq = c->b;
     bq.columns = 0;
+    bq.tgt = nullptr;
     launch_build_grid(c->L, c->sc, bq, c->ds);
     uint32_t* d_cnt = nullptr;
     if ((rc = dmalloc(&d_cnt, n))) return rc;

@@ -9,196 +9,195 @@ namespace sphx {
 //                      P_i = k (rho_i - rho0)
 // (compute_density / compute_pressure, sph_engine.cpp:370-388)
 // ---------------------------------------------------------------------------------------
+// Per warp: the candidate ring as coordinate arrays (the distance test reads four candidates'
+// x, y or z in one 128-bit load), their masses, the lanes' masks, the tile's row segments.
+// 16 chunks (10.9 KB a warp, 20 warps per SM) let the lanes run as far apart as they want to
+// on the lattice; 8 and 12 chunks (24 warps) took 1.08 and 1.03 ms on the 1M dam break where
+// 16 take 0.97, 20 (16 warps) 1.05.
+//
+// Bound: instruction issue (72% of the slots) and the FP32 pipe (56%; a packed instruction
+// holds it two cycles).  Of 841 warp instructions per particle about 210 are distance tests
+// (900 kept candidates per tile, 29 chunks), 80 the walk and box cull, 500 the pair terms
+// (5 turns of two neighbours per lane and particle).  1M dam break: 0.96 ms; with hit lists
+// worked through by the whole warp and folded back lane by lane (1,502 instructions, of which
+// the lists and folds were half) 1.45 ms.
+constexpr int kDensityRing = 16;
 struct DensitySmem {
-    float4 box_lo, box_hi;  // tile box (culling test)
-    uint32_t mcur, mend;    // the warp's region of the hit-mask pool: [mcur, mend)
-    int2 seg[kMaxSegments]; // the tile's row segments
-    float4 cand[32];
-    __align__(8) float cx[32];  // the candidates' coordinates again, as arrays: the exact
-    __align__(8) float cy[32];  // test reads two candidates' x (y, z) in one 64-bit load
-    __align__(8) float cz[32];
-    float4 tpos[32];
-    uint16_t plist[32 * 32];
-    float tbuf[kDensityBatch];
+    float cx[kDensityRing * 32], cy[kDensityRing * 32], cz[kDensityRing * 32];
+    float cm[kDensityRing * 32];
+    uint32_t mask[kDensityRing * 32];
+    int2 seg[kMaxSegments + 1];
 };
+static_assert(sizeof(DensitySmem) % 16 == 0, "per-warp regions stay 16-byte aligned");
 
-// Cells holding more particles than this after the grid build mark a collapsed state, in
-// which whole chunks are dense (every particle of a tile within r of every candidate).
-constexpr uint32_t kDenseOccupancy = 128;
-
-// kDense: the variant with the dense-chunk path.  Both variants are launched every step;
-// each returns at once unless the grid's fullest cell says the state is its case, so the
-// lattice-like states run the leaner code and the collapsed ones get the dense path.
-template <bool kBatch, int kKern, bool kNZ, bool kDense>
-__global__ void __launch_bounds__(128, kDense ? 9 : 10) k_density(
-    const StepConst cp, const Buffers b, DevState* ds) {
+// kNZ: the pair forms' divisions are in range (StepConst::div_nz)
+template <bool kBatch, int kKern, bool kNZ>
+__global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Buffers b,
+                                                    DevState* ds) {
     if (ds->status) return;
-    if (kDense != (ds->max_occ > kDenseOccupancy)) return;
     extern __shared__ __align__(16) unsigned char smem_raw_d[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     DensitySmem* S = reinterpret_cast<DensitySmem*>(smem_raw_d) + warp;
     const uint32_t ntiles = ds->n_tiles;
     // this warp's region of the hit-mask pool, filled tile after tile (record indices fit
     // 32 bits: the pool holds at most 0xffff0000 records)
-    if (lane == 0) {
+    uint32_t mcur, mend;
+    {
         const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
         const uint32_t region = b.hitmask ? (uint32_t)(b.hitmask_cap / nwarps) : 0u;
-        S->mcur = (blockIdx.x * (blockDim.x >> 5) + warp) * region;
-        S->mend = S->mcur + region;
+        mcur = (blockIdx.x * (blockDim.x >> 5) + warp) * region;
+        mend = mcur + region;
     }
-    __syncwarp();
-    const float inf = __int_as_float(0x7f800000);
+    const uint32_t lt = (1u << lane) - 1u;
+    const F2 neg0{cp.lit.neg0};
+    const bool nz = kNZ && !ds->general;
     uint32_t my_max = 0;
     for (uint32_t t = next_tile(&ds->work[0], lane); t < ntiles; t = next_tile(&ds->work[0], lane)) {
-        const uint32_t k0 = b.tile_start[t];
-        const int scene = kBatch ? (int)b.scene_s[k0] : 0;
+        const uint2 tile = b.tiles[t];
+        const int scene = kBatch ? (int)b.scene_s[tile.x] : 0;
         const StepConst& c = kBatch ? b.scenes[scene].c : cp;
         const Geom g = kBatch ? scene_geom(b.scenes[scene], ds) : grid_geom(ds);
         const float r2m = c.r2 * 1.0001f;
         Tile T;
         float4 xi;
         bool valid;
-        tile_setup(c, b, g, k0, lane, T, xi, valid);
-        const int i = T.k0 + lane;
-        {
-            const TileBox B = tile_box(xi, valid);
-            if (lane == 0) {
-                S->box_lo = make_float4(B.lo[0], B.lo[1], B.lo[2], 0.0f);
-                S->box_hi = make_float4(B.hi[0], B.hi[1], B.hi[2], 0.0f);
-            }
-        }
-        S->tpos[lane] = xi;
-        float rho = xmul(xi.w, c.w0);
-        uint32_t nn = 0;
-        // hit-mask records of this tile: from the warp's cursor on, one per chunk
-        __syncwarp();
-        const uint32_t slot = S->mcur, room = S->mend - slot;
-        uint32_t nrec = 0;
+        int i;
+        tile_setup(c, b, g, tile, lane, T, i, xi, valid);
+        const TileBox B = tile_box(xi, valid);
+        __syncwarp();  // the previous tile's segments are read
         const int nseg = build_segments(b, g, T, lane, S->seg);
         __syncwarp();
-        for (int sg = 0; sg < nseg; ++sg) {
-            const int2 se = S->seg[sg];
-            const int a = se.x, e = se.y;
-            for (int s = a; s < e; s += kTile, ++nrec) {
-                const int m = min(kTile, e - s);
-                __syncwarp();
-                const float4 pl = lane < m ? b.pos4_s[s + lane] : make_float4(inf, inf, inf, 0.f);
-                S->cand[lane] = pl;
-                S->cx[lane] = pl.x;
-                S->cy[lane] = pl.y;
-                S->cz[lane] = pl.z;
-                TileBox B;
-                {
-                    const float4 lo = S->box_lo, hi = S->box_hi;
-                    B.lo[0] = lo.x, B.lo[1] = lo.y, B.lo[2] = lo.z;
-                    B.hi[0] = hi.x, B.hi[1] = hi.y, B.hi[2] = hi.z;
+        // records of this tile: ceil(nraw / 32) of kept-candidate words, then the masks
+        const uint32_t hdr = (uint32_t)(raw_chunks(S->seg, nseg, lane) + 31) >> 5;
+        const uint32_t room = mend - mcur;
+        uint32_t* const rec = b.hitmask + (size_t)mcur * 32 + lane;
+        RawStream st(S->seg, nseg);
+        float4 pl = make_float4(0.f, 0.f, 0.f, 0.f);  // the next chunk's candidate, read ahead
+        if (st.more() && lane < st.count()) pl = b.pos4_s[st.s + lane];
+        float rho = xmul(xi.w, c.w0);
+        uint32_t nn = 0, raw = 0, kept_word = 0;
+        int kept = 0, tested = 0, head = 0, self = -1;
+        RingLane<kDensityRing> at;
+        for (;;) {
+            __syncwarp();  // every lane is done with the chunks before head
+            while (st.more() && kept + 32 <= (head + kDensityRing) * 32) {
+                const int m = st.count(), s = st.s;
+                const uint32_t surv =
+                    __ballot_sync(kFull, lane < m && box_near(B, pl, r2m));
+                if ((surv >> lane) & 1u) {
+                    const int slot = ring_slot<kDensityRing>(kept + __popc(surv & lt));
+                    S->cx[slot] = pl.x;
+                    S->cy[slot] = pl.y;
+                    S->cz[slot] = pl.z;
+                    S->cm[slot] = pl.w;
                 }
-                const uint32_t surv = __ballot_sync(kFull, box_near(B, pl, r2m));
-                __syncwarp();
-                uint32_t* rec =
-                    nrec < room ? b.hitmask + (size_t)(slot + nrec) * 32 + lane : nullptr;
-                // streaming stores: the records must not evict the candidate arrays from L2
-                if (!surv) {
-                    if (rec) __stcs(rec, 0u);
-                    continue;
+                if ((unsigned)(i - s) < (unsigned)m) self = kept + __popc(surv & ((1u << (i - s)) - 1u));
+                st.next();
+                if (st.more() && lane < st.count()) pl = b.pos4_s[st.s + lane];
+                if (lane == (int)(raw & 31u)) kept_word = surv;
+                ++raw;
+                if ((raw & 31u) == 0 || !st.more()) {
+                    // streaming stores: the records must not evict the candidates from L2
+                    if ((raw - 1) >> 5 < room) __stcs(rec + ((raw - 1) & ~31u), kept_word);
+                    kept_word = 0;
                 }
-                uint32_t mask = 0u;
-                if (valid) mask = chunk_hits_x2(S->cx, S->cy, S->cz, surv, xi, c.r2);
-                if (rec) __stcs(rec, mask);
-                nn += __popc(mask);
-                const int self = i - s;
-                if ((unsigned)self < 32u) mask &= ~(1u << self);
-                const uint32_t cnt = __popc(mask);
-                uint32_t H;
-                const uint32_t o = warp_excl_scan(cnt, lane, H);
-                if (!H) continue;
-                // dense chunk (collapsed cells): the warp's hits are every (particle,
-                // candidate) pair of the chunk except the self pairs -- the most there can be.
-                // Each lane then adds its own terms in candidate order: the flattened path's
-                // terms and additions, without the hit list and the lane-by-lane fold.
-                const int lo = max(T.k0, s), hi = min(T.k0 + T.cnt, s + m);
-                if (kDense && H == (uint32_t)(T.cnt * m - max(hi - lo, 0))) {
-                    for (int jj = 0; jj < m; ++jj) {
-                        if (!valid || jj == self) continue;
-                        const float4 xj = S->cand[jj];
-                        rho = xadd(rho, xmul(xj.w, pair_w_exact<kKern, kNZ>(c, diff_d2(xi, xj))));
-                    }
-                    continue;
-                }
-                list_hits(S->plist, mask, o, lane);
-                __syncwarp();
-                for (uint32_t base = 0; base < H; base += kDensityBatch) {
-                    const uint32_t end = min(H, base + kDensityBatch);
-                    for (uint32_t f = base + lane; f < end; f += 32) {
-                        const uint32_t pr = S->plist[f];
-                        const float4 xj = S->cand[pr & 31];
-                        const float d2 = diff_d2(S->tpos[pr >> 5], xj);
-                        S->tbuf[f - base] = xmul(xj.w, pair_w_exact<kKern, kNZ>(c, d2));
-                    }
+                kept += __popc(surv);
+                while ((kept >> 5) > tested || (!st.more() && kept > tested * 32)) {
                     __syncwarp();
-                    const uint32_t k1 = min(o + cnt, end);
-                    for (uint32_t k = max(o, base); k < k1; ++k) rho = xadd(rho, S->tbuf[k - base]);
-                    __syncwarp();
+                    const int f = (tested % kDensityRing) * 32;
+                    uint32_t mask = ring_hits(S->cx + f, S->cy + f, S->cz + f, xi, c.r2, neg0);
+                    mask = valid ? mask & chunk_valid(kept - tested * 32) : 0u;
+                    nn += __popc(mask);
+                    if (self >> 5 == tested) mask &= ~(0x80000000u >> (self & 31));
+                    if (hdr + tested < room) __stcs(rec + (size_t)(hdr + tested) * 32, mask);
+                    S->mask[f + lane] = mask;
+                    ++tested;
                 }
             }
+            // the lanes' neighbours in the ring; while candidates are left, until no lane
+            // needs the oldest chunk any more
+            const int until = st.more() ? head + 1 : tested;
+            for (;;) {
+                at.advance(S->mask, tested, lane);
+                if (!__any_sync(kFull, at.need() < until)) break;
+                int qa, qb;
+                bool ha, hb;
+                at.take2(qa, qb, ha, hb);
+                if (nz) {
+                    const F2 d2 = pair_d2(f2(xi.x) - f2(S->cx[qa], S->cx[qb]),
+                                          f2(xi.y) - f2(S->cy[qa], S->cy[qb]),
+                                          f2(xi.z) - f2(S->cz[qa], S->cz[qb]), neg0);
+                    const float2 w = upk2((f2(S->cm[qa], S->cm[qb]) *
+                                           pair_w_exact2<kKern>(cp.lit, c.pair, d2)).v);
+                    if (ha) rho = xadd(rho, w.x);
+                    if (hb) rho = xadd(rho, w.y);
+                } else {
+                    auto add = [&](int q) {
+                        const float4 xj = make_float4(S->cx[q], S->cy[q], S->cz[q], S->cm[q]);
+                        rho = xadd(rho,
+                                   xmul(xj.w, pair_w_exact<kKern>(c, diff_d2(xi, xj))));
+                    };
+                    if (ha) add(qa);
+                    if (hb) add(qb);
+                }
+            }
+            if (!st.more()) break;
+            head = __reduce_min_sync(kFull, at.need());
         }
-        if (b.hitmask && lane == 0) {
-            const bool fits = nrec <= room;
-            b.tile_slot[t] = fits ? slot : kNoSlot;
-            if (fits) S->mcur = slot + nrec;
+        if (b.hitmask) {
+            const bool fits = hdr + (uint32_t)tested <= room;
+            if (lane == 0) b.tile_slot[t] = fits ? mcur : kNoSlot;
+            if (fits) mcur += hdr + (uint32_t)tested;
         }
         if (valid) {
             const float P = xmul(c.gas, xsub(rho, c.rest));
             // the per-candidate factors of the force pass's pair terms, each formed once here
-            // with the rounding the reference applies per pair: (rho, P, 2 rho, (m / rho) mu)
+            // with the rounding the reference applies per pair: (rho, P, (m / rho) mu, 1 / 2 rho)
             const float mr = xdiv(xi.w, rho);
-            b.aux4_s[i] = make_float4(rho, P, xmul(2.0f, rho), xmul(mr, c.visc));
+            b.aux4_s[i] = make_float4(rho, P, xmul(mr, c.visc), __frcp_rn(xmul(2.0f, rho)));
+            // outside these ranges the force pass divides by 2 rho in the general way
+            if (!(rho >= 0x1p-30f && rho <= 0x1p40f) ||
+                !(P == 0.0f || (fabsf(P) >= 0x1p-40f && fabsf(P) <= 0x1p60f)))
+                ds->general = 1;
+            b.vel4_s[i].w = rho;  // read with the candidate's velocity by the force pass
             my_max = max(my_max, nn);
         }
-        __syncwarp();
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) my_max = max(my_max, __shfl_xor_sync(kFull, my_max, o));
     if (lane == 0 && my_max) atomicMax(&ds->max_nn, (unsigned long long)my_max);
 }
 
-template <bool kBatch, int kKern, bool kNZ, bool kDense>
-static void launch_density_v(const LaunchCtx& L, const StepConst& c, const Buffers& b,
+template <bool kBatch, int kKern, bool kNZ>
+static void launch_density_t(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                              DevState* ds) {
     const int threads = 32 * L.warps_per_block;
     const size_t sm = (size_t)L.warps_per_block * sizeof(DensitySmem);
     static LaunchShapeCache cache;
-    const int nb = cached_resident_blocks(
-        cache, L, k_density<kBatch, kKern, kNZ, kDense>, threads, sm);
-    k_density<kBatch, kKern, kNZ, kDense><<<nb, threads, sm, L.stream>>>(c, b, ds);
-}
-
-template <bool kBatch, int kKern, bool kNZ = false>
-static void launch_density_t(const LaunchCtx& L, const StepConst& c, const Buffers& b,
-                             DevState* ds) {
-    launch_density_v<kBatch, kKern, kNZ, false>(L, c, b, ds);
-    launch_density_v<kBatch, kKern, kNZ, true>(L, c, b, ds);
+    const int nb = cached_resident_blocks(cache, L, k_density<kBatch, kKern, kNZ>, threads, sm);
+    k_density<kBatch, kKern, kNZ><<<nb, threads, sm, L.stream>>>(c, b, ds);
 }
 
 template <int kKern>
 static void launch_density_k(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                              DevState* ds) {
-    const bool nz = kKern == SPHX_KERNEL_CUBIC_SPLINE && !c.precise && c.div_nz;
+    // the Gaussian divides by neither h nor h^2
+    constexpr bool kDiv = kKern != SPHX_KERNEL_GAUSSIAN;
+    const bool nz = kDiv && c.div_nz;
     if (b.nscenes > 0) {
-        if (nz) launch_density_t<true, kKern, true>(L, c, b, ds);
-        else launch_density_t<true, kKern>(L, c, b, ds);
-    } else if (nz) launch_density_t<false, kKern, true>(L, c, b, ds);
-    else launch_density_t<false, kKern>(L, c, b, ds);
+        if (nz) launch_density_t<true, kKern, kDiv>(L, c, b, ds);
+        else launch_density_t<true, kKern, false>(L, c, b, ds);
+    } else if (nz) launch_density_t<false, kKern, kDiv>(L, c, b, ds);
+    else launch_density_t<false, kKern, false>(L, c, b, ds);
 }
 
-// Precision mode (single scene) runs the tile sweep (sphx_sweep.cu); exact mode the lean and
-// the dense-chunk variants of k_density.
+// Precision mode (single scene) runs the tile sweep (sphx_sweep.cu); exact mode k_density.
 int launch_density(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds) {
     if (c.precise && b.nscenes == 0) return launch_density_sweep(L, c, b, ds);
     if (c.kern == SPHX_KERNEL_WENDLAND_C2) launch_density_k<SPHX_KERNEL_WENDLAND_C2>(L, c, b, ds);
     else if (c.kern == SPHX_KERNEL_GAUSSIAN) launch_density_k<SPHX_KERNEL_GAUSSIAN>(L, c, b, ds);
     else launch_density_k<SPHX_KERNEL_CUBIC_SPLINE>(L, c, b, ds);
-    return 2;  // the lean and the dense-chunk variant; one of them returns at once
+    return 1;
 }
 
 }  // namespace sphx

@@ -11,23 +11,27 @@ namespace sphx {
 //  sph_engine.cpp:390-443; integrate_leapfrog, cpp:290-310;
 //  ParticleSystem::apply_boundary_conditions, particle.cpp:122-153)
 // ---------------------------------------------------------------------------------------
-// Per-warp shared memory of the force pass.  kBulk: candidates staged by bulk copies into
-// two buffers, the next chunk's copies in flight while the current chunk is worked on;
-// otherwise one buffer filled by the lanes' own loads.
-template <bool kBulk>
+// Per warp: the candidate ring -- positions and mass, velocities and density, the two
+// per-candidate factors -- the lanes' masks and the tile's row segments.  40 bytes a candidate:
+// 12 chunks leave room for 12 warps per SM; 8 chunks (16 warps) take 1.87 ms on the 1M dam
+// break, 10 (14 warps) 1.84, 12 1.71, 16 (8 warps) 2.0.
+//
+// Bound: instruction issue (64% of the slots with 3 warps per scheduler) and the FP32 pipe
+// (58%; a packed instruction holds it two cycles): 1,345 warp instructions per particle in
+// 5.7 turns, each finishing one pair of neighbours per lane and starting the next.  1M dam
+// break, force + leapfrog: 1.71 ms; with hit lists, terms passed through shared memory and
+// in-order folds by their lanes (2,479 instructions) 2.60 ms; one neighbour per turn with the
+// compiler's division and square root 2.72 ms, pairs 2.08, staged by asynchronous copies 1.83,
+// the two halves of a turn overlapped 1.73.
+constexpr int kForceRing = 12;
 struct ForceSmem {
-    uint64_t bar[2];        // mbarriers of the two bulk-copy buffers (kBulk)
-    float4 box_lo, box_hi;  // tile box (the fallback walk's culling test)
-    int2 seg[kMaxSegments]; // the tile's row segments
-    float4 cpos[kBulk ? 2 : 1][32], cvel[kBulk ? 2 : 1][32], caux[kBulk ? 2 : 1][32];
-    float4 tpos[32], tvel[32];  // targets: x,y,z,m and vx,vy,vz,P
-    uint16_t plist[32 * 32];
-    float4 tbA[kForceBatch];  // -(pressure term) x, y and viscosity term x, y
-    float2 tbB[kForceBatch];  // -(pressure term) z, viscosity term z
+    float4 pos[kForceRing * 32];  // x, y, z, m
+    float4 vel[kForceRing * 32];  // vx, vy, vz, rho
+    float2 fac[kForceRing * 32];  // (m / rho) mu, 1 / (2 rho)
+    uint32_t mask[kForceRing * 32];
+    int2 seg[kMaxSegments + 1];
 };
-static_assert(sizeof(ForceSmem<true>) % 16 == 0 && sizeof(ForceSmem<false>) % 16 == 0,
-              "per-warp regions keep the staging buffers 16-byte aligned");
-static_assert(4 * sizeof(ForceSmem<true>) <= 48 * 1024, "four warps within 48 KB");
+static_assert(sizeof(ForceSmem) % 16 == 0, "per-warp regions stay 16-byte aligned");
 
 // The pair term of particle t against candidate j: the pressure-force contribution
 // m_j * (P_t + P_j)/(2 rho_j) * gradW (the caller adds its negation, which equals
@@ -99,354 +103,264 @@ __device__ __forceinline__ void force_term(const StepConst& c, const float4& xt,
     v3[2] = xmul(xmul(sv, xsub(vj.z, vt.z)), lap);
 }
 
-// force_term<CUBIC_SPLINE> with the x and y components of every component-wise step done
-// as packed FP32 pairs (same operations, same rounding, element by element); returns the
-// record (-p.x, -p.y, v.x, v.y), (-p.z, v.z).  The pressure term is stored negated so that
-// the caller's sums are all additions: x - p == x + (-p) in IEEE arithmetic, and the
-// negated products are exact ((-s) * g == -(s * g)).  A skipped term is -0, the negation of
-// the reference's +0 (x + (-0) == x - (+0) == x for every x).
-// kNZ: the divisions by h and h^2 without range tests where bounds keep the dividends in
-// xdiv_fixed_nz's range (|r| of a hit, the Laplacian's numerator); the gradient's
-// components are tested once per pair and take the tested divisions only when one of
-// them is nonzero and below 2^-100 in magnitude.
-template <bool kNZ>
-__device__ __forceinline__ void force_term_cubic_x2(const StepConst& c, const float4& xt,
-                                                    const float4& vt, float Pt,
-                                                    const float4& xj, const float4& vj,
-                                                    const float4& aj, float4& A, float2& B) {
-    const f32x2 dxy = xsub2(pk2(xt.x, xt.y), pk2(xj.x, xj.y));
-    const float dz = xsub(xt.z, xj.z);
-    const float2 sq = upk2(xmul2(dxy, dxy));
-    const float r_len = xsqrt(xadd(xadd(sq.x, sq.y), xmul(dz, dz)));
-    const float q = kNZ ? xdiv_fixed_nz(r_len, c.h, c.rcp_h)
-                        : xdiv_fixed(r_len, c.h, c.rcp_h, c.fast_div_h);
-    f32x2 pxy = pk2(-0.0f, -0.0f);
-    float pz = -0.0f;
-    if (kNZ) {
-        // branch-free: every value is computed and the skipped cases are selected away (a
-        // pair with |r| < 1e-6 may divide by zero here; its results are discarded)
-        const bool live = !(r_len < 1e-6f);
-        const bool in = (q >= 0.0f && q <= 1.0f) || (q > 1.0f && q <= 2.0f);
-        const float sp = xmul(-xj.w, xdiv(xadd(Pt, aj.y), aj.z));  // -(m_j * pt)
-        const float gf = cubic_grad_factor(c, q);
-        const float2 d = upk2(dxy);
-        const f32x2 gq = xmul2(pk2(gf, gf), pk2(xdiv(d.x, r_len), xdiv(d.y, r_len)));
-        const float gzq = xmul(gf, xdiv(dz, r_len));
-        const f32x2 gxy = in ? gq : pk2(0.0f, 0.0f);
-        const float gz = in ? gzq : 0.0f;
-        const float2 g = upk2(gxy);
-        f32x2 pq;
-        float pzq;
-        if (nz_range(g.x) && nz_range(g.y) && nz_range(gz)) {
-            pq = xmul2(pk2(sp, sp), xdiv_fixed2_nz(gxy, c.h, c.rcp_h));
-            pzq = xmul(sp, xsign(xdiv_fixed_nz(gz, c.h, c.rcp_h), gz));
-        } else {
-            pq = xmul2(pk2(sp, sp), xdiv_fixed2(gxy, c.h, c.rcp_h, c.fast_div_h));
-            pzq = xmul(sp, xdiv_fixed(gz, c.h, c.rcp_h, c.fast_div_h));
-        }
-        pxy = live ? pq : pxy;
-        pz = live ? pzq : pz;
-    } else if (!(r_len < 1e-6f)) {
-        const float pt = xdiv(xadd(Pt, aj.y), aj.z);
-        const float sp = xmul(-xj.w, pt);  // -(m_j * pt)
-        f32x2 gxy = pk2(0.0f, 0.0f);
-        float gz = 0.0f;
-        if ((q >= 0.0f && q <= 1.0f) || (q > 1.0f && q <= 2.0f)) {
-            const float gf = cubic_grad_factor(c, q);
-            const float2 d = upk2(dxy);
-            gxy = xmul2(pk2(gf, gf), pk2(xdiv(d.x, r_len), xdiv(d.y, r_len)));
-            gz = xmul(gf, xdiv(dz, r_len));
-        }
-        pxy = xmul2(pk2(sp, sp), xdiv_fixed2(gxy, c.h, c.rcp_h, c.fast_div_h));
-        pz = xmul(sp, xdiv_fixed(gz, c.h, c.rcp_h, c.fast_div_h));
-    }
-    const float lap = cubic_lap<kNZ>(c, q);
-    const float sv = aj.w;  // (m_j / rho_j) * mu, formed by the density pass
-    const f32x2 vxy = xmul2(xmul2(pk2(sv, sv), xsub2(pk2(vj.x, vj.y), pk2(vt.x, vt.y))),
-                            pk2(lap, lap));
-    const float vz = xmul(xmul(sv, xsub(vj.z, vt.z)), lap);
-    const float2 p = upk2(pxy), v = upk2(vxy);
-    A = make_float4(p.x, p.y, v.x, v.y);
-    B = make_float2(pz, vz);
+
+// A lane's running force sums: pressure and viscosity, each in the walk's order.
+struct ForceSums {
+    float px = 0.0f, py = 0.0f, pz = 0.0f, vx = 0.0f, vy = 0.0f, vz = 0.0f;
+};
+
+// force_term added to the sums (the general form; a call of its own, so that the forms below
+// keep their registers)
+template <int K>
+__device__ __noinline__ ForceSums add_term_general(const StepConst& c, float4 xt, float4 vt,
+                                                   float Pt, float4 xj, float4 vj, float4 aj,
+                                                   ForceSums F) {
+    float p3[3], v3[3];
+    force_term<K>(c, xt, vt, Pt, xj, vj, aj, p3, v3);
+    F.px = xsub(F.px, p3[0]);
+    F.py = xsub(F.py, p3[1]);
+    F.pz = xsub(F.pz, p3[2]);
+    F.vx = xadd(F.vx, v3[0]);
+    F.vy = xadd(F.vy, v3[1]);
+    F.vz = xadd(F.vz, v3[2]);
+    return F;
 }
 
-// Cells holding more particles than this after the grid build mark a collapsed state, in
-// which whole chunks are dense (every particle of a tile within r of every candidate).
-constexpr uint32_t kDenseOccupancy = 128;
+// The terms of two neighbours, one in each half of packed FP32 pairs, added to the sums in
+// order (a if ha, b if hb).  The three divisions by |r| (cubic spline) or |r| h (Wendland)
+// share one reciprocal, the division by 2 rho_j has its reciprocal with the candidate, and
+// those by h and h^2 need no range tests.  Valid where StepConst::force_nz holds and
+// DevState::general is 0: a component of x_t - x_j is then 0 or in [2^-68, r], P_t + P_j 0 or
+// in [2^-64, 2^61] and rho in [2^-30, 2^40], and every dividend below stays in the range its
+// division needs.  The signs of zero terms are not kept: the sums start at +0 and so never
+// become -0, and adding a zero of either sign leaves any other value unchanged.  A pair with
+// |r| < 1e-6, whose pressure term the reference skips, gets m_j pt = 0 and with it zero terms
+// (what it multiplies is finite there).
+//
+// The work on a pair of neighbours is split in two (PairStart::start, add_pair): a lane starts
+// its next pair in the same straight-line code that finishes the one before, so that the two
+// chains of dependent operations overlap.
+struct PairStart {
+    F2 dx, dy, dz;  // x_t - x_j
+    F2 m;           // m_j
+    F2 s, ns, hr;   // |r|, -|r|, 1/(2 |r|) scaled (sqrt2_exact)
+    int qa, qb;     // ring slots
+    bool ha = false, hb = false;
+    __device__ __forceinline__ void start(const PairLits& k, const float4& xt, const float4& xa,
+                                          const float4& xb) {
+        dx = f2(xt.x) - f2(xa.x, xb.x);
+        dy = f2(xt.y) - f2(xa.y, xb.y);
+        dz = f2(xt.z) - f2(xa.z, xb.z);
+        m = f2(xa.w, xb.w);
+        s = sqrt2_exact(k, pair_d2(dx, dy, dz, F2{k.neg0}), hr, ns);
+    }
+};
+template <int K>
+__device__ __forceinline__ void add_pair(const PairLits& k, const PairConst& c, const float4& vt, float Pt,
+                                         const PairStart& p, const float4& va, const float4& vb,
+                                         const float2& fa, const float2& fb, ForceSums& F) {
+    const F2 zero = f2(0.0f), neg0{k.neg0};
+    const F2 dx = p.dx, dy = p.dy, dz = p.dz, ns = p.ns;
+    const bool ha = p.ha, hb = p.hb;
+    const F2 q = div_fixed2(p.s, F2{c.neg_h}, F2{c.rcp_h});
+    const float2 su = upk2(p.s.v), qu = upk2(q.v);
+    const bool la = !(su.x < 1e-6f), lb = !(su.y < 1e-6f);
+    const F2 rho = f2(va.w, vb.w);
+    const F2 Pj = pmul(F2{c.gas}, rho - F2{c.rest}, neg0);
+    const F2 pt = div_rcp2(f2(Pt) + Pj, F2{k.neg2} * rho, f2(fa.y, fb.y));
+    const F2 sp = select2(la, lb, p.m * pt, zero);  // m_j pt
+    const F2 y1 = p.hr * F2{k.p2p21};               // ~ 1/|r|
+    F2 px, py, pz, lap;
+    // beyond the support q = 2 the clamped 2 - q (1 - q/2) makes the terms the zeros that the
+    // reference returns there
+    if (K == SPHX_KERNEL_WENDLAND_C2) {
+        // norm dW/dq (r / (|r| h)), dW/dq = -5 t^3 q (kernels.cpp:180-192)
+        const F2 t = max0(F2{k.one} - F2{k.half} * q);
+        const F2 gsc = F2{c.wnorm} * (F2{k.neg5} * t * t * t * q);
+        const F2 nden = ns * F2{c.h};
+        const F2 y = rcp2_exact(k, nden, y1 * F2{c.rcp_h});
+        px = sp * (gsc * div_rcp2(dx, nden, y));
+        py = sp * (gsc * div_rcp2(dy, nden, y));
+        pz = sp * (gsc * div_rcp2(dz, nden, y));
+        lap = F2{c.wl} * t * t * (pmul(F2{k.five}, q, neg0) - F2{k.three});
+    } else {
+        // gradient factor (kernels.cpp:96-108): sigma (-2 q + 1.5 q q) or -sigma (0.5 t) t
+        const bool ia = qu.x <= 1.0f, ib = qu.y <= 1.0f;
+        const F2 t = max0(F2{k.two} - q);
+        const F2 g1 = F2{c.sigma} * (F2{k.neg2} * q + pmul(F2{k.onehalf} * q, q, neg0));
+        const F2 g2 = F2{c.neg_sigma} * (F2{k.half} * t * t);
+        const F2 gf = select2(ia, ib, g1, g2);
+        const F2 y = rcp2_exact(k, ns, y1);
+        px = sp * div_fixed2(gf * div_rcp2(dx, ns, y), F2{c.neg_h}, F2{c.rcp_h});
+        py = sp * div_fixed2(gf * div_rcp2(dy, ns, y), F2{c.neg_h}, F2{c.rcp_h});
+        pz = sp * div_fixed2(gf * div_rcp2(dz, ns, y), F2{c.neg_h}, F2{c.rcp_h});
+        // Laplacian (kernels.cpp:130-138)
+        const F2 l = select2(ia, ib, F2{k.neg2} + pmul(F2{k.three}, q, neg0), t);
+        lap = div_fixed2(F2{c.sigma} * l, F2{c.neg_hsq}, F2{c.rcp_hsq});
+    }
+    const F2 mv = f2(fa.x, fb.x);  // (m_j / rho_j) mu, formed by the density pass
+    const F2 wx = mv * (f2(va.x, vb.x) - f2(vt.x)) * lap, wy = mv * (f2(va.y, vb.y) - f2(vt.y)) * lap,
+             wz = mv * (f2(va.z, vb.z) - f2(vt.z)) * lap;
+    const float2 ax = upk2(px.v), ay = upk2(py.v), az = upk2(pz.v);
+    const float2 bx = upk2(wx.v), by = upk2(wy.v), bz = upk2(wz.v);
+    if (ha) {
+        F.px = xsub(F.px, ax.x);
+        F.py = xsub(F.py, ay.x);
+        F.pz = xsub(F.pz, az.x);
+        F.vx = xadd(F.vx, bx.x);
+        F.vy = xadd(F.vy, by.x);
+        F.vz = xadd(F.vz, bz.x);
+    }
+    if (hb) {
+        F.px = xsub(F.px, ax.y);
+        F.py = xsub(F.py, ay.y);
+        F.pz = xsub(F.pz, az.y);
+        F.vx = xadd(F.vx, bx.y);
+        F.vy = xadd(F.vy, by.y);
+        F.vz = xadd(F.vz, bz.y);
+    }
+}
 
-// kDense: the variant with the dense-chunk path (lane-load staging only).  With lane-load
-// staging both variants are launched every step and each returns at once unless the grid's
-// fullest cell says the state is its case.
-template <bool kIntegrate, bool kBatch, int kKern, bool kNZ, bool kBulk, bool kDense>
-__global__ void __launch_bounds__(128, kBulk || kDense ? 6 : 7) k_force(
-    const StepConst cp, const Buffers b, DevState* ds) {
+// Candidates go from global to shared memory by asynchronous copies (cp.async), a round of the
+// ring ahead of their use.
+template <bool kIntegrate, bool kBatch, int kKern, bool kNZ>
+__global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buffers b,
+                                                  DevState* ds) {
     if (ds->status) return;
-    if (!kBulk && kDense != (ds->max_occ > kDenseOccupancy)) return;
     extern __shared__ __align__(16) unsigned char smem_raw_f[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    ForceSmem<kBulk>* S = reinterpret_cast<ForceSmem<kBulk>*>(smem_raw_f) + warp;
-    if constexpr (kBulk) {
-        if (lane == 0) {
-            mbar_init(&S->bar[0], 1);
-            mbar_init(&S->bar[1], 1);
-            fence_mbar_init();
-        }
-        __syncwarp();
-    }
-    uint32_t parity = 0;  // bit q: the phase of buffer q's mbarrier to wait for next
+    ForceSmem* S = reinterpret_cast<ForceSmem*>(smem_raw_f) + warp;
     const uint32_t ntiles = ds->n_tiles;
-    const float inf = __int_as_float(0x7f800000);
+    const uint32_t lt = (1u << lane) - 1u;
+    const PairLits& lit = cp.lit;
+    const bool nz = kNZ && !ds->general;
     for (uint32_t t = next_tile(&ds->work[1], lane); t < ntiles; t = next_tile(&ds->work[1], lane)) {
-        const uint32_t k0 = b.tile_start[t];
-        const int scene = kBatch ? (int)b.scene_s[k0] : 0;
+        const uint2 tile = b.tiles[t];
+        const int scene = kBatch ? (int)b.scene_s[tile.x] : 0;
         const StepConst& c = kBatch ? b.scenes[scene].c : cp;
         const Geom g = kBatch ? scene_geom(b.scenes[scene], ds) : grid_geom(ds);
-        const float r2m = c.r2 * 1.0001f;
         Tile T;
         float4 xi;
         bool valid;
-        tile_setup(c, b, g, k0, lane, T, xi, valid);
-        const int i = T.k0 + lane;
+        int i;
+        tile_setup(c, b, g, tile, lane, T, i, xi, valid);
         const float4 vi0 = valid ? b.vel4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float Pi = valid ? b.aux4_s[i].y : 0.0f;
-        // hit masks of the density pass (same walk, same chunks, same tests)
+        // the density pass's records of this tile (same walk, same candidates kept)
         const uint32_t slot = b.tile_slot ? b.tile_slot[t] : kNoSlot;
-        if (slot == kNoSlot) {
-            const TileBox B = tile_box(xi, valid);
-            if (lane == 0) {
-                S->box_lo = make_float4(B.lo[0], B.lo[1], B.lo[2], 0.0f);
-                S->box_hi = make_float4(B.hi[0], B.hi[1], B.hi[2], 0.0f);
-            }
-        }
-        S->tpos[lane] = xi;
-        S->tvel[lane] = make_float4(vi0.x, vi0.y, vi0.z, Pi);
-        // force sums, packed: pressure (x, y), viscosity (x, y), (pressure z, viscosity z)
-        f32x2 fpxy = pk2(0.0f, 0.0f), fvxy = pk2(0.0f, 0.0f), fz = pk2(0.0f, 0.0f);
+        __syncwarp();  // the previous tile's segments are read
         const int nseg = build_segments(b, g, T, lane, S->seg);
         __syncwarp();
-        // One chunk's work once its candidates are staged (cpos/cvel/caux) and this lane's
-        // hit mask is known: list the warp's hits, compute the pair terms flattened, and
-        // add every lane's own terms in candidate order.
-        auto process = [&](uint32_t mask, int s, int m, const float4* cpos, const float4* cvel,
-                           const float4* caux) {
-            const int self = i - s;
-            if ((unsigned)self < 32u) mask &= ~(1u << self);
-            const uint32_t cnt = __popc(mask);
-            uint32_t H;
-            const uint32_t o = warp_excl_scan(cnt, lane, H);
-            if (!H) return;
-            // dense chunk (collapsed cells): the warp's hits are every (particle, candidate)
-            // pair of the chunk except the self pairs.  Each lane then forms its own terms,
-            // candidate after candidate, and adds them to its sums: the flattened path's
-            // terms (same inputs from shared memory) and additions, in the same order.  The
-            // additions are scalar IEEE adds on the unpacked sums: the packed FP32x2 add fed
-            // directly with the term values in registers gave last-bit differences in some
-            // collapsed states (measured against the reference's fixtures), while scalar adds
-            // (or a round trip of the terms through shared memory, as the flattened fold
-            // does) are exact.
-            const int lo = max(T.k0, s), hi = min(T.k0 + T.cnt, s + m);
-            if (kDense && H == (uint32_t)(T.cnt * m - max(hi - lo, 0))) {
-                const float4 xt = S->tpos[lane], vt = S->tvel[lane];
-                float2 sp = upk2(fpxy), sv = upk2(fvxy), sz = upk2(fz);
-                for (int jj = 0; jj < m; ++jj) {
-                    if (!valid || jj == self) continue;
-                    float4 A;
-                    float2 Bv;
-                    if (kKern == SPHX_KERNEL_CUBIC_SPLINE) {
-                        force_term_cubic_x2<kNZ>(c, xt, vt, vt.w, cpos[jj], cvel[jj], caux[jj], A,
-                                                 Bv);
-                    } else {
-                        float p3[3], v3[3];
-                        force_term<kKern>(c, xt, vt, vt.w, cpos[jj], cvel[jj], caux[jj], p3, v3);
-                        A = make_float4(-p3[0], -p3[1], v3[0], v3[1]);
-                        Bv = make_float2(-p3[2], v3[2]);
-                    }
-                    sp.x = xadd(sp.x, A.x);
-                    sp.y = xadd(sp.y, A.y);
-                    sv.x = xadd(sv.x, A.z);
-                    sv.y = xadd(sv.y, A.w);
-                    sz.x = xadd(sz.x, Bv.x);
-                    sz.y = xadd(sz.y, Bv.y);
-                }
-                fpxy = pk2(sp.x, sp.y);
-                fvxy = pk2(sv.x, sv.y);
-                fz = pk2(sz.x, sz.y);
-                return;
-            }
-            list_hits(S->plist, mask, o, lane);
-            __syncwarp();
-            for (uint32_t base = 0; base < H; base += kForceBatch) {
-                const uint32_t end = min(H, base + kForceBatch);
-                for (uint32_t f = base + lane; f < end; f += 32) {
-                    const uint32_t pr = S->plist[f];
-                    const int tt = pr >> 5, jj = pr & 31;
-                    float p3[3], v3[3];
-                    const float4 vt = S->tvel[tt];
-                    const uint32_t u = f - base;
-                    if (kKern == SPHX_KERNEL_CUBIC_SPLINE) {
-                        float4 A;
-                        float2 Bp;
-                        force_term_cubic_x2<kNZ>(c, S->tpos[tt], vt, vt.w, cpos[jj],
-                                            cvel[jj], caux[jj], A, Bp);
-                        S->tbA[u] = A;
-                        S->tbB[u] = Bp;
-                        continue;
-                    }
-                    force_term<kKern>(c, S->tpos[tt], vt, vt.w, cpos[jj], cvel[jj],
-                                      caux[jj], p3, v3);
-                    S->tbA[u] = make_float4(-p3[0], -p3[1], v3[0], v3[1]);
-                    S->tbB[u] = make_float2(-p3[2], v3[2]);
-                }
-                __syncwarp();
-                const uint32_t k1 = min(o + cnt, end);
-                for (uint32_t k = max(o, base); k < k1; ++k) {
-                    const uint32_t u = k - base;
-                    const float4 A = S->tbA[u];
-                    const float2 Bv = S->tbB[u];
-                    // the records hold -(pressure term): three packed additions
-                    fpxy = xadd2(fpxy, pk2(A.x, A.y));
-                    fvxy = xadd2(fvxy, pk2(A.z, A.w));
-                    fz = xadd2(fz, pk2(Bv.x, Bv.y));
-                }
-                __syncwarp();
-            }
-        };
-        const uint32_t* rec = slot != kNoSlot ? b.hitmask + (size_t)slot * 32 + lane : nullptr;
-        const size_t pool_words = (size_t)b.hitmask_cap * 32;
-        auto record = [&](const uint32_t* r) -> uint32_t {  // a lane's word, if in the pool
-            return r && (size_t)(r - b.hitmask) < pool_words ? __ldcs(r) : 0u;
-        };
-        if constexpr (!kBulk) {
-            uint32_t mnext = record(rec);
-            for (int sg = 0; sg < nseg; ++sg) {
-                const int2 se = S->seg[sg];
-                const int a = se.x, e = se.y;
-                for (int s = a; s < e; s += kTile, rec += rec ? 32 : 0) {
-                    const int m = min(kTile, e - s);
-                    uint32_t mask;
-                    __syncwarp();
-                    if (rec) {
-                        mask = mnext;
-                        // the next chunk's record, loaded a chunk ahead (past the tile's
-                        // last chunk it reads another tile's record, or nothing at the end)
-                        mnext = record(rec + 32);
-                        const uint32_t used = __reduce_or_sync(kFull, mask);  // candidates hit
-                        if (!used) continue;
-                        if (used & (1u << lane)) {
-                            S->cpos[0][lane] = b.pos4_s[s + lane];
-                            S->cvel[0][lane] = b.vel4_s[s + lane];
-                            S->caux[0][lane] = b.aux4_s[s + lane];
-                        }
-                        __syncwarp();
-                    } else {
-                        const bool in = lane < m;
-                        const float4 pl = in ? b.pos4_s[s + lane] : make_float4(inf, inf, inf, 0.f);
-                        S->cpos[0][lane] = pl;
-                        __syncwarp();
-                        TileBox B;
-                        const float4 lo = S->box_lo, hi = S->box_hi;
-                        B.lo[0] = lo.x, B.lo[1] = lo.y, B.lo[2] = lo.z;
-                        B.hi[0] = hi.x, B.hi[1] = hi.y, B.hi[2] = hi.z;
-                        const uint32_t surv = __ballot_sync(kFull, box_near(B, pl, r2m));
-                        if (!surv) continue;
-                        if (surv & (1u << lane)) {
-                            S->cvel[0][lane] = b.vel4_s[s + lane];
-                            S->caux[0][lane] = b.aux4_s[s + lane];
-                        }
-                        __syncwarp();
-                        mask = valid ? chunk_hits(S->cpos[0], surv, xi, c.r2) : 0u;
-                    }
-                    process(mask, s, m, S->cpos[0], S->cvel[0], S->caux[0]);
-                }
-            }
-        } else {
-            // Bulk copies (exact mode): chunks are bulk-copied (pos, vel, aux: contiguous ranges of the
-            // sorted arrays) into the two buffers.  A chunk some particle of the tile needs
-            // is copied while the chunk before it is worked on; the records (this lane's
-            // mask words) are read two chunks ahead, so the decision never waits on a load.
-            auto stage = [&](int qb, int s, int m) {
-                if (lane == 0) {
-                    const uint32_t bytes = (uint32_t)m * 16u;
-                    fence_proxy_async_smem();
-                    mbar_arrive_expect_tx(&S->bar[qb], 3u * bytes);
-                    bulk_copy_g2s(S->cpos[qb], b.pos4_s + s, bytes, &S->bar[qb]);
-                    bulk_copy_g2s(S->cvel[qb], b.vel4_s + s, bytes, &S->bar[qb]);
-                    bulk_copy_g2s(S->caux[qb], b.aux4_s + s, bytes, &S->bar[qb]);
-                }
-            };
-            int sg = 0, s = nseg ? S->seg[0].x : 0;
-            uint32_t m_cur = record(rec), m_next = record(rec ? rec + 32 : nullptr);
-            int q = 0;
-            bool cur_staged = false;
-            while (sg < nseg) {
-                const int m = min(kTile, S->seg[sg].y - s);
-                int sg_n = sg, s_n = s + kTile;  // the chunk after this one
-                if (s_n >= S->seg[sg].y) {
-                    ++sg_n;
-                    if (sg_n < nseg) s_n = S->seg[sg_n].x;
-                }
-                const bool has_next = sg_n < nseg;
-                const int m_n = has_next ? min(kTile, S->seg[sg_n].y - s_n) : 0;
-                uint32_t mask = m_cur, used, used_next;
+        const int hdr = (raw_chunks(S->seg, nseg, lane) + 31) >> 5;
+        const uint32_t* const rec =
+            slot != kNoSlot ? b.hitmask + (size_t)slot * 32 + lane : nullptr;
+        RawStream st(S->seg, nseg);
+        TileBox B;
+        if (!rec) B = tile_box(xi, valid);
+        ForceSums F;
+        uint32_t kept_word = 0;
+        int raw = 0, kept = 0, ready = 0, staged = 0, head = 0, self = -1;
+        RingLane<kForceRing> at;
+        PairStart pair;  // started, not yet added
+        pair.qa = pair.qb = 0;
+        pair.start(lit, xi, xi, xi);
+        int need = 0;  // first chunk the lane still needs
+        for (;;) {
+            cp_async_wait_all();
+            __syncwarp();  // staged chunks are in place, every lane is done with those before head
+            ready = staged;
+            while (st.more() && kept + 32 <= (head + kForceRing) * 32) {
+                const int m = st.count(), s = st.s;
+                uint32_t surv;
                 if (rec) {
-                    used = __reduce_or_sync(kFull, m_cur);  // candidates some lane hits
-                    used_next = __reduce_or_sync(kFull, has_next ? m_next : 0u);
-                    const uint32_t m_after = record(rec + 64);
-                    m_cur = m_next;
-                    m_next = m_after;
-                    rec += 32;
-                } else {  // no records: every chunk is staged and culled by the tile's box
-                    used = ~0u;
-                    used_next = has_next ? ~0u : 0u;
-                }
-                if (used) {
-                    if (!cur_staged) stage(q, s, m);
-                    const bool next_staged = used_next != 0u;
-                    if (next_staged) stage(q ^ 1, s_n, m_n);
-                    const bool arrived = mbar_wait(&S->bar[q], (parity >> q) & 1u);
-                    if (!__all_sync(kFull, arrived)) {
-                        // a bulk copy did not complete in time: record it, wait (bounded)
-                        // for the copies in flight into the other buffer, leave the pass
-                        if (lane == 0) atomicCAS(&ds->status, 0, SPHX_ERR_TIMEOUT);
-                        if (next_staged) mbar_wait(&S->bar[q ^ 1], (parity >> (q ^ 1)) & 1u);
-                        return;
-                    }
-                    parity ^= 1u << q;
-                    const float4* cpos = S->cpos[q];
-                    if (!rec) {
-                        TileBox B;
-                        const float4 lo = S->box_lo, hi = S->box_hi;
-                        B.lo[0] = lo.x, B.lo[1] = lo.y, B.lo[2] = lo.z;
-                        B.hi[0] = hi.x, B.hi[1] = hi.y, B.hi[2] = hi.z;
-                        const uint32_t surv =
-                            __ballot_sync(kFull, lane < m && box_near(B, cpos[lane], r2m));
-                        mask = valid && surv ? chunk_hits(cpos, surv, xi, c.r2) : 0u;
-                    }
-                    process(mask, s, m, cpos, S->cvel[q], S->caux[q]);
-                    __syncwarp();  // buffer q is free once every lane is past this point
-                    if (next_staged) q ^= 1;
-                    cur_staged = next_staged;
+                    if ((raw & 31) == 0) kept_word = __ldcs(rec + raw);
+                    surv = __shfl_sync(kFull, kept_word, raw & 31);
                 } else {
-                    // nothing to do here; start the next chunk's copies now if it is needed
-                    cur_staged = used_next != 0u;
-                    if (cur_staged) stage(q, s_n, m_n);
+                    bool near = false;
+                    if (lane < m) near = box_near(B, b.pos4_s[s + lane], c.r2 * 1.0001f);
+                    surv = __ballot_sync(kFull, near);
+                    if ((unsigned)(i - s) < (unsigned)m)
+                        self = kept + __popc(surv & ((1u << (i - s)) - 1u));
                 }
-                sg = sg_n;
-                s = s_n;
+                ++raw;
+                if ((surv >> lane) & 1u) {
+                    const int q = ring_slot<kForceRing>(kept + __popc(surv & lt));
+                    const int j = s + lane;
+                    cp_async16(&S->pos[q], &b.pos4_s[j]);
+                    cp_async16(&S->vel[q], &b.vel4_s[j]);
+                    cp_async8(&S->fac[q], &b.aux4_s[j].z);
+                }
+                st.next();
+                kept += __popc(surv);
+                while ((kept >> 5) > staged || (!st.more() && kept > staged * 32)) {
+                    const int f = (staged % kForceRing) * 32;
+                    if (rec) {
+                        const uint32_t* w = rec + (size_t)(hdr + staged) * 32;
+                        cp_async4(&S->mask[f + lane], w);
+                    } else {
+                        cp_async_wait_all();
+                        __syncwarp();
+                        uint32_t mask = 0;
+                        for (int q = 0; q < 32; ++q)
+                            if (diff_d2(xi, S->pos[f + q]) <= c.r2) mask |= 1u << q;
+                        mask = valid ? mask & chunk_valid(kept - staged * 32) : 0u;
+                        if (self >> 5 == staged) mask &= ~(0x80000000u >> (self & 31));
+                        S->mask[f + lane] = mask;
+                    }
+                    ++staged;
+                }
             }
+            const bool all = !st.more() && ready == staged;
+            const int until = all ? ready : min(head + 1, ready);
+            if (nz) {
+                // starts `next` and adds `done`; false when no lane needs a chunk before `until`
+                auto turn = [&](PairStart& next, const PairStart& done) -> bool {
+                    at.advance(S->mask, ready, lane);
+                    at.take2(next.qa, next.qb, next.ha, next.hb);
+                    next.start(lit, xi, S->pos[next.qa], S->pos[next.qb]);
+                    add_pair<kKern>(lit, c.pair, vi0, Pi, done, S->vel[done.qa], S->vel[done.qb],
+                                    S->fac[done.qa], S->fac[done.qb], F);
+                    need = at.next - (next.ha ? 1 : 0);
+                    return __any_sync(kFull, need < until);
+                };
+                for (;;) {
+                    PairStart other;
+                    if (!turn(other, pair)) {
+                        pair = other;
+                        break;
+                    }
+                    if (!turn(pair, other)) break;
+                }
+            } else {
+                for (;;) {
+                    at.advance(S->mask, ready, lane);
+                    need = at.need();
+                    if (!__any_sync(kFull, need < until)) break;
+                    int q[2];
+                    bool h[2];
+                    at.take2(q[0], q[1], h[0], h[1]);
+                    for (int k = 0; k < 2; ++k) {
+                        if (!h[k]) continue;
+                        const float4 vj = S->vel[q[k]];
+                        const float Pj = xmul(c.gas, xsub(vj.w, c.rest));
+                        F = add_term_general<kKern>(
+                            c, xi, vi0, Pi, S->pos[q[k]], vj,
+                            make_float4(vj.w, Pj, xmul(2.0f, vj.w), S->fac[q[k]].x), F);
+                    }
+                }
+            }
+            if (all) break;
+            head = __reduce_min_sync(kFull, need);
         }
-        __syncwarp();
         if (!valid) continue;
         const float mi = xi.w;
-        const float2 fp = upk2(fpxy), fv = upk2(fvxy), fzz = upk2(fz);
-        const float fpz = fzz.x, fvz = fzz.y;
-        const float ax = xdiv(xadd(xadd(fp.x, fv.x), xmul(0.0f, mi)), mi);
-        const float ay = xdiv(xadd(xadd(fp.y, fv.y), xmul(c.grav, mi)), mi);
-        const float az = xdiv(xadd(xadd(fpz, fvz), xmul(0.0f, mi)), mi);
+        const float ax = xdiv(xadd(xadd(F.px, F.vx), xmul(0.0f, mi)), mi);
+        const float ay = xdiv(xadd(xadd(F.py, F.vy), xmul(c.grav, mi)), mi);
+        const float az = xdiv(xadd(xadd(F.pz, F.vz), xmul(0.0f, mi)), mi);
         b.acc4_s[i] = make_float4(ax, ay, az, 0.0f);
         if (!kIntegrate) continue;
         const float dt = kBatch ? b.scenes[scene].dt : ds->dt;
-        const float4 vi = S->tvel[lane];
+        const float4 vi = vi0;
         const uint32_t id = b.id_s[i];
         float x[3] = {xi.x, xi.y, xi.z}, v[3] = {vi.x, vi.y, vi.z};
         const float acc[3] = {ax, ay, az};
@@ -481,57 +395,45 @@ __global__ void __launch_bounds__(128, kBulk || kDense ? 6 : 7) k_force(
     }
 }
 
-template <bool kIntegrate, bool kBatch, int kKern, bool kNZ, bool kBulk, bool kDense>
-static void launch_force_v(const LaunchCtx& L, const StepConst& c, const Buffers& b,
+template <bool kIntegrate, bool kBatch, int kKern, bool kNZ>
+static void launch_force_t(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                            DevState* ds) {
     const int threads = 32 * L.warps_per_block;
-    const size_t sm = (size_t)L.warps_per_block * sizeof(ForceSmem<kBulk>);
+    const size_t sm = (size_t)L.warps_per_block * sizeof(ForceSmem);
     static LaunchShapeCache cache;
     const int nb = cached_resident_blocks(
-        cache, L, k_force<kIntegrate, kBatch, kKern, kNZ, kBulk, kDense>, threads, sm);
-    k_force<kIntegrate, kBatch, kKern, kNZ, kBulk, kDense>
-        <<<nb, threads, sm, L.stream>>>(c, b, ds);
+        cache, L, k_force<kIntegrate, kBatch, kKern, kNZ>, threads, sm);
+    k_force<kIntegrate, kBatch, kKern, kNZ><<<nb, threads, sm, L.stream>>>(c, b, ds);
 }
 
-// Candidates are staged by the lanes' own loads or by bulk copies (L.bulk_copy, a tuning
-// choice).  Returns the kernels launched.
-template <bool kIntegrate, bool kBatch, int kKern, bool kNZ = false>
-static int launch_force_t(const LaunchCtx& L, const StepConst& c, const Buffers& b,
-                          DevState* ds) {
-    if (L.bulk_copy) {
-        launch_force_v<kIntegrate, kBatch, kKern, kNZ, true, false>(L, c, b, ds);
-        return 1;
-    }
-    launch_force_v<kIntegrate, kBatch, kKern, kNZ, false, false>(L, c, b, ds);
-    launch_force_v<kIntegrate, kBatch, kKern, kNZ, false, true>(L, c, b, ds);
-    return 2;
-}
-
-template <int kKern>
-static int launch_force_k(const LaunchCtx& L, const StepConst& c, const Buffers& b,
-                          DevState* ds, int integrate) {
-    const bool nz = kKern == SPHX_KERNEL_CUBIC_SPLINE && c.div_nz;
+template <int kKern, bool kNZ>
+static void launch_force_n(const LaunchCtx& L, const StepConst& c, const Buffers& b,
+                           DevState* ds, int integrate) {
     const bool batch = b.nscenes > 0;
     if (integrate) {
-        if (batch) return nz ? launch_force_t<true, true, kKern, true>(L, c, b, ds)
-                             : launch_force_t<true, true, kKern>(L, c, b, ds);
-        return nz ? launch_force_t<true, false, kKern, true>(L, c, b, ds)
-                  : launch_force_t<true, false, kKern>(L, c, b, ds);
+        if (batch) launch_force_t<true, true, kKern, kNZ>(L, c, b, ds);
+        else launch_force_t<true, false, kKern, kNZ>(L, c, b, ds);
+    } else {
+        if (batch) launch_force_t<false, true, kKern, kNZ>(L, c, b, ds);
+        else launch_force_t<false, false, kKern, kNZ>(L, c, b, ds);
     }
-    if (batch) return launch_force_t<false, true, kKern>(L, c, b, ds);
-    return nz ? launch_force_t<false, false, kKern, true>(L, c, b, ds)
-              : launch_force_t<false, false, kKern>(L, c, b, ds);
 }
 
 // Precision mode (single scene) runs the tile sweep (sphx_sweep.cu); exact mode k_force.
 int launch_force(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
                  int integrate) {
     if (c.precise && b.nscenes == 0) return launch_force_sweep(L, c, b, ds, integrate);
-    if (c.kern == SPHX_KERNEL_WENDLAND_C2)
-        return launch_force_k<SPHX_KERNEL_WENDLAND_C2>(L, c, b, ds, integrate);
-    if (c.kern == SPHX_KERNEL_GAUSSIAN)
-        return launch_force_k<SPHX_KERNEL_GAUSSIAN>(L, c, b, ds, integrate);
-    return launch_force_k<SPHX_KERNEL_CUBIC_SPLINE>(L, c, b, ds, integrate);
+    if (c.kern == SPHX_KERNEL_WENDLAND_C2) {
+        if (c.force_nz) launch_force_n<SPHX_KERNEL_WENDLAND_C2, true>(L, c, b, ds, integrate);
+        else launch_force_n<SPHX_KERNEL_WENDLAND_C2, false>(L, c, b, ds, integrate);
+    } else if (c.kern == SPHX_KERNEL_GAUSSIAN) {
+        launch_force_n<SPHX_KERNEL_GAUSSIAN, false>(L, c, b, ds, integrate);
+    } else if (c.force_nz) {
+        launch_force_n<SPHX_KERNEL_CUBIC_SPLINE, true>(L, c, b, ds, integrate);
+    } else {
+        launch_force_n<SPHX_KERNEL_CUBIC_SPLINE, false>(L, c, b, ds, integrate);
+    }
+    return 1;
 }
 
 }  // namespace sphx

@@ -40,6 +40,7 @@ __global__ void k_begin_step(DevState* ds, int reset_bbox) {
     ds->work[0] = ds->work[1] = 0;
     ds->spread_work[0] = ds->spread_work[1] = 0;
     ds->n_spread = 0;
+    ds->general = 0;
 }
 
 int launch_begin_step(const LaunchCtx& L, DevState* ds, int reset_bbox) {
@@ -135,8 +136,10 @@ __global__ void k_bbox(const float4* __restrict__ pos4, int n, float inv_cell, D
     int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
     int mx[3] = {-0x7fffffff - 1, -0x7fffffff - 1, -0x7fffffff - 1};
     uint32_t bad = 0;
+    bool tiny = false;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 p = pos4[i];
+        tiny = tiny || tiny_coord(p.x) || tiny_coord(p.y) || tiny_coord(p.z);
         if (!finite3(p.x, p.y, p.z)) {
             ++bad;
             continue;
@@ -166,6 +169,7 @@ __global__ void k_bbox(const float4* __restrict__ pos4, int n, float inv_cell, D
         }
         if (bad) atomicAdd(&ds->nonfinite, bad);
     }
+    if (tiny) ds->general = 1;
 }
 
 // Grid extent.  The occupied-cell box is laid out densely when it has at most max_cells
@@ -276,19 +280,25 @@ __global__ void k_keys(const float4* __restrict__ pos4, int n, float inv_cell,
     }
 }
 
-// Gathers the state into cell-sorted order and keeps the sorted keys and permutation.
+// Gathers the state into cell-sorted order, keeps the sorted keys and permutation, and writes
+// the cell offsets: off[c] = first sorted position whose key is >= c, for c in
+// [0, ncells + 1]; off[ncells] is the number of finite particles and off[ncells + 1] == n.
 __global__ void k_reorder(const Buffers b, int n, DevState* ds) {
     if (ds->status) return;
     const int sel = ds->passes & 1;
+    const uint32_t nc = ds->ncells;
     const uint32_t* __restrict__ ks = b.key[sel];
     const uint32_t* __restrict__ vs = b.val[sel];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= n; k += gridDim.x * blockDim.x) {
+        const uint32_t hi = k == n ? nc + 1u : ks[k];
+        for (uint32_t c = k == 0 ? 0u : ks[k - 1] + 1u; c <= hi; ++c) b.off[c] = (uint32_t)k;
+        if (k == n) break;
         uint32_t id = vs[k];
         if (id >= (uint32_t)n) {  // never for a valid permutation: record, do not fault
             atomicExch(&ds->status, SPHX_ERR_CUDA);
             id = 0;
         }
-        b.key_s[k] = ks[k];
+        b.key_s[k] = hi;
         b.id_s[k] = id;
         b.pos4_s[k] = b.pos4[id];
         b.vel4_s[k] = b.vel4[id];
@@ -297,37 +307,127 @@ __global__ void k_reorder(const Buffers b, int n, DevState* ds) {
     }
 }
 
-// off[c] = first sorted position whose key is >= c, for c in [0, ncells + 1];
-// off[ncells] is the number of finite particles and off[ncells + 1] == n.
-__global__ void k_offsets(const uint32_t* __restrict__ key_s, int n, const DevState* ds,
-                          uint32_t* __restrict__ off) {
-    if (ds->status) return;
-    const uint32_t nc = ds->ncells;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= n; k += gridDim.x * blockDim.x) {
-        const uint32_t lo = (k == 0) ? 0u : key_s[k - 1] + 1u;
-        const uint32_t hi = (k == n) ? nc + 1u : key_s[k];
-        for (uint32_t c = lo; c <= hi; ++c) off[c] = (uint32_t)k;
+// ---- in-cell order and tile list --------------------------------------------------------
+// A tile is a run of at most tile_n consecutive positions of a cell (b.columns == 0) or of a
+// cell column (x, y, *).  Whether a tile starts at position k is decided from the keys and
+// cell offsets alone (no scan over the particles): at every tile_n-th position of the column
+// and, so that no tile reaches far from its first cell, where a sparse stretch of the column
+// is cut (kRunWindow / kRunAlign).  A tile whose first particle lies in cell z_a ends by cell
+// z_a + kRunCells: the first multiple z_m of kRunAlign at or above z_a + kRunWindow + 1 is at
+// most that plus kRunAlign - 1, and were the tile to reach cell z_m, the kRunWindow cells
+// below z_m would lie wholly in it, fewer than tile_n particles, so a tile starts at z_m.
+struct ColumnInfo {
+    uint32_t base, d2;  // first cell of the scene's block, cells along z
+    bool each_cell;     // tiles within one cell
+    float inv_cell;
+};
+__device__ __forceinline__ ColumnInfo column_info(const Buffers& b, const DevState* ds, int k,
+                                                  float inv_cell, bool folded_cells) {
+    if (b.nscenes) {
+        const SceneInfo& sc = b.scenes[b.scene_s[k]];
+        return ColumnInfo{sc.base, (uint32_t)sc.dim[2], !b.columns, sc.c.inv_cell};
     }
+    return ColumnInfo{0u, (uint32_t)ds->dim[2], !b.columns || folded_cells, inv_cell};
+}
+__device__ __forceinline__ bool tile_starts(const Buffers& b, const ColumnInfo& g, uint32_t nc,
+                                            int k, uint32_t key, uint32_t prev, bool new_cell) {
+    const uint32_t tn = (uint32_t)b.tile_n;
+    if (key >= nc || g.each_cell) return ((uint32_t)k - b.off[key]) % tn == 0;
+    const uint32_t z = (key - g.base) % g.d2, cb = key - z;
+    if (((uint32_t)k - b.off[cb]) % tn == 0) return true;
+    if (!new_cell) return false;
+    // the cells between the last particle's and this one are empty: only the last multiple of
+    // kRunAlign among them can be undecided (an earlier one implies an empty window there)
+    const uint32_t zm = z - z % kRunAlign;
+    return zm > (uint32_t)kRunWindow && cb + zm > prev &&
+           b.off[cb + zm] - b.off[cb + zm - kRunWindow] < tn;
 }
 
-// Precision-mode step (b.columns): each cell's particles put in z order (the in-cell
-// offset quantised to 16 levels of cs/16, stable within a level), so that a run of
-// consecutive particles of a cell column -- a tile -- is a compact slab across the cells.
-// The order within a cell is free in this mode (its sums are judged against FP64, not
-// against the reference's order).  One warp per cell; cells of more than kZOrderMax
-// particles (collapsed states, whose tiles are dense anyway) keep their order.
+// One block per 256 positions; a warp puts the cells that start in its 32 positions in z order
+// (the in-cell offset quantised to 16 levels, stable within a level), so that a tile is a
+// compact slab across the cells of its column.  kCells (precision mode, whose sums are judged
+// against FP64): the particles themselves are moved.  Otherwise the particles keep the
+// reference's insertion order, in which they are met as neighbours, and only the order in
+// which they are taken as targets changes (b.tgt).  Cells of more than kZOrderMax particles
+// (collapsed states, whose tiles are dense anyway) keep their order.
 constexpr int kZOrderMax = 128;
-__global__ void __launch_bounds__(256) k_cell_zorder(const Buffers b, const DevState* ds,
-                                                     float levels_per_unit) {
+template <bool kCells>
+__global__ void __launch_bounds__(256) k_order_tiles(const Buffers b, int n, DevState* ds,
+                                                     float inv_cell, float levels) {
     if (ds->status) return;
     constexpr int kPer = kZOrderMax / 32;
+    __shared__ uint32_t flags[9];
+    __shared__ uint32_t s_occ, s_max, s_base;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) s_occ = s_max = 0;
     const uint32_t nc = ds->ncells;
-    const int lane = threadIdx.x & 31;
-    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-    const uint32_t lt = (1u << lane) - 1u;
-    for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < nc; c += nwarps) {
-        const uint32_t a = b.off[c], cnt = b.off[c + 1] - a;
-        if (cnt < 2 || cnt > (uint32_t)kZOrderMax) continue;
+    // an exact step on a grid folded along z keeps one-cell tiles: a row that wraps is met in
+    // each cell's own dz order
+    const bool folded_cells = !kCells && ds->wrap[2];
+    const int k = blockIdx.x * 256 + tid;
+    uint32_t key = 0, cnt = 0;
+    bool new_cell = false, flag = false;
+    if (k < n) {
+        key = b.key_s[k];
+        const uint32_t prev = k ? b.key_s[k - 1] : 0u;
+        new_cell = k == 0 || prev != key;
+        const ColumnInfo g = column_info(b, ds, k, inv_cell, folded_cells);
+        inv_cell = g.inv_cell;
+        flag = tile_starts(b, g, nc, k, key, prev, new_cell);
+        cnt = key < nc ? b.off[key + 1] - b.off[key] : 0u;
+    }
+    {
+        const uint32_t f = __ballot_sync(0xffffffffu, flag);
+        if (lane == 0) flags[warp] = f;
+    }
+    if (warp == 0) {  // the first 32 positions past the block end its last tiles
+        const int q = blockIdx.x * 256 + 256 + lane;
+        bool fq = false;
+        if (q < n) {
+            const uint32_t kq = b.key_s[q], pq = b.key_s[q - 1];
+            const ColumnInfo g = column_info(b, ds, q, inv_cell, folded_cells);
+            fq = tile_starts(b, g, nc, q, kq, pq, pq != kq);
+        }
+        const uint32_t f = __ballot_sync(0xffffffffu, fq);
+        if (lane == 0) flags[8] = f;
+    }
+    __syncthreads();
+    {   // occupied cells, fullest cell
+        const uint32_t starts = __ballot_sync(0xffffffffu, new_cell && key < nc);
+        const uint32_t occ = __reduce_max_sync(0xffffffffu, new_cell ? cnt : 0u);
+        if (lane == 0 && starts) {
+            atomicAdd(&s_occ, (uint32_t)__popc(starts));
+            atomicMax(&s_max, occ);
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        uint32_t nt = 0;
+        for (int w = 0; w < 8; ++w) nt += __popc(flags[w]);
+        s_base = atomicAdd(&ds->n_tiles, nt);
+        if (s_occ) {
+            atomicAdd(&ds->occupied, s_occ);
+            atomicMax(&ds->max_occ, s_max);
+        }
+    }
+    __syncthreads();
+    if (flag) {
+        uint32_t t = s_base + __popc(flags[warp] & ((1u << lane) - 1u));
+        for (int w = 0; w < warp; ++w) t += __popc(flags[w]);
+        const unsigned long long rest =
+            (flags[warp] | (unsigned long long)flags[warp + 1] << 32) >> lane >> 1;
+        uint32_t m = min((uint32_t)b.tile_n, (uint32_t)(n - k));
+        if (rest) m = min(m, (uint32_t)__ffsll((long long)rest));
+        b.tiles[t] = make_uint2((uint32_t)k, m);
+    }
+    if (!b.columns) return;
+    const bool ordered = cnt >= 2 && cnt <= (uint32_t)kZOrderMax;
+    if (!kCells && k < n && !ordered) b.tgt[k] = (uint32_t)k;
+    for (uint32_t todo = __ballot_sync(0xffffffffu, new_cell && ordered); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        const uint32_t a = (uint32_t)__shfl_sync(0xffffffffu, k, src);
+        const uint32_t c = __shfl_sync(0xffffffffu, cnt, src);
+        const float ic = __shfl_sync(0xffffffffu, inv_cell, src);
         float4 p[kPer], v[kPer];
         int4 ce[kPer];
         uint32_t id[kPer];
@@ -336,12 +436,16 @@ __global__ void __launch_bounds__(256) k_cell_zorder(const Buffers b, const DevS
         for (int j = 0; j < kPer; ++j) {
             const uint32_t q = (uint32_t)(j * 32 + lane);
             lev[j] = 16;  // no element
-            if (q < cnt) {
+            if (q >= c) continue;
+            if (kCells) {
                 p[j] = b.pos4_s[a + q];
                 v[j] = b.vel4_s[a + q];
                 ce[j] = b.cell4_s[a + q];
                 id[j] = b.id_s[a + q];
-                lev[j] = min(15, max(0, (int)(p[j].z * levels_per_unit)));
+                lev[j] = min(15, max(0, (int)(p[j].z * levels)));
+            } else {
+                const float u = b.pos4_s[a + q].z * ic;
+                lev[j] = min(15, max(0, (int)((u - floorf(u)) * 16.0f)));
             }
         }
         // stable counting sort over the 16 levels: an element's place is the number of
@@ -354,7 +458,7 @@ __global__ void __launch_bounds__(256) k_cell_zorder(const Buffers b, const DevS
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
                 const uint32_t m = __ballot_sync(0xffffffffu, lev[j] == L);
-                if (lev[j] == L) dest[j] = (int)(seen + __popc(m & lt));
+                if (lev[j] == L) dest[j] = (int)(seen + __popc(m & ((1u << lane) - 1u)));
                 seen += __popc(m);
             }
             below = seen;
@@ -363,11 +467,15 @@ __global__ void __launch_bounds__(256) k_cell_zorder(const Buffers b, const DevS
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
             if (lev[j] == 16) continue;
-            const uint32_t k = a + (uint32_t)dest[j];
-            b.pos4_s[k] = p[j];
-            b.vel4_s[k] = v[j];
-            b.cell4_s[k] = ce[j];
-            b.id_s[k] = id[j];
+            const uint32_t to = a + (uint32_t)dest[j];
+            if (kCells) {
+                b.pos4_s[to] = p[j];
+                b.vel4_s[to] = v[j];
+                b.cell4_s[to] = ce[j];
+                b.id_s[to] = id[j];
+            } else {
+                b.tgt[to] = a + (uint32_t)(j * 32 + lane);
+            }
         }
     }
 }
@@ -381,90 +489,22 @@ int launch_build_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b,
     k_grid_setup<<<1, 32, 0, L.stream>>>(n, c.max_cells, ds);
     if (c.precise) k_keys_cells<<<gb, 256, 0, L.stream>>>(b.cell4, n, ds, b.key[0]);
     else k_keys<<<gb, 256, 0, L.stream>>>(b.pos4, n, c.inv_cell, ds, b.key[0]);
-    return 3 + launch_grid_sort(L, b, ds, n, c.cs);
+    return 3 + launch_grid_sort(L, b, ds, n, c);
 }
 
-static int launch_cell_zorder(const LaunchCtx& L, const Buffers& b, DevState* ds, int n,
-                              float cs) {
-    if (!b.columns || !b.cell4_s) return 0;
-    // one warp per cell: blocks of 8 warps, enough of them for the occupied cells
-    k_cell_zorder<<<grid_blocks(L, n, 256, 8), 256, 0, L.stream>>>(b, ds, 16.0f / cs);
-    return 1;
-}
-
-// Precision-mode step, single scene: the runs of each cell column.  Cell z of a column
-// starts a run when it is the column's first cell, or when z is a multiple of A =
-// kRunAlign and the W = kRunWindow cells below z hold fewer than tile_n particles.  A tile
-// whose first particle lies in cell z_a then ends by cell z_a + W + A - 1: the first
-// multiple of A at or above z_a + W + 1, z_m, is at most z_a + W + A, and were the tile
-// to reach cell z_m, cells z_m - W .. z_m - 1 would lie wholly in it, fewer than tile_n
-// particles, so z_m starts a run.  Dense stretches stay one run; a sparse one is cut every
-// A cells (a window of one cell and A = 1 would cut it at every cell).  runs[c] = the
-// sorted positions where c's run starts and ends (the off of its first cell and of the
-// next run's).  One warp per column: a max-scan over its cells 32 at a time upward for
-// the starts, a min-scan downward for the ends.
-__device__ __forceinline__ bool run_starts_at(const uint32_t* __restrict__ off, uint32_t cb,
-                                              uint32_t z, uint32_t tile_n) {
-    return z == 0 || (z > (uint32_t)kRunWindow && z % kRunAlign == 0 &&
-                      off[cb + z] - off[cb + z - kRunWindow] < tile_n);
-}
-__global__ void __launch_bounds__(256) k_column_runs(const uint32_t* __restrict__ off,
-                                                     const DevState* ds, uint32_t tile_n,
-                                                     uint2* __restrict__ runs) {
-    if (ds->status) return;
-    const int d2 = ds->dim[2];
-    if (d2 <= 0) return;
-    const uint32_t ncol = ds->ncells / (uint32_t)d2;
-    const int lane = threadIdx.x & 31;
-    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); col < ncol;
-         col += nwarps) {
-        const uint32_t cb = col * (uint32_t)d2;
-        int carry = 0;  // first cell of the run (column-relative)
-        for (int z0 = 0; z0 < d2; z0 += 32) {
-            const int z = z0 + lane;
-            int v = (z < d2 && run_starts_at(off, cb, (uint32_t)z, tile_n)) ? z : carry;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v = max(v, u);
-            }
-            if (z < d2) runs[cb + z].x = off[cb + v];
-            carry = __shfl_sync(0xffffffffu, v, 31);
-        }
-        carry = d2;  // first cell of the next run (d2: the column's end)
-        for (int z0 = (d2 - 1) & ~31; z0 >= 0; z0 -= 32) {
-            const int z = z0 + lane;
-            int v = (z + 1 < d2 && run_starts_at(off, cb, (uint32_t)(z + 1), tile_n)) ? z + 1
-                                                                                     : carry;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_down_sync(0xffffffffu, v, o);
-                if (lane + o < 32) v = min(v, u);
-            }
-            if (z < d2) runs[cb + z].y = off[cb + v];
-            carry = __shfl_sync(0xffffffffu, v, 0);
-        }
-    }
-}
-
-static int launch_column_runs(const LaunchCtx& L, const Buffers& b, DevState* ds, int n) {
-    if (!b.columns || !b.runs || b.nscenes) return 0;
-    k_column_runs<<<grid_blocks(L, n, 256, 2), 256, 0, L.stream>>>(b.off, ds,
-                                                                   (uint32_t)b.tile_n, b.runs);
-    return 1;
-}
-
-// Shared tail of the grid build: stable sort of the keys, gather into cell-sorted order,
-// cell offsets, (b.columns) z order within the cells and column runs, tile list.
-int launch_grid_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, float cs) {
+// Shared tail of the grid build: stable sort of the keys, gather into cell-sorted order with
+// the cell offsets, in-cell order and tile list.
+int launch_grid_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n,
+                     const StepConst& c) {
     const int r = launch_radix_sort(L, b, ds, n);
-    k_reorder<<<grid_blocks(L, n, 256, 8), 256, 0, L.stream>>>(b, n, ds);
-    k_offsets<<<grid_blocks(L, n + 1, 256, 8), 256, 0, L.stream>>>(b.key_s, n, ds, b.off);
-    const int z = launch_cell_zorder(L, b, ds, n, cs) + launch_column_runs(L, b, ds, n);
-    return 2 + r + z + launch_tile_scan(L, b, ds, n);
+    k_reorder<<<grid_blocks(L, n + 1, 256, 8), 256, 0, L.stream>>>(b, n, ds);
+    const int nb = (n + 255) / 256;
+    if (b.columns && b.cell4_s)
+        k_order_tiles<true><<<nb, 256, 0, L.stream>>>(b, n, ds, c.inv_cell, 16.0f / c.cs);
+    else
+        k_order_tiles<false><<<nb, 256, 0, L.stream>>>(b, n, ds, c.inv_cell, 0.0f);
+    return 2 + r;
 }
-
 
 // ---- FP64 diagnostics of the state after a step -----------------------------------------
 // sums: mass, momentum x/y/z, kinetic energy, potential energy (-m g y), density.

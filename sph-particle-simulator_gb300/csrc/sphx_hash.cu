@@ -106,7 +106,7 @@ int galloc(T** p, size_t count) {
 void grid_free(sphx_grid* g) {
     Buffers& b = g->b;
     void* ptrs[] = {b.pos4, b.vel4, b.pos4_s, b.vel4_s, b.key[0], b.key[1], b.val[0], b.val[1],
-                    b.key_s, b.id_s, b.off, b.tile_start, b.hist, b.scan_part, g->ds, g->stage};
+                    b.key_s, b.id_s, b.off, b.tiles, b.hist, b.scan_part, g->ds, g->stage};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (g->stream) cudaStreamDestroy(g->stream);
@@ -158,7 +158,7 @@ int sphx_grid_create(sphx_grid** out, size_t capacity) {
         (rc = galloc(&b.vel4_s, C)) || (rc = galloc(&b.key[0], C)) || (rc = galloc(&b.key[1], C)) ||
         (rc = galloc(&b.val[0], C)) || (rc = galloc(&b.val[1], C)) || (rc = galloc(&b.key_s, C)) ||
         (rc = galloc(&b.id_s, C)) || (rc = galloc(&b.off, (size_t)max_cells + 2)) ||
-        (rc = galloc(&b.tile_start, C)) || (rc = galloc(&b.hist, hist_n)) ||
+        (rc = galloc(&b.tiles, C)) || (rc = galloc(&b.hist, hist_n)) ||
         (rc = galloc(&b.scan_part, (size_t)b.scan_part_cap)) || (rc = galloc(&g->ds, 1)) ||
         (rc = galloc(&g->stage, 4 * C)))
         return fail(rc);

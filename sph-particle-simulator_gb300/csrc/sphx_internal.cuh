@@ -22,7 +22,22 @@ constexpr int kScanItems = 8;
 constexpr int kScanTileN = kScanThreads * kScanItems;
 constexpr int kDiagThreads = 256;
 constexpr int kDiagSums = 8;
+// A nonzero coordinate below this (in magnitude) sends a step's exact passes to the general
+// pair forms (DevState::general): the others rely on x_i - x_j being 0 or at least 2^-68.
+constexpr float kTiny = 0x1p-45f;
 constexpr int kCellClamp = 1 << 30;    // |cell coordinate| clamp for finite positions
+
+// Operands of the packed pair arithmetic (F2), both halves equal: read as 64-bit operands from
+// the kernel parameters, where a pair built from a scalar would cost two moves at each use.
+typedef unsigned long long f32x2;
+struct PairLits {  // numbers
+    f32x2 neg0;    // -0: see F2
+    f32x2 half, one, two, neg2, three, onehalf, neg2p40, p2p20, neg2p20, p2p21, two_thirds,
+        one_sixth, neg5, five;
+};
+struct PairConst {  // of the step's parameters
+    f32x2 neg_h, h, rcp_h, neg_hsq, rcp_hsq, sigma, neg_sigma, gas, rest, wnorm, wl;
+};
 
 // Constants of one step, computed on the host in float exactly as the reference does
 // (SpatialHash::set_cell_size, spatial_hash.h:63-66; CubicSplineKernel ctor,
@@ -49,6 +64,8 @@ struct StepConst {
     float sw_cs, sw_r2, sw_r2m, sw_skip2;
     int fast_div_h, fast_div_hsq;  // 1: the one-correction sequence is verified for it
     // smoothing kernel (SPHX_KERNEL_*) and the constants its constructor computes in float
+    PairLits lit;
+    PairConst pair;
     int kern;
     float wnorm;  // Wendland norm_factor_ 21/(2 pi h^3); Gaussian norm_ 1/(pi h^2)^1.5
     float wl;     // Wendland norm_factor_ * (5 / h_sq)
@@ -56,7 +73,10 @@ struct StepConst {
     float gg;     // Gaussian -2 sigma_sq_inv_ norm_
     float gl;     // Gaussian 2 sigma_sq_inv_ norm_
     float g2s;    // Gaussian 2 sigma_sq_inv_
-    int div_nz;   // 1: the cubic passes' dividends are in xdiv_fixed_nz's range by bounds
+    // 1: the pair forms' divisions by h and h^2 (div_fixed2) are in range: |r| of a hit is +0
+    // or in [2^-74.5, r (1 + 2^-23)] (div_nz); the gradient's and the Laplacian's dividends of
+    // pairs without tiny coordinates are, too (force_nz)
+    int div_nz, force_nz;
 };
 
 // Device-resident scalars written and read by the kernels of a step.
@@ -82,6 +102,7 @@ struct DevState {
     unsigned long long vmax64;  // precision mode: max |v| (FP64 bits)
     uint32_t n_spread;          // precision mode: spread tiles listed this step
     uint32_t spread_work[2];    // precision mode: tile counters of the spread-tile kernels
+    uint32_t general;           // exact mode: 1 if a value lies outside the pair forms' ranges
 };
 
 // Batched mode: one record per scene (device memory).  Scenes are contiguous ranges of
@@ -112,7 +133,7 @@ struct Buffers {
     float4* vel4;     // insertion order: vx, vy, vz, 0
     float4* pos4_s;   // cell-sorted copies
     float4* vel4_s;
-    float4* aux4_s;   // cell-sorted: rho, P, 2*rho, mass/rho
+    float4* aux4_s;   // cell-sorted: rho, P, (m/rho) mu, 1/(2 rho); precision mode: see density_out
     float4* acc4_s;   // cell-sorted accelerations of the last step/eval
     int4* cell4;      // precision mode, insertion order: cell (x, y, z), w = 1 if not finite
     int4* cell4_s;    // precision mode, cell-sorted copy
@@ -121,7 +142,10 @@ struct Buffers {
     uint32_t* key_s;  // sorted cell keys
     uint32_t* id_s;   // sorted position -> insertion index
     uint32_t* off;    // dense cell grid: first sorted position of each cell (max_cells + 2)
-    uint32_t* tile_start;
+    uint2* tiles;     // warp work items: first target position and number of targets
+    // Target order: the particle of target position k is sorted position tgt[k]; null: k.
+    // (k_order_tiles: a permutation within each cell, so position k's cell is key_s[k].)
+    uint32_t* tgt = nullptr;
     uint32_t* hist;   // radix histograms / offsets
     uint32_t* scan_part;
     double* diag_part;
@@ -129,12 +153,13 @@ struct Buffers {
     uint32_t* scene_s;   // batched mode: scene of each particle (cell-sorted)
     SceneInfo* scenes;   // batched mode: per-scene records
     int nscenes;         // 0: single scene
-    // Hit masks of the density pass, reused by the force pass of the same step: record r
-    // holds 32 words (word = lane: bit j set if candidate j of the chunk is within r of the
-    // lane's particle).  Every warp of the density grid owns an equal region of the pool
-    // and stores its tiles' records one after another, one record per chunk of the tile's
-    // walk; tile_slot[t] = first record, or kNoSlot when the tile did not fit in what was
-    // left of the region (the force pass then repeats the distance tests for that tile).
+    // Hit masks of the density pass, reused by the force pass of the same step.  A tile owns
+    // consecutive records of 32 words: first one word per 32-candidate chunk of the tile's
+    // walk (which candidates the tile's box keeps), then one record per 32 kept candidates
+    // (word = lane: bit 31 - j set if the j-th of them is a neighbour of the lane's particle).
+    // Every warp of the density grid owns an equal region of the pool and stores its tiles
+    // one after another; tile_slot[t] = first record, or kNoSlot when the tile did not fit in
+    // what was left of the region (the force pass then repeats the tests for that tile).
     uint32_t* hitmask = nullptr;
     uint32_t* tile_slot = nullptr;
     unsigned long long hitmask_cap = 0;  // records
@@ -142,21 +167,16 @@ struct Buffers {
     int scan_part_cap;
     int diag_blocks;
     int tile_n = kTile;  // particles per warp work item (1 .. kTile)
-    // 1 (precision-mode step): each cell's particles are put in z order after the sort and
-    // the tiles run along cell columns (x, y, *), spanning cells; 0: the reference's
-    // insertion order within each cell and tiles within one cell
+    // 1: the tiles run along cell columns (x, y, *), spanning cells, with each cell's particles
+    // taken in z order; 0: insertion order within each cell and tiles within one cell
     int columns = 0;
     // precision mode: the tiles whose particles lie in cells far apart (listed by the density
     // sweep, swept by the spread-tile kernels), one entry per tile at most
     uint32_t* spread_tiles = nullptr;
-    // precision mode, single scene (max_cells + 1): per cell, the sorted positions where its
-    // column run -- the stretch of its column that one sequence of tiles fills
-    // (k_column_runs) -- starts and ends; null: runs are whole columns
-    uint2* runs = nullptr;
 };
-// A column run ends before cell z when z is a multiple of kRunAlign and the kRunWindow
-// cells below z hold fewer particles than a tile: no tile of a run then reaches more than
-// kRunCells = kRunWindow + kRunAlign - 1 cells past its first one (k_column_runs).
+// A column's tiles restart at cell z when z is a multiple of kRunAlign and the kRunWindow
+// cells below z hold fewer particles than a tile (tile_starts): no tile then reaches more
+// than kRunCells = kRunWindow + kRunAlign - 1 cells past its first one.
 constexpr int kRunWindow = 2, kRunAlign = 3;
 constexpr int kRunCells = kRunWindow + kRunAlign - 1;
 constexpr uint32_t kNoSlot = 0xffffffffu;
@@ -232,26 +252,8 @@ __device__ __forceinline__ float xdiv_fixed(float a, float b, float y, int verif
     return __fdiv_rn(a, b);
 }
 
-// xdiv_fixed without the range test, for dividends known to be +-0 or of magnitude in
-// [2^-100, 2^100] with a verified divisor b in [2^-20, 2^20].  In that range q0 and the
-// quotient are normal and the residual r is exact (a multiple of 2^(e_a - 46) >= 2^-146,
-// at most about 2^-22 |a|), so the sequence scales exactly with powers of two of a and
-// the verification on one binade covers every binade.  A zero dividend gives +0 whatever
-// its sign; the callers whose dividend can be -0 restore the sign (xsign).
-__device__ __forceinline__ float xdiv_fixed_nz(float a, float b, float y) {
-    const float q0 = __fmul_rn(a, y);
-    const float r = __fmaf_rn(-q0, b, a);
-    return __fmaf_rn(r, y, q0);
-}
-
-// q with the sign bit of a (q = a / b for b > 0: only a zero quotient can lose it)
-__device__ __forceinline__ float xsign(float q, float a) {
-    return __int_as_float((__float_as_int(q) & 0x7fffffff) | (__float_as_int(a) & (int)0x80000000));
-}
-
 // Packed FP32 pairs (Blackwell f32x2 instructions): two IEEE round-to-nearest operations in
 // one instruction, each element rounded exactly as the scalar __f*_rn would.
-typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pk2(float a, float b) {
     f32x2 r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -284,28 +286,99 @@ __device__ __forceinline__ f32x2 xfma2(f32x2 a, f32x2 b, f32x2 c) {
     return d;
 }
 
-// xdiv_fixed of a pair of dividends: the one-correction sequence with packed FP32 pairs
-// when both dividends are in its range (-b is passed pre-negated: fma(q0, -b, a) is the
-// exact a - q0 b), else element by element.
-__device__ __forceinline__ f32x2 xdiv_fixed2(f32x2 a2, float b, float y, int verified) {
-    const float2 a = upk2(a2);
-    const float ax = fabsf(a.x), ay = fabsf(a.y);
-    if (verified && ax >= 0x1p-60f && ax <= 0x1p60f && ay >= 0x1p-60f && ay <= 0x1p60f) {
-        const f32x2 y2 = pk2(y, y);
-        const f32x2 q0 = xmul2(a2, y2);
-        const f32x2 r = xfma2(q0, pk2(-b, -b), a2);
-        return xfma2(r, y2, q0);
-    }
-    return pk2(xdiv_fixed(a.x, b, y, verified), xdiv_fixed(a.y, b, y, verified));
+// ---- packed FP32 pairs as a value type ------------------------------------------------
+// Two pair terms, or two components, side by side: half the instructions of the scalar form
+// (the FP32 pipe still spends a cycle on each half).
+//
+// The compiler (CUDA 13.0) contracts a packed product and the packed addition that uses it
+// into one fma.rn.f32x2 although both are written with .rn (found by comparing sums of
+// products in a loop with the scalar form: 68% differed).  Exact code therefore forms a
+// product that is added or subtracted by pmul, an FMA with a -0 addend which the compiler
+// cannot see through (PairLits::neg0): RN(a b + -0) = RN(a b), zeros' signs included, and
+// an FMA's result is not contracted further.  Unpacked halves added by __fadd_rn are safe.
+struct F2 {
+    f32x2 v;
+};
+__device__ __forceinline__ F2 f2(float a) { return {pk2(a, a)}; }
+__device__ __forceinline__ F2 f2(float a, float b) { return {pk2(a, b)}; }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return {xadd2(a.v, b.v)}; }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return {xsub2(a.v, b.v)}; }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return {xmul2(a.v, b.v)}; }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return {xfma2(a.v, b.v, c.v)}; }
+__device__ __forceinline__ F2 pmul(F2 a, F2 b, F2 neg0) { return {xfma2(a.v, b.v, neg0.v)}; }
+__device__ __forceinline__ F2 select2(bool ka, bool kb, F2 a, F2 b) {
+    const float2 u = upk2(a.v), w = upk2(b.v);
+    return f2(ka ? u.x : w.x, kb ? u.y : w.y);
 }
 
-// xdiv_fixed_nz of a pair of dividends, signs restored
-__device__ __forceinline__ f32x2 xdiv_fixed2_nz(f32x2 a2, float b, float y) {
-    const f32x2 y2 = pk2(y, y);
-    const f32x2 q0 = xmul2(a2, y2);
-    const f32x2 r = xfma2(q0, pk2(-b, -b), a2);
-    const f32x2 q = xfma2(r, y2, q0);
-    return (q & 0x7fffffff7fffffffull) | (a2 & 0x8000000080000000ull);
+__device__ __forceinline__ F2 max0(F2 a) {
+    const float2 u = upk2(a.v);
+    return f2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f));
+}
+
+// xdiv_fixed of both halves without the range test, nb = -b, y = RN(1/b), for dividends known
+// to be +-0 or of magnitude in [2^-100, 2^100] with a verified divisor b in [2^-20, 2^20].  In
+// that range q0 and the quotient are normal and the residual r is exact (a multiple of
+// 2^(e_a - 46) >= 2^-146, at most about 2^-22 |a|), so the sequence scales exactly with powers
+// of two of a and the verification on one binade covers every binade.  A zero dividend gives
+// a zero whose sign is not kept.
+__device__ __forceinline__ F2 div_fixed2(F2 a, F2 nb, F2 y) {
+    const F2 q0 = a * y;
+    return fma2(fma2(q0, nb, a), y, q0);
+}
+
+// a / b, correctly rounded, from the correctly rounded reciprocal y = RN(1/b), nb = -b: two
+// FMA corrections.  The first brings RN(a y) (at most 1.5 ulp off) within an ulp of a / b;
+// the second is then correctly rounded (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990: with y the correctly
+// rounded reciprocal and q within an ulp of a / b, RN(q + RN(a - q b) y) = RN(a / b)).  For
+// dividends that are 0 or at least 2^-100 in magnitude and quotients in the normal range (a
+// zero's sign is not kept).
+__device__ __forceinline__ F2 div_rcp2(F2 a, F2 nb, F2 y) {
+    const F2 q0 = a * y;
+    const F2 q1 = fma2(fma2(q0, nb, a), y, q0);
+    return fma2(fma2(q1, nb, a), y, q1);
+}
+
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Correctly rounded square roots of a pair in [0, 2^86], by Goldschmidt's iteration with a
+// final residual correction (Markstein, "Software division and square root using
+// Goldschmidt's algorithms", RNC6, 2004): from y0 ~ 1/sqrt(x), g ~ sqrt(x) and h ~ 1/(2
+// sqrt(x)) are refined once and g gets the correction (x - g g) h.  x is scaled by 2^40 (the
+// result by 2^-20, both exact), which keeps the residuals of all x that occur out of the
+// subnormal range; the clamp gives sqrt(0) = 0.  Equal to sqrt.rn for every float in the
+// range (all of them compared, test_gpu_kernels).  h: 1/(2 sqrt(2^40 x)), a few ulp.
+// ns: the negated roots (the iteration runs on -g and -x: an FMA needs no negated operand).
+__device__ __forceinline__ F2 sqrt2_exact(const PairLits& k, F2 x, F2& h, F2& ns) {
+    const F2 nx = x * F2{k.neg2p40};
+    const float2 u = upk2(nx.v);
+    const F2 y0 = f2(rsqrt_approx(fmaxf(-u.x, 0x1p-126f)), rsqrt_approx(fmaxf(-u.y, 0x1p-126f)));
+    const F2 ng0 = nx * y0, h0 = y0 * F2{k.half};
+    const F2 r = fma2(ng0, h0, F2{k.half});
+    const F2 ng = fma2(ng0, r, ng0);
+    h = fma2(h0, r, h0);
+    const F2 t = fma2(fma2(ng, ng, nx), h, ng);  // -(g + (x - g g) h)
+    ns = t * F2{k.p2p20};
+    return t * F2{k.neg2p20};
+}
+
+// Correctly rounded reciprocals of b = -nb from approximations y1 within a few ulp: two
+// Newton steps (the first leaves less than an ulp, after which the second is correctly
+// rounded for every significand but all ones, where it ends an ulp below: Markstein 1990).
+__device__ __forceinline__ F2 rcp2_exact(const PairLits& k, F2 nb, F2 y1) {
+    const F2 one{k.one};
+    const F2 y2 = fma2(fma2(nb, y1, one), y1, y1);
+    const float2 y = upk2(fma2(fma2(nb, y2, one), y2, y2).v), s = upk2(nb.v);
+    auto fix = [](float q, float b) {
+        return __uint_as_float(__float_as_uint(q) +
+                               (((__float_as_uint(b) & 0x7fffffu) + 1u) >> 23));
+    };
+    return f2(fix(y.x, s.x), fix(y.y, s.y));
 }
 
 // glm::dot(v, v) = (x*x + y*y) + z*z (products rounded first)
@@ -343,16 +416,11 @@ __device__ __forceinline__ float cubic_grad_factor(const StepConst& c, float q) 
 // numerator, one division follows: lanes of a warp hold q on both sides of 1, and a
 // division per branch would run twice.  Outside both ranges (and for NaN q) the numerator
 // is 0 and 0 / h_sq = +0, the reference's 0.0f.
-template <bool kNZ = false>
 __device__ __forceinline__ float cubic_lap(const StepConst& c, float q) {
     const float a = (q > 1.0f) ? xsub(2.0f, q) : xadd(-2.0f, xmul(3.0f, q));
     const bool in = (q >= 0.0f && q <= 1.0f) || (q > 1.0f && q <= 2.0f);
     const float num = in ? xmul(c.sigma, a) : 0.0f;
-    // kNZ: a is 0 or at least 2^-23 in magnitude (2 - q and 3q - 2 are exact multiples of
-    // ulp(q) or of ulp(3q)), so num is +0 or in [sigma 2^-24, 2 sigma], inside
-    // xdiv_fixed_nz's range for the sigma the host admits
-    return kNZ ? xdiv_fixed_nz(num, c.h_sq, c.rcp_hsq)
-               : xdiv_fixed(num, c.h_sq, c.rcp_hsq, c.fast_div_hsq);
+    return xdiv_fixed(num, c.h_sq, c.rcp_hsq, c.fast_div_hsq);
 }
 
 // WendlandC2Kernel::W after q = length(r)/h (kernels.cpp:172-178):
@@ -384,60 +452,28 @@ __device__ __forceinline__ int cell_coord(float x, float inv_cell) {
     return (int)f;
 }
 
-// ---- bulk copies (cp.async.bulk: the TMA unit's 1-D form) and mbarriers ----------------
-// A warp stages a contiguous range of a cell-sorted array into its shared memory with one
-// bulk copy per array, completed on an mbarrier (one arrival: the issuing lane's
-// arrive.expect_tx with the byte count).  Source and destination 16-byte aligned, size a
-// multiple of 16 bytes: whole float4 elements of cudaMalloc'd arrays.  The threads only
-// read the staged buffers; a buffer is reused once every lane has passed a __syncwarp
-// after its last read.
+// a nonzero coordinate below kTiny in magnitude
+__device__ __forceinline__ bool tiny_coord(float x) { return x != 0.0f && fabsf(x) < kTiny; }
+
+// ---- asynchronous copies of single elements, global to shared memory -------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(arrivals)
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
                  : "memory");
 }
-// makes mbarrier initialisation visible to the bulk-copy (async) proxy
-__device__ __forceinline__ void fence_mbar_init() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src)
+                 : "memory");
 }
-// orders this thread's earlier shared-memory accesses before later async-proxy accesses
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src)
+                 : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile(
-        "{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
-            smem_u32(bar)),
-        "r"(bytes)
-        : "memory");
-}
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes,
-                                              uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ bool mbar_test_parity(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Waits for the phase `parity` of bar to complete, giving up after kMbarWaitLimit polls
-// (each poll may suspend the thread for a short, hardware-defined time): false = gave up.
-constexpr uint32_t kMbarWaitLimit = 1u << 20;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    for (uint32_t it = 0; it < kMbarWaitLimit; ++it)
-        if (mbar_test_parity(bar, parity)) return true;
-    return false;
+// waits for this thread's copies
+__device__ __forceinline__ void cp_async_wait_all() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // ---- precision mode helpers ----------------------------------------------------------
@@ -470,7 +506,6 @@ struct LaunchCtx {
     int num_sms;
     int warps_per_block;
     int blocks_per_sm;
-    int bulk_copy;  // 1: the force pass stages candidates with bulk copies (exact mode)
 };
 
 int launch_begin_step(const LaunchCtx& L, DevState* ds, int reset_bbox);
@@ -478,8 +513,7 @@ int launch_cfl(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevStat
                 float host_dt);
 int launch_build_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                        DevState* ds);
-// cs: the precision mode's cell size (the in-cell z order of b.columns; else unused)
-int launch_grid_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, float cs);
+int launch_grid_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, const StepConst& c);
 int launch_density(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds);
 int launch_force(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
                   int integrate);
@@ -503,7 +537,6 @@ int launch_batch_diag(const LaunchCtx& L, const Buffers& b, DevState* ds);
 
 // radix sort + scan (sphx_sort.cu)
 int launch_radix_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n);
-int launch_tile_scan(const LaunchCtx& L, const Buffers& b, DevState* ds, int n);
 
 // io (sphx_grid.cu)
 void launch_pack(const LaunchCtx& L, int n, const float* pos3, const float* vel3,

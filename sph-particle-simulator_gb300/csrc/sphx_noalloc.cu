@@ -65,7 +65,8 @@ constexpr size_t kOffVal1 = kOffVal0 + align_up(kN * sizeof(uint32_t));
 constexpr size_t kOffKeyS = kOffVal1 + align_up(kN * sizeof(uint32_t));
 constexpr size_t kOffIdS = kOffKeyS + align_up(kN * sizeof(uint32_t));
 constexpr size_t kOffTiles = kOffIdS + align_up(kN * sizeof(uint32_t));
-constexpr size_t kOffOff = kOffTiles + align_up(kN * sizeof(uint32_t));
+constexpr size_t kOffTgt = kOffTiles + align_up(kN * sizeof(uint2));
+constexpr size_t kOffOff = kOffTgt + align_up(kN * sizeof(uint32_t));
 constexpr size_t kOffHist = kOffOff + align_up((kCells + 2) * sizeof(uint32_t));
 constexpr size_t kOffScan = kOffHist + align_up(kHist * sizeof(uint32_t));
 constexpr size_t kNoAllocScratchBytes = kOffScan + align_up(kScanPart * sizeof(uint32_t));
@@ -151,7 +152,9 @@ extern "C" int sphx_density_noalloc(const sphx_params* p, size_t n, const float*
     b.val[1] = reinterpret_cast<uint32_t*>(base + kOffVal1);
     b.key_s = reinterpret_cast<uint32_t*>(base + kOffKeyS);
     b.id_s = reinterpret_cast<uint32_t*>(base + kOffIdS);
-    b.tile_start = reinterpret_cast<uint32_t*>(base + kOffTiles);
+    b.tiles = reinterpret_cast<uint2*>(base + kOffTiles);
+    b.tgt = reinterpret_cast<uint32_t*>(base + kOffTgt);
+    b.columns = 1;
     b.off = reinterpret_cast<uint32_t*>(base + kOffOff);
     b.hist = reinterpret_cast<uint32_t*>(base + kOffHist);
     b.scan_part = reinterpret_cast<uint32_t*>(base + kOffScan);

@@ -17,15 +17,15 @@ __global__ void __launch_bounds__(128) k_pairs(const StepConst c, const Buffers 
     const int nwarps = gridDim.x * (blockDim.x >> 5);
     const uint32_t ntiles = ds->n_tiles;
     for (uint32_t t = blockIdx.x * (blockDim.x >> 5) + warp; t < ntiles; t += nwarps) {
-        const uint32_t k0 = b.tile_start[t];
+        const uint2 tile = b.tiles[t];
         const Geom g = grid_geom(ds);
         Tile T;
         float4 xi;
         bool valid;
         int4 frame = make_int4(0, 0, 0, 0);
-        if (kPrecise) tile_setup_cells(c, b, g, k0, lane, T, xi, valid, frame);
-        else tile_setup(c, b, g, k0, lane, T, xi, valid);
-        const int i = T.k0 + lane;
+        int i = (int)tile.x + lane;
+        if (kPrecise) tile_setup_cells(c, b, g, tile, lane, T, xi, valid, frame);
+        else tile_setup(c, b, g, tile, lane, T, i, xi, valid);
         const uint32_t id = valid ? b.id_s[i] : 0u;
         uint64_t pos = (kFill && valid) ? off_by_id[id] : 0ull;
         const bool want = !kFill || pos != kNoPairs;  // fill: particles with an offset only

@@ -1,14 +1,14 @@
 // Shared device code of the neighbour passes (density + pressure in sphx_density.cu, force +
-// leapfrog + wall clamp in sphx_force.cu, the neighbour-list dump in sphx_passes.cu): tiles,
-// the stencil walk, the chunk machinery, the pair arithmetic helpers and the launch-shape
-// cache.
+// leapfrog + wall clamp in sphx_force.cu, the precision mode's in sphx_sweep.cu, the
+// neighbour-list dump in sphx_passes.cu): tiles, the stencil walk, the candidate rings, the
+// pair arithmetic helpers and the launch-shape cache.
 //
-// Work decomposition: one warp owns one tile (up to 32 consecutive cell-sorted particles of
-// one cell column (x, y, *), one particle per lane; a tile may span several cells of its
-// column).  All lanes of a tile share the tile's stencil: for each row (dx, dy) the cells
-// cz+lo..cz+hi (covering every lane's cell +-1, +-2 near a face) are one contiguous range
-// of the sorted arrays; the warp stages that range through shared memory 32 candidates at
-// a time and every lane tests every candidate against its own particle.
+// Work decomposition: one warp owns one tile (up to 32 particles of one cell column
+// (x, y, *), one particle per lane; a tile may span several cells of its column).  All lanes
+// of a tile share the tile's stencil: for each row (dx, dy) the cells cz+lo..cz+hi (covering
+// every lane's cell +-1, +-2 near a face) are one contiguous range of the sorted arrays; the
+// warp reads that range 32 candidates at a time, drops those the tile's box cannot reach and
+// keeps the rest in a shared-memory ring from which every lane takes its own neighbours.
 //
 // Exactness.  The reference walks, for particle i, the cells (dx, dy, dz) of its stencil
 // in lexicographic order and each cell's particles in insertion order
@@ -16,7 +16,8 @@
 // (sph_engine.cpp:370-432).  The sorted arrays hold each cell's particles in insertion
 // order (stable sort from insertion order), the rows are walked in (dx, dy) order and
 // each row in increasing z, so a lane meets its neighbours in exactly the reference's
-// order.  The reference scans a 5x5x5 block (cell_radius = 2); a neighbour at distance
+// order, whichever particles share its tile.  The reference scans a 5x5x5 block
+// (cell_radius = 2); a neighbour at distance
 // <= r can only sit two cells away when the particle lies within rounding distance of a
 // cell face, so the tile's stencil is the 3x3x3 block of each of its cells, widened on an
 // axis to the second layer when some lane is that close to a face (guard band eps below).
@@ -64,16 +65,6 @@ __device__ __forceinline__ Geom scene_geom(const SceneInfo& sc, const DevState* 
     return g;
 }
 
-// End (sorted position) of the run a tile of cell `key` may fill: the cell, or (b.columns)
-// its cell column -- its column run where b.runs holds them (single scene) -- (the
-// non-finite group is its own column).
-__device__ __forceinline__ uint32_t tile_run_end(const Buffers& b, const Geom& g, uint32_t key) {
-    if (!b.columns || key >= g.sentinel) return b.off[key + 1];
-    if (b.runs && !b.nscenes) return b.runs[key].y;
-    const uint32_t d2 = (uint32_t)g.dim[2];
-    return b.off[g.base + ((key - g.base) / d2 + 1u) * d2];
-}
-
 // The tile's z range relative to its first particle's cell: every lane's cell +-1, or +-2
 // on the side where the lane lies within the guard band of a cell face.
 __device__ __forceinline__ void tile_z_range(const Buffers& b, const Geom& g, uint32_t k0,
@@ -85,17 +76,19 @@ __device__ __forceinline__ void tile_z_range(const Buffers& b, const Geom& g, ui
     T.hi[2] = __reduce_max_sync(0xffffffffu, rz + (near_hi ? 2 : 1));
 }
 
-// Sets up the tile starting at sorted position k0; returns the lane's particle (valid
-// lanes only).
+// Sets up a tile; returns the sorted position i of the lane's particle and the particle
+// (valid lanes only).
 __device__ __forceinline__ void tile_setup(const StepConst& c, const Buffers& b, const Geom& g,
-                                           uint32_t k0, int lane, Tile& T, float4& xi,
+                                           uint2 tile, int lane, Tile& T, int& i, float4& xi,
                                            bool& valid) {
+    const uint32_t k0 = tile.x;
     const uint32_t key = b.key_s[k0];
-    const uint32_t end = tile_run_end(b, g, key);
     T.k0 = (int)k0;
-    T.cnt = (int)min(end - k0, (uint32_t)b.tile_n);
+    T.cnt = (int)tile.y;
     valid = lane < T.cnt;
-    xi = valid ? b.pos4_s[k0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    i = (int)k0 + lane;
+    if (b.tgt && valid) i = (int)b.tgt[k0 + lane];
+    xi = valid ? b.pos4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     T.cells = key < g.sentinel;
     if (!T.cells) return;
     const uint32_t local = key - g.base;
@@ -135,14 +128,14 @@ __device__ __forceinline__ float4 frame_pos(const int4& cell, const int4& frame,
 }
 
 __device__ __forceinline__ void tile_setup_cells(const StepConst& c, const Buffers& b,
-                                                 const Geom& g, uint32_t k0, int lane,
+                                                 const Geom& g, uint2 tile, int lane,
                                                  Tile& T, float4& xi, bool& valid,
                                                  int4& frame) {
+    const uint32_t k0 = tile.x;
     const uint32_t key = b.key_s[k0];
     const uint32_t nc = g.sentinel;
-    const uint32_t end = tile_run_end(b, g, key);
     T.k0 = (int)k0;
-    T.cnt = (int)min(end - k0, (uint32_t)b.tile_n);
+    T.cnt = (int)tile.y;
     valid = lane < T.cnt;
     frame = b.cell4_s[k0];
     const float4 o = valid ? b.pos4_s[k0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -320,55 +313,7 @@ __device__ __forceinline__ float diff_d2(const float4& xi, const float4& xj) {
     return xadd(xadd(sq.x, sq.y), xmul(dz, dz));
 }
 
-// a gradient component inside xdiv_fixed_nz's range: zero, or at least 2^-100 in
-// magnitude (its upper bound, sigma, is the host's business)
-__device__ __forceinline__ bool nz_range(float g) { return !(fabsf(g) < 0x1p-100f) || g == 0.0f; }
-
-// ---------------------------------------------------------------------------------------
-// Chunk machinery shared by the density and force passes.
-//
-// A row segment is consumed in chunks of 32 candidates staged in shared memory.  For a
-// chunk, every lane first builds a 32-bit mask of its hits (the exact distance test; the
-// candidates a warp-uniform bounding-box test rules out for the whole tile are skipped).
-// The expensive per-pair terms are then computed FLATTENED: the warp's hits are listed
-// (lane, candidate) in lane-then-candidate order and the 32 lanes work through that list
-// together, writing each term to shared memory.  Finally every lane adds its own terms in
-// candidate order -- the reference's order -- so each particle's sums are the same
-// sequence of IEEE additions as in the reference, while the SIMT lanes stay busy on the
-// costly terms regardless of how unevenly the hits fall on lanes.
-// ---------------------------------------------------------------------------------------
-
 constexpr uint32_t kFull = 0xffffffffu;
-constexpr int kDensityBatch = 256;  // flattened terms computed per round (density)
-constexpr int kForceBatch = 96;     // flattened terms computed per round (force)
-
-__device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, int lane, uint32_t& total) {
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, x, o);
-        if (lane >= o) x += y;
-    }
-    total = __shfl_sync(kFull, x, 31);
-    return x - v;
-}
-
-// Writes this lane's hits (mask) to plist[o, o + popc(mask)) as (lane << 5) | candidate,
-// in candidate order, two per iteration.
-__device__ __forceinline__ void list_hits(uint16_t* plist, uint32_t mask, uint32_t o, int lane) {
-    const uint32_t tag = (uint32_t)lane << 5;
-    uint32_t mm = mask, k = o;
-    while (mm) {
-        const uint32_t a = __ffs(mm) - 1;
-        mm &= mm - 1;
-        plist[k] = (uint16_t)(tag | a);
-        if (!mm) break;
-        const uint32_t b = __ffs(mm) - 1;
-        mm &= mm - 1;
-        plist[k + 1] = (uint16_t)(tag | b);
-        k += 2;
-    }
-}
 
 // Axis-aligned box of the tile's particles (valid lanes).
 struct TileBox {
@@ -402,53 +347,162 @@ __device__ __forceinline__ bool box_near(const TileBox& B, const float4& p, floa
     return ex * ex + ey * ey + ez * ez <= r2_margin;
 }
 
-// Hit mask of this lane's particle against the staged chunk (candidates in `surv` only):
-// the reference's rounded test.
-__device__ __forceinline__ uint32_t chunk_hits(const float4* cand, uint32_t surv,
-                                               const float4& xi, float r2) {
-    uint32_t mask = 0;
-#pragma unroll
-    for (int jj = 0; jj < 32; ++jj) {
-        if (surv & (1u << jj)) {
-            if (diff(xi, cand[jj]).d2 <= r2) mask |= 1u << jj;
+// ---------------------------------------------------------------------------------------
+// Candidate rings (density and force passes).
+//
+// The candidates of the tile's walk that its box keeps are appended, in order, to a ring of
+// kRing chunks of 32 in shared memory, and each complete chunk gets one 32-bit mask per lane:
+// bit p is set when the candidate in slot p of the chunk is a neighbour of the lane's
+// particle.  The j-th candidate of a chunk sits in slot 31 - j, so that the highest set bit is
+// the next neighbour in order.  Every lane then takes its own neighbours one after another,
+// each at its own place in the ring, forms the term and adds it to its sums in registers: no
+// hit list, no staging of terms, and the additions happen in the walk's order by construction.
+//
+// What bounds the split: all lanes of a warp issue together, so a pass costs the largest
+// number of terms any lane has between two points where the lanes must meet.  The lanes of a
+// tile have about the same number of neighbours in all (270 on the lattice, within 7%) but
+// meet them at different times: a particle on the low-x side of the tile meets its first
+// third of the stream before one on the high side meets any.  The ring is what lets a lane
+// run ahead; its length trades resident warps (shared memory) for that freedom.  Iterations
+// per particle on the lattice (ideal 7.5): 21 with one chunk, 13 with 4, 11 with 8, 9.1 with
+// 12, 8.0 with 16.
+// ---------------------------------------------------------------------------------------
+
+// The walk's row segments, 32 candidates at a time (warp-uniform).
+struct RawStream {
+    const int2* seg;
+    int nseg, sg, s, e;
+    __device__ __forceinline__ RawStream(const int2* segs, int n) : seg(segs), nseg(n), sg(0) {
+        s = n ? segs[0].x : 0;
+        e = n ? segs[0].y : 0;
+    }
+    __device__ __forceinline__ bool more() const { return sg < nseg; }
+    __device__ __forceinline__ int count() const { return min(32, e - s); }
+    __device__ __forceinline__ void next() {
+        s += 32;
+        if (s < e) return;
+        if (++sg < nseg) {
+            s = seg[sg].x;
+            e = seg[sg].y;
         }
     }
-    return mask;
+};
+
+// 32-candidate chunks of all segments (all lanes call it, all get the sum)
+__device__ __forceinline__ int raw_chunks(const int2* seg, int nseg, int lane) {
+    int n = 0;
+    for (int q = lane; q < nseg; q += 32) n += (seg[q].y - seg[q].x + 31) >> 5;
+    return __reduce_add_sync(kFull, n);
 }
 
-// chunk_hits two candidates at a time with packed FP32 pairs: the same exact test
-// (x_i - x_j per axis, (dx*dx + dy*dy) + dz*dz, <= r^2), element by element.  Candidates
-// outside `surv` are farther than r from every lane (the box cull is conservative), so a
-// pair is skipped only when both of its candidates are.
-__device__ __forceinline__ uint32_t chunk_hits_x2(const float* cx, const float* cy,
-                                                  const float* cz, uint32_t surv,
-                                                  const float4& xi, float r2) {
-    const f32x2 X = pk2(xi.x, xi.x), Y = pk2(xi.y, xi.y), Z = pk2(xi.z, xi.z);
-    uint32_t mask = 0;
+// Ring slot of the a-th candidate kept (a counts from the tile's start).
+template <int kRing>
+__device__ __forceinline__ int ring_slot(int a) {
+    return ((a >> 5) % kRing) * 32 + (31 - (a & 31));
+}
+
+// glm::dot(d, d) of two separations
+__device__ __forceinline__ F2 pair_d2(F2 dx, F2 dy, F2 dz, F2 neg0) {
+    return (pmul(dx, dx, neg0) + pmul(dy, dy, neg0)) + pmul(dz, dz, neg0);
+}
+
+// Neighbour mask of the lane's particle against a complete chunk (32 slots of cx, cy, cz): the
+// reference's rounded test (x_i - x_j per axis, (dx*dx + dy*dy) + dz*dz, <= r^2), two
+// candidates per packed FP32 instruction, element by element.  d2 <= r2 is read from the sign
+// of r2 - d2 (exact: a rounded difference keeps its sign), shifted into the mask.
+__device__ __forceinline__ uint32_t ring_hits(const float* cx, const float* cy, const float* cz,
+                                              const float4& xi, float r2, F2 neg0) {
+    const F2 X = f2(xi.x), Y = f2(xi.y), Z = f2(xi.z), R2 = f2(r2);
+    uint32_t miss = 0;
 #pragma unroll
-    for (int jj = 0; jj < 32; jj += 2) {
-        if ((surv >> jj) & 3u) {
-            const f32x2 dx = xsub2(X, *reinterpret_cast<const f32x2*>(cx + jj));
-            const f32x2 dy = xsub2(Y, *reinterpret_cast<const f32x2*>(cy + jj));
-            const f32x2 dz = xsub2(Z, *reinterpret_cast<const f32x2*>(cz + jj));
-            const float2 d2 = upk2(xadd2(xadd2(xmul2(dx, dx), xmul2(dy, dy)), xmul2(dz, dz)));
-            if (d2.x <= r2) mask |= 1u << jj;
-            if (d2.y <= r2) mask |= 2u << jj;
+    for (int q = 28; q >= 0; q -= 4) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(cx + q);
+        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(cy + q);
+        const ulonglong2 z = *reinterpret_cast<const ulonglong2*>(cz + q);
+#pragma unroll
+        for (int h = 1; h >= 0; --h) {
+            const F2 dx = X - F2{h ? x.y : x.x}, dy = Y - F2{h ? y.y : y.x},
+                     dz = Z - F2{h ? z.y : z.x};
+            const float2 t = upk2((R2 - pair_d2(dx, dy, dz, neg0)).v);
+            miss = __funnelshift_l(__float_as_uint(t.y), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(t.x), miss, 1);
         }
     }
-    return mask;
+    return ~miss;
 }
 
-// W of the pair (x_i - x_j = (dx, dy, dz), d2 = |.|^2) for smoothing kernel K, with the
-// reference's float operations (Kernel::W, kernels.cpp:140-143, 172-178, 210-213).
-// kNZ: d2 <= r^2 (a hit), so |r| is +0 or in [2^-74.5, r (1 + 2^-23)], which the host
-// keeps inside xdiv_fixed_nz's range
-template <int K, bool kNZ = false>
+// slots of a chunk that hold candidates when `left` of the stream remain from its start
+__device__ __forceinline__ uint32_t chunk_valid(int left) {
+    return left >= 32 ? kFull : ~(kFull >> left);
+}
+
+// position of the highest set bit
+__device__ __forceinline__ uint32_t top_bit(uint32_t m) {
+    uint32_t p;
+    asm("bfind.u32 %0, %1;" : "=r"(p) : "r"(m));
+    return p;
+}
+
+// A lane's place in the ring: the next chunk to load and what is left of the mask of the one
+// before it.
+template <int kRing>
+struct RingLane {
+    int next = 0;  // chunks from the tile's start
+    int at = 0;    // first slot of the chunk being worked through
+    int at_next = 0;
+    uint32_t m = 0;
+    // first chunk still needed
+    __device__ __forceinline__ int need() const { return next - (m != 0); }
+    // loads the next of the first n chunks when the last one is used up
+    __device__ __forceinline__ void advance(const uint32_t* mask, int n, int lane) {
+        if (m == 0 && next < n) {
+            m = mask[at_next + lane];
+            at = at_next;
+            at_next = at == (kRing - 1) * 32 ? 0 : at + 32;
+            ++next;
+        }
+    }
+    // Slots of the next two neighbours of the chunk, removed from the mask; a: there is one,
+    // b: there are two (otherwise the slot is some slot of the ring).
+    __device__ __forceinline__ void take2(int& qa, int& qb, bool& a, bool& b) {
+        a = m != 0;
+        const uint32_t pa = top_bit(m) & 31u;
+        m &= ~(1u << pa);
+        b = m != 0;
+        const uint32_t pb = top_bit(m) & 31u;
+        m &= ~(1u << pb);
+        qa = at + (int)pa;
+        qb = at + (int)pb;
+    }
+};
+
+// W of the pair with |x_i - x_j|^2 = d2 for smoothing kernel K, with the reference's float
+// operations (Kernel::W, kernels.cpp:140-143, 172-178, 210-213).
+template <int K>
 __device__ __forceinline__ float pair_w_exact(const StepConst& c, float d2) {
     if (K == SPHX_KERNEL_GAUSSIAN) return xmul(c.wnorm, expf(xmul(-d2, c.gs)));
-    const float q = kNZ ? xdiv_fixed_nz(xsqrt(d2), c.h, c.rcp_h)
-                        : xdiv_fixed(xsqrt(d2), c.h, c.rcp_h, c.fast_div_h);
+    const float q = xdiv_fixed(xsqrt(d2), c.h, c.rcp_h, c.fast_div_h);
     return K == SPHX_KERNEL_WENDLAND_C2 ? wendland_w(c, q) : cubic_w(c, q);
+}
+
+// pair_w_exact of two neighbours of the cubic spline or Wendland kernel (StepConst::div_nz and
+// no tiny coordinate: d2 is 0 or at least 2^-136)
+template <int K>
+__device__ __forceinline__ F2 pair_w_exact2(const PairLits& k, const PairConst& c, F2 d2) {
+    const F2 neg0{k.neg0};
+    F2 hr, ns;
+    const F2 q = div_fixed2(sqrt2_exact(k, d2, hr, ns), F2{c.neg_h}, F2{c.rcp_h});
+    const float2 u = upk2(q.v);
+    // beyond the support q = 2 the clamped 2 - q (1 - q/2) makes the outer branch the 0 that
+    // the reference returns there; 0.5 q and 2 q are exact: contraction changes nothing
+    if (K == SPHX_KERNEL_WENDLAND_C2) {
+        const F2 t = max0(F2{k.one} - F2{k.half} * q);
+        return F2{c.wnorm} * t * t * t * t * (F2{k.two} * q + F2{k.one});
+    }
+    const F2 t = max0(F2{k.two} - q);
+    const F2 w1 = (F2{k.two_thirds} - pmul(q, q, neg0)) + pmul(F2{k.half} * q * q, q, neg0);
+    const F2 w2 = F2{k.one_sixth} * t * t * t;
+    return F2{c.sigma} * select2(u.x <= 1.0f, u.y <= 1.0f, w1, w2);
 }
 
 // Precision-mode leapfrog + wall clamp on cell + offset positions (FP64 clamp).
@@ -503,6 +557,8 @@ __device__ __forceinline__ uint32_t next_tile(uint32_t* ctr, int lane) {
 template <class K>
 inline int resident_blocks(const LaunchCtx& L, K kernel, int threads, size_t smem) {
     int per_sm = 0;
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) !=
             cudaSuccess ||
         per_sm < 1)

@@ -234,76 +234,4 @@ int launch_radix_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n)
     return launches;
 }
 
-// ---------------------------------------------------------------------------------------
-// tile list: a tile starts at every tile_n-th particle of a cell, or (b.columns) of a cell
-// column (x, y, *) -- of a column run (b.runs, k_column_runs) in a single-scene precision
-// step -- contiguous in cell-sorted order; the non-finite group (key == ncells) is tiled
-// the same way.  A column tile may span several cells: the passes walk the union of its
-// particles' stencils.
-// ---------------------------------------------------------------------------------------
-
-// first cell of the column of cell `key` (the non-finite group is its own column)
-__device__ __forceinline__ uint32_t column_base(uint32_t key, uint32_t k, const DevState* ds,
-                                                const uint32_t* scene_s,
-                                                const SceneInfo* scenes) {
-    if (key >= ds->ncells) return key;
-    uint32_t base = 0, d2 = (uint32_t)ds->dim[2];
-    if (scenes) {
-        const SceneInfo& sc = scenes[scene_s[k]];
-        base = sc.base;
-        d2 = (uint32_t)sc.dim[2];
-    }
-    return base + (key - base) / d2 * d2;
-}
-
-struct TileSrc {
-    const uint32_t* key_s;
-    const uint32_t* off;
-    const DevState* ds;
-    const uint32_t* scene_s;  // batched mode (else null)
-    const SceneInfo* scenes;
-    uint32_t tile_n;        // particles per tile
-    int columns;            // 1: tiles along cell columns, else within cells
-    const uint2* runs;      // columns: each cell's run (null: the whole column)
-    __device__ bool active() const { return !ds->status; }
-    __device__ uint32_t operator()(uint32_t k) const {
-        const uint32_t key = key_s[k];
-        uint32_t st;
-        if (!columns || key >= ds->ncells) st = off[key];
-        else if (runs) st = runs[key].x;
-        else st = off[column_base(key, k, ds, scene_s, scenes)];
-        return (k - st) % tile_n == 0 ? 1u : 0u;
-    }
-};
-// Writes the tile starts and counts the occupied cells and the fullest one (the threads
-// of a warp call it together: one atomic of each kind per warp and call).
-struct TileSink {
-    const uint32_t* key_s;
-    const uint32_t* off;
-    uint32_t* tile_start;
-    DevState* ds;
-    __device__ void operator()(uint32_t k, uint32_t excl, uint32_t v) const {
-        if (v) tile_start[excl] = k;
-        const uint32_t c = key_s[k];
-        const bool start = c < ds->ncells && off[c] == k;
-        const unsigned am = __activemask();
-        const unsigned starts = __ballot_sync(am, start);
-        if (!starts) return;
-        const uint32_t occ = __reduce_max_sync(am, start ? off[c + 1] - k : 0u);
-        if ((threadIdx.x & 31) == (uint32_t)(__ffs(am) - 1)) {
-            atomicAdd(&ds->occupied, (uint32_t)__popc(starts));
-            atomicMax(&ds->max_occ, occ);
-        }
-    }
-};
-
-int launch_tile_scan(const LaunchCtx& L, const Buffers& b, DevState* ds, int n) {
-    const bool batched = b.nscenes > 0;
-    const TileSrc src{b.key_s, b.off, ds, batched ? b.scene_s : nullptr,
-                      batched ? b.scenes : nullptr, (uint32_t)b.tile_n, b.columns,
-                      batched ? nullptr : b.runs};
-    return scan(L, src, TileSink{b.key_s, b.off, b.tile_start, ds},
-         (uint32_t)n, b.scan_part, &ds->n_tiles);
-}
-
 }  // namespace sphx

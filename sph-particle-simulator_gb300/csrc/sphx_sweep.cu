@@ -40,34 +40,15 @@ namespace sphx {
 
 namespace {
 
-// ---- packed FP32 pairs ----------------------------------------------------------------
-struct F2 {
-    f32x2 v;
-};
-__device__ __forceinline__ F2 f2(float a) { return {pk2(a, a)}; }
-__device__ __forceinline__ F2 f2(float a, float b) { return {pk2(a, b)}; }
-__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return {xadd2(a.v, b.v)}; }
-__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return {xsub2(a.v, b.v)}; }
-__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return {xmul2(a.v, b.v)}; }
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return {xfma2(a.v, b.v, c.v)}; }
-__device__ __forceinline__ F2 max0(F2 a) {
-    const float2 u = upk2(a.v);
-    return f2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f));
-}
 __device__ __forceinline__ F2 keep(bool ka, bool kb, F2 a) {
     const float2 u = upk2(a.v);
     return f2(ka ? u.x : 0.0f, kb ? u.y : 0.0f);
 }
 
-// hardware square root and reciprocal square root (a few ulp; precision mode only)
+// hardware square root (a few ulp; precision mode only)
 __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 __device__ __forceinline__ float exp_approx(float x) { return __expf(x); }
@@ -249,7 +230,7 @@ __global__ void __launch_bounds__(128, 6) k_density_sweep(const StepConst c, con
         float4 xi;
         bool valid;
         int4 frame;
-        tile_setup_cells(c, b, g, b.tile_start[t], lane, T, xi, valid, frame);
+        tile_setup_cells(c, b, g, b.tiles[t], lane, T, xi, valid, frame);
         const int i = T.k0 + lane;
         if (spread_tile(b, T, i, valid, frame)) {
             if (lane == 0) b.spread_tiles[atomicAdd(&ds->n_spread, 1u)] = t;
@@ -348,7 +329,7 @@ __global__ void __launch_bounds__(128, 4) k_density_sweep_spread(const StepConst
         float4 xi;
         bool valid;
         int4 frame;
-        tile_setup_cells(c, b, g, b.tile_start[b.spread_tiles[t]], lane, T, xi, valid, frame);
+        tile_setup_cells(c, b, g, b.tiles[b.spread_tiles[t]], lane, T, xi, valid, frame);
         const int i = T.k0 + lane;
         const int4 ct = valid ? b.cell4_s[i] : frame;
         const float4 o = valid ? b.pos4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -573,7 +554,7 @@ __global__ void __launch_bounds__(128, 5) k_force_sweep(const StepConst c, const
         float4 xi;
         bool valid;
         int4 frame;
-        tile_setup_cells(c, b, g, b.tile_start[t], lane, T, xi, valid, frame);
+        tile_setup_cells(c, b, g, b.tiles[t], lane, T, xi, valid, frame);
         const int i = T.k0 + lane;
         if (spread_tile(b, T, i, valid, frame))
             continue;  // listed by the density launch, swept by the spread launch
@@ -687,7 +668,7 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep_spread(const StepConst c
         float4 xi;
         bool valid;
         int4 frame;
-        tile_setup_cells(c, b, g, b.tile_start[b.spread_tiles[t]], lane, T, xi, valid, frame);
+        tile_setup_cells(c, b, g, b.tiles[b.spread_tiles[t]], lane, T, xi, valid, frame);
         const int i = T.k0 + lane;
         const int4 ct = valid ? b.cell4_s[i] : frame;
         const float4 o = valid ? b.pos4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);

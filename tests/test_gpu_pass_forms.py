@@ -1,0 +1,94 @@
+"""The exact passes' forms and limits, bit for bit against the oracle: the packed pair
+arithmetic itself (every square root and reciprocal compared with CUDA's), and states that
+leave its ranges or stress the candidate ring."""
+import subprocess
+
+import numpy as np
+import pytest
+
+import sph_oracle as O
+import sphx
+import sphx_build
+import sphx_inputs as I
+
+pytestmark = pytest.mark.gpu
+
+
+def test_pair_arithmetic_is_correctly_rounded(built, tmp_path):
+    src = sphx_build.REPO / "tests" / "cpp" / "pair_math_check.cu"
+    exe = tmp_path / "pair_math_check"
+    subprocess.run([sphx_build._nvcc(), *sphx_build.NVCC_FLAGS, *sphx_build.ARCH,
+                    f"-I{sphx_build.PKG / 'csrc'}", str(src), "-o", str(exe),
+                    f"-L{sphx_build.LIB}", "-lsphx", f"-Xlinker=-rpath={sphx_build.LIB}"],
+                   check=True, capture_output=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+    assert out.split() == ["roots", "0", "reciprocals", "0", "quotients", "0", "products", "0"]
+
+
+def block(n_side, seed, jitter=5e-4, origin=0.1):
+    rng = np.random.default_rng(seed)
+    pos = I.lattice(n_side, n_side, n_side, seed=seed, jitter=jitter, origin=(origin,) * 3)
+    vel = (0.1 * rng.standard_normal(pos.shape)).astype(np.float32)
+    return pos, vel, np.full(len(pos), 1e-3, np.float32), I.params16()
+
+
+def state(name):
+    if name in ("one", "two", "thirty_three"):  # fewer and one more than a warp
+        pos, vel, mass, prm = block(4, 3)
+        n = {"one": 1, "two": 2, "thirty_three": 33}[name]
+        return pos[:n], vel[:n], mass[:n], prm
+    if name == "tiny_coordinates":  # the general forms: separations down to the subnormals
+        pos, vel, mass, prm = block(12, 4, origin=0.0)
+        pos[5] = (1e-20, 0.0, 1e-41)
+        pos[6] = (0.0, -1e-30, 0.0)
+        pos[7] = (1e-20, 0.0, 1e-41)
+        return pos, vel, mass, prm
+    if name == "light":  # densities outside the shared reciprocals' range
+        pos, vel, mass, prm = block(12, 5)
+        return pos, vel, np.full(len(pos), 1e-15, np.float32), prm
+    if name == "zero_pressure":  # P_i + P_j = 0 among infinities of neither sign
+        pos, vel, mass, prm = block(12, 6)
+        return pos, vel, mass, I.params16(gas_constant=0.0)
+    if name == "close_pairs":  # |r| around the 1e-6 below which the pressure term is skipped
+        pos, vel, mass, prm = block(12, 7)
+        pos[1::3] = pos[0::3][: len(pos[1::3])] + np.float32(1e-6) * \
+            np.random.default_rng(1).random((len(pos[1::3]), 3)).astype(np.float32)
+        return pos, vel, mass, prm
+    if name == "wide_radius":  # twice the support: 2,100 neighbours, most of zero weight
+        pos, vel, mass, prm = block(24, 8)
+        return pos, vel, mass, I.params16(neighbor_search_radius=0.08)
+    if name == "ties":  # many pairs at |r| = r_search exactly, on cell faces
+        k = np.arange(14, dtype=np.float32) * np.float32(0.0078125)
+        pos = np.stack(np.meshgrid(k, k, k, indexing="ij"), -1).reshape(-1, 3)
+        vel = (0.1 * np.random.default_rng(2).standard_normal(pos.shape)).astype(np.float32)
+        return (pos, vel, np.full(len(pos), 1e-3, np.float32),
+                I.params16(smoothing_length=0.015625, neighbor_search_radius=0.03125))
+    if name == "sparse_column":  # tiles cut along a column of mostly empty cells
+        rng = np.random.default_rng(9)
+        pos = np.zeros((700, 3), np.float32)
+        pos[:, 2] = np.sort(rng.random(700) * 40).astype(np.float32)
+        pos[:, :2] = (0.02 * rng.random((700, 2))).astype(np.float32)
+        return pos, np.zeros_like(pos), np.full(700, 1e-3, np.float32), I.params16()
+    # a dense clump beside a lattice: lanes of one tile with very different neighbour counts
+    pos, vel, mass, prm = block(16, 10)
+    pos[:1500] = (0.14 + 0.01 * np.random.default_rng(3).random((1500, 3))).astype(np.float32)
+    return pos, vel, mass, prm
+
+
+@pytest.mark.parametrize("kernel", [sphx.KERNEL_CUBIC_SPLINE, sphx.KERNEL_WENDLAND_C2])
+@pytest.mark.parametrize("name", ["one", "two", "thirty_three", "tiny_coordinates", "light",
+                                  "zero_pressure", "close_pairs", "wide_radius", "ties",
+                                  "sparse_column", "clump"])
+def test_fields_bit_identical(port, name, kernel):
+    pos, vel, mass, prm = state(name)
+    ctx = sphx.Context(len(pos))
+    ctx.set_params(prm)
+    ctx.set_kernel(kernel)
+    ctx.upload(pos, vel, mass)
+    ctx.eval()
+    out = ctx.download()
+    rho, p, acc = port.fields(pos, vel, mass, prm, kernel=kernel)
+    for got, want, key in ((out["rho"], rho, "rho"), (out["pressure"], p, "P"),
+                           (out["acc"], acc, "acc")):
+        assert O.bits_equal(got, want), O.mismatch_report(got, want, key)
+    ctx.close()
