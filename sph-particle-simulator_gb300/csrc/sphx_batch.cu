@@ -19,160 +19,145 @@ static inline int blocks_for(const LaunchCtx& L, int n, int threads, int per_sm 
     return need < 1 ? 1 : (need < cap ? need : cap);
 }
 
-__global__ void k_batch_begin(SceneInfo* scenes, int nscenes, DevState* ds) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) {
-        ds->status = 0;
-        ds->nonfinite = 0;
-        ds->occupied = 0;
-        ds->max_occ = 0;
-        ds->n_tiles = 0;
-        ds->work[0] = 0;
-        ds->work[1] = 0;
-        ds->general = 0;
-    }
-    if (s >= nscenes) return;
-    SceneInfo& sc = scenes[s];
+// ---- the step's first kernel --------------------------------------------------------------
+
+// What a warp has gathered of one scene.
+struct SceneAcc {
+    uint32_t scene;
+    int mn[3], mx[3];
+    uint32_t bad, vmax;
+};
+__device__ __forceinline__ void clear(SceneAcc& s, uint32_t scene) {
+    s.scene = scene;
     for (int a = 0; a < 3; ++a) {
-        sc.cmin[a] = 0x7fffffff;
-        sc.cmax[a] = -0x7fffffff - 1;
+        s.mn[a] = 0x7fffffff;
+        s.mx[a] = -0x7fffffff - 1;
     }
-    sc.nonfinite = 0;
-    sc.vmax_bits = 0;
+    s.bad = s.vmax = 0;
 }
-
-int launch_batch_begin(const LaunchCtx& L, const Buffers& b, DevState* ds) {
-    k_batch_begin<<<(b.nscenes + 255) / 256, 256, 0, L.stream>>>(b.scenes, b.nscenes, ds);
-    return 1;
-}
-
-// ---- CFL per scene --------------------------------------------------------------------
-
-__global__ void k_batch_vmax(const float4* __restrict__ vel4, const uint32_t* __restrict__ scene_of,
-                             int n, SceneInfo* scenes) {
-    const int lane = threadIdx.x & 31;
-    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base < n;
-         base += gridDim.x * blockDim.x) {
-        const int i = base + lane;
-        uint32_t m = 0, s = 0xffffffffu;
-        if (i < n) {
-            const float4 v = vel4[i];
-            const float len = xsqrt(xdot3(v.x, v.y, v.z));
-            if (!isnan(len)) m = __float_as_uint(len);  // NaN ignored like std::max
-            s = scene_of[i];
-        }
-        // lanes of one scene combine, then one atomic per scene per warp
-        const uint32_t peers = __match_any_sync(0xffffffffu, s);
-        uint32_t mm = m;
-        for (uint32_t rest = peers; rest; rest &= rest - 1) {
-            const int src = __ffs(rest) - 1;
-            mm = max(mm, __shfl_sync(peers, m, src));
-        }
-        if (s != 0xffffffffu && lane == __ffs(peers) - 1 && mm) atomicMax(&scenes[s].vmax_bits, mm);
-    }
-}
-
-// Per scene: dt = min({dt_cfl, dt_force, timestep}) (SPHEngine::compute_cfl_timestep,
-// sph_engine.cpp:312-333) or the host dt; current_time_ += dt.
-__global__ void k_batch_set_dt(SceneInfo* scenes, int nscenes, float host_dt) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nscenes) return;
-    SceneInfo& sc = scenes[s];
-    const StepConst& c = sc.c;
-    float dt = host_dt;
-    if (host_dt <= 0.0f) {
-        const float vmax = __uint_as_float(sc.vmax_bits);
-        const float dt_cfl = xdiv(xmul(c.cfl, c.h), xadd(vmax, 1e-6f));
-        const float alen = xsqrt(xdot3(sc.a0[0], sc.a0[1], sc.a0[2]));
-        const float dt_force = xmul(c.cfl, xsqrt(xdiv(c.h, xadd(alen, 1e-6f))));
-        dt = dt_cfl;
-        if (dt_force < dt) dt = dt_force;
-        if (c.timestep < dt) dt = c.timestep;
-    }
-    if (sc.count == 0) return;  // SPHEngine::step is a no-op on an empty scene
-    sc.dt = dt;
-    sc.time = xadd(sc.time, dt);
-}
-
-int launch_batch_cfl(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, float host_dt) {
-    int k = 1;
-    if (host_dt <= 0.0f) {
-        k_batch_vmax<<<blocks_for(L, n, 256), 256, 0, L.stream>>>(b.vel4, b.scene_of, n, b.scenes);
-        ++k;
-    }
-    k_batch_set_dt<<<(b.nscenes + 255) / 256, 256, 0, L.stream>>>(b.scenes, b.nscenes, host_dt);
-    return k;
-}
-
-// ---- grid ------------------------------------------------------------------------------
-
-__global__ void k_batch_bbox(const float4* __restrict__ pos4, const uint32_t* __restrict__ scene_of,
-                             int n, SceneInfo* scenes, DevState* ds) {
-    const int lane = threadIdx.x & 31;
-    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base < n;
-         base += gridDim.x * blockDim.x) {
-        const int i = base + lane;
-        uint32_t s = 0xffffffffu;
-        bool fin = false;
-        int c[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
-        int d[3] = {-0x7fffffff - 1, -0x7fffffff - 1, -0x7fffffff - 1};
-        if (i < n) {
-            s = scene_of[i];
-            const float4 p = pos4[i];
-            fin = finite3(p.x, p.y, p.z);
-            if (tiny_coord(p.x) || tiny_coord(p.y) || tiny_coord(p.z)) ds->general = 1;
-            if (fin) {
-                const float ic = scenes[s].c.inv_cell;
-                c[0] = d[0] = cell_coord(p.x, ic);
-                c[1] = d[1] = cell_coord(p.y, ic);
-                c[2] = d[2] = cell_coord(p.z, ic);
-            }
-        }
-        const uint32_t peers = __match_any_sync(0xffffffffu, s);
-        const uint32_t bad = __popc(__ballot_sync(0xffffffffu, i < n && !fin) & peers);
-        int mn[3] = {c[0], c[1], c[2]}, mx[3] = {d[0], d[1], d[2]};
-        for (uint32_t rest = peers; rest; rest &= rest - 1) {
-            const int src = __ffs(rest) - 1;
+__device__ __forceinline__ void flush(const SceneAcc& s, SceneInfo* scenes, int lane) {
+    SceneInfo& sc = scenes[s.scene];
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                mn[a] = min(mn[a], __shfl_sync(peers, c[a], src));
-                mx[a] = max(mx[a], __shfl_sync(peers, d[a], src));
+    for (int a = 0; a < 3; ++a) {
+        const int mn = __reduce_min_sync(0xffffffffu, s.mn[a]);
+        const int mx = __reduce_max_sync(0xffffffffu, s.mx[a]);
+        if (lane == 0 && mn != 0x7fffffff) atomicMin(&sc.acc_min[a], mn);
+        if (lane == 0 && mx != -0x7fffffff - 1) atomicMax(&sc.acc_max[a], mx);
+    }
+    const uint32_t bad = __reduce_add_sync(0xffffffffu, s.bad);
+    const uint32_t vm = __reduce_max_sync(0xffffffffu, s.vmax);
+    if (lane == 0 && bad) atomicAdd(&sc.acc_bad, bad);
+    if (lane == 0 && vm) atomicMax(&sc.acc_vmax, vm);
+}
+__device__ __forceinline__ void gather(SceneAcc& s, const float4& p, const float4* vel, int i,
+                                       float inv_cell, bool& tiny) {
+    if (vel) {
+        const float4 v = vel[i];
+        const float len = xsqrt(xdot3(v.x, v.y, v.z));
+        if (!isnan(len)) s.vmax = max(s.vmax, __float_as_uint(len));  // NaN ignored like std::max
+    }
+    tiny = tiny || tiny_coord(p.x) || tiny_coord(p.y) || tiny_coord(p.z);
+    if (!finite3(p.x, p.y, p.z)) {
+        ++s.bad;
+        return;
+    }
+    const int c[3] = {cell_coord(p.x, inv_cell), cell_coord(p.y, inv_cell),
+                      cell_coord(p.z, inv_cell)};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        s.mn[a] = min(s.mn[a], c[a]);
+        s.mx[a] = max(s.mx[a], c[a]);
+    }
+}
+
+// Per scene: box of occupied cells, non-finite count, max |v| (a warp takes consecutive
+// particles, so it meets few scenes and adds each to the scene's record once); the block that
+// finishes last sets every scene's dt and time and lays the scenes' cell blocks end to end.
+__global__ void __launch_bounds__(kPrepThreads) k_batch_prepare(const Buffers b, DevState* ds,
+                                                                int n, int how, float host_dt,
+                                                                uint32_t max_cells) {
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * (kPrepThreads / 32);
+    const int w = blockIdx.x * (kPrepThreads / 32) + (threadIdx.x >> 5);
+    const long long rows = (n + 31) / 32;  // of 32 particles
+    const int r0 = (int)(rows * w / warps), r1 = (int)(rows * (w + 1) / warps);
+    SceneInfo* scenes = b.scenes;
+    const float4* vel = how == kCflDt ? b.vel4 : nullptr;
+    bool tiny = false;
+    if (r0 < r1) {
+        SceneAcc acc;
+        clear(acc, b.scene_of[r0 * 32]);
+        for (int r = r0; r < r1; ++r) {
+            const int i = r * 32 + lane;
+            const bool in = i < n;
+            const uint32_t s = in ? b.scene_of[i] : b.scene_of[n - 1];
+            const float4 p = in ? b.pos4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            uint32_t todo = __ballot_sync(0xffffffffu, in);
+            while (todo) {  // scenes are contiguous: usually one round
+                const uint32_t cur = __shfl_sync(0xffffffffu, s, __ffs(todo) - 1);
+                if (cur != acc.scene) {
+                    flush(acc, scenes, lane);
+                    clear(acc, cur);
+                }
+                if (in && s == cur) gather(acc, p, vel, i, scenes[cur].c.inv_cell, tiny);
+                todo &= ~__ballot_sync(0xffffffffu, s == cur);
             }
         }
-        if (s != 0xffffffffu && lane == __ffs(peers) - 1) {
+        flush(acc, scenes, lane);
+    }
+    if (tiny) b.sync->general = 1;
+    if (!last_block(b.sync)) return;
+    reset_step(ds, b);
+    __shared__ unsigned long long warp_cells[kPrepThreads / 32];
+    unsigned long long total = 0;  // cells of the scenes before this round's
+    for (int s0 = 0; s0 < b.nscenes; s0 += kPrepThreads) {
+        const int s = s0 + (int)threadIdx.x;
+        unsigned long long cells = 0;
+        if (s < b.nscenes) {
             SceneInfo& sc = scenes[s];
-#pragma unroll
+            const bool none = sc.acc_bad >= sc.count;  // no finite particle: one cell
+            cells = 1;
             for (int a = 0; a < 3; ++a) {
-                if (mn[a] != 0x7fffffff) atomicMin(&sc.cmin[a], mn[a]);
-                if (mx[a] != -0x7fffffff - 1) atomicMax(&sc.cmax[a], mx[a]);
+                sc.cmin[a] = none ? 0 : sc.acc_min[a];
+                sc.cmax[a] = none ? 0 : sc.acc_max[a];
+                sc.acc_min[a] = 0x7fffffff;
+                sc.acc_max[a] = -0x7fffffff - 1;
+                const long long d = (long long)sc.cmax[a] - (long long)sc.cmin[a] + 1;
+                sc.dim[a] = (int)(d < 0x7fffffff ? d : 0x7fffffff);
+                cells *= (unsigned long long)(d < (long long)max_cells ? d : (long long)max_cells + 1);
+                if (cells > (unsigned long long)max_cells) cells = (unsigned long long)max_cells + 1;
             }
-            if (bad) atomicAdd(&sc.nonfinite, bad);
+            sc.ncells = (uint32_t)cells;
+            // SPHEngine::step is a no-op on an empty scene
+            if (how != kNoStep && sc.count) {
+                const float dt = how == kCflDt ? cfl_dt(sc.c, __uint_as_float(sc.acc_vmax), sc.a0)
+                                               : host_dt;
+                sc.dt = dt;
+                sc.time = xadd(sc.time, dt);
+            }
+            sc.acc_bad = sc.acc_vmax = 0;
         }
+        unsigned long long x = cells;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_cells[threadIdx.x >> 5] = x;
+        __syncthreads();
+        unsigned long long before = total, all = 0;
+        for (int v = 0; v < kPrepThreads / 32; ++v) {
+            if (v < (int)(threadIdx.x >> 5)) before += warp_cells[v];
+            all += warp_cells[v];
+        }
+        const unsigned long long base = before + x - cells;
+        if (s < b.nscenes) scenes[s].base = (uint32_t)(base < 0xffffffffull ? base : 0xffffffffull);
+        total += all;
+        __syncthreads();
     }
-}
-
-// One thread lays the scenes' blocks end to end (scenes are few: a serial scan is cheap).
-__global__ void k_batch_grid_setup(SceneInfo* scenes, int nscenes, uint32_t max_cells,
-                                   DevState* ds) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    unsigned long long total = 0;
-    for (int s = 0; s < nscenes; ++s) {
-        SceneInfo& sc = scenes[s];
-        if (sc.nonfinite >= sc.count) {  // no finite particle: one cell, all keys sentinel
-            for (int a = 0; a < 3; ++a) sc.cmin[a] = sc.cmax[a] = 0;
-        }
-        unsigned long long cells = 1;
-        for (int a = 0; a < 3; ++a) {
-            const long long d = (long long)sc.cmax[a] - (long long)sc.cmin[a] + 1;
-            sc.dim[a] = (int)(d < 0x7fffffff ? d : 0x7fffffff);
-            cells *= (unsigned long long)(d < (long long)max_cells ? d : (long long)max_cells + 1);
-            if (cells > (unsigned long long)max_cells) cells = (unsigned long long)max_cells + 1;
-        }
-        sc.base = (uint32_t)(total < 0xffffffffull ? total : 0xffffffffull);
-        sc.ncells = (uint32_t)(cells < 0xffffffffull ? cells : 0xffffffffull);
-        total += cells;
-        if (total > (unsigned long long)max_cells) break;
-    }
+    if (threadIdx.x != 0) return;
+    ds->general = b.sync->general;
+    b.sync->general = 0;
+    ds->nonfinite = 0;
     if (total > (unsigned long long)max_cells) {  // each scene's box must fit unfolded
         ds->status = SPHX_ERR_DOMAIN;
         ds->ncells = 0;
@@ -188,33 +173,46 @@ __global__ void k_batch_grid_setup(SceneInfo* scenes, int nscenes, uint32_t max_
     ds->passes = (uint32_t)((bits + kRadixBits - 1) / kRadixBits);
 }
 
-__global__ void k_batch_keys(const float4* __restrict__ pos4, const uint32_t* __restrict__ scene_of,
-                             int n, const SceneInfo* __restrict__ scenes, const DevState* ds,
-                             uint32_t* __restrict__ keys) {
-    if (ds->status) return;
-    const uint32_t sentinel = ds->ncells;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const SceneInfo& sc = scenes[scene_of[i]];
-        const float4 p = pos4[i];
-        uint32_t key = sentinel;
-        if (finite3(p.x, p.y, p.z)) {
-            const float ic = sc.c.inv_cell;
-            const uint32_t x = (uint32_t)(cell_coord(p.x, ic) - sc.cmin[0]);
-            const uint32_t y = (uint32_t)(cell_coord(p.y, ic) - sc.cmin[1]);
-            const uint32_t z = (uint32_t)(cell_coord(p.z, ic) - sc.cmin[2]);
-            key = sc.base + (x * (uint32_t)sc.dim[1] + y) * (uint32_t)sc.dim[2] + z;
-        }
-        keys[i] = key;
-    }
+int launch_batch_prepare(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, int how,
+                         float host_dt, uint32_t max_cells) {
+    int nb = (n + 4 * kPrepThreads - 1) / (4 * kPrepThreads);
+    nb = nb < 1 ? 1 : (nb > kMaxPrepBlocks ? kMaxPrepBlocks : nb);
+    k_batch_prepare<<<nb, kPrepThreads, 0, L.stream>>>(b, ds, n, how, host_dt, max_cells);
+    return 1;
 }
 
-int launch_batch_grid(const LaunchCtx& L, const Buffers& b, DevState* ds, int n,
-                      uint32_t max_cells) {
-    const int gb = blocks_for(L, n, 256);
-    k_batch_bbox<<<gb, 256, 0, L.stream>>>(b.pos4, b.scene_of, n, b.scenes, ds);
-    k_batch_grid_setup<<<1, 32, 0, L.stream>>>(b.scenes, b.nscenes, max_cells, ds);
-    k_batch_keys<<<gb, 256, 0, L.stream>>>(b.pos4, b.scene_of, n, b.scenes, ds, b.key[0]);
-    return 3 + launch_grid_sort(L, b, ds, n, StepConst{});  // (scenes carry their own)
+// ---- grid ------------------------------------------------------------------------------
+
+__global__ void __launch_bounds__(256) k_batch_keys(const Buffers b, int n, const DevState* ds) {
+    if (ds->status) return;
+    __shared__ uint32_t h[kMaxPasses][kRadixBuckets];
+    for (int i = threadIdx.x; i < kMaxPasses * kRadixBuckets; i += 256) (&h[0][0])[i] = 0;
+    __syncthreads();
+    const uint32_t sentinel = ds->ncells, passes = ds->passes;
+    for (int i0 = blockIdx.x * 256; i0 < n; i0 += gridDim.x * 256) {
+        const int i = i0 + (int)threadIdx.x;
+        uint32_t key = sentinel;
+        if (i < n) {
+            const SceneInfo& sc = b.scenes[b.scene_of[i]];
+            const float4 p = b.pos4[i];
+            if (finite3(p.x, p.y, p.z)) {
+                const float ic = sc.c.inv_cell;
+                const uint32_t x = (uint32_t)(cell_coord(p.x, ic) - sc.cmin[0]);
+                const uint32_t y = (uint32_t)(cell_coord(p.y, ic) - sc.cmin[1]);
+                const uint32_t z = (uint32_t)(cell_coord(p.z, ic) - sc.cmin[2]);
+                key = sc.base + (x * (uint32_t)sc.dim[1] + y) * (uint32_t)sc.dim[2] + z;
+            }
+            b.key[0][i] = key;
+        }
+        count_digits(h, key, i < n, passes);
+    }
+    __syncthreads();
+    add_digits(h, b.hist, passes);
+}
+
+int launch_batch_grid(const LaunchCtx& L, const Buffers& b, DevState* ds, int n) {
+    k_batch_keys<<<blocks_for(L, n, 256, 2), 256, 0, L.stream>>>(b, n, ds);
+    return 1 + launch_grid_sort(L, b, ds, n, StepConst{});  // (scenes carry their own)
 }
 
 // ---- FP64 diagnostics per scene (one block per scene, fixed order) ----------------------

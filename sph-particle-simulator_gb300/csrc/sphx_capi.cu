@@ -224,7 +224,8 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
     };
     s.lit = PairLits{both(-0.0f), both(0.5f), both(1.0f), both(2.0f), both(-2.0f), both(3.0f),
                      both(1.5f), both(-0x1p40f), both(0x1p-20f), both(-0x1p-20f), both(0x1p21f),
-                     both(kTwoThirds), both(kOneSixth), both(-5.0f), both(5.0f)};
+                     both(kTwoThirds), both(kOneSixth), both(-5.0f), both(5.0f), both(-0.5f), both(-1.0f),
+                     both(-3.0f), both(kCoincident)};
     s.pair = PairConst{both(-h), both(h), both(s.rcp_h), both(-s.h_sq), both(s.rcp_hsq),
                        both(s.sigma), both(-s.sigma), both(s.gas), both(s.rest), both(s.wnorm),
                        both(s.wl)};
@@ -263,10 +264,10 @@ void free_all(sphx_ctx* c) {
     Buffers& b = c->b;
     void* ptrs[] = {b.pos4, b.vel4,   b.pos4_s, b.vel4_s,     b.aux4_s,    b.acc4_s,
                     b.key[0], b.key[1], b.val[0], b.val[1],   b.key_s,     b.id_s,
-                    b.off,  b.tiles, b.tgt, b.hist, b.scan_part, b.diag_part, c->ds,
+                    b.off,  b.tiles, b.tgt, b.sync, b.diag_part, c->ds,
                     c->stage, c->snap_pos, c->snap_vel, c->snap_cell, b.cell4, b.cell4_s,
                     b.spread_tiles,
-                    b.scene_of, b.scene_s, b.scenes, b.hitmask, b.tile_slot,
+                    b.scene_of, b.scene_s, b.scenes, b.records, b.tile_list,
                     c->r_colors, c->r_inst, c->r_keys, c->r_rgba};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -356,13 +357,12 @@ int run_phases(sphx_ctx* c, float dt, bool integrate) {
         c->sc.force_nz = c->scenes_force_nz ? 1 : 0;
     }
     int k = 0;
+    const int how = !integrate ? kNoStep : (dt <= 0.0f ? kCflDt : kHostDt);
     if (batch) {
-        k += launch_batch_begin(c->L, c->b, c->ds);
-        if (integrate) k += launch_batch_cfl(c->L, c->b, c->ds, (int)c->n, dt);
-        k += launch_batch_grid(c->L, c->b, c->ds, (int)c->n, c->sc.max_cells);
+        k += launch_batch_prepare(c->L, c->b, c->ds, (int)c->n, how, dt, c->sc.max_cells);
+        k += launch_batch_grid(c->L, c->b, c->ds, (int)c->n);
     } else {
-        k += launch_begin_step(c->L, c->ds, 1);
-        if (integrate) k += launch_cfl(c->L, c->sc, c->b, c->ds, dt);
+        k += launch_prepare(c->L, c->sc, c->b, c->ds, how, dt);
         k += launch_build_grid(c->L, c->sc, c->b, c->ds);
     }
     if (slot) SPHX_CUDA(cudaEventRecord(slot->ev[1], c->stream));
@@ -677,49 +677,47 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     c->sc.max_cells = (uint32_t)max_cells;
     Buffers& b = c->b;
     const size_t C = capacity;
-    b.radix_blocks = (int)((C + kRadixTileN - 1) / kRadixTileN);
-    const size_t hist_n = (size_t)b.radix_blocks * kRadixBuckets;
-    const size_t part_a = (hist_n + kScanTileN - 1) / kScanTileN;
-    const size_t part_b = (C + kScanTileN - 1) / kScanTileN;
-    b.scan_part_cap = (int)((part_a > part_b ? part_a : part_b) + 1);
     b.diag_blocks = c->L.num_sms * 2;
+    b.num_sms = c->L.num_sms;
     if ((rc = dmalloc(&b.pos4, C)) || (rc = dmalloc(&b.vel4, C)) || (rc = dmalloc(&b.pos4_s, C)) ||
         (rc = dmalloc(&b.vel4_s, C)) || (rc = dmalloc(&b.aux4_s, C)) ||
         (rc = dmalloc(&b.acc4_s, C)) || (rc = dmalloc(&b.key[0], C)) ||
         (rc = dmalloc(&b.key[1], C)) || (rc = dmalloc(&b.val[0], C)) ||
         (rc = dmalloc(&b.val[1], C)) || (rc = dmalloc(&b.key_s, C)) ||
         (rc = dmalloc(&b.id_s, C)) || (rc = dmalloc(&b.off, (size_t)max_cells + 2)) ||
-        (rc = dmalloc(&b.tiles, C)) || (rc = dmalloc(&b.hist, hist_n)) ||
-        (rc = dmalloc(&b.scan_part, (size_t)b.scan_part_cap)) ||
-        (rc = dmalloc(&b.diag_part, (size_t)b.diag_blocks * kDiagSums)) ||
+        (rc = dmalloc(&b.tiles, C)) ||         (rc = dmalloc(&b.diag_part, (size_t)b.diag_blocks * kDiagSums)) ||
         (rc = dmalloc(&c->ds, 1)) || (rc = dmalloc(&c->stage, 11 * C)))
         return fail(rc);
     if (c->tuning.mode != SPHX_MODE_EXACT &&
         ((rc = dmalloc(&b.cell4, C)) || (rc = dmalloc(&b.cell4_s, C)) ||
          (rc = dmalloc(&b.spread_tiles, C))))
         return fail(rc);
-    if (c->tuning.mode == SPHX_MODE_EXACT && (rc = dmalloc(&b.tgt, C))) return fail(rc);
-    // Hit-mask pool (exact mode; the precision mode's sweeps keep no records): 4 records
-    // (128 B each) per particle of capacity.  A dense state needs about 1.7-2.6 per particle
-    // (32-particle tiles, 27-cell stencil); the rest is slack for the uneven split of tiles
-    // over the warps.  Without the pool (or where a warp's region runs out) the force pass
-    // repeats the distance tests.
-    if (c->tuning.mode == SPHX_MODE_EXACT) {
-        if (dmalloc(&b.tile_slot, C) == SPHX_OK) {
-            unsigned long long cap = 4ull * C;
-            if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
-            if (dmalloc(&b.hitmask, (size_t)cap * 32) == SPHX_OK) {
-                b.hitmask_cap = cap;
-            } else {
-                cudaGetLastError();
-                cudaFree(b.tile_slot);
-                b.tile_slot = nullptr;
-            }
+    if ((rc = dmalloc(&b.tgt, C))) return fail(rc);
+    // Record pool (Buffers::records): 4 records (128 B each) per particle of capacity.  The
+    // lattice and uniform states need about 2 per particle in exact mode (32-particle tiles,
+    // the candidates their boxes keep) and 1 in the precision mode; the rest is room for
+    // denser states and for the uneven split of tiles over the warps.  Without the pool (or
+    // where a warp's region runs out) the force pass walks the candidates itself.
+    if (dmalloc(&b.tile_list, C) == SPHX_OK) {
+        unsigned long long cap = 4ull * C;
+        if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
+        if (dmalloc(&b.records, (size_t)cap * 32) == SPHX_OK) {
+            b.record_cap = cap;
         } else {
             cudaGetLastError();
+            cudaFree(b.tile_list);
+            b.tile_list = nullptr;
         }
+    } else {
+        cudaGetLastError();
     }
-    if (cudaMemset(c->ds, 0, sizeof(DevState)) != cudaSuccess) return fail(SPHX_ERR_CUDA);
+    // (look-back words of an absent epoch: an epoch is at least kMaxPasses)
+    unsigned char* scratch = nullptr;
+    if ((rc = dmalloc(&scratch, grid_scratch_bytes(C)))) return fail(rc);
+    set_grid_scratch(b, scratch);
+    if (cudaMemset(c->ds, 0, sizeof(DevState)) != cudaSuccess ||
+        cudaMemset(scratch, 0, grid_scratch_bytes(C)) != cudaSuccess)
+        return fail(SPHX_ERR_CUDA);
     if (cudaHostAlloc(reinterpret_cast<void**>(&c->h_status), sizeof(int), cudaHostAllocDefault) !=
         cudaSuccess) {
         c->h_status = nullptr;
@@ -955,6 +953,10 @@ int sphx_set_scenes(sphx_ctx* c, uint32_t nscenes, const uint64_t* scene_start,
     for (uint32_t s = 0; s < nscenes; ++s) {
         SceneInfo& si = info[s];
         std::memset(&si, 0, sizeof(si));
+        for (int a = 0; a < 3; ++a) {
+            si.acc_min[a] = 0x7fffffff;
+            si.acc_max[a] = -0x7fffffff - 1;
+        }
         si.start = (uint32_t)scene_start[s];
         si.count = (uint32_t)(scene_start[s + 1] - scene_start[s]);
         fill_step_const_from(c, params[s], si.count, si.c);
@@ -1351,11 +1353,11 @@ int sphx_debug_pairs(sphx_ctx* c, int64_t* counts, int64_t* idx, size_t* total_i
     }
     fill_step_const(c);
     c->have_fields = false;  // the grid rebuild below replaces the sorted permutation
-    launch_begin_step(c->L, c->ds, 1);
     // the lists come in the reference's order: insertion order within each cell
     Buffers bq = c->b;
     bq.columns = 0;
     bq.tgt = nullptr;
+    launch_prepare(c->L, c->sc, bq, c->ds, kNoStep, 0.0f);
     launch_build_grid(c->L, c->sc, bq, c->ds);
     uint32_t* d_cnt = nullptr;
     if ((rc = dmalloc(&d_cnt, n))) return rc;
@@ -1414,11 +1416,11 @@ int sphx_debug_pairs_subset(sphx_ctx* c, size_t nsel, const int64_t* sel, int64_
     }
     fill_step_const(c);
     c->have_fields = false;  // the grid rebuild below replaces the sorted permutation
-    launch_begin_step(c->L, c->ds, 1);
     // the lists come in the reference's order: insertion order within each cell
     Buffers bq = c->b;
     bq.columns = 0;
     bq.tgt = nullptr;
+    launch_prepare(c->L, c->sc, bq, c->ds, kNoStep, 0.0f);
     launch_build_grid(c->L, c->sc, bq, c->ds);
     uint32_t* d_cnt = nullptr;
     if ((rc = dmalloc(&d_cnt, n))) return rc;

@@ -39,20 +39,13 @@ __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Bu
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     DensitySmem* S = reinterpret_cast<DensitySmem*>(smem_raw_d) + warp;
     const uint32_t ntiles = ds->n_tiles;
-    // this warp's region of the hit-mask pool, filled tile after tile (record indices fit
-    // 32 bits: the pool holds at most 0xffff0000 records)
-    uint32_t mcur, mend;
-    {
-        const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-        const uint32_t region = b.hitmask ? (uint32_t)(b.hitmask_cap / nwarps) : 0u;
-        mcur = (blockIdx.x * (blockDim.x >> 5) + warp) * region;
-        mend = mcur + region;
-    }
     const uint32_t lt = (1u << lane) - 1u;
     const F2 neg0{cp.lit.neg0};
     const bool nz = kNZ && !ds->general;
     uint32_t my_max = 0;
-    for (uint32_t t = next_tile(&ds->work[0], lane); t < ntiles; t = next_tile(&ds->work[0], lane)) {
+    const TileQueue queue(&ds->work[0], b.num_sms);
+    RecordRegion region(b, queue, ntiles);
+    for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         const uint2 tile = b.tiles[t];
         const int scene = kBatch ? (int)b.scene_s[tile.x] : 0;
         const StepConst& c = kBatch ? b.scenes[scene].c : cp;
@@ -67,15 +60,15 @@ __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Bu
         __syncwarp();  // the previous tile's segments are read
         const int nseg = build_segments(b, g, T, lane, S->seg);
         __syncwarp();
-        // records of this tile: ceil(nraw / 32) of kept-candidate words, then the masks
-        const uint32_t hdr = (uint32_t)(raw_chunks(S->seg, nseg, lane) + 31) >> 5;
-        const uint32_t room = mend - mcur;
-        uint32_t* const rec = b.hitmask + (size_t)mcur * 32 + lane;
+        // records of this tile: per chunk of 32 kept candidates their sorted positions, then
+        // the lanes' masks
+        const int room = (int)((region.end - region.cur) >> 1);  // chunks
+        uint32_t* const rec = b.records + (size_t)region.cur * 32;
         RawStream st(S->seg, nseg);
         float4 pl = make_float4(0.f, 0.f, 0.f, 0.f);  // the next chunk's candidate, read ahead
         if (st.more() && lane < st.count()) pl = b.pos4_s[st.s + lane];
         float rho = xmul(xi.w, c.w0);
-        uint32_t nn = 0, raw = 0, kept_word = 0;
+        uint32_t nn = 0;
         int kept = 0, tested = 0, head = 0, self = -1;
         RingLane<kDensityRing> at;
         for (;;) {
@@ -85,22 +78,18 @@ __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Bu
                 const uint32_t surv =
                     __ballot_sync(kFull, lane < m && box_near(B, pl, r2m));
                 if ((surv >> lane) & 1u) {
-                    const int slot = ring_slot<kDensityRing>(kept + __popc(surv & lt));
+                    const int a = kept + __popc(surv & lt);
+                    const int slot = ring_slot<kDensityRing>(a);
                     S->cx[slot] = pl.x;
                     S->cy[slot] = pl.y;
                     S->cz[slot] = pl.z;
                     S->cm[slot] = pl.w;
+                    // streaming stores: the records must not evict the candidates from L2
+                    if ((a >> 5) < room) __stcs(rec + (a >> 5) * 64 + (a & 31), (uint32_t)(s + lane));
                 }
                 if ((unsigned)(i - s) < (unsigned)m) self = kept + __popc(surv & ((1u << (i - s)) - 1u));
                 st.next();
                 if (st.more() && lane < st.count()) pl = b.pos4_s[st.s + lane];
-                if (lane == (int)(raw & 31u)) kept_word = surv;
-                ++raw;
-                if ((raw & 31u) == 0 || !st.more()) {
-                    // streaming stores: the records must not evict the candidates from L2
-                    if ((raw - 1) >> 5 < room) __stcs(rec + ((raw - 1) & ~31u), kept_word);
-                    kept_word = 0;
-                }
                 kept += __popc(surv);
                 while ((kept >> 5) > tested || (!st.more() && kept > tested * 32)) {
                     __syncwarp();
@@ -109,7 +98,7 @@ __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Bu
                     mask = valid ? mask & chunk_valid(kept - tested * 32) : 0u;
                     nn += __popc(mask);
                     if (self >> 5 == tested) mask &= ~(0x80000000u >> (self & 31));
-                    if (hdr + tested < room) __stcs(rec + (size_t)(hdr + tested) * 32, mask);
+                    if (tested < room) __stcs(rec + tested * 64 + 32 + lane, mask);
                     S->mask[f + lane] = mask;
                     ++tested;
                 }
@@ -144,10 +133,10 @@ __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Bu
             if (!st.more()) break;
             head = __reduce_min_sync(kFull, at.need());
         }
-        if (b.hitmask) {
-            const bool fits = hdr + (uint32_t)tested <= room;
-            if (lane == 0) b.tile_slot[t] = fits ? mcur : kNoSlot;
-            if (fits) mcur += hdr + (uint32_t)tested;
+        if (b.records) {
+            const bool fits = tested <= room;
+            if (lane == 0) b.tile_list[t] = make_uint2(fits ? region.cur : kNoSlot, (uint32_t)kept);
+            if (fits) region.cur += 2u * (uint32_t)tested;
         }
         if (valid) {
             const float P = xmul(c.gas, xsub(rho, c.rest));

@@ -13,13 +13,14 @@ namespace sphx {
 // ---------------------------------------------------------------------------------------
 // Per warp: the candidate ring -- positions and mass, velocities and density, the two
 // per-candidate factors -- the lanes' masks and the tile's row segments.  40 bytes a candidate:
-// 12 chunks leave room for 12 warps per SM; 8 chunks (16 warps) take 1.87 ms on the 1M dam
-// break, 10 (14 warps) 1.84, 12 1.71, 16 (8 warps) 2.0.
+// 12 chunks leave room for 12 warps per SM; 8 chunks (16 warps) took 9% longer on the 1M dam
+// break, 10 (14 warps) 8%, 16 (8 warps) 17%.
 //
 // Bound: instruction issue (64% of the slots with 3 warps per scheduler) and the FP32 pipe
-// (58%; a packed instruction holds it two cycles): 1,345 warp instructions per particle in
-// 5.7 turns, each finishing one pair of neighbours per lane and starting the next.  1M dam
-// break, force + leapfrog: 1.71 ms; with hit lists, terms passed through shared memory and
+// (58%; a packed instruction holds it two cycles): about 1,200 warp instructions per particle
+// in 5.7 turns, each finishing one pair of neighbours per lane and starting the next.  1M dam
+// break, force + leapfrog: 1.52 ms; walking and culling the candidates again instead of
+// reading the density pass's list 1.71 ms; with hit lists, terms passed through shared memory and
 // in-order folds by their lanes (2,479 instructions) 2.60 ms; one neighbour per turn with the
 // compiler's division and square root 2.72 ms, pairs 2.08, staged by asynchronous copies 1.83,
 // the two halves of a turn overlapped 1.73.
@@ -234,7 +235,8 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
     const uint32_t lt = (1u << lane) - 1u;
     const PairLits& lit = cp.lit;
     const bool nz = kNZ && !ds->general;
-    for (uint32_t t = next_tile(&ds->work[1], lane); t < ntiles; t = next_tile(&ds->work[1], lane)) {
+    const TileQueue queue(&ds->work[1], b.num_sms);
+    for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         const uint2 tile = b.tiles[t];
         const int scene = kBatch ? (int)b.scene_s[tile.x] : 0;
         const StepConst& c = kBatch ? b.scenes[scene].c : cp;
@@ -246,20 +248,23 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
         tile_setup(c, b, g, tile, lane, T, i, xi, valid);
         const float4 vi0 = valid ? b.vel4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float Pi = valid ? b.aux4_s[i].y : 0.0f;
-        // the density pass's records of this tile (same walk, same candidates kept)
-        const uint32_t slot = b.tile_slot ? b.tile_slot[t] : kNoSlot;
-        __syncwarp();  // the previous tile's segments are read
-        const int nseg = build_segments(b, g, T, lane, S->seg);
-        __syncwarp();
-        const int hdr = (raw_chunks(S->seg, nseg, lane) + 31) >> 5;
-        const uint32_t* const rec =
-            slot != kNoSlot ? b.hitmask + (size_t)slot * 32 + lane : nullptr;
-        RawStream st(S->seg, nseg);
+        // the density pass's records of this tile: its kept candidates and the lanes' masks
+        const uint2 list = b.records ? b.tile_list[t] : make_uint2(kNoSlot, 0u);
+        const bool listed = list.x != kNoSlot;
+        const uint32_t* rec = b.records + (size_t)list.x * 32 + lane;
+        const int nlist = listed ? (int)list.y : 0;  // candidates
+        uint32_t ahead = lane < nlist ? __ldcs(rec) : 0u;  // the next chunk's, read ahead
         TileBox B;
-        if (!rec) B = tile_box(xi, valid);
+        int nseg = 0;
+        if (!listed) {
+            B = tile_box(xi, valid);
+            __syncwarp();  // the previous tile's segments are read
+            nseg = build_segments(b, g, T, lane, S->seg);
+            __syncwarp();
+        }
+        RawStream st(S->seg, nseg);
         ForceSums F;
-        uint32_t kept_word = 0;
-        int raw = 0, kept = 0, ready = 0, staged = 0, head = 0, self = -1;
+        int kept = 0, ready = 0, staged = 0, head = 0, self = -1;
         RingLane<kForceRing> at;
         PairStart pair;  // started, not yet added
         pair.qa = pair.qb = 0;
@@ -269,48 +274,44 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
             cp_async_wait_all();
             __syncwarp();  // staged chunks are in place, every lane is done with those before head
             ready = staged;
+            auto copy = [&](int q, uint32_t j) {  // candidate j to ring slot q
+                cp_async16(&S->pos[q], &b.pos4_s[j]);
+                cp_async16(&S->vel[q], &b.vel4_s[j]);
+                cp_async8(&S->fac[q], &b.aux4_s[j].z);
+            };
+            for (; staged * 32 < nlist && staged < head + kForceRing; ++staged) {
+                const int f = (staged % kForceRing) * 32;
+                if (staged * 32 + lane < nlist) copy(f + 31 - lane, ahead);
+                cp_async4(&S->mask[f + lane], rec + 32);
+                rec += 64;
+                if ((staged + 1) * 32 + lane < nlist) ahead = __ldcs(rec);
+            }
+            // without records: the walk, culled and tested again
             while (st.more() && kept + 32 <= (head + kForceRing) * 32) {
                 const int m = st.count(), s = st.s;
-                uint32_t surv;
-                if (rec) {
-                    if ((raw & 31) == 0) kept_word = __ldcs(rec + raw);
-                    surv = __shfl_sync(kFull, kept_word, raw & 31);
-                } else {
-                    bool near = false;
-                    if (lane < m) near = box_near(B, b.pos4_s[s + lane], c.r2 * 1.0001f);
-                    surv = __ballot_sync(kFull, near);
-                    if ((unsigned)(i - s) < (unsigned)m)
-                        self = kept + __popc(surv & ((1u << (i - s)) - 1u));
-                }
-                ++raw;
-                if ((surv >> lane) & 1u) {
-                    const int q = ring_slot<kForceRing>(kept + __popc(surv & lt));
-                    const int j = s + lane;
-                    cp_async16(&S->pos[q], &b.pos4_s[j]);
-                    cp_async16(&S->vel[q], &b.vel4_s[j]);
-                    cp_async8(&S->fac[q], &b.aux4_s[j].z);
-                }
+                bool near = false;
+                if (lane < m) near = box_near(B, b.pos4_s[s + lane], c.r2 * 1.0001f);
+                const uint32_t surv = __ballot_sync(kFull, near);
+                if ((unsigned)(i - s) < (unsigned)m)
+                    self = kept + __popc(surv & ((1u << (i - s)) - 1u));
+                if ((surv >> lane) & 1u)
+                    copy(ring_slot<kForceRing>(kept + __popc(surv & lt)), (uint32_t)(s + lane));
                 st.next();
                 kept += __popc(surv);
                 while ((kept >> 5) > staged || (!st.more() && kept > staged * 32)) {
                     const int f = (staged % kForceRing) * 32;
-                    if (rec) {
-                        const uint32_t* w = rec + (size_t)(hdr + staged) * 32;
-                        cp_async4(&S->mask[f + lane], w);
-                    } else {
-                        cp_async_wait_all();
-                        __syncwarp();
-                        uint32_t mask = 0;
-                        for (int q = 0; q < 32; ++q)
-                            if (diff_d2(xi, S->pos[f + q]) <= c.r2) mask |= 1u << q;
-                        mask = valid ? mask & chunk_valid(kept - staged * 32) : 0u;
-                        if (self >> 5 == staged) mask &= ~(0x80000000u >> (self & 31));
-                        S->mask[f + lane] = mask;
-                    }
+                    cp_async_wait_all();
+                    __syncwarp();
+                    uint32_t mask = 0;
+                    for (int q = 0; q < 32; ++q)
+                        if (diff_d2(xi, S->pos[f + q]) <= c.r2) mask |= 1u << q;
+                    mask = valid ? mask & chunk_valid(kept - staged * 32) : 0u;
+                    if (self >> 5 == staged) mask &= ~(0x80000000u >> (self & 31));
+                    S->mask[f + lane] = mask;
                     ++staged;
                 }
             }
-            const bool all = !st.more() && ready == staged;
+            const bool all = !st.more() && staged * 32 >= nlist && ready == staged;
             const int until = all ? ready : min(head + 1, ready);
             if (nz) {
                 // starts `next` and adds `done`; false when no lane needs a chunk before `until`

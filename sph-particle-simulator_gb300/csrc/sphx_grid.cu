@@ -5,7 +5,7 @@
 // Cells are the reference's own: floor(x * inv_cell) per axis with
 // inv_cell = 1.0f / neighbor_search_radius (spatial_hash.h:30-36, 63-66).  Instead of a
 // hash map of index vectors the occupied-cell box is laid out as a dense grid (folded
-// per axis when the box is huge, see k_grid_setup) with a linear key
+// per axis when the box is huge, see grid_setup) with a linear key
 // ((cx * dy + cy) * dz + cz), the keys are radix-sorted stably from insertion order, and
 // off[c] holds the first sorted position of cell c.  z is the fastest axis, so
 // the three cells (cx+dx, cy+dy, cz-1..cz+1) of one stencil row are one contiguous range
@@ -22,155 +22,7 @@ static inline int grid_blocks(const LaunchCtx& L, int n, int threads, int per_sm
     return need < 1 ? 1 : (need < cap ? need : cap);
 }
 
-__global__ void k_begin_step(DevState* ds, int reset_bbox) {
-    if (threadIdx.x != 0) return;
-    ds->status = 0;
-    if (reset_bbox) {
-        for (int a = 0; a < 3; ++a) {
-            ds->cmin[a] = 0x7fffffff;
-            ds->cmax[a] = -0x7fffffff - 1;
-        }
-    }
-    ds->nonfinite = 0;
-    ds->vmax_bits = 0;
-    ds->vmax64 = 0ull;
-    ds->occupied = 0;
-    ds->max_occ = 0;
-    ds->n_tiles = 0;
-    ds->work[0] = ds->work[1] = 0;
-    ds->spread_work[0] = ds->spread_work[1] = 0;
-    ds->n_spread = 0;
-    ds->general = 0;
-}
-
-int launch_begin_step(const LaunchCtx& L, DevState* ds, int reset_bbox) {
-    k_begin_step<<<1, 32, 0, L.stream>>>(ds, reset_bbox);
-    return 1;
-}
-
-// ---- CFL ------------------------------------------------------------------------------
-
-// max |v_i| over the particles, NaN lengths ignored: std::max(m, v) keeps m when v is NaN
-// (sph_engine.cpp:316-322).  Non-negative floats order like their bit patterns.
-__global__ void k_vmax(const float4* __restrict__ vel4, int n, DevState* ds) {
-    uint32_t m = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 v = vel4[i];
-        const float len = xsqrt(xdot3(v.x, v.y, v.z));
-        if (!isnan(len)) m = max(m, __float_as_uint(len));
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(&ds->vmax_bits, m);
-}
-
-// dt = min({dt_cfl, dt_force, timestep}) with std::min's first-smallest rule; then
-// current_time_ += dt.
-__global__ void k_set_dt(StepConst c, DevState* ds, float host_dt) {
-    if (threadIdx.x != 0) return;
-    float dt = host_dt;  // a NaN dt is used as given, like SPHEngine::step (cpp:99-101)
-    if (host_dt <= 0.0f) {
-        const float vmax = __uint_as_float(ds->vmax_bits);
-        const float dt_cfl = xdiv(xmul(c.cfl, c.h), xadd(vmax, 1e-6f));
-        const float alen = xsqrt(xdot3(ds->a0[0], ds->a0[1], ds->a0[2]));
-        const float dt_force = xmul(c.cfl, xsqrt(xdiv(c.h, xadd(alen, 1e-6f))));
-        dt = dt_cfl;
-        if (dt_force < dt) dt = dt_force;
-        if (c.timestep < dt) dt = c.timestep;
-    }
-    ds->dt = dt;
-    ds->time = xadd(ds->time, dt);
-}
-
-// Precision mode: max |v| in FP64 (NaN ignored), then the same rule in FP64; time in FP64.
-__global__ void k_vmax64(const float4* __restrict__ vel4, int n, DevState* ds) {
-    unsigned long long m = 0ull;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 v = vel4[i];
-        const double len = sqrt((double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z);
-        if (!isnan(len)) m = max(m, (unsigned long long)__double_as_longlong(len));
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(&ds->vmax64, m);
-}
-
-__global__ void k_set_dt64(StepConst c, DevState* ds, float host_dt) {
-    if (threadIdx.x != 0) return;
-    double dt = host_dt;
-    if (host_dt <= 0.0f) {
-        const double vmax = __longlong_as_double((long long)ds->vmax64);
-        const double cfl = c.cfl, h = c.h;
-        const double dt_cfl = cfl * h / (vmax + 1e-6);
-        const double a0 = sqrt((double)ds->a0[0] * ds->a0[0] + (double)ds->a0[1] * ds->a0[1] +
-                               (double)ds->a0[2] * ds->a0[2]);
-        const double dt_force = cfl * sqrt(h / (a0 + 1e-6));
-        dt = dt_cfl;
-        if (dt_force < dt) dt = dt_force;
-        if ((double)c.timestep < dt) dt = c.timestep;
-    }
-    ds->dt64 = dt;
-    ds->time64 += dt;
-    ds->dt = (float)dt;
-    ds->time = (float)ds->time64;
-}
-
-int launch_cfl(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
-               float host_dt) {
-    int launches = 1;
-    if (host_dt <= 0.0f) {
-        if (c.precise)
-            k_vmax64<<<grid_blocks(L, c.n, 256), 256, 0, L.stream>>>(b.vel4, c.n, ds);
-        else
-            k_vmax<<<grid_blocks(L, c.n, 256), 256, 0, L.stream>>>(b.vel4, c.n, ds);
-        ++launches;
-    }
-    if (c.precise) k_set_dt64<<<1, 32, 0, L.stream>>>(c, ds, host_dt);
-    else k_set_dt<<<1, 32, 0, L.stream>>>(c, ds, host_dt);
-    return launches;
-}
-
-// ---- grid -----------------------------------------------------------------------------
-
-__global__ void k_bbox(const float4* __restrict__ pos4, int n, float inv_cell, DevState* ds) {
-    int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
-    int mx[3] = {-0x7fffffff - 1, -0x7fffffff - 1, -0x7fffffff - 1};
-    uint32_t bad = 0;
-    bool tiny = false;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 p = pos4[i];
-        tiny = tiny || tiny_coord(p.x) || tiny_coord(p.y) || tiny_coord(p.z);
-        if (!finite3(p.x, p.y, p.z)) {
-            ++bad;
-            continue;
-        }
-        const int c[3] = {cell_coord(p.x, inv_cell), cell_coord(p.y, inv_cell),
-                          cell_coord(p.z, inv_cell)};
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            mn[a] = min(mn[a], c[a]);
-            mx[a] = max(mx[a], c[a]);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-            mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
-        }
-        bad += __shfl_xor_sync(0xffffffffu, bad, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (mn[a] != 0x7fffffff) atomicMin(&ds->cmin[a], mn[a]);
-            if (mx[a] != -0x7fffffff - 1) atomicMax(&ds->cmax[a], mx[a]);
-        }
-        if (bad) atomicAdd(&ds->nonfinite, bad);
-    }
-    if (tiny) ds->general = 1;
-}
+// ---- the step's first kernel --------------------------------------------------------------
 
 // Grid extent.  The occupied-cell box is laid out densely when it has at most max_cells
 // cells.  Otherwise (particles spread over a huge box) every axis longer than F =
@@ -178,59 +30,7 @@ __global__ void k_bbox(const float4* __restrict__ pos4, int n, float inv_cell, D
 // that fold onto each other are at least F - 2 cells apart, so a candidate from a folded
 // neighbour fails the distance test; sets and visiting order are unchanged, only the
 // number of candidates grows.
-// Precision mode: the cells are stored; w != 0 marks a particle with no finite position.
-__global__ void k_bbox_cells(const int4* __restrict__ cell4, int n, DevState* ds) {
-    int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
-    int mx[3] = {-0x7fffffff - 1, -0x7fffffff - 1, -0x7fffffff - 1};
-    uint32_t bad = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int4 c = cell4[i];
-        if (c.w) {
-            ++bad;
-            continue;
-        }
-        mn[0] = min(mn[0], c.x); mn[1] = min(mn[1], c.y); mn[2] = min(mn[2], c.z);
-        mx[0] = max(mx[0], c.x); mx[1] = max(mx[1], c.y); mx[2] = max(mx[2], c.z);
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-            mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
-        }
-        bad += __shfl_xor_sync(0xffffffffu, bad, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (mn[a] != 0x7fffffff) atomicMin(&ds->cmin[a], mn[a]);
-            if (mx[a] != -0x7fffffff - 1) atomicMax(&ds->cmax[a], mx[a]);
-        }
-        if (bad) atomicAdd(&ds->nonfinite, bad);
-    }
-}
-
-__global__ void k_keys_cells(const int4* __restrict__ cell4, int n, const DevState* ds,
-                             uint32_t* __restrict__ keys) {
-    if (ds->status) return;
-    const int cx0 = ds->cmin[0], cy0 = ds->cmin[1], cz0 = ds->cmin[2];
-    const uint32_t dx = ds->dim[0], dy = ds->dim[1], dz = ds->dim[2], nc = ds->ncells;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int4 c = cell4[i];
-        uint32_t key = nc;
-        if (!c.w) {
-            const uint32_t x = (uint32_t)(c.x - cx0) % dx;
-            const uint32_t y = (uint32_t)(c.y - cy0) % dy;
-            const uint32_t z = (uint32_t)(c.z - cz0) % dz;
-            key = (x * dy + y) * dz + z;
-        }
-        keys[i] = key;
-    }
-}
-
-__global__ void k_grid_setup(int n, uint32_t max_cells, DevState* ds) {
-    if (threadIdx.x != 0) return;
+__device__ void grid_setup(int n, uint32_t max_cells, DevState* ds) {
     if ((int)ds->nonfinite >= n) {  // no finite particle: a one-cell grid, all keys sentinel
         for (int a = 0; a < 3; ++a) {
             ds->cmin[a] = 0;
@@ -261,23 +61,199 @@ __global__ void k_grid_setup(int n, uint32_t max_cells, DevState* ds) {
     ds->passes = (uint32_t)((bits + kRadixBits - 1) / kRadixBits);
 }
 
-__global__ void k_keys(const float4* __restrict__ pos4, int n, float inv_cell,
-                       const DevState* ds, uint32_t* __restrict__ keys) {
+// dt of the step, then current_time_ += dt; precision mode: the same rule and the time in FP64.
+__device__ void set_dt(const StepConst& c, DevState* ds, int how, float host_dt,
+                       unsigned long long vmax) {
+    if (!c.precise) {
+        // (a NaN dt is used as given, like SPHEngine::step, cpp:99-101)
+        const float dt = how == kCflDt ? cfl_dt(c, __uint_as_float((uint32_t)vmax), ds->a0)
+                                       : host_dt;
+        ds->dt = dt;
+        ds->time = xadd(ds->time, dt);
+        return;
+    }
+    double dt = host_dt;
+    if (how == kCflDt) {
+        const double vm = __longlong_as_double((long long)vmax);
+        const double cfl = c.cfl, h = c.h;
+        const double dt_cfl = cfl * h / (vm + 1e-6);
+        const double a0 = sqrt((double)ds->a0[0] * ds->a0[0] + (double)ds->a0[1] * ds->a0[1] +
+                               (double)ds->a0[2] * ds->a0[2]);
+        const double dt_force = cfl * sqrt(h / (a0 + 1e-6));
+        dt = dt_cfl;
+        if (dt_force < dt) dt = dt_force;
+        if ((double)c.timestep < dt) dt = c.timestep;
+    }
+    ds->dt64 = dt;
+    ds->time64 += dt;
+    ds->dt = (float)dt;
+    ds->time = (float)ds->time64;
+}
+
+__device__ __forceinline__ PrepPart prep_empty() {
+    PrepPart p;
+    for (int a = 0; a < 3; ++a) {
+        p.mn[a] = 0x7fffffff;
+        p.mx[a] = -0x7fffffff - 1;
+    }
+    p.bad = p.general = 0;
+    p.vmax = 0;
+    return p;
+}
+__device__ __forceinline__ void merge(PrepPart& p, const PrepPart& q) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        p.mn[a] = min(p.mn[a], q.mn[a]);
+        p.mx[a] = max(p.mx[a], q.mx[a]);
+    }
+    p.bad += q.bad;
+    p.general |= q.general;
+    p.vmax = max(p.vmax, q.vmax);
+}
+__device__ __forceinline__ PrepPart merge_block(PrepPart p) {
+    __shared__ PrepPart part[kPrepThreads / 32];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        PrepPart q;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            q.mn[a] = __shfl_xor_sync(0xffffffffu, p.mn[a], o);
+            q.mx[a] = __shfl_xor_sync(0xffffffffu, p.mx[a], o);
+        }
+        q.bad = __shfl_xor_sync(0xffffffffu, p.bad, o);
+        q.general = __shfl_xor_sync(0xffffffffu, p.general, o);
+        q.vmax = __shfl_xor_sync(0xffffffffu, p.vmax, o);
+        merge(p, q);
+    }
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = p;
+    __syncthreads();
+    p = part[0];
+    for (int w = 1; w < kPrepThreads / 32; ++w) merge(p, part[w]);
+    return p;
+}
+
+// Box of occupied cells, non-finite count and max |v| over the particles: per-block partials,
+// joined by the block that finishes last, which then lays out the grid and sets dt (one
+// launch where a reset, two reductions by atomics and two one-thread kernels were five: 1M
+// particles 0.036 -> 0.011 ms, 10k 0.012 -> 0.007).  kCells (precision mode): the stored cells.  kVmax: NaN
+// lengths are ignored, as std::max(m, v) keeps m when v is NaN (sph_engine.cpp:316-322);
+// non-negative floats order like their bit patterns.
+template <bool kCells, bool kVmax>
+__global__ void __launch_bounds__(kPrepThreads) k_prepare(const StepConst c, const Buffers b,
+                                                          DevState* ds, int how, float host_dt) {
+    PrepPart p = prep_empty();
+    const int n = c.n;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (kVmax) {
+            const float4 v = b.vel4[i];
+            if (kCells) {
+                const double len = sqrt((double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z);
+                if (!isnan(len)) p.vmax = max(p.vmax, (unsigned long long)__double_as_longlong(len));
+            } else {
+                const float len = xsqrt(xdot3(v.x, v.y, v.z));
+                if (!isnan(len)) p.vmax = max(p.vmax, (unsigned long long)__float_as_uint(len));
+            }
+        }
+        int cell[3];
+        if (kCells) {
+            const int4 q = b.cell4[i];
+            if (q.w) {
+                ++p.bad;
+                continue;
+            }
+            cell[0] = q.x, cell[1] = q.y, cell[2] = q.z;
+        } else {
+            const float4 q = b.pos4[i];
+            p.general |= tiny_coord(q.x) || tiny_coord(q.y) || tiny_coord(q.z);
+            if (!finite3(q.x, q.y, q.z)) {
+                ++p.bad;
+                continue;
+            }
+            cell[0] = cell_coord(q.x, c.inv_cell);
+            cell[1] = cell_coord(q.y, c.inv_cell);
+            cell[2] = cell_coord(q.z, c.inv_cell);
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            p.mn[a] = min(p.mn[a], cell[a]);
+            p.mx[a] = max(p.mx[a], cell[a]);
+        }
+    }
+    p = merge_block(p);
+    if (threadIdx.x == 0) b.prep[blockIdx.x] = p;
+    if (!last_block(b.sync)) return;
+    reset_step(ds, b);
+    p = prep_empty();
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) merge(p, b.prep[k]);
+    p = merge_block(p);
+    if (threadIdx.x != 0) return;
+    for (int a = 0; a < 3; ++a) {
+        ds->cmin[a] = p.mn[a];
+        ds->cmax[a] = p.mx[a];
+    }
+    ds->nonfinite = p.bad;
+    ds->general = p.general;
+    grid_setup(n, c.max_cells, ds);
+    if (how != kNoStep) set_dt(c, ds, how, host_dt, p.vmax);
+}
+
+int launch_prepare(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
+                   int how, float host_dt) {
+    // at least 4 particles a thread, so that the partials of small sets are few
+    int nb = (c.n + 4 * kPrepThreads - 1) / (4 * kPrepThreads);
+    nb = nb < 1 ? 1 : (nb > kMaxPrepBlocks ? kMaxPrepBlocks : nb);
+    const bool cfl = how == kCflDt;
+    if (c.precise && cfl) k_prepare<true, true><<<nb, kPrepThreads, 0, L.stream>>>(c, b, ds, how, host_dt);
+    else if (c.precise) k_prepare<true, false><<<nb, kPrepThreads, 0, L.stream>>>(c, b, ds, how, host_dt);
+    else if (cfl) k_prepare<false, true><<<nb, kPrepThreads, 0, L.stream>>>(c, b, ds, how, host_dt);
+    else k_prepare<false, false><<<nb, kPrepThreads, 0, L.stream>>>(c, b, ds, how, host_dt);
+    return 1;
+}
+
+// ---- grid -----------------------------------------------------------------------------
+
+// Cell keys and their digit histograms.  kCells (precision mode): the stored cells; w != 0
+// marks a particle with no finite position.
+template <bool kCells>
+__global__ void __launch_bounds__(256) k_keys(const Buffers b, int n, float inv_cell,
+                                              const DevState* ds) {
     if (ds->status) return;
+    __shared__ uint32_t h[kMaxPasses][kRadixBuckets];
+    for (int i = threadIdx.x; i < kMaxPasses * kRadixBuckets; i += 256) (&h[0][0])[i] = 0;
+    __syncthreads();
     const int cx0 = ds->cmin[0], cy0 = ds->cmin[1], cz0 = ds->cmin[2];
     const uint32_t dx = ds->dim[0], dy = ds->dim[1], dz = ds->dim[2], nc = ds->ncells;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 p = pos4[i];
+    const uint32_t passes = ds->passes;
+    for (int i0 = blockIdx.x * 256; i0 < n; i0 += gridDim.x * 256) {
+        const int i = i0 + (int)threadIdx.x;
         uint32_t key = nc;
-        if (finite3(p.x, p.y, p.z)) {
-            // relative cell index (< 2^31), folded on the axes that wrap
-            const uint32_t x = (uint32_t)(cell_coord(p.x, inv_cell) - cx0) % dx;
-            const uint32_t y = (uint32_t)(cell_coord(p.y, inv_cell) - cy0) % dy;
-            const uint32_t z = (uint32_t)(cell_coord(p.z, inv_cell) - cz0) % dz;
-            key = (x * dy + y) * dz + z;
+        if (i < n) {
+            int cx = 0, cy = 0, cz = 0;
+            bool fin;
+            if (kCells) {
+                const int4 q = b.cell4[i];
+                cx = q.x, cy = q.y, cz = q.z;
+                fin = !q.w;
+            } else {
+                const float4 p = b.pos4[i];
+                fin = finite3(p.x, p.y, p.z);
+                if (fin) {
+                    cx = cell_coord(p.x, inv_cell);
+                    cy = cell_coord(p.y, inv_cell);
+                    cz = cell_coord(p.z, inv_cell);
+                }
+            }
+            if (fin) {  // relative cell index (< 2^31), folded on the axes that wrap
+                const uint32_t x = (uint32_t)(cx - cx0) % dx, y = (uint32_t)(cy - cy0) % dy,
+                               z = (uint32_t)(cz - cz0) % dz;
+                key = (x * dy + y) * dz + z;
+            }
+            b.key[0][i] = key;
         }
-        keys[i] = key;
+        count_digits(h, key, i < n, passes);
     }
+    __syncthreads();
+    add_digits(h, b.hist, passes);
 }
 
 // Gathers the state into cell-sorted order, keeps the sorted keys and permutation, and writes
@@ -319,15 +295,14 @@ __global__ void k_reorder(const Buffers b, int n, DevState* ds) {
 struct ColumnInfo {
     uint32_t base, d2;  // first cell of the scene's block, cells along z
     bool each_cell;     // tiles within one cell
-    float inv_cell;
 };
 __device__ __forceinline__ ColumnInfo column_info(const Buffers& b, const DevState* ds, int k,
-                                                  float inv_cell, bool folded_cells) {
+                                                  bool folded_cells) {
     if (b.nscenes) {
         const SceneInfo& sc = b.scenes[b.scene_s[k]];
-        return ColumnInfo{sc.base, (uint32_t)sc.dim[2], !b.columns, sc.c.inv_cell};
+        return ColumnInfo{sc.base, (uint32_t)sc.dim[2], !b.columns};
     }
-    return ColumnInfo{0u, (uint32_t)ds->dim[2], !b.columns || folded_cells, inv_cell};
+    return ColumnInfo{0u, (uint32_t)ds->dim[2], !b.columns || folded_cells};
 }
 __device__ __forceinline__ bool tile_starts(const Buffers& b, const ColumnInfo& g, uint32_t nc,
                                             int k, uint32_t key, uint32_t prev, bool new_cell) {
@@ -343,50 +318,62 @@ __device__ __forceinline__ bool tile_starts(const Buffers& b, const ColumnInfo& 
            b.off[cb + zm] - b.off[cb + zm - kRunWindow] < tn;
 }
 
-// One block per 256 positions; a warp puts the cells that start in its 32 positions in z order
-// (the in-cell offset quantised to 16 levels, stable within a level), so that a tile is a
-// compact slab across the cells of its column.  kCells (precision mode, whose sums are judged
-// against FP64): the particles themselves are moved.  Otherwise the particles keep the
-// reference's insertion order, in which they are met as neighbours, and only the order in
-// which they are taken as targets changes (b.tgt).  Cells of more than kZOrderMax particles
-// (collapsed states, whose tiles are dense anyway) keep their order.
+// One block per 256 positions: the tile list, and the order in which each cell's particles are
+// taken as targets: z order (the in-cell offset quantised to 16 levels, stable within a
+// level), so that a tile is a compact slab across the cells of its column.  The particles
+// themselves keep the reference's insertion order, in which they are met as neighbours.  A
+// particle's place is the number of its cell's particles before it in that order, counted by
+// one thread per particle from the levels in shared memory (a counting sort per cell by one
+// warp took 0.038 ms at 1M for this kernel, 0.014 at 10k).  Cells of more than kZOrderMax particles (collapsed
+// states, whose tiles are dense anyway) keep their order.
 constexpr int kZOrderMax = 128;
-template <bool kCells>
+__device__ __forceinline__ uint8_t z_level(const Buffers& b, int k, float inv_cell, float levels) {
+    if (b.cell4_s) return (uint8_t)min(15, max(0, (int)(b.pos4_s[k].z * levels)));
+    if (b.nscenes) inv_cell = b.scenes[b.scene_s[k]].c.inv_cell;
+    const float u = b.pos4_s[k].z * inv_cell;
+    return (uint8_t)min(15, max(0, (int)((u - floorf(u)) * 16.0f)));
+}
 __global__ void __launch_bounds__(256) k_order_tiles(const Buffers b, int n, DevState* ds,
                                                      float inv_cell, float levels) {
     if (ds->status) return;
-    constexpr int kPer = kZOrderMax / 32;
     __shared__ uint32_t flags[9];
     __shared__ uint32_t s_occ, s_max, s_base;
+    __shared__ uint8_t lev[256 + 2 * kZOrderMax];  // positions k0 - kZOrderMax ...
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_occ = s_max = 0;
     const uint32_t nc = ds->ncells;
     // an exact step on a grid folded along z keeps one-cell tiles: a row that wraps is met in
     // each cell's own dz order
-    const bool folded_cells = !kCells && ds->wrap[2];
-    const int k = blockIdx.x * 256 + tid;
-    uint32_t key = 0, cnt = 0;
+    const bool folded_cells = !b.cell4_s && ds->wrap[2];
+    const int k0 = blockIdx.x * 256, k = k0 + tid;
+    uint32_t key = 0, cnt = 0, first = 0;
     bool new_cell = false, flag = false;
     if (k < n) {
         key = b.key_s[k];
         const uint32_t prev = k ? b.key_s[k - 1] : 0u;
         new_cell = k == 0 || prev != key;
-        const ColumnInfo g = column_info(b, ds, k, inv_cell, folded_cells);
-        inv_cell = g.inv_cell;
-        flag = tile_starts(b, g, nc, k, key, prev, new_cell);
-        cnt = key < nc ? b.off[key + 1] - b.off[key] : 0u;
+        flag = tile_starts(b, column_info(b, ds, k, folded_cells), nc, k, key, prev, new_cell);
+        if (key < nc) {
+            first = b.off[key];
+            cnt = b.off[key + 1] - first;
+        }
+    }
+    if (b.columns) {
+        if (k < n) lev[kZOrderMax + tid] = z_level(b, k, inv_cell, levels);
+        const int h = tid < kZOrderMax ? tid : 256 + tid;  // the halo on both sides
+        const int q = k0 - kZOrderMax + h;
+        if (q >= 0 && q < n) lev[h] = z_level(b, q, inv_cell, levels);
     }
     {
         const uint32_t f = __ballot_sync(0xffffffffu, flag);
         if (lane == 0) flags[warp] = f;
     }
     if (warp == 0) {  // the first 32 positions past the block end its last tiles
-        const int q = blockIdx.x * 256 + 256 + lane;
+        const int q = k0 + 256 + lane;
         bool fq = false;
         if (q < n) {
             const uint32_t kq = b.key_s[q], pq = b.key_s[q - 1];
-            const ColumnInfo g = column_info(b, ds, q, inv_cell, folded_cells);
-            fq = tile_starts(b, g, nc, q, kq, pq, pq != kq);
+            fq = tile_starts(b, column_info(b, ds, q, folded_cells), nc, q, kq, pq, pq != kq);
         }
         const uint32_t f = __ballot_sync(0xffffffffu, fq);
         if (lane == 0) flags[8] = f;
@@ -410,6 +397,17 @@ __global__ void __launch_bounds__(256) k_order_tiles(const Buffers b, int n, Dev
             atomicMax(&ds->max_occ, s_max);
         }
     }
+    if (b.columns && k < n) {
+        uint32_t to = (uint32_t)k;
+        if (cnt >= 2 && cnt <= (uint32_t)kZOrderMax) {
+            const uint8_t* l = lev + kZOrderMax + ((int)first - k0);  // the cell's levels
+            const uint32_t mine = lev[kZOrderMax + tid], own = (uint32_t)k - first;
+            to = first;
+            for (uint32_t q = 0; q < own; ++q) to += l[q] <= mine;
+            for (uint32_t q = own + 1; q < cnt; ++q) to += l[q] < mine;
+        }
+        b.tgt[to] = (uint32_t)k;
+    }
     __syncthreads();
     if (flag) {
         uint32_t t = s_base + __popc(flags[warp] & ((1u << lane) - 1u));
@@ -420,76 +418,15 @@ __global__ void __launch_bounds__(256) k_order_tiles(const Buffers b, int n, Dev
         if (rest) m = min(m, (uint32_t)__ffsll((long long)rest));
         b.tiles[t] = make_uint2((uint32_t)k, m);
     }
-    if (!b.columns) return;
-    const bool ordered = cnt >= 2 && cnt <= (uint32_t)kZOrderMax;
-    if (!kCells && k < n && !ordered) b.tgt[k] = (uint32_t)k;
-    for (uint32_t todo = __ballot_sync(0xffffffffu, new_cell && ordered); todo; todo &= todo - 1) {
-        const int src = __ffs(todo) - 1;
-        const uint32_t a = (uint32_t)__shfl_sync(0xffffffffu, k, src);
-        const uint32_t c = __shfl_sync(0xffffffffu, cnt, src);
-        const float ic = __shfl_sync(0xffffffffu, inv_cell, src);
-        float4 p[kPer], v[kPer];
-        int4 ce[kPer];
-        uint32_t id[kPer];
-        int lev[kPer];
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            const uint32_t q = (uint32_t)(j * 32 + lane);
-            lev[j] = 16;  // no element
-            if (q >= c) continue;
-            if (kCells) {
-                p[j] = b.pos4_s[a + q];
-                v[j] = b.vel4_s[a + q];
-                ce[j] = b.cell4_s[a + q];
-                id[j] = b.id_s[a + q];
-                lev[j] = min(15, max(0, (int)(p[j].z * levels)));
-            } else {
-                const float u = b.pos4_s[a + q].z * ic;
-                lev[j] = min(15, max(0, (int)((u - floorf(u)) * 16.0f)));
-            }
-        }
-        // stable counting sort over the 16 levels: an element's place is the number of
-        // elements of lower levels plus those of its level before it
-        int dest[kPer];
-        uint32_t below = 0;
-#pragma unroll 1
-        for (int L = 0; L < 16; ++L) {
-            uint32_t seen = below;
-#pragma unroll
-            for (int j = 0; j < kPer; ++j) {
-                const uint32_t m = __ballot_sync(0xffffffffu, lev[j] == L);
-                if (lev[j] == L) dest[j] = (int)(seen + __popc(m & ((1u << lane) - 1u)));
-                seen += __popc(m);
-            }
-            below = seen;
-        }
-        __syncwarp();  // every lane holds its elements: the cell's range can be rewritten
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            if (lev[j] == 16) continue;
-            const uint32_t to = a + (uint32_t)dest[j];
-            if (kCells) {
-                b.pos4_s[to] = p[j];
-                b.vel4_s[to] = v[j];
-                b.cell4_s[to] = ce[j];
-                b.id_s[to] = id[j];
-            } else {
-                b.tgt[to] = a + (uint32_t)(j * 32 + lane);
-            }
-        }
-    }
 }
 
 int launch_build_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                       DevState* ds) {
     const int n = c.n;
-    const int gb = grid_blocks(L, n, 256);
-    if (c.precise) k_bbox_cells<<<gb, 256, 0, L.stream>>>(b.cell4, n, ds);
-    else k_bbox<<<gb, 256, 0, L.stream>>>(b.pos4, n, c.inv_cell, ds);
-    k_grid_setup<<<1, 32, 0, L.stream>>>(n, c.max_cells, ds);
-    if (c.precise) k_keys_cells<<<gb, 256, 0, L.stream>>>(b.cell4, n, ds, b.key[0]);
-    else k_keys<<<gb, 256, 0, L.stream>>>(b.pos4, n, c.inv_cell, ds, b.key[0]);
-    return 3 + launch_grid_sort(L, b, ds, n, c);
+    const int gb = grid_blocks(L, n, 256, 2);
+    if (c.precise) k_keys<true><<<gb, 256, 0, L.stream>>>(b, n, c.inv_cell, ds);
+    else k_keys<false><<<gb, 256, 0, L.stream>>>(b, n, c.inv_cell, ds);
+    return 1 + launch_grid_sort(L, b, ds, n, c);
 }
 
 // Shared tail of the grid build: stable sort of the keys, gather into cell-sorted order with
@@ -498,11 +435,7 @@ int launch_grid_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n,
                      const StepConst& c) {
     const int r = launch_radix_sort(L, b, ds, n);
     k_reorder<<<grid_blocks(L, n + 1, 256, 8), 256, 0, L.stream>>>(b, n, ds);
-    const int nb = (n + 255) / 256;
-    if (b.columns && b.cell4_s)
-        k_order_tiles<true><<<nb, 256, 0, L.stream>>>(b, n, ds, c.inv_cell, 16.0f / c.cs);
-    else
-        k_order_tiles<false><<<nb, 256, 0, L.stream>>>(b, n, ds, c.inv_cell, 0.0f);
+    k_order_tiles<<<(n + 255) / 256, 256, 0, L.stream>>>(b, n, ds, c.inv_cell, 16.0f / c.cs);
     return 2 + r;
 }
 

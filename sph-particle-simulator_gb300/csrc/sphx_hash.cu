@@ -106,7 +106,7 @@ int galloc(T** p, size_t count) {
 void grid_free(sphx_grid* g) {
     Buffers& b = g->b;
     void* ptrs[] = {b.pos4, b.vel4, b.pos4_s, b.vel4_s, b.key[0], b.key[1], b.val[0], b.val[1],
-                    b.key_s, b.id_s, b.off, b.tiles, b.hist, b.scan_part, g->ds, g->stage};
+                    b.key_s, b.id_s, b.off, b.tiles, b.sync, g->ds, g->stage};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (g->stream) cudaStreamDestroy(g->stream);
@@ -149,20 +149,20 @@ int sphx_grid_create(sphx_grid** out, size_t capacity) {
     g->sc.max_cells = (uint32_t)max_cells;
     Buffers& b = g->b;
     const size_t C = capacity;
-    b.radix_blocks = (int)((C + kRadixTileN - 1) / kRadixTileN);
-    const size_t hist_n = (size_t)b.radix_blocks * kRadixBuckets;
-    const size_t pa = (hist_n + kScanTileN - 1) / kScanTileN, pb = (C + kScanTileN - 1) / kScanTileN;
-    b.scan_part_cap = (int)((pa > pb ? pa : pb) + 1);
     int rc;
     if ((rc = galloc(&b.pos4, C)) || (rc = galloc(&b.vel4, C)) || (rc = galloc(&b.pos4_s, C)) ||
         (rc = galloc(&b.vel4_s, C)) || (rc = galloc(&b.key[0], C)) || (rc = galloc(&b.key[1], C)) ||
         (rc = galloc(&b.val[0], C)) || (rc = galloc(&b.val[1], C)) || (rc = galloc(&b.key_s, C)) ||
         (rc = galloc(&b.id_s, C)) || (rc = galloc(&b.off, (size_t)max_cells + 2)) ||
-        (rc = galloc(&b.tiles, C)) || (rc = galloc(&b.hist, hist_n)) ||
-        (rc = galloc(&b.scan_part, (size_t)b.scan_part_cap)) || (rc = galloc(&g->ds, 1)) ||
+        (rc = galloc(&b.tiles, C)) ||  (rc = galloc(&g->ds, 1)) ||
         (rc = galloc(&g->stage, 4 * C)))
         return fail(rc);
-    if (cudaMemset(g->ds, 0, sizeof(DevState)) != cudaSuccess) return fail(SPHX_ERR_CUDA);
+    unsigned char* scratch = nullptr;
+    if ((rc = galloc(&scratch, grid_scratch_bytes(C)))) return fail(rc);
+    set_grid_scratch(b, scratch);
+    if (cudaMemset(g->ds, 0, sizeof(DevState)) != cudaSuccess ||
+        cudaMemset(scratch, 0, grid_scratch_bytes(C)) != cudaSuccess)
+        return fail(SPHX_ERR_CUDA);
     *out = g;
     return SPHX_OK;
 }
@@ -193,7 +193,7 @@ int sphx_grid_build(sphx_grid* g, size_t n, const float* pos_xyz, float cell_siz
     GRID_CUDA(cudaMemcpyAsync(s_pos, pos_xyz, 3 * n * sizeof(float), cudaMemcpyHostToDevice, g->stream));
     GRID_CUDA(cudaMemsetAsync(s_mass, 0, n * sizeof(float), g->stream));
     launch_pack(g->L, (int)n, s_pos, nullptr, s_mass, g->b.pos4, g->b.vel4);
-    launch_begin_step(g->L, g->ds, 1);
+    launch_prepare(g->L, g->sc, g->b, g->ds, kNoStep, 0.0f);
     launch_build_grid(g->L, g->sc, g->b, g->ds);
     GRID_CUDA(cudaGetLastError());
     GRID_CUDA(cudaStreamSynchronize(g->stream));

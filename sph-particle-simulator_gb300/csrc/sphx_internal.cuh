@@ -17,11 +17,11 @@ constexpr int kRadixThreads = 256;
 constexpr int kRadixItems = 16;
 constexpr int kRadixTileN = kRadixThreads * kRadixItems;  // keys per radix block
 constexpr int kMaxPasses = 4;                             // 32-bit keys
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
-constexpr int kScanTileN = kScanThreads * kScanItems;
+constexpr int kSmallSort = 1 << 18;                       // keys: see launch_radix_sort
+constexpr int kPrepThreads = 256, kMaxPrepBlocks = 608;   // first kernel of a step
 constexpr int kDiagThreads = 256;
 constexpr int kDiagSums = 8;
+constexpr float kCoincident = 1e-30f;  // see sweep_d2
 // A nonzero coordinate below this (in magnitude) sends a step's exact passes to the general
 // pair forms (DevState::general): the others rely on x_i - x_j being 0 or at least 2^-68.
 constexpr float kTiny = 0x1p-45f;
@@ -33,7 +33,7 @@ typedef unsigned long long f32x2;
 struct PairLits {  // numbers
     f32x2 neg0;    // -0: see F2
     f32x2 half, one, two, neg2, three, onehalf, neg2p40, p2p20, neg2p20, p2p21, two_thirds,
-        one_sixth, neg5, five;
+        one_sixth, neg5, five, neg_half, neg1, neg3, coincident;
 };
 struct PairConst {  // of the step's parameters
     f32x2 neg_h, h, rcp_h, neg_hsq, rcp_hsq, sigma, neg_sigma, gas, rest, wnorm, wl;
@@ -89,7 +89,6 @@ struct DevState {
     uint32_t passes;            // radix passes needed this step
     uint32_t n_tiles;           // warp work items
     uint32_t nonfinite;         // particles with a NaN/inf coordinate
-    uint32_t vmax_bits;         // max |v| (float bits) for the CFL rule
     uint32_t occupied;          // occupied cells
     uint32_t max_occ;           // particles in the fullest cell
     uint32_t work[2];           // tile counters of the density and force passes
@@ -99,10 +98,24 @@ struct DevState {
     unsigned long long max_nn;  // max |N(i)| since the last stats reset
     double sums[kDiagSums];     // FP64 diagnostics of the state after the last step
     double dt64, time64;        // precision mode: dt and current time in FP64
-    unsigned long long vmax64;  // precision mode: max |v| (FP64 bits)
     uint32_t n_spread;          // precision mode: spread tiles listed this step
     uint32_t spread_work[2];    // precision mode: tile counters of the spread-tile kernels
     uint32_t general;           // exact mode: 1 if a value lies outside the pair forms' ranges
+};
+
+// What blocks of one grid-build kernel tell each other; not part of the step's state (never
+// saved or restored, zero once at creation).
+struct GridSync {
+    uint32_t done;               // blocks of the step's first kernel that have finished
+    uint32_t epoch;              // sorts started: tags the look-back words (sphx_sort.cu)
+    uint32_t tile[kMaxPasses];   // sort tickets of each pass
+    uint32_t general;            // batched mode: see DevState::general
+};
+// One block's share of the first kernel's reductions.
+struct PrepPart {
+    int mn[3], mx[3];
+    uint32_t bad, general;
+    unsigned long long vmax;     // max |v|: float or (precision mode) double bits
 };
 
 // Batched mode: one record per scene (device memory).  Scenes are contiguous ranges of
@@ -110,11 +123,12 @@ struct DevState {
 struct SceneInfo {
     StepConst c;                // the scene's parameters and constants (c.n = count)
     uint32_t start, count;      // particle range in insertion order
+    // reductions of the step's first kernel, reset when they have been read
+    int acc_min[3], acc_max[3];
+    uint32_t acc_bad, acc_vmax;
     int cmin[3], cmax[3];       // box of occupied cells
     int dim[3];                 // grid extent of the scene
     uint32_t base, ncells;      // first grid cell, number of cells
-    uint32_t nonfinite;
-    uint32_t vmax_bits;
     float dt, time;             // the scene's dt of the current step and current_time_
     float a0[4];                // acceleration of the scene's first particle
     double sums[kDiagSums];     // FP64 diagnostics of the scene after the last step
@@ -146,26 +160,28 @@ struct Buffers {
     // Target order: the particle of target position k is sorted position tgt[k]; null: k.
     // (k_order_tiles: a permutation within each cell, so position k's cell is key_s[k].)
     uint32_t* tgt = nullptr;
-    uint32_t* hist;   // radix histograms / offsets
-    uint32_t* scan_part;
+    uint32_t* hist;   // radix digit histograms, one per pass
+    unsigned long long* look;  // radix look-back words: one per (tile, digit)
+    GridSync* sync;
+    PrepPart* prep;   // kMaxPrepBlocks
     double* diag_part;
     uint32_t* scene_of;  // batched mode: scene of each particle (insertion order)
     uint32_t* scene_s;   // batched mode: scene of each particle (cell-sorted)
     SceneInfo* scenes;   // batched mode: per-scene records
     int nscenes;         // 0: single scene
-    // Hit masks of the density pass, reused by the force pass of the same step.  A tile owns
-    // consecutive records of 32 words: first one word per 32-candidate chunk of the tile's
-    // walk (which candidates the tile's box keeps), then one record per 32 kept candidates
-    // (word = lane: bit 31 - j set if the j-th of them is a neighbour of the lane's particle).
-    // Every warp of the density grid owns an equal region of the pool and stores its tiles
-    // one after another; tile_slot[t] = first record, or kNoSlot when the tile did not fit in
-    // what was left of the region (the force pass then repeats the tests for that tile).
-    uint32_t* hitmask = nullptr;
-    uint32_t* tile_slot = nullptr;
-    unsigned long long hitmask_cap = 0;  // records
-    int radix_blocks;
-    int scan_part_cap;
+    // What the density pass tells the force pass of the same step about each tile, in records
+    // of 32 words: exact mode, per chunk of 32 candidates that the tile's box keeps their
+    // sorted positions and the lanes' neighbour masks (word = lane: bit 31 - j set if the j-th
+    // of them is a neighbour of the lane's particle); precision mode, the sorted positions of
+    // the kept candidates that are a neighbour of some lane.  Every warp of the density grid
+    // owns an equal region of the pool and stores its tiles one after another; tile_list[t] =
+    // first record and candidates, or kNoSlot when the tile did not fit in what was left of
+    // the region (the force pass then walks and tests that tile itself).
+    uint32_t* records = nullptr;
+    uint2* tile_list = nullptr;
+    unsigned long long record_cap = 0;
     int diag_blocks;
+    int num_sms = 1;
     int tile_n = kTile;  // particles per warp work item (1 .. kTile)
     // 1: the tiles run along cell columns (x, y, *), spanning cells, with each cell's particles
     // taken in z order; 0: insertion order within each cell and tiles within one cell
@@ -455,6 +471,67 @@ __device__ __forceinline__ int cell_coord(float x, float inv_cell) {
 // a nonzero coordinate below kTiny in magnitude
 __device__ __forceinline__ bool tiny_coord(float x) { return x != 0.0f && fabsf(x) < kTiny; }
 
+// ---- pieces of the step's first kernel (single scene and batched) -----------------------
+
+// true in every thread of the block that finishes last; its reads then see what the other
+// blocks wrote before their call
+__device__ __forceinline__ bool last_block(GridSync* sync) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(&sync->done, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+// resets the step's counters (one block, all threads)
+__device__ __forceinline__ void reset_step(DevState* ds, const Buffers& b) {
+    for (int i = threadIdx.x; i < kMaxPasses * kRadixBuckets; i += blockDim.x) b.hist[i] = 0;
+    if (threadIdx.x != 0) return;
+    ds->status = 0;
+    ds->occupied = 0;
+    ds->max_occ = 0;
+    ds->n_tiles = 0;
+    ds->work[0] = ds->work[1] = 0;
+    ds->spread_work[0] = ds->spread_work[1] = 0;
+    ds->n_spread = 0;
+    b.sync->epoch++;
+    for (int p = 0; p < kMaxPasses; ++p) b.sync->tile[p] = 0;
+}
+// dt = min({dt_cfl, dt_force, timestep}) with std::min's first-smallest rule
+// (SPHEngine::compute_cfl_timestep, sph_engine.cpp:312-333)
+__device__ __forceinline__ float cfl_dt(const StepConst& c, float vmax, const float* a0) {
+    const float dt_cfl = xdiv(xmul(c.cfl, c.h), xadd(vmax, 1e-6f));
+    const float alen = xsqrt(xdot3(a0[0], a0[1], a0[2]));
+    const float dt_force = xmul(c.cfl, xsqrt(xdiv(c.h, xadd(alen, 1e-6f))));
+    float dt = dt_cfl;
+    if (dt_force < dt) dt = dt_force;
+    if (c.timestep < dt) dt = c.timestep;
+    return dt;
+}
+// digit counts of a key for the sort's passes, gathered in shared memory; the lanes of a warp
+// that all hold the same digit (the high digits of neighbouring particles) count once
+__device__ __forceinline__ void count_digits(uint32_t (*h)[kRadixBuckets], uint32_t key, bool ok,
+                                             uint32_t passes) {
+    const uint32_t act = __ballot_sync(0xffffffffu, ok);
+    if (!act) return;
+    const int first = __ffs(act) - 1;
+    for (uint32_t p = 0; p < passes; ++p) {
+        const uint32_t d = (key >> (p * kRadixBits)) & (kRadixBuckets - 1);
+        const uint32_t d0 = __shfl_sync(0xffffffffu, d, first);
+        if (__all_sync(0xffffffffu, !ok || d == d0)) {
+            if ((threadIdx.x & 31) == (unsigned)first) atomicAdd(&h[p][d0], (uint32_t)__popc(act));
+        } else if (ok) {
+            atomicAdd(&h[p][d], 1u);
+        }
+    }
+}
+__device__ __forceinline__ void add_digits(uint32_t (*h)[kRadixBuckets], uint32_t* hist,
+                                           uint32_t passes) {
+    for (uint32_t i = threadIdx.x; i < passes * kRadixBuckets; i += blockDim.x)
+        if ((&h[0][0])[i]) atomicAdd(&hist[i], (&h[0][0])[i]);
+}
+
 // ---- asynchronous copies of single elements, global to shared memory -------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -508,9 +585,12 @@ struct LaunchCtx {
     int blocks_per_sm;
 };
 
-int launch_begin_step(const LaunchCtx& L, DevState* ds, int reset_bbox);
-int launch_cfl(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
-                float host_dt);
+// How a step gets its dt.
+constexpr int kNoStep = 0, kHostDt = 1, kCflDt = 2;
+// The step's first kernel: resets the step's counters, finds the box of occupied cells and
+// lays out the grid, and (how != kNoStep) sets dt and advances the time.
+int launch_prepare(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
+                   int how, float host_dt);
 int launch_build_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                        DevState* ds);
 int launch_grid_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, const StepConst& c);
@@ -529,13 +609,16 @@ void launch_pair_fill(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                       DevState* ds, const uint64_t* offsets_by_id, int64_t* out_idx);
 
 // batched mode (sphx_batch.cu)
-int launch_batch_begin(const LaunchCtx& L, const Buffers& b, DevState* ds);
-int launch_batch_cfl(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, float host_dt);
-int launch_batch_grid(const LaunchCtx& L, const Buffers& b, DevState* ds, int n,
-                      uint32_t max_cells);
+int launch_batch_prepare(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, int how,
+                         float host_dt, uint32_t max_cells);
+int launch_batch_grid(const LaunchCtx& L, const Buffers& b, DevState* ds, int n);
 int launch_batch_diag(const LaunchCtx& L, const Buffers& b, DevState* ds);
 
-// radix sort + scan (sphx_sort.cu)
+// The grid build's working memory besides the per-particle arrays, one block: GridSync (first),
+// PrepPart, digit histograms and the sort's look-back words; zero once at creation (sphx_sort.cu).
+size_t grid_scratch_bytes(size_t capacity);
+void set_grid_scratch(Buffers& b, unsigned char* base);
+// radix sort (sphx_sort.cu)
 int launch_radix_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n);
 
 // io (sphx_grid.cu)

@@ -19,8 +19,9 @@
 //  - the cell grid has SPHX_NOALLOC_MAX_CELLS cells; a larger box of occupied cells is
 //    folded onto it (results unchanged, more candidates to test);
 //  - all calls share the one array, which keeps the previous call's contents: the
-//    device-side step state is cleared at the start of every call, every other region is
-//    fully written before it is read.  Calls whose work overlaps on the GPU (two streams,
+//    device-side step state is cleared at the start of every call, and every other region is
+//    fully written before it is read, but for the sort's look-back words and the counters
+//    that tag them (zero when the library is loaded, then only counted up).  Calls whose work overlaps on the GPU (two streams,
 //    two host threads) race on the array and must be serialised by the caller;
 //  - the first call on a device looks up the array's device address
 //    (cudaGetSymbolAddress) with that device current; make that first call before any
@@ -44,12 +45,13 @@ constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign;
 
 constexpr size_t kN = SPHX_NOALLOC_MAX_PARTICLES;
 constexpr size_t kCells = SPHX_NOALLOC_MAX_CELLS;
-constexpr size_t kRadixBlocks = (kN + kRadixTileN - 1) / kRadixTileN;
-constexpr size_t kHist = kRadixBlocks * kRadixBuckets;
-constexpr size_t kScanPart =
-    ((kHist + kScanTileN - 1) / kScanTileN > (kN + kScanTileN - 1) / kScanTileN
-         ? (kHist + kScanTileN - 1) / kScanTileN
-         : (kN + kScanTileN - 1) / kScanTileN) + 1;
+// grid_scratch_bytes(kN): kN <= kSmallSort, so the sort's tiles are of 1024 keys
+constexpr size_t kLook = (kN + kRadixThreads * 4 - 1) / (kRadixThreads * 4) * kRadixBuckets;
+static_assert(kN <= (size_t)kSmallSort, "kLook");
+constexpr size_t kGridScratch = align_up(sizeof(GridSync)) +
+                                align_up(kMaxPrepBlocks * sizeof(PrepPart)) +
+                                align_up((size_t)kMaxPasses * kRadixBuckets * sizeof(uint32_t)) +
+                                align_up(kLook * sizeof(unsigned long long));
 
 // byte offsets of the regions inside the scratch array
 constexpr size_t kOffState = 0;
@@ -67,9 +69,8 @@ constexpr size_t kOffIdS = kOffKeyS + align_up(kN * sizeof(uint32_t));
 constexpr size_t kOffTiles = kOffIdS + align_up(kN * sizeof(uint32_t));
 constexpr size_t kOffTgt = kOffTiles + align_up(kN * sizeof(uint2));
 constexpr size_t kOffOff = kOffTgt + align_up(kN * sizeof(uint32_t));
-constexpr size_t kOffHist = kOffOff + align_up((kCells + 2) * sizeof(uint32_t));
-constexpr size_t kOffScan = kOffHist + align_up(kHist * sizeof(uint32_t));
-constexpr size_t kNoAllocScratchBytes = kOffScan + align_up(kScanPart * sizeof(uint32_t));
+constexpr size_t kOffGrid = kOffOff + align_up((kCells + 2) * sizeof(uint32_t));
+constexpr size_t kNoAllocScratchBytes = kOffGrid + kGridScratch;
 
 // The scratch.  In host code this name is only a host-side stand-in for the device
 // array: its device address comes from cudaGetSymbolAddress.
@@ -156,12 +157,10 @@ extern "C" int sphx_density_noalloc(const sphx_params* p, size_t n, const float*
     b.tgt = reinterpret_cast<uint32_t*>(base + kOffTgt);
     b.columns = 1;
     b.off = reinterpret_cast<uint32_t*>(base + kOffOff);
-    b.hist = reinterpret_cast<uint32_t*>(base + kOffHist);
-    b.scan_part = reinterpret_cast<uint32_t*>(base + kOffScan);
+    set_grid_scratch(b, base + kOffGrid);
     b.diag_part = nullptr;
-    b.radix_blocks = (int)kRadixBlocks;
-    b.scan_part_cap = (int)kScanPart;
     b.diag_blocks = 0;
+    b.num_sms = sms;
     DevState* ds = reinterpret_cast<DevState*>(base + kOffState);
 
     LaunchCtx L{};
@@ -174,7 +173,7 @@ extern "C" int sphx_density_noalloc(const sphx_params* p, size_t n, const float*
     // the previous call's device-side state must not leak into this one
     if (cudaMemsetAsync(ds, 0, sizeof(DevState), L.stream) != cudaSuccess) return SPHX_ERR_CUDA;
     launch_pack(L, (int)n, pos_xyz, nullptr, mass, b.pos4, b.vel4);
-    launch_begin_step(L, ds, 1);
+    launch_prepare(L, c, b, ds, kNoStep, 0.0f);
     launch_build_grid(L, c, b, ds);
     launch_density(L, c, b, ds);
     const int ub = (int)((n + 255) / 256) < 4 * sms ? (int)((n + 255) / 256) : 4 * sms;

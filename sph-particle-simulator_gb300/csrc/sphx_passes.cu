@@ -24,8 +24,12 @@ __global__ void __launch_bounds__(128) k_pairs(const StepConst c, const Buffers 
         bool valid;
         int4 frame = make_int4(0, 0, 0, 0);
         int i = (int)tile.x + lane;
-        if (kPrecise) tile_setup_cells(c, b, g, tile, lane, T, xi, valid, frame);
-        else tile_setup(c, b, g, tile, lane, T, i, xi, valid);
+        if (kPrecise) {
+            int4 ci;
+            float4 o;
+            tile_setup_cells(c, b, g, tile, lane, T, i, ci, o, valid, frame);
+            xi = T.cells ? frame_pos(ci, frame, o, c.cs) : o;
+        } else tile_setup(c, b, g, tile, lane, T, i, xi, valid);
         const uint32_t id = valid ? b.id_s[i] : 0u;
         uint64_t pos = (kFill && valid) ? off_by_id[id] : 0ull;
         const bool want = !kFill || pos != kNoPairs;  // fill: particles with an offset only

@@ -1,21 +1,23 @@
-// Precision-mode neighbour passes as tile sweeps: density + pressure, and force +
-// acceleration + leapfrog + wall clamp, of the cell + offset step (compute_densities /
-// compute_pressures / compute_forces, sph_engine.cpp:203-244, 370-443; integrate_leapfrog,
-// cpp:290-310; apply_boundary_conditions, particle.cpp:122-153).
+// Precision-mode neighbour passes: density + pressure, and force + acceleration + leapfrog +
+// wall clamp, of the cell + offset step (compute_densities / compute_pressures /
+// compute_forces, sph_engine.cpp:203-244, 370-443; integrate_leapfrog, cpp:290-310;
+// apply_boundary_conditions, particle.cpp:122-153).
 //
 // The precision mode is judged against an FP64 evaluation, not against the reference's
-// summation order, so its passes need neither the hit lists nor the in-order folds of the
-// exact passes.  One warp owns one tile (up to 32 cell-sorted particles of one cell, one
-// per lane) and sweeps the tile's stencil 32 candidates at a time: a chunk is staged in
-// shared memory in the tile's frame, the candidates that no particle of the tile can reach
-// are culled by the tile's box, and every lane evaluates every remaining candidate against
-// its own particle, two candidates per packed FP32x2 instruction and without branches: the
+// summation order, so its passes sweep: one warp owns one tile (up to 32 particles of one cell
+// column, one per lane), appends the candidates its box can reach to a small buffer in shared
+// memory in the tile's frame, and whenever 32 have come together every lane evaluates all of
+// them against its own particle, two per packed FP32 instruction and without branches: the
 // pair's term is formed whatever the distance and is zero (or zeroed) when the candidate is
-// not a neighbour.  Every lane is busy on every instruction; the price is the terms of the
-// culled box's non-neighbours, which costs less than listing the neighbours.
+// not a neighbour.  Every lane is busy on every instruction and the terms are independent of
+// one another; the price is the terms of the non-neighbours (about two of three), which costs
+// less here than taking each lane's neighbours one by one (the exact passes' way, whose terms
+// are four times as long: 0.90 and 1.49 ms for density and force on the 1M dam break).  The
+// density pass also lists the kept candidates that are a neighbour of some lane at all (750 of
+// 920 per tile); the force pass sweeps only those.
 //
-// The self pair is swept like any other: its W is W(0) (the reference's m_i W(0) term) and
-// its force terms are zero (r = 0 skips the pressure term; v_i - v_i = 0).
+// The particle itself is swept like any other: its W is W(0) (the reference's m_i W(0)
+// term) and its force terms are zero (r = 0 gives a zero gradient; v_i - v_i = 0).
 //
 // Smoothing kernels in the "max form" (a = max(2 - q, 0), b = max(1 - q, 0) for the cubic
 // spline), which is zero beyond the support without a test:
@@ -27,13 +29,13 @@
 //                                                             (kernels.cpp:210-225)
 // A pair is a neighbour when |r|^2 <= r_search^2 (spatial_hash.cpp:46-50); when the search
 // radius is at least the support 2h, the max form already zeroes every non-neighbour and
-// the force sweep skips the test (kCut = false).
+// the terms need no selection (kCut = false).
 //
-// Positions are swept in units of h (the tile's frame scaled by 1/h): |r|/h = q comes
-// without a multiplication, and every force term that needs the direction uses r_vec / |r|,
-// which is the same in any unit.  The pressure term of a pair closer than 1e-6 m, which the
-// reference skips, is formed here (it is at most |grad W| 1e-6 m, far below the stated
-// bound; a coincident pair, |r| = 0, gives exactly 0 as in the reference).
+// Positions are in units of h (the tile's frame scaled by 1/h): |r|/h = q comes without a
+// multiplication, and every force term that needs the direction uses r_vec / |r|, which is
+// the same in any unit.  The pressure term of a pair closer than 1e-6 m, which the reference
+// skips, is formed here (it is at most |grad W| 1e-6 m, far below the stated bound; a
+// coincident pair, |r| = 0, gives exactly 0 as in the reference).
 #include "sphx_passes.cuh"
 
 namespace sphx {
@@ -45,7 +47,7 @@ __device__ __forceinline__ F2 keep(bool ka, bool kb, F2 a) {
     return f2(ka ? u.x : 0.0f, kb ? u.y : 0.0f);
 }
 
-// hardware square root (a few ulp; precision mode only)
+// hardware square root (a few ulp)
 __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -53,7 +55,7 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 }
 __device__ __forceinline__ float exp_approx(float x) { return __expf(x); }
 
-// position of the empty slots of a chunk: far enough to be no particle's neighbour, near
+// position of an empty slot: far enough to be no particle's neighbour, near
 // enough that every term formed from it stays finite (|r|^2 of 3e30)
 constexpr float kFar = 1.0e15f;
 
@@ -88,13 +90,13 @@ __device__ __forceinline__ F2 sweep_w(const StepConst& c, F2 d2) {
     if (K == SPHX_KERNEL_GAUSSIAN) return f2(exp_approx(-e.x), exp_approx(-e.y));
     const F2 q = f2(sqrt_approx(e.x), sqrt_approx(e.y));
     if (K == SPHX_KERNEL_WENDLAND_C2) {
-        const F2 t = max0(fma2(q, f2(-0.5f), f2(1.0f)));
+        const F2 t = max0(fma2(q, F2{c.lit.neg_half}, F2{c.lit.one}));
         const F2 t2 = t * t;
-        return (t2 * t2) * fma2(q, f2(2.0f), f2(1.0f));
+        return (t2 * t2) * fma2(q, F2{c.lit.two}, F2{c.lit.one});
     }
-    const F2 w1 = fma2(q * q, fma2(q, f2(0.5f), f2(-1.0f)), f2(2.0f / 3.0f));
-    const F2 t = max0(f2(2.0f) - q);
-    const F2 w2 = (t * t) * (t * f2(1.0f / 6.0f));
+    const F2 w1 = fma2(q * q, fma2(q, F2{c.lit.half}, F2{c.lit.neg1}), F2{c.lit.two_thirds});
+    const F2 t = max0(F2{c.lit.two} - q);
+    const F2 w2 = (t * t) * (t * F2{c.lit.one_sixth});
     const float2 qv = upk2(q.v), a = upk2(w1.v), bb = upk2(w2.v);
     return f2(qv.x <= 1.0f ? a.x : bb.x, qv.y <= 1.0f ? a.y : bb.y);
 }
@@ -105,14 +107,15 @@ __host__ __device__ __forceinline__ float sweep_w_scale(const StepConst& c) {
 // ---------------------------------------------------------------------------------------
 // density + pressure
 // ---------------------------------------------------------------------------------------
+// Candidates kept by the tile wait in a buffer of two chunks of 32; a chunk is swept once
+// complete (the last one padded with empty slots: far, without mass).
 struct SweepDensitySmem {
-    float4 box_lo, box_hi;  // the tile's box (kept here, not in registers, across the sweep)
-    int2 seg[kMaxSegments];
-    float4 xy[16];  // candidates 2p, 2p+1 of the chunk: x, x, y, y (tile frame)
-    float4 zm[16];  // z, z, m, m
+    float cx[64], cy[64], cz[64], cm[64];  // tile frame; mass
+    uint32_t idx[64];                      // sorted position
+    int2 seg[kMaxSegments + 1];
 };
-// The spread tiles' launch (sweep_density_spread) stages whole candidates; its own layout
-// keeps the main launch's shared memory (and so its L1 share) as small as before.
+static_assert(sizeof(SweepDensitySmem) % 16 == 0, "per-warp regions stay 16-byte aligned");
+// The spread tiles' launch (sweep_density_spread) stages whole candidates.
 struct SweepDensitySpreadSmem {
     int2 seg[kMaxSegments];
     int4 scell[32];   // candidate j of the chunk: its cell
@@ -205,15 +208,52 @@ __device__ __forceinline__ void density_out(const StepConst& c, const Buffers& b
 }
 
 // A tile with a particle more than kSpreadCells cells from its frame (listed for the
-// spread launch by the density sweep, skipped by both sweeps).
-__device__ __forceinline__ bool spread_tile(const Buffers& b, const Tile& T, int i, bool valid,
+// spread launch by the density pass, skipped by both passes).
+__device__ __forceinline__ bool spread_tile(const Tile& T, const int4& cell, bool valid,
                                             const int4& frame) {
-    return T.cells && __any_sync(kFull, valid && far_cell(b.cell4_s[i], frame));
+    return T.cells && __any_sync(kFull, valid && far_cell(cell, frame));
+}
+
+// A chunk's terms added to acc; returns the mask of the lane's neighbours in it (bit 31 - j:
+// slot j; quads past nq unset).
+template <int kKern, bool kCut>
+__device__ __forceinline__ uint32_t sweep_density_chunk(const StepConst& c, const float* cx,
+                                                        const float* cy, const float* cz,
+                                                        const float* cm, int nq, F2 X, F2 Y, F2 Z,
+                                                        float r2, F2& acc) {
+    const F2 R2 = f2(r2);
+    uint32_t miss = 0;
+#pragma unroll 4
+    for (int q = 0; q < nq; ++q) {
+        const ulonglong2 x = reinterpret_cast<const ulonglong2*>(cx)[q];
+        const ulonglong2 y = reinterpret_cast<const ulonglong2*>(cy)[q];
+        const ulonglong2 z = reinterpret_cast<const ulonglong2*>(cz)[q];
+        const ulonglong2 m = reinterpret_cast<const ulonglong2*>(cm)[q];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const F2 dx = X - F2{h ? x.y : x.x}, dy = Y - F2{h ? y.y : y.x},
+                     dz = Z - F2{h ? z.y : z.x};
+            const F2 d2 = fma2(dx, dx, fma2(dy, dy, dz * dz));
+            const float2 t = upk2((R2 - d2).v);  // negative: not a neighbour
+            miss = __funnelshift_l(__float_as_uint(t.x), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(t.y), miss, 1);
+            F2 w = sweep_w<kKern>(c, d2);
+            if (kCut) w = keep(!(t.x < 0.0f), !(t.y < 0.0f), w);
+            acc = fma2(F2{h ? m.y : m.x}, w, acc);
+        }
+    }
+    return ~miss << (32 - 4 * nq);
 }
 
 // kCut: the search radius is below the support 2h (or the kernel is the Gaussian): W is
 // selected by the neighbour test; otherwise W is already 0 beyond 2h and the test only
-// counts the neighbours.
+// counts the neighbours and finds the candidates some lane needs.
+//
+// Bound: instruction issue (73% of the slots) and the FP32 pipe: 653 warp instructions per
+// particle, of which 415 are the chunks (27.7 per pair of candidates, 29 chunks a tile) and
+// most of the rest the walk of 55 chunks of 32, its conversion to the tile's frame and its box
+// cull.  1M dam break: 0.74 ms (0.76 with a sweep of each culled chunk on its own, without the
+// list for the force pass).
 template <int kKern, bool kCut>
 __global__ void __launch_bounds__(128, 6) k_density_sweep(const StepConst c, const Buffers b,
                                                           DevState* ds) {
@@ -222,87 +262,90 @@ __global__ void __launch_bounds__(128, 6) k_density_sweep(const StepConst c, con
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     SweepDensitySmem* S = reinterpret_cast<SweepDensitySmem*>(smem_sweep_d) + warp;
     const uint32_t ntiles = ds->n_tiles;
+    const uint32_t lt = (1u << lane) - 1u;
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
     uint32_t my_max = 0;
-    for (uint32_t t = next_tile(&ds->work[0], lane); t < ntiles; t = next_tile(&ds->work[0], lane)) {
+    const TileQueue queue(&ds->work[0], b.num_sms);
+    RecordRegion region(b, queue, ntiles);
+    for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
-        float4 xi;
+        int i;
+        int4 cell, frame;
+        float4 o;
         bool valid;
-        int4 frame;
-        tile_setup_cells(c, b, g, b.tiles[t], lane, T, xi, valid, frame);
-        const int i = T.k0 + lane;
-        if (spread_tile(b, T, i, valid, frame)) {
+        tile_setup_cells(c, b, g, b.tiles[t], lane, T, i, cell, o, valid, frame);
+        if (spread_tile(T, cell, valid, frame)) {
             if (lane == 0) b.spread_tiles[atomicAdd(&ds->n_spread, 1u)] = t;
             continue;  // swept by the spread launch
         }
-        if (valid && T.cells) xi = frame_pos_h(b.cell4_s[i], frame, b.pos4_s[i], U);
-        {
-            const TileBox B = tile_box(xi, valid);
-            if (lane == 0) {
-                S->box_lo = make_float4(B.lo[0], B.lo[1], B.lo[2], 0.0f);
-                S->box_hi = make_float4(B.hi[0], B.hi[1], B.hi[2], 0.0f);
-            }
-        }
-        const F2 X = f2(xi.x), Y = f2(xi.y), Z = f2(xi.z);
-        KSum rk;  // sum of m_j W_ij / scale over the stencil, the particle itself included
-        uint32_t nn = 0;
+        const float4 xi = frame_pos_h(cell, frame, o, U);
+        const TileBox B = tile_box(xi, valid);
+        __syncwarp();  // the previous tile's segments are read
         const int nseg = build_segments(b, g, T, lane, S->seg);
         __syncwarp();
+        // the tile's list of needed candidates, one after another in its records
+        uint32_t* const list = b.records + (size_t)region.cur * 32;
+        const uint32_t room = (region.end - region.cur) * 32;
+        const F2 X = f2(xi.x), Y = f2(xi.y), Z = f2(xi.z);
+        KSum rk;  // sum of m_j W_ij / scale over the stencil, the particle itself included
+        uint32_t nn = 0, needed = 0;
+        int kept = 0, swept = 0;
+        auto put = [&](int q, float x, float y, float z, float m) {
+            S->cx[q] = x;
+            S->cy[q] = y;
+            S->cz[q] = z;
+            S->cm[q] = m;
+        };
+        auto sweep = [&](int left) {  // chunk `swept`, `left` candidates
+            const int f = (swept & 1) * 32;
+            __syncwarp();
+            F2 acc = f2(0.0f);
+            uint32_t mask = sweep_density_chunk<kKern, kCut>(c, S->cx + f, S->cy + f, S->cz + f,
+                                                             S->cm + f, (left + 3) >> 2, X, Y, Z,
+                                                             U.r2, acc);
+            const float2 a2 = upk2(acc.v);
+            rk.add(a2.x + a2.y);  // compensated across chunks
+            mask = valid ? mask & chunk_valid(left) : 0u;
+            nn += __popc(mask);
+            const uint32_t used = __brev(__reduce_or_sync(kFull, mask));
+            const uint32_t at = needed + __popc(used & lt);
+            // (streaming stores: the lists must not evict the candidates from L2)
+            if (((used >> lane) & 1u) && at < room) __stcs(list + at, S->idx[f + lane]);
+            needed += __popc(used);
+            ++swept;
+            __syncwarp();  // the chunk's slots may be written again
+        };
         for (int sg = 0; sg < nseg; ++sg) {
             const int2 se = S->seg[sg];
             for (int s = se.x; s < se.y; s += 32) {
                 const bool in = lane < se.y - s;
                 float4 pl = make_float4(kFar, kFar, kFar, 0.0f);
                 if (in) pl = frame_pos_h(b.cell4_s[s + lane], frame, b.pos4_s[s + lane], U);
-                TileBox B;
-                {
-                    const float4 lo = S->box_lo, hi = S->box_hi;
-                    B.lo[0] = lo.x, B.lo[1] = lo.y, B.lo[2] = lo.z;
-                    B.hi[0] = hi.x, B.hi[1] = hi.y, B.hi[2] = hi.z;
-                }
                 const uint32_t surv = __ballot_sync(kFull, in && box_near(B, pl, U.r2m));
-                if (!surv) continue;
-                const int nsv = __popc(surv);
-                __syncwarp();  // the previous chunk's reads are done
-                {
-                    // survivors packed to slots 0 .. nsv-1; an odd count is padded with an
-                    // empty slot (written by lane 0 besides its own)
-                    auto put = [&](int k, const float4& v) {
-                        float* xy = reinterpret_cast<float*>(&S->xy[k >> 1]);
-                        float* zm = reinterpret_cast<float*>(&S->zm[k >> 1]);
-                        const int h = k & 1;
-                        xy[h] = v.x;
-                        xy[2 + h] = v.y;
-                        zm[h] = v.z;
-                        zm[2 + h] = v.w;
-                    };
-                    if ((surv >> lane) & 1u) put(__popc(surv & ((1u << lane) - 1u)), pl);
-                    if (lane == 0 && (nsv & 1)) put(nsv, make_float4(kFar, kFar, kFar, 0.0f));
+                if ((surv >> lane) & 1u) {
+                    const int q = (kept + __popc(surv & lt)) & 63;
+                    put(q, pl.x, pl.y, pl.z, pl.w);
+                    S->idx[q] = (uint32_t)(s + lane);
                 }
-                __syncwarp();
-                F2 acc = f2(0.0f);
-                const int np = (nsv + 1) >> 1;
-                for (int p = 0; p < np; ++p) {
-                    const ulonglong2 u0 = *reinterpret_cast<const ulonglong2*>(&S->xy[p]);
-                    const ulonglong2 u1 = *reinterpret_cast<const ulonglong2*>(&S->zm[p]);
-                    const F2 dx = X - F2{u0.x}, dy = Y - F2{u0.y}, dz = Z - F2{u1.x};
-                    const F2 d2 = fma2(dx, dx, fma2(dy, dy, dz * dz));
-                    const float2 e = upk2(d2.v);
-                    const bool ha = e.x <= U.r2, hb = e.y <= U.r2;
-                    nn += (uint32_t)ha + (uint32_t)hb;
-                    const F2 w = sweep_w<kKern>(c, d2);
-                    acc = fma2(F2{u1.y}, kCut ? keep(ha, hb, w) : w, acc);
-                }
-                const float2 a2 = upk2(acc.v);
-                rk.add(a2.x + a2.y);  // compensated across chunks
+                kept += __popc(surv);
+                if ((kept >> 5) > swept) sweep(32);
             }
         }
+        if (kept > swept * 32) {
+            const int left = kept - swept * 32;
+            if (lane >= left) put((swept & 1) * 32 + lane, kFar, kFar, kFar, 0.0f);
+            sweep(left);
+        }
+        if (b.records) {
+            const bool fits = needed <= room;
+            if (lane == 0) b.tile_list[t] = make_uint2(fits ? region.cur : kNoSlot, needed);
+            if (fits) region.cur += (needed + 31) >> 5;
+        }
         if (valid) {
-            density_out(c, b, i, T.cells, xi.w, rk);
+            density_out(c, b, i, T.cells, o.w, rk);
             my_max = max(my_max, nn);
         }
-        __syncwarp();
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) my_max = max(my_max, __shfl_xor_sync(kFull, my_max, o));
@@ -323,23 +366,21 @@ __global__ void __launch_bounds__(128, 4) k_density_sweep_spread(const StepConst
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
     uint32_t my_max = 0;
-    for (uint32_t t = next_tile(&ds->spread_work[0], lane); t < ntiles;
-         t = next_tile(&ds->spread_work[0], lane)) {
+    const TileQueue queue(&ds->spread_work[0], b.num_sms);
+    for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
-        float4 xi;
+        int i;
+        int4 ct, frame;
+        float4 o;
         bool valid;
-        int4 frame;
-        tile_setup_cells(c, b, g, b.tiles[b.spread_tiles[t]], lane, T, xi, valid, frame);
-        const int i = T.k0 + lane;
-        const int4 ct = valid ? b.cell4_s[i] : frame;
-        const float4 o = valid ? b.pos4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        tile_setup_cells(c, b, g, b.tiles[b.spread_tiles[t]], lane, T, i, ct, o, valid, frame);
         KSum rk;
         uint32_t nn = 0;
         const int nseg = build_segments(b, g, T, lane, S->seg);
         __syncwarp();
         sweep_density_spread<kKern>(c, b, U, S, nseg, lane, valid, ct, spread_off(o, U), rk, nn);
         if (valid) {
-            density_out(c, b, i, T.cells, xi.w, rk);
+            density_out(c, b, i, T.cells, o.w, rk);
             my_max = max(my_max, nn);
         }
         __syncwarp();
@@ -352,25 +393,19 @@ __global__ void __launch_bounds__(128, 4) k_density_sweep_spread(const StepConst
 // ---------------------------------------------------------------------------------------
 // force + acceleration (+ leapfrog + wall clamp when kIntegrate)
 // ---------------------------------------------------------------------------------------
-struct SweepForceSmem {
-    float4 box_lo, box_hi;  // the tile's box (kept here, not in registers, across the sweep)
-    int2 seg[kMaxSegments];
-    float4 xy[16];  // candidates 2p, 2p+1: x, x, y, y (tile frame)
-    float4 zv[16];  // z, z, vx, vx
-    float4 vv[16];  // vy, vy, vz, vz
-    float4 pa[16];  // P, P, kg m/(2 rho), kg m/(2 rho)
-    float2 va[16];  // kl (m/rho) mu, kl (m/rho) mu
+struct SweepForceSmem {  // one chunk of candidates
+    float cx[32], cy[32], cz[32];  // tile frame
+    float vx[32], vy[32], vz[32];
+    float pf[32], cf[32];          // kg m / (2 rho), the same times P
+    int2 seg[kMaxSegments + 1];
 };
-// The spread tiles' launch (sweep_force_spread): candidate j's cell and offset (sweep
-// units) in place of the frame coordinates; zv's z slots unused.
+static_assert(sizeof(SweepForceSmem) % 16 == 0, "per-warp regions stay 16-byte aligned");
+// The spread tiles' launch (sweep_force_spread) stages whole candidates.
 struct SweepForceSpreadSmem {
-    int2 seg[kMaxSegments];
-    int4 scell[32];
-    float4 soff[32];
-    float4 zv[16];
-    float4 vv[16];
-    float4 pa[16];
-    float2 va[16];
+    int2 seg[kMaxSegments + 1];
+    int4 scell[32];   // candidate j of the chunk: its cell
+    float4 soff[32];  // its offset in sweep units, P
+    float4 svel[32];  // its velocity, kg m / (2 rho)
 };
 
 // Pressure and viscosity factors of the kernel: the force on particle t from candidate j is
@@ -388,119 +423,128 @@ __host__ __device__ __forceinline__ float sweep_kl(const StepConst& c) {
     return c.sigma * c.rcp_hsq;
 }
 
-// One packed pair of candidates against the lane's particle; F accumulates.  kMask: zero
-// the terms of non-neighbours by selection (needed when the search radius is below the
-// support, for the Gaussian, and when a staged candidate carries a non-finite velocity or
-// factor, which a zero factor would not cancel).
-// The terms of a candidate pair from the separations x_t - x_j (dx, dy, dz, sweep units)
-// and the candidates' velocities (vx, vy, vz) and factors (P, kg m/(2 rho); va).
-template <int K, bool kMask>
-__device__ __forceinline__ void sweep_force_terms(const SweepUnits& U, F2 dx, F2 dy, F2 dz,
-                                                  F2 VX, F2 VY, F2 VZ, F2 PT, F2 vx, F2 vy,
-                                                  F2 vz, F2 pj, F2 cpf, F2 va, F2& Fx, F2& Fy,
-                                                  F2& Fz) {
-    const F2 d2 = fma2(dx, dx, fma2(dy, dy, dz * dz));
+// The viscosity factor kl (m_j / rho_j) mu is the pressure factor kg m_j / (2 rho_j) times
+// this constant.
+__host__ __device__ __forceinline__ float sweep_kappa(const StepConst& c) {
+    return 2.0f * sweep_kl(c) * c.visc / sweep_kg(c);
+}
+
+// (|r|/h)^2 of a pair is formed with kCoincident added: far below the rounding of any other pair
+__device__ __forceinline__ F2 sweep_d2(const PairLits& k, F2 dx, F2 dy, F2 dz) {
+    return fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, F2{k.coincident})));
+}
+
+// The gradient shape over |r| and the Laplacian shape of two pairs, from their (|r|/h)^2.
+template <int K>
+__device__ __forceinline__ void sweep_shapes(const PairLits& k, const SweepUnits& U, F2 d2, F2& G, F2& L) {
     const float2 e = upk2(d2.v);
-    F2 G, L;
     if (K == SPHX_KERNEL_GAUSSIAN) {
         const F2 ex = f2(exp_approx(-e.x), exp_approx(-e.y));
         G = keep(e.x >= U.skip2, e.y >= U.skip2, ex);
-        L = ex * fma2(d2, f2(2.0f), f2(-3.0f));  // 2 |r|^2 / h^2 - 3
-    } else {
-        // 1/|r| (h units); a coincident pair gets a finite value and q = 0, where the
-        // gradient shapes below are 0
-        const F2 dd = d2 + f2(1e-30f);
-        const float2 de = upk2(dd.v);
-        const F2 R = f2(rsqrt_approx(de.x), rsqrt_approx(de.y));
-        const F2 q = d2 * R;
-        if (K == SPHX_KERNEL_WENDLAND_C2) {
-            const F2 t = max0(fma2(q, f2(-0.5f), f2(1.0f)));
-            const F2 t2 = t * t;
-            G = ((t2 * t) * q) * R;
-            L = t2 * fma2(q, f2(5.0f), f2(-3.0f));
-        } else {
-            const F2 a = max0(f2(2.0f) - q), b2 = max0(fma2(q, f2(-2.0f), f2(2.0f)));  // b2 = 2b
-            G = ((b2 - a) * (b2 + a)) * R;  // 4 b^2 - a^2
-            L = fma2(b2, f2(-2.0f), a);     // a - 4 b
-        }
+        L = ex * fma2(d2, F2{k.two}, F2{k.neg3});  // 2 |r|^2 / h^2 - 3
+        return;
     }
-    F2 cp = (PT + pj) * cpf * G;
-    F2 cv = va * L;
-    F2 dvx = vx - VX, dvy = vy - VY, dvz = vz - VZ;
+    // 1/|r| (h units); a coincident pair (d2 = kCoincident) gets a finite value and q = 1e-15,
+    // where the gradient shapes below are 0
+    const F2 R = f2(rsqrt_approx(e.x), rsqrt_approx(e.y));
+    const F2 q = d2 * R;
+    if (K == SPHX_KERNEL_WENDLAND_C2) {
+        const F2 t = max0(fma2(q, F2{k.neg_half}, F2{k.one}));
+        const F2 t2 = t * t;
+        G = ((t2 * t) * q) * R;
+        L = t2 * fma2(q, F2{k.five}, F2{k.neg3});
+    } else {
+        const F2 a = max0(F2{k.two} - q), b2 = max0(fma2(q, F2{k.neg2}, F2{k.two}));  // b2 = 2b
+        G = ((b2 - a) * (b2 + a)) * R;  // 4 b^2 - a^2
+        L = fma2(b2, F2{k.neg2}, a);     // a - 4 b
+    }
+}
+
+// The terms of two candidates from the separations x_t - x_j (dx, dy, dz, sweep units) and the
+// candidates' velocities and factors (pf = kg m / (2 rho), cf = pf P), added to the packed
+// sums.  kMask: zero the terms of non-neighbours by selection (needed when the search radius
+// is below the support, for the Gaussian, and when a candidate carries a non-finite velocity
+// or factor, which a zero factor would not cancel).
+template <int K, bool kMask>
+__device__ __forceinline__ void sweep_force_terms(const PairLits& k, const SweepUnits& U, F2 kappa, F2 dx, F2 dy,
+                                                  F2 dz, const float4& vt, float Pt, F2 vx, F2 vy,
+                                                  F2 vz, F2 pf, F2 cf, F2& Fx, F2& Fy, F2& Fz) {
+    const F2 d2 = sweep_d2(k, dx, dy, dz);
+    F2 G, L;
+    sweep_shapes<K>(k, U, d2, G, L);
+    F2 cp = fma2(f2(Pt), pf, cf) * G, cv = (pf * kappa) * L;
+    F2 ux = vx - f2(vt.x), uy = vy - f2(vt.y), uz = vz - f2(vt.z);
     if (kMask) {
+        const float2 e = upk2(d2.v);
         const bool ha = e.x <= U.r2, hb = e.y <= U.r2;
         cp = keep(ha, hb, cp);
         cv = keep(ha, hb, cv);
-        dvx = keep(ha, hb, dvx);
-        dvy = keep(ha, hb, dvy);
-        dvz = keep(ha, hb, dvz);
+        ux = keep(ha, hb, ux);
+        uy = keep(ha, hb, uy);
+        uz = keep(ha, hb, uz);
     }
-    Fx = fma2(cv, dvx, fma2(cp, dx, Fx));
-    Fy = fma2(cv, dvy, fma2(cp, dy, Fy));
-    Fz = fma2(cv, dvz, fma2(cp, dz, Fz));
+    Fx = fma2(cv, ux, fma2(cp, dx, Fx));
+    Fy = fma2(cv, uy, fma2(cp, dy, Fy));
+    Fz = fma2(cv, uz, fma2(cp, dz, Fz));
 }
 
-// Staged pair p (candidates 2p, 2p+1, tile frame) against the lane's particle.
+// The staged chunk (nq quads) against the lane's particle.
 template <int K, bool kMask>
-__device__ __forceinline__ void sweep_force_pair(const SweepUnits& U, F2 X, F2 Y, F2 Z, F2 VX,
-                                                 F2 VY, F2 VZ, F2 PT, const SweepForceSmem* S,
-                                                 int p, F2& Fx, F2& Fy, F2& Fz) {
-    const ulonglong2 u0 = *reinterpret_cast<const ulonglong2*>(&S->xy[p]);
-    const ulonglong2 u1 = *reinterpret_cast<const ulonglong2*>(&S->zv[p]);
-    const ulonglong2 u2 = *reinterpret_cast<const ulonglong2*>(&S->vv[p]);
-    const ulonglong2 u3 = *reinterpret_cast<const ulonglong2*>(&S->pa[p]);
-    const F2 va{*reinterpret_cast<const f32x2*>(&S->va[p])};
-    sweep_force_terms<K, kMask>(U, X - F2{u0.x}, Y - F2{u0.y}, Z - F2{u1.x}, VX, VY, VZ, PT,
-                                F2{u1.y}, F2{u2.x}, F2{u2.y}, F2{u3.x}, F2{u3.y}, va, Fx, Fy, Fz);
+__device__ __forceinline__ void sweep_force_chunk(const PairLits& k, const SweepUnits& U, F2 kappa,
+                                                  const SweepForceSmem* S, int nq, F2 X,
+                                                  F2 Y, F2 Z, const float4& vt, float Pt, F2& Fx,
+                                                  F2& Fy, F2& Fz) {
+    auto quad = [&](const float* a, int q) {
+        return reinterpret_cast<const ulonglong2*>(a)[q];
+    };
+#pragma unroll 4
+    for (int q = 0; q < nq; ++q) {
+        const ulonglong2 x = quad(S->cx, q), y = quad(S->cy, q), z = quad(S->cz, q),
+                         vx = quad(S->vx, q), vy = quad(S->vy, q), vz = quad(S->vz, q),
+                         pf = quad(S->pf, q), cf = quad(S->cf, q);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            sweep_force_terms<K, kMask>(k, U, kappa, X - F2{h ? x.y : x.x}, Y - F2{h ? y.y : y.x},
+                                        Z - F2{h ? z.y : z.x}, vt, Pt, F2{h ? vx.y : vx.x},
+                                        F2{h ? vy.y : vy.x}, F2{h ? vz.y : vz.x},
+                                        F2{h ? pf.y : pf.x}, F2{h ? cf.y : cf.x}, Fx, Fy, Fz);
+    }
 }
 
 // The force sweep of a spread tile: every candidate of every chunk against the lane's
 // particle in the lane's own frame (ct, ot), masked by the neighbour test.
 template <int kKern>
-__device__ __forceinline__ void sweep_force_spread(const Buffers& b, const SweepUnits& U, float kg,
-                                                float kl, SweepForceSpreadSmem* S, int nseg,
-                                                int lane, int4 ct, float4 ot, F2 VX, F2 VY,
-                                                F2 VZ, F2 PT,
-                                                KSum& Sx, KSum& Sy, KSum& Sz) {
+__device__ __forceinline__ void sweep_force_spread(const PairLits& k, const Buffers& b, const SweepUnits& U, float kg,
+                                                   F2 kappa, SweepForceSpreadSmem* S, int nseg,
+                                                   int lane, int4 ct, float4 ot, const float4& vt,
+                                                   float Pt, KSum& Sx, KSum& Sy, KSum& Sz) {
     for (int sg = 0; sg < nseg; ++sg) {
         const int2 se = S->seg[sg];
         for (int s = se.x; s < se.y; s += 32) {
             const int m = min(32, se.y - s);
-            int4 cl = ct;
-            float4 ol = make_float4(kFar, kFar, kFar, 0.0f), vl = make_float4(0.f, 0.f, 0.f, 0.f),
-                   al = make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncwarp();
             if (lane < m) {
-                const float4 o = b.pos4_s[s + lane];
-                cl = b.cell4_s[s + lane];
-                ol = spread_off(o, U);
-                vl = b.vel4_s[s + lane];
-                al = b.aux4_s[s + lane];
+                const float4 o = spread_off(b.pos4_s[s + lane], U), v = b.vel4_s[s + lane],
+                             a = b.aux4_s[s + lane];
+                S->scell[lane] = b.cell4_s[s + lane];
+                S->soff[lane] = make_float4(o.x, o.y, o.z, a.y);
+                S->svel[lane] = make_float4(v.x, v.y, v.z, kg * a.z);
+            } else {  // empty slot: far
+                S->scell[lane] = ct;
+                S->soff[lane] = make_float4(kFar, kFar, kFar, 0.0f);
+                S->svel[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
             __syncwarp();
-            {
-                const int p = lane >> 1, h = lane & 1;
-                S->scell[lane] = cl;
-                S->soff[lane] = ol;
-                reinterpret_cast<float*>(&S->zv[p])[2 + h] = vl.x;
-                reinterpret_cast<float*>(&S->vv[p])[h] = vl.y;
-                reinterpret_cast<float*>(&S->vv[p])[2 + h] = vl.z;
-                reinterpret_cast<float*>(&S->pa[p])[h] = al.y;
-                reinterpret_cast<float*>(&S->pa[p])[2 + h] = kg * al.z;
-                reinterpret_cast<float*>(&S->va[p])[h] = kl * al.w;
-            }
-            __syncwarp();
-            F2 Fx = f2(0.0f), Fy = f2(0.0f), Fz = f2(0.0f);
+            F2 Fx = f2(0.0f), Fy = Fx, Fz = Fx;
             for (int j = 0; j < m; j += 2) {
-                const int p = j >> 1;
+                const float4 oa = S->soff[j], ob = S->soff[j + 1];
                 F2 dx, dy, dz;
-                spread_sep(U, ct, ot, S->scell[j], S->soff[j], S->scell[j + 1], S->soff[j + 1],
-                           dx, dy, dz);
-                const ulonglong2 u1 = *reinterpret_cast<const ulonglong2*>(&S->zv[p]);
-                const ulonglong2 u2 = *reinterpret_cast<const ulonglong2*>(&S->vv[p]);
-                const ulonglong2 u3 = *reinterpret_cast<const ulonglong2*>(&S->pa[p]);
-                const F2 va{*reinterpret_cast<const f32x2*>(&S->va[p])};
-                sweep_force_terms<kKern, true>(U, dx, dy, dz, VX, VY, VZ, PT, F2{u1.y}, F2{u2.x},
-                                               F2{u2.y}, F2{u3.x}, F2{u3.y}, va, Fx, Fy, Fz);
+                spread_sep(U, ct, ot, S->scell[j], oa, S->scell[j + 1], ob, dx, dy, dz);
+                const float4 va = S->svel[j], vb = S->svel[j + 1];
+                const F2 pf = f2(va.w, vb.w);
+                sweep_force_terms<kKern, true>(k, U, kappa, dx, dy, dz, vt, Pt, f2(va.x, vb.x),
+                                               f2(va.y, vb.y), f2(va.z, vb.z), pf,
+                                               pf * f2(oa.w, ob.w), Fx, Fy, Fz);
             }
             const float2 fx = upk2(Fx.v), fy = upk2(Fy.v), fz = upk2(Fz.v);
             Sx.add(fx.x + fx.y);
@@ -538,8 +582,12 @@ __device__ __forceinline__ void force_out(const StepConst& c, const Buffers& b, 
     }
 }
 
+// Bound: the FP32 pipe (27 packed instructions of two cycles per pair of candidates, 374 pairs
+// a tile and lane).  1M dam break: 0.82 ms; walking and culling the candidates again instead
+// of reading the density pass's list (1.8 times the instructions) 1.14 ms, sweeping all kept
+// candidates 1.20 ms.
 template <bool kIntegrate, int kKern, bool kCut>
-__global__ void __launch_bounds__(128, 5) k_force_sweep(const StepConst c, const Buffers b,
+__global__ void __launch_bounds__(128, 4) k_force_sweep(const StepConst c, const Buffers b,
                                                         DevState* ds) {
     if (ds->status) return;
     extern __shared__ __align__(16) unsigned char smem_sweep_f[];
@@ -548,105 +596,99 @@ __global__ void __launch_bounds__(128, 5) k_force_sweep(const StepConst c, const
     const uint32_t ntiles = ds->n_tiles;
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
-    const float kg = sweep_kg(c), kl = sweep_kl(c);
-    for (uint32_t t = next_tile(&ds->work[1], lane); t < ntiles; t = next_tile(&ds->work[1], lane)) {
+    const float kg = sweep_kg(c);
+    const F2 kappa = f2(sweep_kappa(c));
+    const TileQueue queue(&ds->work[1], b.num_sms);
+    for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
-        float4 xi;
+        int i;
+        int4 cell, frame;
+        float4 o;
         bool valid;
-        int4 frame;
-        tile_setup_cells(c, b, g, b.tiles[t], lane, T, xi, valid, frame);
-        const int i = T.k0 + lane;
-        if (spread_tile(b, T, i, valid, frame))
+        tile_setup_cells(c, b, g, b.tiles[t], lane, T, i, cell, o, valid, frame);
+        if (spread_tile(T, cell, valid, frame))
             continue;  // listed by the density launch, swept by the spread launch
-        if (valid && T.cells) xi = frame_pos_h(b.cell4_s[i], frame, b.pos4_s[i], U);
-        {
-            const TileBox B = tile_box(xi, valid);
-            if (lane == 0) {
-                S->box_lo = make_float4(B.lo[0], B.lo[1], B.lo[2], 0.0f);
-                S->box_hi = make_float4(B.hi[0], B.hi[1], B.hi[2], 0.0f);
-            }
-        }
-        F2 VX, VY, VZ, PT;
-        {
-            const float4 vi = valid ? b.vel4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float Pi = valid ? b.aux4_s[i].y : 0.0f;
-            VX = f2(vi.x), VY = f2(vi.y), VZ = f2(vi.z), PT = f2(Pi);
-        }
+        const float4 xi = frame_pos_h(cell, frame, o, U);
+        const float4 vi = b.vel4_s[i];
+        const float Pi = b.aux4_s[i].y;
         const F2 X = f2(xi.x), Y = f2(xi.y), Z = f2(xi.z);
-        KSum Sx, Sy, Sz;  // force sums, compensated across chunks
-        const int nseg = build_segments(b, g, T, lane, S->seg);
-        __syncwarp();
-        for (int sg = 0; sg < nseg; ++sg) {
-            const int2 se = S->seg[sg];
-            for (int s = se.x; s < se.y; s += 32) {
-                const bool in = lane < se.y - s;
-                float4 pl = make_float4(kFar, kFar, kFar, 0.0f);
-                if (in) pl = frame_pos_h(b.cell4_s[s + lane], frame, b.pos4_s[s + lane], U);
-                TileBox B;
-                {
-                    const float4 lo = S->box_lo, hi = S->box_hi;
-                    B.lo[0] = lo.x, B.lo[1] = lo.y, B.lo[2] = lo.z;
-                    B.hi[0] = hi.x, B.hi[1] = hi.y, B.hi[2] = hi.z;
+        KSum Sx, Sy, Sz;  // force sums, compensated
+        // a candidate as loaded, and how a chunk of them is staged and swept (`left` of them in
+        // lane order; an empty lane's has no factor and lies far away)
+        struct Cand {
+            int4 cell;
+            float4 o, v, a;
+        };
+        const Cand empty{frame, make_float4(kFar, kFar, kFar, 0.0f),
+                         make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        auto load = [&](bool has, uint32_t j) {
+            Cand d = empty;
+            if (has) {
+                d.cell = b.cell4_s[j];
+                d.o = b.pos4_s[j];
+                d.v = b.vel4_s[j];
+                d.a = b.aux4_s[j];
+            }
+            return d;
+        };
+        auto stage = [&](const Cand& d) {  // returns whether the chunk needs the masked sweep
+            const float4 x = frame_pos_h(d.cell, frame, d.o, U);
+            const float pf = kg * d.a.z;
+            __syncwarp();  // the previous chunk's reads are done
+            S->cx[lane] = x.x;
+            S->cy[lane] = x.y;
+            S->cz[lane] = x.z;
+            S->vx[lane] = d.v.x;
+            S->vy[lane] = d.v.y;
+            S->vz[lane] = d.v.z;
+            S->pf[lane] = pf;
+            S->cf[lane] = pf * d.a.y;
+            __syncwarp();
+            // a non-finite velocity or factor is not cancelled by a zero factor
+            return kCut || __any_sync(kFull, !isfinite(d.v.x + d.v.y + d.v.z + d.a.y + pf));
+        };
+        auto sweep = [&](bool masked, int left) {
+            F2 Fx = f2(0.0f), Fy = Fx, Fz = Fx;
+            const int nq = (left + 3) >> 2;
+            if (masked) sweep_force_chunk<kKern, true>(c.lit, U, kappa, S, nq, X, Y, Z, vi, Pi, Fx, Fy, Fz);
+            else sweep_force_chunk<kKern, false>(c.lit, U, kappa, S, nq, X, Y, Z, vi, Pi, Fx, Fy, Fz);
+            const float2 fx = upk2(Fx.v), fy = upk2(Fy.v), fz = upk2(Fz.v);
+            Sx.add(fx.x + fx.y);  // compensated across chunks
+            Sy.add(fy.x + fy.y);
+            Sz.add(fz.x + fz.y);
+        };
+        // the candidates that some lane needs, listed by the density pass: positions read two
+        // chunks ahead, their data one
+        const uint2 list = b.records ? b.tile_list[t] : make_uint2(kNoSlot, 0u);
+        if (list.x != kNoSlot) {
+            const uint32_t* p = b.records + (size_t)list.x * 32;
+            const uint32_t n = list.y;
+            auto at = [&](uint32_t q) { return q < n ? __ldcs(p + q) : 0u; };
+            Cand d = load((uint32_t)lane < n, at(lane));
+            uint32_t j = at(32 + lane);
+            for (uint32_t q = 0; q < n; q += 32) {
+                const bool masked = stage(d);
+                d = load(q + 32 + lane < n, j);
+                j = at(q + 64 + lane);
+                sweep(masked, (int)min(32u, n - q));
+            }
+        } else {  // no list: every chunk of the walk that the tile's box reaches
+            const TileBox B = tile_box(xi, valid);
+            __syncwarp();  // the previous tile's segments are read
+            const int nseg = build_segments(b, g, T, lane, S->seg);
+            __syncwarp();
+            for (int sg = 0; sg < nseg; ++sg) {
+                const int2 se = S->seg[sg];
+                for (int s = se.x; s < se.y; s += 32) {
+                    const bool in = lane < se.y - s;
+                    const Cand d = load(in, (uint32_t)(s + lane));
+                    const bool near = in && box_near(B, frame_pos_h(d.cell, frame, d.o, U), U.r2m);
+                    if (__any_sync(kFull, near)) sweep(stage(d), min(32, se.y - s));
                 }
-                const uint32_t surv = __ballot_sync(kFull, in && box_near(B, pl, U.r2m));
-                if (!surv) continue;
-                const int nsv = __popc(surv);
-                const bool mine = (surv >> lane) & 1u;
-                float4 vl = make_float4(0.f, 0.f, 0.f, 0.f), al = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (mine) {
-                    vl = b.vel4_s[s + lane];
-                    al = b.aux4_s[s + lane];
-                }
-                const float cpf = kg * al.z, cvf = kl * al.w;
-                // a non-finite velocity or factor is not cancelled by a zero factor: such a
-                // chunk takes the masked sweep
-                const bool odd = !isfinite(vl.x + vl.y + vl.z + al.y + cpf + cvf);
-                const bool masked = kCut || __any_sync(kFull, odd);
-                __syncwarp();  // the previous chunk's reads are done
-                // survivors packed to slots 0 .. nsv-1; an odd count is padded with an empty
-                // slot (written by lane 0 besides its own)
-                auto put = [&](int k, const float4& x, const float4& v, const float4& a3) {
-                    const int p = k >> 1, h = k & 1;
-                    float* xy = reinterpret_cast<float*>(&S->xy[p]);
-                    float* zv = reinterpret_cast<float*>(&S->zv[p]);
-                    float* vv = reinterpret_cast<float*>(&S->vv[p]);
-                    float* pa = reinterpret_cast<float*>(&S->pa[p]);
-                    float* va = reinterpret_cast<float*>(&S->va[p]);
-                    xy[h] = x.x;
-                    xy[2 + h] = x.y;
-                    zv[h] = x.z;
-                    zv[2 + h] = v.x;
-                    vv[h] = v.y;
-                    vv[2 + h] = v.z;
-                    pa[h] = a3.x;
-                    pa[2 + h] = a3.y;
-                    va[h] = a3.z;
-                };
-                if (mine)
-                    put(__popc(surv & ((1u << lane) - 1u)), pl, vl, make_float4(al.y, cpf, cvf, 0.f));
-                if (lane == 0 && (nsv & 1)) {
-                    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-                    put(nsv, make_float4(kFar, kFar, kFar, 0.0f), z, z);
-                }
-                __syncwarp();
-                F2 Fx = f2(0.0f), Fy = f2(0.0f), Fz = f2(0.0f);
-                const int np = (nsv + 1) >> 1;
-                if (masked) {
-                    for (int p = 0; p < np; ++p)
-                        sweep_force_pair<kKern, true>(U, X, Y, Z, VX, VY, VZ, PT, S, p, Fx, Fy, Fz);
-                } else {
-                    for (int p = 0; p < np; ++p)
-                        sweep_force_pair<kKern, false>(U, X, Y, Z, VX, VY, VZ, PT, S, p, Fx, Fy, Fz);
-                }
-                const float2 fx = upk2(Fx.v), fy = upk2(Fy.v), fz = upk2(Fz.v);
-                Sx.add(fx.x + fx.y);
-                Sy.add(fy.x + fy.y);
-                Sz.add(fz.x + fz.y);
             }
         }
-        __syncwarp();
         if (!valid) continue;
-        force_out<kIntegrate>(c, b, ds, i, xi.w, Sx, Sy, Sz);
+        force_out<kIntegrate>(c, b, ds, i, o.w, Sx, Sy, Sz);
     }
 }
 
@@ -661,31 +703,24 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep_spread(const StepConst c
     const uint32_t ntiles = ds->n_spread;
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
-    const float kg = sweep_kg(c), kl = sweep_kl(c);
-    for (uint32_t t = next_tile(&ds->spread_work[1], lane); t < ntiles;
-         t = next_tile(&ds->spread_work[1], lane)) {
+    const float kg = sweep_kg(c);
+    const F2 kappa = f2(sweep_kappa(c));
+    const TileQueue queue(&ds->spread_work[1], b.num_sms);
+    for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
-        float4 xi;
+        int i;
+        int4 ct, frame;
+        float4 o;
         bool valid;
-        int4 frame;
-        tile_setup_cells(c, b, g, b.tiles[b.spread_tiles[t]], lane, T, xi, valid, frame);
-        const int i = T.k0 + lane;
-        const int4 ct = valid ? b.cell4_s[i] : frame;
-        const float4 o = valid ? b.pos4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        F2 VX, VY, VZ, PT;
-        {
-            const float4 vi = valid ? b.vel4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float Pi = valid ? b.aux4_s[i].y : 0.0f;
-            VX = f2(vi.x), VY = f2(vi.y), VZ = f2(vi.z), PT = f2(Pi);
-        }
+        tile_setup_cells(c, b, g, b.tiles[b.spread_tiles[t]], lane, T, i, ct, o, valid, frame);
         KSum Sx, Sy, Sz;
         const int nseg = build_segments(b, g, T, lane, S->seg);
         __syncwarp();
-        sweep_force_spread<kKern>(b, U, kg, kl, S, nseg, lane, ct, spread_off(o, U), VX, VY, VZ,
-                                  PT, Sx, Sy, Sz);
+        sweep_force_spread<kKern>(c.lit, b, U, kg, kappa, S, nseg, lane, ct, spread_off(o, U),
+                                  b.vel4_s[i], b.aux4_s[i].y, Sx, Sy, Sz);
         __syncwarp();
         if (!valid) continue;
-        force_out<kIntegrate>(c, b, ds, i, xi.w, Sx, Sy, Sz);
+        force_out<kIntegrate>(c, b, ds, i, o.w, Sx, Sy, Sz);
     }
 }
 
@@ -696,6 +731,13 @@ void launch_sweep(const LaunchCtx& L, LaunchShapeCache& cache, K kernel, size_t 
     const size_t sm = (size_t)L.warps_per_block * smem_per_warp;
     const int nb = cached_resident_blocks(cache, L, kernel, threads, sm);
     kernel<<<nb, threads, sm, L.stream>>>(c, b, ds);
+}
+
+// the max form zeroes every pair beyond the support 2h; a search radius below it needs the
+// neighbour test (the Gaussian has no compact support)
+template <int kKern>
+bool cut(const StepConst& c) {
+    return kKern == SPHX_KERNEL_GAUSSIAN || c.r2 < 4.0f * c.h_sq;
 }
 
 template <int kKern, bool kCut>
@@ -710,10 +752,8 @@ void launch_density_sweep_v(const LaunchCtx& L, const StepConst& c, const Buffer
 template <int kKern>
 void launch_density_sweep_k(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                             DevState* ds) {
-    if (kKern == SPHX_KERNEL_GAUSSIAN || c.r2 < 4.0f * c.h_sq)
-        launch_density_sweep_v<kKern, true>(L, c, b, ds);
-    else
-        launch_density_sweep_v<kKern, false>(L, c, b, ds);
+    if (cut<kKern>(c)) launch_density_sweep_v<kKern, true>(L, c, b, ds);
+    else launch_density_sweep_v<kKern, false>(L, c, b, ds);
 }
 
 template <bool kIntegrate, int kKern, bool kCut>
@@ -729,14 +769,12 @@ void launch_force_sweep_v(const LaunchCtx& L, const StepConst& c, const Buffers&
 template <int kKern>
 void launch_force_sweep_k(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                           DevState* ds, int integrate) {
-    // the max form zeroes every pair beyond the support 2h; a search radius below it needs
-    // the neighbour test (the Gaussian has no compact support)
-    const bool cut = kKern == SPHX_KERNEL_GAUSSIAN || c.r2 < 4.0f * c.h_sq;
+    const bool k = cut<kKern>(c);
     if (integrate) {
-        if (cut) launch_force_sweep_v<true, kKern, true>(L, c, b, ds);
+        if (k) launch_force_sweep_v<true, kKern, true>(L, c, b, ds);
         else launch_force_sweep_v<true, kKern, false>(L, c, b, ds);
     } else {
-        if (cut) launch_force_sweep_v<false, kKern, true>(L, c, b, ds);
+        if (k) launch_force_sweep_v<false, kKern, true>(L, c, b, ds);
         else launch_force_sweep_v<false, kKern, false>(L, c, b, ds);
     }
 }
