@@ -92,3 +92,28 @@ def test_fields_bit_identical(port, name, kernel):
                            (out["acc"], acc, "acc")):
         assert O.bits_equal(got, want), O.mismatch_report(got, want, key)
     ctx.close()
+
+
+@pytest.mark.parametrize("name", ["faces", "wide_stencil", "large_cells", "tiny_radius", "folded"])
+def test_grid_query_lists_match_the_reference_walk(port, name):
+    """The query's cell culling and ranked writes: every particle's list, in order."""
+    rng = np.random.default_rng(11)
+    cell, radius = {"faces": (0.03125, 0.03125), "wide_stencil": (0.013, 0.04),
+                    "large_cells": (0.1, 0.04), "tiny_radius": (0.04, 1e-6),
+                    "folded": (0.04, 0.04)}[name]
+    if name == "faces":  # points on cell faces, many pairs at the radius exactly
+        k = np.arange(16, dtype=np.float32) * np.float32(0.015625) - np.float32(0.125)
+        pos = np.stack(np.meshgrid(k, k, k, indexing="ij"), -1).reshape(-1, 3)
+    elif name == "folded":  # clusters far apart: the box has far more cells than the grid
+        centre = (2e3 * rng.standard_normal((40, 1, 3))).astype(np.float32)
+        pos = (centre + 0.05 * rng.random((40, 60, 3))).astype(np.float32).reshape(-1, 3)
+    else:
+        pos = I.lattice(16, 16, 16, seed=12)
+        pos[7::7] = pos[1::7][: len(pos[7::7])]  # coincident points
+    g = sphx.Grid(len(pos))
+    g.build(pos, cell)
+    r = np.float32(radius)
+    counts, idx = g.query(pos, float(r * r))
+    want_counts, want_idx = port.query(pos, radius, cell_size=cell)
+    assert np.array_equal(counts, want_counts) and np.array_equal(idx, want_idx)
+    g.close()
