@@ -74,7 +74,8 @@ typedef struct sphx_params {
 
 typedef struct sphx_tuning {
     int mode;              /* SPHX_MODE_* (default EXACT) */
-    int warps_per_block;   /* neighbour-pass CTA size in warps; 0 = default (4) */
+    int warps_per_block;   /* neighbour-pass CTA size in warps; 0 = default (4); not used by
+                              the passes on tiles of up to 8 particles, one CTA per SM */
     int blocks_per_sm;     /* persistent CTAs per SM for the neighbour passes; 0 = auto */
     int64_t max_grid_cells;/* cap on the dense cell grid (cells), >= 125; a larger box of
                               occupied cells is folded per axis; 0 = default */
@@ -82,7 +83,8 @@ typedef struct sphx_tuning {
     int graph;             /* 1 = run steps as a captured CUDA graph (recaptured when n,
                               dt, parameters or scenes change) */
     int tile_particles;    /* particles of one cell column per warp work item (tile), 1..32;
-                              0 = default (32) */
+                              0 = chosen by the set's size (8 up to 65,536 particles in exact
+                              mode, else 32; reported as 32) */
     int bulk_copy;         /* accepted and reported back; the force pass stages its candidates
                               by asynchronous copies whatever its value */
 } sphx_tuning;

@@ -53,6 +53,7 @@ struct sphx_ctx {
     uint64_t graph_version = ~0ull;
     float graph_dt = 0.0f;
     int graph_launches = 0;
+    bool tile_auto = false;  // tile size left to pass_tile
     uint64_t version = 0;  // bumped by every change the graph depends on
     // headless rendering: colour staging, instance buffer, depth keys and image
     float* r_colors = nullptr;
@@ -352,6 +353,7 @@ int run_phases(sphx_ctx* c, float dt, bool integrate) {
         SPHX_CUDA(cudaEventRecord(slot->ev[0], c->stream));
     }
     const bool batch = c->b.nscenes > 0;
+    if (c->tile_auto) c->b.tile_n = pass_tile((int)c->n, c->sc.precise && !batch);
     if (batch) {  // the passes' kernels serve all scenes
         c->sc.div_nz = c->scenes_div_nz ? 1 : 0;
         c->sc.force_nz = c->scenes_force_nz ? 1 : 0;
@@ -644,8 +646,8 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     }
     if (c->tuning.warps_per_block <= 0 || c->tuning.warps_per_block > 4)
         c->tuning.warps_per_block = kDefaultWarpsPerBlock;
-    if (c->tuning.tile_particles <= 0 || c->tuning.tile_particles > kTile)
-        c->tuning.tile_particles = kTile;
+    c->tile_auto = c->tuning.tile_particles <= 0 || c->tuning.tile_particles > kTile;
+    if (c->tile_auto) c->tuning.tile_particles = kTile;
     c->b.tile_n = c->tuning.tile_particles;
     c->b.columns = 1;
     c->tuning.bulk_copy = c->tuning.bulk_copy ? 1 : 0;
@@ -696,10 +698,13 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     // Record pool (Buffers::records): 4 records (128 B each) per particle of capacity.  The
     // lattice and uniform states need about 2 per particle in exact mode (32-particle tiles,
     // the candidates their boxes keep) and 1 in the precision mode; the rest is room for
-    // denser states and for the uneven split of tiles over the warps.  Without the pool (or
+    // denser states and for the uneven split of tiles over the warps.  The small sets' lists
+    // (270 neighbours of 4 bytes a particle) take 8.5, so up to that size 12 are held.  Without the pool (or
     // where a warp's region runs out) the force pass walks the candidates itself.
     if (dmalloc(&b.tile_list, C) == SPHX_OK) {
-        unsigned long long cap = 4ull * C;
+        unsigned long long cap = std::max<unsigned long long>(
+            4ull * C, c->tuning.mode != SPHX_MODE_EXACT
+                          ? 0ull : 12ull * std::min<unsigned long long>(C, kTeamMax));
         if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
         if (dmalloc(&b.records, (size_t)cap * 32) == SPHX_OK) {
             b.record_cap = cap;
@@ -1050,10 +1055,12 @@ int sphx_autotune(sphx_ctx* c, float dt, int* warps_per_block, int* blocks_per_s
     // then the tile size at the chosen launch shape
     c->L.warps_per_block = bw;
     c->L.blocks_per_sm = bb;
-    int bt = c->b.tile_n;
+    int bt = c->tuning.tile_particles;
+    const bool was_auto = c->tile_auto;
     const int tiles[] = {16, 24};
     for (const int tn : tiles) {
         if (rc) break;
+        c->tile_auto = false;
         c->b.tile_n = tn;
         if ((rc = reset()) || (rc = run_phases(c, dt, true))) break;  // warm-up
         if ((rc = reset())) break;
@@ -1070,6 +1077,7 @@ int sphx_autotune(sphx_ctx* c, float dt, int* warps_per_block, int* blocks_per_s
             bt = tn;
         }
     }
+    c->tile_auto = was_auto && bt == c->tuning.tile_particles;
     c->b.tile_n = bt;
     c->tuning.tile_particles = bt;
     cudaEventDestroy(e0);

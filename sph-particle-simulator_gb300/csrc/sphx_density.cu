@@ -180,9 +180,11 @@ static void launch_density_k(const LaunchCtx& L, const StepConst& c, const Buffe
     else launch_density_t<false, kKern, false>(L, c, b, ds);
 }
 
-// Precision mode (single scene) runs the tile sweep (sphx_sweep.cu); exact mode k_density.
+// Precision mode (single scene) runs the tile sweep (sphx_sweep.cu); exact mode k_density, or on
+// tiles of at most 8 particles (small sets: pass_tile) k_density_team.
 int launch_density(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds) {
     if (c.precise && b.nscenes == 0) return launch_density_sweep(L, c, b, ds);
+    if (b.tile_n <= kTeamTile) return launch_density_team(L, c, b, ds);
     if (c.kern == SPHX_KERNEL_WENDLAND_C2) launch_density_k<SPHX_KERNEL_WENDLAND_C2>(L, c, b, ds);
     else if (c.kern == SPHX_KERNEL_GAUSSIAN) launch_density_k<SPHX_KERNEL_GAUSSIAN>(L, c, b, ds);
     else launch_density_k<SPHX_KERNEL_CUBIC_SPLINE>(L, c, b, ds);

@@ -11,6 +11,9 @@ namespace sphx {
 
 constexpr int kWarp = 32;
 constexpr int kTile = 32;              // particles of one cell handled by one warp
+constexpr int kTeam = 4;                // lanes per particle of the small sets' exact passes
+constexpr int kTeamTile = kWarp / kTeam;
+constexpr int kTeamMax = 1 << 16, kTeamMaxDensity = 40000;  // see pass_tile
 constexpr int kRadixBits = 8;
 constexpr int kRadixBuckets = 1 << kRadixBits;
 constexpr int kRadixThreads = 256;
@@ -172,10 +175,11 @@ struct Buffers {
     // What the density pass tells the force pass of the same step about each tile, in records
     // of 32 words: exact mode, per chunk of 32 candidates that the tile's box keeps their
     // sorted positions and the lanes' neighbour masks (word = lane: bit 31 - j set if the j-th
-    // of them is a neighbour of the lane's particle); precision mode, the sorted positions of
-    // the kept candidates that are a neighbour of some lane.  Every warp of the density grid
+    // of them is a neighbour of the lane's particle), on tiles of up to 8 the neighbours
+    // themselves, rows of 16 per particle (4 records: sphx_team.cuh); precision mode, the
+    // sorted positions of the kept candidates that are a neighbour of some lane.  Every warp of the density grid
     // owns an equal region of the pool and stores its tiles one after another; tile_list[t] =
-    // first record and candidates, or kNoSlot when the tile did not fit in what was left of
+    // first record and candidates (or rows), or kNoSlot when the tile did not fit in what was left of
     // the region (the force pass then walks and tests that tile itself).
     uint32_t* records = nullptr;
     uint2* tile_list = nullptr;
@@ -548,6 +552,14 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src)
                  : "memory");
 }
+// closes a group of this thread's copies; waits until at most N groups are outstanding
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 // waits for this thread's copies
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -597,6 +609,18 @@ int launch_grid_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, 
 int launch_density(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds);
 int launch_force(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
                   int integrate);
+// Particles per tile where the caller leaves the choice: the exact passes take tiles of 8, four
+// lanes a particle, on sets too small to fill the GPU with a lane per particle.  Density +
+// force with tiles of 8 and of 32, lattice, us: 4k 45 and 122, 10k 57 and 133, 33k 138 and
+// 179, 47k 178 and 199, 64k 234 and 243; the density pass alone, which has no list to gain
+// by: 22k 55 and 77, 33k 73 and 79, 47k 94 and 91, 64k 122 and 105.
+inline int pass_tile(int n, bool precise, bool density_only = false) {
+    return !precise && n <= (density_only ? kTeamMaxDensity : kTeamMax) ? kTeamTile : kTile;
+}
+// the same passes with four lanes per particle (sphx_team_density.cu, sphx_team_force.cu)
+int launch_density_team(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds);
+int launch_force_team(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
+                      int integrate);
 int launch_diag(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds);
 // precision mode (single scene): the tile-sweep passes (sphx_sweep.cu)
 int launch_density_sweep(const LaunchCtx& L, const StepConst& c, const Buffers& b,

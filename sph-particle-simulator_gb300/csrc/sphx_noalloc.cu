@@ -156,6 +156,7 @@ extern "C" int sphx_density_noalloc(const sphx_params* p, size_t n, const float*
     b.tiles = reinterpret_cast<uint2*>(base + kOffTiles);
     b.tgt = reinterpret_cast<uint32_t*>(base + kOffTgt);
     b.columns = 1;
+    b.tile_n = pass_tile((int)n, false, true);
     b.off = reinterpret_cast<uint32_t*>(base + kOffOff);
     set_grid_scratch(b, base + kOffGrid);
     b.diag_part = nullptr;

@@ -499,6 +499,26 @@ __device__ __forceinline__ F2 pair_w_exact2(const PairLits& k, const PairConst& 
     return F2{c.sigma} * select2(u.x <= 1.0f, u.y <= 1.0f, w1, w2);
 }
 
+// integrate_leapfrog and the wall clamp (sph_engine.cpp:290-310, particle.cpp:122-153)
+__device__ __forceinline__ void leapfrog_exact(const StepConst& c, float dt, const float* acc,
+                                               float* x, float* v) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float half = xmul(xmul(0.5f, acc[a]), dt);
+        float vv = xadd(v[a], half);
+        x[a] = xadd(x[a], xmul(vv, dt));
+        vv = xadd(vv, half);
+        v[a] = xmul(vv, c.damping);
+        if (x[a] < c.lo[a]) {
+            x[a] = c.lo[a];
+            v[a] = xmul(v[a], -0.8f);
+        } else if (x[a] > c.hi[a]) {
+            x[a] = c.hi[a];
+            v[a] = xmul(v[a], -0.8f);
+        }
+    }
+}
+
 // Precision-mode leapfrog + wall clamp on cell + offset positions (FP64 clamp).
 __device__ __forceinline__ void integrate_cells(const StepConst& c, float dt, const float* acc,
                                                 float* o, float* v, int4& cell) {

@@ -94,6 +94,36 @@ def test_fields_bit_identical(port, name, kernel):
     ctx.close()
 
 
+@pytest.mark.parametrize("kernel", [sphx.KERNEL_CUBIC_SPLINE, sphx.KERNEL_GAUSSIAN])
+@pytest.mark.parametrize("name", ["thirty_three", "clump", "crowd"])
+@pytest.mark.parametrize("tile", [1, 8, 9, 32])
+def test_tile_sizes_bit_identical(built, port, tile, name, kernel):
+    """Both forms of the exact passes (four lanes per particle up to tiles of 8, one above), and
+    tiles whose neighbours do not fit in what the density pass leaves for the force pass."""
+    if name == "crowd":  # everything within reach of everything
+        rng = np.random.default_rng(21)
+        pos = (0.05 + 0.02 * rng.random((2500, 3))).astype(np.float32)
+        vel = (0.1 * rng.standard_normal(pos.shape)).astype(np.float32)
+        mass, prm = np.full(len(pos), 1e-3, np.float32), I.params16(gas_constant=2e-3)
+    else:
+        pos, vel, mass, prm = state(name)
+    def fields(t):
+        ctx = sphx.Context(len(pos), tile_particles=t)
+        ctx.set_params(prm)
+        ctx.set_kernel(kernel)
+        ctx.upload(pos, vel, mass)
+        ctx.eval()
+        out = ctx.download()
+        ctx.close()
+        return out["rho"], out["pressure"], out["acc"]
+
+    # the Gaussian's exp is CUDA's, not the host's: there the two forms are compared
+    want = (port.fields(pos, vel, mass, prm, kernel=kernel)
+            if kernel != sphx.KERNEL_GAUSSIAN else fields(32))
+    for g, w, key in zip(fields(tile), want, ("rho", "P", "acc")):
+        assert O.bits_equal(g, w), O.mismatch_report(g, w, key)
+
+
 @pytest.mark.parametrize("name", ["faces", "wide_stencil", "large_cells", "tiny_radius", "folded"])
 def test_grid_query_lists_match_the_reference_walk(port, name):
     """The query's cell culling and ranked writes: every particle's list, in order."""
