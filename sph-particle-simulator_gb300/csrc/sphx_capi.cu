@@ -364,8 +364,7 @@ int run_phases(sphx_ctx* c, float dt, bool integrate) {
         k += launch_batch_prepare(c->L, c->b, c->ds, (int)c->n, how, dt, c->sc.max_cells);
         k += launch_batch_grid(c->L, c->b, c->ds, (int)c->n);
     } else {
-        k += launch_prepare(c->L, c->sc, c->b, c->ds, how, dt);
-        k += launch_build_grid(c->L, c->sc, c->b, c->ds);
+        k += launch_grid(c->L, c->sc, c->b, c->ds, how, dt);
     }
     if (slot) SPHX_CUDA(cudaEventRecord(slot->ev[1], c->stream));
     k += launch_density(c->L, c->sc, c->b, c->ds);
@@ -1365,8 +1364,7 @@ int sphx_debug_pairs(sphx_ctx* c, int64_t* counts, int64_t* idx, size_t* total_i
     Buffers bq = c->b;
     bq.columns = 0;
     bq.tgt = nullptr;
-    launch_prepare(c->L, c->sc, bq, c->ds, kNoStep, 0.0f);
-    launch_build_grid(c->L, c->sc, bq, c->ds);
+    launch_grid(c->L, c->sc, bq, c->ds, kNoStep, 0.0f);
     uint32_t* d_cnt = nullptr;
     if ((rc = dmalloc(&d_cnt, n))) return rc;
     launch_pair_counts(c->L, c->sc, bq, c->ds, d_cnt);
@@ -1428,8 +1426,7 @@ int sphx_debug_pairs_subset(sphx_ctx* c, size_t nsel, const int64_t* sel, int64_
     Buffers bq = c->b;
     bq.columns = 0;
     bq.tgt = nullptr;
-    launch_prepare(c->L, c->sc, bq, c->ds, kNoStep, 0.0f);
-    launch_build_grid(c->L, c->sc, bq, c->ds);
+    launch_grid(c->L, c->sc, bq, c->ds, kNoStep, 0.0f);
     uint32_t* d_cnt = nullptr;
     if ((rc = dmalloc(&d_cnt, n))) return rc;
     launch_pair_counts(c->L, c->sc, bq, c->ds, d_cnt);

@@ -12,7 +12,7 @@
 // of the sorted arrays.  Particles with a NaN/inf coordinate get key == ncells: they sort
 // last and are never anyone's neighbour (every distance test with them fails in the
 // reference too).
-#include "sphx_internal.cuh"
+#include "sphx_grid.cuh"
 
 namespace sphx {
 
@@ -24,168 +24,24 @@ static inline int grid_blocks(const LaunchCtx& L, int n, int threads, int per_sm
 
 // ---- the step's first kernel --------------------------------------------------------------
 
-// Grid extent.  The occupied-cell box is laid out densely when it has at most max_cells
-// cells.  Otherwise (particles spread over a huge box) every axis longer than F =
-// floor(cbrt(max_cells)) >= 256 cells is folded: its cell index is taken modulo F.  Cells
-// that fold onto each other are at least F - 2 cells apart, so a candidate from a folded
-// neighbour fails the distance test; sets and visiting order are unchanged, only the
-// number of candidates grows.
-__device__ void grid_setup(int n, uint32_t max_cells, DevState* ds) {
-    if ((int)ds->nonfinite >= n) {  // no finite particle: a one-cell grid, all keys sentinel
-        for (int a = 0; a < 3; ++a) {
-            ds->cmin[a] = 0;
-            ds->cmax[a] = 0;
-        }
-    }
-    long long d[3];
-    unsigned long long cells = 1;
-    bool fits = true;
-    for (int a = 0; a < 3; ++a) {
-        d[a] = (long long)ds->cmax[a] - (long long)ds->cmin[a] + 1;
-        if (d[a] > (long long)max_cells) fits = false;
-        else if ((cells *= (unsigned long long)d[a]) > (unsigned long long)max_cells) fits = false;
-    }
-    long long fold = 1;
-    if (!fits) {
-        while ((fold + 1) * (fold + 1) * (fold + 1) <= (long long)max_cells) ++fold;
-    }
-    cells = 1;
-    for (int a = 0; a < 3; ++a) {
-        const bool w = !fits && d[a] > fold;
-        ds->wrap[a] = w ? 1 : 0;
-        ds->dim[a] = (int)(w ? fold : d[a]);
-        cells *= (unsigned long long)ds->dim[a];
-    }
-    ds->ncells = (uint32_t)cells;
-    const int bits = 32 - __clz(ds->ncells);  // key range is [0, ncells]
-    ds->passes = (uint32_t)((bits + kRadixBits - 1) / kRadixBits);
-}
-
-// dt of the step, then current_time_ += dt; precision mode: the same rule and the time in FP64.
-__device__ void set_dt(const StepConst& c, DevState* ds, int how, float host_dt,
-                       unsigned long long vmax) {
-    if (!c.precise) {
-        // (a NaN dt is used as given, like SPHEngine::step, cpp:99-101)
-        const float dt = how == kCflDt ? cfl_dt(c, __uint_as_float((uint32_t)vmax), ds->a0)
-                                       : host_dt;
-        ds->dt = dt;
-        ds->time = xadd(ds->time, dt);
-        return;
-    }
-    double dt = host_dt;
-    if (how == kCflDt) {
-        const double vm = __longlong_as_double((long long)vmax);
-        const double cfl = c.cfl, h = c.h;
-        const double dt_cfl = cfl * h / (vm + 1e-6);
-        const double a0 = sqrt((double)ds->a0[0] * ds->a0[0] + (double)ds->a0[1] * ds->a0[1] +
-                               (double)ds->a0[2] * ds->a0[2]);
-        const double dt_force = cfl * sqrt(h / (a0 + 1e-6));
-        dt = dt_cfl;
-        if (dt_force < dt) dt = dt_force;
-        if ((double)c.timestep < dt) dt = c.timestep;
-    }
-    ds->dt64 = dt;
-    ds->time64 += dt;
-    ds->dt = (float)dt;
-    ds->time = (float)ds->time64;
-}
-
-__device__ __forceinline__ PrepPart prep_empty() {
-    PrepPart p;
-    for (int a = 0; a < 3; ++a) {
-        p.mn[a] = 0x7fffffff;
-        p.mx[a] = -0x7fffffff - 1;
-    }
-    p.bad = p.general = 0;
-    p.vmax = 0;
-    return p;
-}
-__device__ __forceinline__ void merge(PrepPart& p, const PrepPart& q) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        p.mn[a] = min(p.mn[a], q.mn[a]);
-        p.mx[a] = max(p.mx[a], q.mx[a]);
-    }
-    p.bad += q.bad;
-    p.general |= q.general;
-    p.vmax = max(p.vmax, q.vmax);
-}
-__device__ __forceinline__ PrepPart merge_block(PrepPart p) {
-    __shared__ PrepPart part[kPrepThreads / 32];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        PrepPart q;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            q.mn[a] = __shfl_xor_sync(0xffffffffu, p.mn[a], o);
-            q.mx[a] = __shfl_xor_sync(0xffffffffu, p.mx[a], o);
-        }
-        q.bad = __shfl_xor_sync(0xffffffffu, p.bad, o);
-        q.general = __shfl_xor_sync(0xffffffffu, p.general, o);
-        q.vmax = __shfl_xor_sync(0xffffffffu, p.vmax, o);
-        merge(p, q);
-    }
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = p;
-    __syncthreads();
-    p = part[0];
-    for (int w = 1; w < kPrepThreads / 32; ++w) merge(p, part[w]);
-    return p;
-}
-
 // Box of occupied cells, non-finite count and max |v| over the particles: per-block partials,
 // joined by the block that finishes last, which then lays out the grid and sets dt (one
 // launch where a reset, two reductions by atomics and two one-thread kernels were five: 1M
-// particles 0.036 -> 0.011 ms, 10k 0.012 -> 0.007).  kCells (precision mode): the stored cells.  kVmax: NaN
-// lengths are ignored, as std::max(m, v) keeps m when v is NaN (sph_engine.cpp:316-322);
-// non-negative floats order like their bit patterns.
+// particles 0.036 -> 0.011 ms, 10k 0.012 -> 0.007).
 template <bool kCells, bool kVmax>
 __global__ void __launch_bounds__(kPrepThreads) k_prepare(const StepConst c, const Buffers b,
                                                           DevState* ds, int how, float host_dt) {
     PrepPart p = prep_empty();
     const int n = c.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (kVmax) {
-            const float4 v = b.vel4[i];
-            if (kCells) {
-                const double len = sqrt((double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z);
-                if (!isnan(len)) p.vmax = max(p.vmax, (unsigned long long)__double_as_longlong(len));
-            } else {
-                const float len = xsqrt(xdot3(v.x, v.y, v.z));
-                if (!isnan(len)) p.vmax = max(p.vmax, (unsigned long long)__float_as_uint(len));
-            }
-        }
-        int cell[3];
-        if (kCells) {
-            const int4 q = b.cell4[i];
-            if (q.w) {
-                ++p.bad;
-                continue;
-            }
-            cell[0] = q.x, cell[1] = q.y, cell[2] = q.z;
-        } else {
-            const float4 q = b.pos4[i];
-            p.general |= tiny_coord(q.x) || tiny_coord(q.y) || tiny_coord(q.z);
-            if (!finite3(q.x, q.y, q.z)) {
-                ++p.bad;
-                continue;
-            }
-            cell[0] = cell_coord(q.x, c.inv_cell);
-            cell[1] = cell_coord(q.y, c.inv_cell);
-            cell[2] = cell_coord(q.z, c.inv_cell);
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            p.mn[a] = min(p.mn[a], cell[a]);
-            p.mx[a] = max(p.mx[a], cell[a]);
-        }
-    }
-    p = merge_block(p);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        prep_add<kCells, kVmax>(p, c, b, i);
+    p = merge_block<kPrepThreads>(p);
     if (threadIdx.x == 0) b.prep[blockIdx.x] = p;
     if (!last_block(b.sync)) return;
     reset_step(ds, b);
     p = prep_empty();
     for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) merge(p, b.prep[k]);
-    p = merge_block(p);
+    p = merge_block<kPrepThreads>(p);
     if (threadIdx.x != 0) return;
     for (int a = 0; a < 3; ++a) {
         ds->cmin[a] = p.mn[a];
@@ -197,7 +53,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const StepConst c, con
     if (how != kNoStep) set_dt(c, ds, how, host_dt, p.vmax);
 }
 
-int launch_prepare(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
+static int launch_prepare(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
                    int how, float host_dt) {
     // at least 4 particles a thread, so that the partials of small sets are few
     int nb = (c.n + 4 * kPrepThreads - 1) / (4 * kPrepThreads);
@@ -212,8 +68,7 @@ int launch_prepare(const LaunchCtx& L, const StepConst& c, const Buffers& b, Dev
 
 // ---- grid -----------------------------------------------------------------------------
 
-// Cell keys and their digit histograms.  kCells (precision mode): the stored cells; w != 0
-// marks a particle with no finite position.
+// Cell keys and their digit histograms.
 template <bool kCells>
 __global__ void __launch_bounds__(256) k_keys(const Buffers b, int n, float inv_cell,
                                               const DevState* ds) {
@@ -221,33 +76,13 @@ __global__ void __launch_bounds__(256) k_keys(const Buffers b, int n, float inv_
     __shared__ uint32_t h[kMaxPasses][kRadixBuckets];
     for (int i = threadIdx.x; i < kMaxPasses * kRadixBuckets; i += 256) (&h[0][0])[i] = 0;
     __syncthreads();
-    const int cx0 = ds->cmin[0], cy0 = ds->cmin[1], cz0 = ds->cmin[2];
-    const uint32_t dx = ds->dim[0], dy = ds->dim[1], dz = ds->dim[2], nc = ds->ncells;
+    const KeyGrid g(ds);
     const uint32_t passes = ds->passes;
     for (int i0 = blockIdx.x * 256; i0 < n; i0 += gridDim.x * 256) {
         const int i = i0 + (int)threadIdx.x;
-        uint32_t key = nc;
+        uint32_t key = 0;
         if (i < n) {
-            int cx = 0, cy = 0, cz = 0;
-            bool fin;
-            if (kCells) {
-                const int4 q = b.cell4[i];
-                cx = q.x, cy = q.y, cz = q.z;
-                fin = !q.w;
-            } else {
-                const float4 p = b.pos4[i];
-                fin = finite3(p.x, p.y, p.z);
-                if (fin) {
-                    cx = cell_coord(p.x, inv_cell);
-                    cy = cell_coord(p.y, inv_cell);
-                    cz = cell_coord(p.z, inv_cell);
-                }
-            }
-            if (fin) {  // relative cell index (< 2^31), folded on the axes that wrap
-                const uint32_t x = (uint32_t)(cx - cx0) % dx, y = (uint32_t)(cy - cy0) % dy,
-                               z = (uint32_t)(cz - cz0) % dz;
-                key = (x * dy + y) * dz + z;
-            }
+            key = cell_key<kCells>(b, i, inv_cell, g);
             b.key[0][i] = key;
         }
         count_digits(h, key, i < n, passes);
@@ -284,61 +119,20 @@ __global__ void k_reorder(const Buffers b, int n, DevState* ds) {
 }
 
 // ---- in-cell order and tile list --------------------------------------------------------
-// A tile is a run of at most tile_n consecutive positions of a cell (b.columns == 0) or of a
-// cell column (x, y, *).  Whether a tile starts at position k is decided from the keys and
-// cell offsets alone (no scan over the particles): at every tile_n-th position of the column
-// and, so that no tile reaches far from its first cell, where a sparse stretch of the column
-// is cut (kRunWindow / kRunAlign).  A tile whose first particle lies in cell z_a ends by cell
-// z_a + kRunCells: the first multiple z_m of kRunAlign at or above z_a + kRunWindow + 1 is at
-// most that plus kRunAlign - 1, and were the tile to reach cell z_m, the kRunWindow cells
-// below z_m would lie wholly in it, fewer than tile_n particles, so a tile starts at z_m.
-struct ColumnInfo {
-    uint32_t base, d2;  // first cell of the scene's block, cells along z
-    bool each_cell;     // tiles within one cell
-};
-__device__ __forceinline__ ColumnInfo column_info(const Buffers& b, const DevState* ds, int k,
-                                                  bool folded_cells) {
-    if (b.nscenes) {
-        const SceneInfo& sc = b.scenes[b.scene_s[k]];
-        return ColumnInfo{sc.base, (uint32_t)sc.dim[2], !b.columns};
-    }
-    return ColumnInfo{0u, (uint32_t)ds->dim[2], !b.columns || folded_cells};
-}
-__device__ __forceinline__ bool tile_starts(const Buffers& b, const ColumnInfo& g, uint32_t nc,
-                                            int k, uint32_t key, uint32_t prev, bool new_cell) {
-    const uint32_t tn = (uint32_t)b.tile_n;
-    if (key >= nc || g.each_cell) return ((uint32_t)k - b.off[key]) % tn == 0;
-    const uint32_t z = (key - g.base) % g.d2, cb = key - z;
-    if (((uint32_t)k - b.off[cb]) % tn == 0) return true;
-    if (!new_cell) return false;
-    // the cells between the last particle's and this one are empty: only the last multiple of
-    // kRunAlign among them can be undecided (an earlier one implies an empty window there)
-    const uint32_t zm = z - z % kRunAlign;
-    return zm > (uint32_t)kRunWindow && cb + zm > prev &&
-           b.off[cb + zm] - b.off[cb + zm - kRunWindow] < tn;
-}
-
 // One block per 256 positions: the tile list, and the order in which each cell's particles are
 // taken as targets: z order (the in-cell offset quantised to 16 levels, stable within a
 // level), so that a tile is a compact slab across the cells of its column.  The particles
 // themselves keep the reference's insertion order, in which they are met as neighbours.  A
 // particle's place is the number of its cell's particles before it in that order, counted by
-// one thread per particle from the levels in shared memory (a counting sort per cell by one
-// warp took 0.038 ms at 1M for this kernel, 0.014 at 10k).  Cells of more than kZOrderMax particles (collapsed
+// one thread per particle from the levels in shared memory, four at a time (a counting sort per
+// cell by one warp took 0.038 ms at 1M for this kernel, 0.014 at 10k).  Cells of more than kZOrderMax particles (collapsed
 // states, whose tiles are dense anyway) keep their order.
-constexpr int kZOrderMax = 128;
-__device__ __forceinline__ uint8_t z_level(const Buffers& b, int k, float inv_cell, float levels) {
-    if (b.cell4_s) return (uint8_t)min(15, max(0, (int)(b.pos4_s[k].z * levels)));
-    if (b.nscenes) inv_cell = b.scenes[b.scene_s[k]].c.inv_cell;
-    const float u = b.pos4_s[k].z * inv_cell;
-    return (uint8_t)min(15, max(0, (int)((u - floorf(u)) * 16.0f)));
-}
 __global__ void __launch_bounds__(256) k_order_tiles(const Buffers b, int n, DevState* ds,
                                                      float inv_cell, float levels) {
     if (ds->status) return;
     __shared__ uint32_t flags[9];
     __shared__ uint32_t s_occ, s_max, s_base;
-    __shared__ uint8_t lev[256 + 2 * kZOrderMax];  // positions k0 - kZOrderMax ...
+    __shared__ __align__(4) uint8_t lev[256 + 2 * kZOrderMax];  // positions k0 - kZOrderMax ...
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_occ = s_max = 0;
     const uint32_t nc = ds->ncells;
@@ -399,13 +193,8 @@ __global__ void __launch_bounds__(256) k_order_tiles(const Buffers b, int n, Dev
     }
     if (b.columns && k < n) {
         uint32_t to = (uint32_t)k;
-        if (cnt >= 2 && cnt <= (uint32_t)kZOrderMax) {
-            const uint8_t* l = lev + kZOrderMax + ((int)first - k0);  // the cell's levels
-            const uint32_t mine = lev[kZOrderMax + tid], own = (uint32_t)k - first;
-            to = first;
-            for (uint32_t q = 0; q < own; ++q) to += l[q] <= mine;
-            for (uint32_t q = own + 1; q < cnt; ++q) to += l[q] < mine;
-        }
+        if (cnt >= 2 && cnt <= (uint32_t)kZOrderMax)
+            to = ordered_place(lev, k0 - kZOrderMax, (uint32_t)k, first, cnt);
         b.tgt[to] = (uint32_t)k;
     }
     __syncthreads();
@@ -420,13 +209,23 @@ __global__ void __launch_bounds__(256) k_order_tiles(const Buffers b, int n, Dev
     }
 }
 
-int launch_build_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b,
-                      DevState* ds) {
+static int launch_build_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b,
+                             DevState* ds) {
     const int n = c.n;
     const int gb = grid_blocks(L, n, 256, 2);
     if (c.precise) k_keys<true><<<gb, 256, 0, L.stream>>>(b, n, c.inv_cell, ds);
     else k_keys<false><<<gb, 256, 0, L.stream>>>(b, n, c.inv_cell, ds);
     return 1 + launch_grid_sort(L, b, ds, n, c);
+}
+
+int launch_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds, int how,
+                float host_dt) {
+    // up to kSmallMax one cluster's shared memory holds the sort, and one launch is faster than
+    // eight over the whole GPU (k_grid_small: 0.019 against 0.036 ms at 4k, 0.035 against 0.052
+    // at 33k, 0.042 against 0.054 at 64k)
+    if (c.n >= 1 && c.n <= kSmallMax && launch_grid_small(L, c, b, ds, how, host_dt)) return 1;
+    const int k = launch_prepare(L, c, b, ds, how, host_dt);
+    return k + launch_build_grid(L, c, b, ds);
 }
 
 // Shared tail of the grid build: stable sort of the keys, gather into cell-sorted order with

@@ -276,8 +276,7 @@ int sphx_grid_build(sphx_grid* g, size_t n, const float* pos_xyz, float cell_siz
     GRID_CUDA(cudaMemcpyAsync(s_pos, pos_xyz, 3 * n * sizeof(float), cudaMemcpyHostToDevice, g->stream));
     GRID_CUDA(cudaMemsetAsync(s_mass, 0, n * sizeof(float), g->stream));
     launch_pack(g->L, (int)n, s_pos, nullptr, s_mass, g->b.pos4, g->b.vel4);
-    launch_prepare(g->L, g->sc, g->b, g->ds, kNoStep, 0.0f);
-    launch_build_grid(g->L, g->sc, g->b, g->ds);
+    launch_grid(g->L, g->sc, g->b, g->ds, kNoStep, 0.0f);
     GRID_CUDA(cudaGetLastError());
     GRID_CUDA(cudaStreamSynchronize(g->stream));
     GRID_CUDA(cudaMemcpy(&g->host, g->ds, sizeof(DevState), cudaMemcpyDeviceToHost));

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "sphx.h"
 
 namespace sphx {
@@ -21,6 +23,7 @@ constexpr int kRadixItems = 16;
 constexpr int kRadixTileN = kRadixThreads * kRadixItems;  // keys per radix block
 constexpr int kMaxPasses = 4;                             // 32-bit keys
 constexpr int kSmallSort = 1 << 18;                       // keys: see launch_radix_sort
+constexpr int kSmallMax = 1 << 16;     // particles: see k_grid_small
 constexpr int kPrepThreads = 256, kMaxPrepBlocks = 608;   // first kernel of a step
 constexpr int kDiagThreads = 256;
 constexpr int kDiagSums = 8;
@@ -488,10 +491,7 @@ __device__ __forceinline__ bool last_block(GridSync* sync) {
     if (last) __threadfence();
     return last;
 }
-// resets the step's counters (one block, all threads)
-__device__ __forceinline__ void reset_step(DevState* ds, const Buffers& b) {
-    for (int i = threadIdx.x; i < kMaxPasses * kRadixBuckets; i += blockDim.x) b.hist[i] = 0;
-    if (threadIdx.x != 0) return;
+__device__ __forceinline__ void reset_counters(DevState* ds) {
     ds->status = 0;
     ds->occupied = 0;
     ds->max_occ = 0;
@@ -499,6 +499,12 @@ __device__ __forceinline__ void reset_step(DevState* ds, const Buffers& b) {
     ds->work[0] = ds->work[1] = 0;
     ds->spread_work[0] = ds->spread_work[1] = 0;
     ds->n_spread = 0;
+}
+// resets what the step's kernels count in (one block, all threads)
+__device__ __forceinline__ void reset_step(DevState* ds, const Buffers& b) {
+    for (int i = threadIdx.x; i < kMaxPasses * kRadixBuckets; i += blockDim.x) b.hist[i] = 0;
+    if (threadIdx.x != 0) return;
+    reset_counters(ds);
     b.sync->epoch++;
     for (int p = 0; p < kMaxPasses; ++p) b.sync->tile[p] = 0;
 }
@@ -597,14 +603,25 @@ struct LaunchCtx {
     int blocks_per_sm;
 };
 
+// A flag per device, filled by whichever thread comes first.
+constexpr int kMaxCacheDevices = 64;
+struct LaunchShapeFlag {
+    std::atomic<int> v[kMaxCacheDevices];
+    std::atomic<int>& at(int device) {
+        return v[device >= 0 && device < kMaxCacheDevices ? device : 0];
+    }
+};
+
 // How a step gets its dt.
 constexpr int kNoStep = 0, kHostDt = 1, kCflDt = 2;
-// The step's first kernel: resets the step's counters, finds the box of occupied cells and
-// lays out the grid, and (how != kNoStep) sets dt and advances the time.
-int launch_prepare(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
-                   int how, float host_dt);
-int launch_build_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b,
-                       DevState* ds);
+// The grid build (single scene): resets the step's counters, finds the box of occupied cells,
+// lays out the grid, sorts the particles and lists the tiles; how != kNoStep: sets dt and
+// advances the time.
+int launch_grid(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds, int how,
+                float host_dt);
+// the same in one launch, for sets of 1 to kSmallMax particles; false: the device cannot
+bool launch_grid_small(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
+                       int how, float host_dt);
 int launch_grid_sort(const LaunchCtx& L, const Buffers& b, DevState* ds, int n, const StepConst& c);
 int launch_density(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds);
 int launch_force(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,

@@ -174,8 +174,7 @@ extern "C" int sphx_density_noalloc(const sphx_params* p, size_t n, const float*
     // the previous call's device-side state must not leak into this one
     if (cudaMemsetAsync(ds, 0, sizeof(DevState), L.stream) != cudaSuccess) return SPHX_ERR_CUDA;
     launch_pack(L, (int)n, pos_xyz, nullptr, mass, b.pos4, b.vel4);
-    launch_prepare(L, c, b, ds, kNoStep, 0.0f);
-    launch_build_grid(L, c, b, ds);
+    launch_grid(L, c, b, ds, kNoStep, 0.0f);
     launch_density(L, c, b, ds);
     const int ub = (int)((n + 255) / 256) < 4 * sms ? (int)((n + 255) / 256) : 4 * sms;
     k_noalloc_unpack<<<ub, 256, 0, L.stream>>>((int)n, ds, b.id_s, b.aux4_s, rho, pressure);

@@ -27,8 +27,6 @@
 // every term uses the reference's float operations in the reference's order with
 // IEEE round-to-nearest and no contraction, so each lane's sums are bit-identical.
 #pragma once
-#include <atomic>
-
 #include "sphx_internal.cuh"
 
 namespace sphx {
@@ -614,7 +612,6 @@ inline int resident_blocks(const LaunchCtx& L, K kernel, int threads, size_t sme
 // Grid sizes of the persistent passes, found once per (device, kernel instantiation, warps
 // per block, requested CTAs per SM) and kept: one cache object per instantiation, indexed
 // by device; any host thread may fill an entry (a racing fill stores the same value).
-constexpr int kMaxCacheDevices = 64;
 struct LaunchShapeCache {
     std::atomic<int> nb[kMaxCacheDevices][5][33];
     std::atomic<int>& at(const LaunchCtx& L) {

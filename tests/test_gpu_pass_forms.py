@@ -147,3 +147,32 @@ def test_grid_query_lists_match_the_reference_walk(port, name):
     want_counts, want_idx = port.query(pos, radius, cell_size=cell)
     assert np.array_equal(counts, want_counts) and np.array_equal(idx, want_idx)
     g.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 1024, 1025, 16384, 16385, 65536, 65537])
+@pytest.mark.parametrize("spread", ["dense", "sparse", "nonfinite"])
+def test_grid_build_forms_list_the_reference_neighbours(built, port, n, spread):
+    """The one-launch grid build at the edges of its blocks, rounds and range: one to four sort
+    passes, cells across block ends, particles without a cell."""
+    rng = np.random.default_rng(n)
+    side = {"dense": 0.04 * (n / 30) ** (1 / 3), "sparse": 6.0, "nonfinite": 0.5}[spread]
+    pos = (side * rng.random((n, 3))).astype(np.float32)
+    if spread == "nonfinite":
+        pos[::3] = np.nan
+    g = sphx.Grid(n)
+    g.build(pos, 0.04)
+    r = np.float32(0.02)
+    counts, idx = g.query(pos, float(r * r))
+    want_counts, want_idx = port.query(pos, 0.02, cell_size=0.04)
+    assert np.array_equal(counts, want_counts) and np.array_equal(idx, want_idx)
+    g.close()
+    if spread == "dense":
+        mass = np.full(n, 1e-3, np.float32)
+        ctx = sphx.Context(n)
+        ctx.set_params(I.params16())
+        ctx.upload(pos, np.zeros_like(pos), mass)
+        ctx.eval()
+        rho = ctx.download()["rho"]
+        want, _, _ = port.fields(pos, np.zeros_like(pos), mass, I.params16())
+        assert O.bits_equal(rho, want), O.mismatch_report(rho, want, "rho")
+        ctx.close()
