@@ -154,23 +154,45 @@ __device__ __forceinline__ void raster_triangle(const RenderConst& r, float3 a, 
     }
     const float xmin = fminf(a.x, fminf(b.x, c.x)), xmax = fmaxf(a.x, fmaxf(b.x, c.x));
     const float ymin = fminf(a.y, fminf(b.y, c.y)), ymax = fmaxf(a.y, fmaxf(b.y, c.y));
-    // pixel (px, py) has its centre at (px + 0.5, py + 0.5); clamp in float before the
-    // integer conversion (window coordinates of far off-screen corners can be huge)
-    const float fx0 = fmaxf(floorf(xsub(xmin, 0.5f)), 0.0f);
-    const float fx1 = fminf(ceilf(xsub(xmax, 0.5f)), (float)(r.width - 1));
-    const float fy0 = fmaxf(floorf(xsub(ymin, 0.5f)), 0.0f);
-    const float fy1 = fminf(ceilf(xsub(ymax, 0.5f)), (float)(r.height - 1));
+    // Pixel (px, py) has its centre at (px + 0.5, py + 0.5).  The centres tried: all within a
+    // pixel of the triangle's box, or only those within kSlack of it where no other can pass
+    // the tests below.  For a centre outside the box by kSlack, say in x, the barycentric
+    // coordinates l (sum 1, sum l_i (x_i - px) = 0) include a negative one of at least
+    // kSlack / (2 (W + 1.5)), so an edge function is at most -A kSlack / (W + 1.5); its rounding
+    // error is at most 10 2^-24 (W + 1.5) (H + 1.5) (W, H: the box, A: the area).  The test
+    // compares with six times that.
+    constexpr float kSlack = 0x1p-6f;
+    const float W = xmax - xmin + 2.0f, H = ymax - ymin + 2.0f;
+    const bool tight = area * kSlack >= 0x1p-17f * W * H * fmaxf(W, H) &&
+                       fmaxf(xmax, ymax) < 16384.0f;
+    // clamp in float before the integer conversion (window coordinates of far off-screen
+    // corners can be huge)
+    const float lx = xsub(xmin, 0.5f), hx = xsub(xmax, 0.5f), ly = xsub(ymin, 0.5f),
+                hy = xsub(ymax, 0.5f);
+    const float fx0 = fmaxf(tight ? ceilf(lx - kSlack) : floorf(lx), 0.0f);
+    const float fx1 = fminf(tight ? floorf(hx + kSlack) : ceilf(hx), (float)(r.width - 1));
+    const float fy0 = fmaxf(tight ? ceilf(ly - kSlack) : floorf(ly), 0.0f);
+    const float fy1 = fminf(tight ? floorf(hy + kSlack) : ceilf(hy), (float)(r.height - 1));
     if (!(fx0 <= fx1 && fy0 <= fy1)) return;
     const int x0 = (int)fx0, x1 = (int)fx1, y0 = (int)fy0, y1 = (int)fy1;
-    const bool tab = top_left(a, b), tbc = top_left(b, c), tca = top_left(c, a);
+    // a centre is inside an edge if its function is above 0, or 0 on a top or left edge: above
+    // the largest float below 0
+    const float below = -__uint_as_float(1u);
+    const float t0 = top_left(b, c) ? below : 0.0f, t1 = top_left(c, a) ? below : 0.0f,
+                t2 = top_left(a, b) ? below : 0.0f;
+    const float dx0 = xsub(c.x, b.x), dy0 = xsub(c.y, b.y), dx1 = xsub(a.x, c.x),
+                dy1 = xsub(a.y, c.y), dx2 = xsub(b.x, a.x), dy2 = xsub(b.y, a.y);
     for (int py = y0; py <= y1; ++py) {
         const float cy = (float)py + 0.5f;
+        const float r0 = xmul(dx0, xsub(cy, b.y)), r1 = xmul(dx1, xsub(cy, c.y)),
+                    r2 = xmul(dx2, xsub(cy, a.y));
         for (int px = x0; px <= x1; ++px) {
             const float cx = (float)px + 0.5f;
-            const float w0 = edge(b, c, cx, cy), w1 = edge(c, a, cx, cy), w2 = edge(a, b, cx, cy);
-            const bool in = (w0 > 0.0f || (w0 == 0.0f && tbc)) && (w1 > 0.0f || (w1 == 0.0f && tca)) &&
-                            (w2 > 0.0f || (w2 == 0.0f && tab));
-            if (!in) continue;
+            // edge(b, c), edge(c, a), edge(a, b)
+            const float w0 = xsub(r0, xmul(dy0, xsub(cx, b.x)));
+            const float w1 = xsub(r1, xmul(dy1, xsub(cx, c.x)));
+            const float w2 = xsub(r2, xmul(dy2, xsub(cx, a.x)));
+            if (!((w0 > t0) & (w1 > t1) & (w2 > t2))) continue;
             // depth: barycentric interpolation of window z (affine in window space)
             // (+ 0 turns a -0 into +0, whose bits order correctly in the key)
             const float z =
@@ -183,9 +205,13 @@ __device__ __forceinline__ void raster_triangle(const RenderConst& r, float3 a, 
     }
 }
 
-__global__ void k_render_raster(const RenderConst r, const RenderArgs a,
-                                unsigned long long* keys) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
+// A thread per particle.  Bound: instruction issue (0.76 per cycle; 1,240 per warp of particles,
+// the fragments' path and the corners' transforms).  1M particles of 2.5 x 2.5 pixels, 1280 x
+// 720: 45 us; trying every pixel around the quad with each edge function in full 169 us.
+__global__ void __launch_bounds__(128) k_render_raster(const RenderConst r, const RenderArgs a,
+                                                       unsigned long long* keys) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < a.n) {
         const float3 w = world_pos(a, i);
         float4 c[4];
         bool ok = true;
@@ -194,7 +220,7 @@ __global__ void k_render_raster(const RenderConst r, const RenderArgs a,
             c[k] = corner(r, w, kQuad[k][0], kQuad[k][1]);
             ok = ok && in_clip(c[k]);
         }
-        if (!ok) continue;
+        if (!ok) return;
         float3 s[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) s[k] = to_window(r, c[k]);
@@ -258,8 +284,7 @@ int launch_render_image(const LaunchCtx& L, const RenderConst& r, const RenderAr
     k_fill_u64<<<pblocks, 256, 0, L.stream>>>(keys, npix, kClearedKey);
     int k = 1;
     if (a.n > 0) {
-        const int blocks = min((a.n + 127) / 128, L.num_sms * 16);
-        k_render_raster<<<blocks, 128, 0, L.stream>>>(r, a, keys);
+        k_render_raster<<<(a.n + 127) / 128, 128, 0, L.stream>>>(r, a, keys);
         ++k;
     }
     k_render_resolve<<<pblocks, 256, 0, L.stream>>>(r, a, keys, rgba);

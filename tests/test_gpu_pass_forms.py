@@ -176,3 +176,27 @@ def test_grid_build_forms_list_the_reference_neighbours(built, port, n, spread):
         want, _, _ = port.fields(pos, np.zeros_like(pos), mass, I.params16())
         assert O.bits_equal(rho, want), O.mismatch_report(rho, want, "rho")
         ctx.close()
+
+
+@pytest.mark.parametrize("size", [1e-5, 1e-3, 0.02, 0.4, 6.0])
+@pytest.mark.parametrize("image", [(333, 217), (64, 1000)])
+def test_render_quad_sizes_match_the_oracle(built, port, size, image):
+    """Quads from a fraction of a pixel to several images wide: pixels tried within a slack of
+    the quad's box and, where that is not provably enough, all around it."""
+    rng = np.random.default_rng(31)
+    pos = rng.random((400, 3)).astype(np.float32)
+    vel = rng.standard_normal(pos.shape).astype(np.float32)
+    ctx = sphx.Context(len(pos))
+    ctx.set_params(I.params16())
+    ctx.upload(pos, vel, np.full(len(pos), 1e-3, np.float32))
+    for view, proj in (sphx.camera_matrices((0.5, 0.4, 2.0), -90.0, 0.0, 45.0, 16 / 9),
+                       sphx.camera_matrices((1.8, 1.2, 1.6), -135.0, -25.0, 35.0, 4 / 3)):
+        # the second projection is also squeezed: quads a few hundredths as wide as high
+        for squeeze in (1.0, 0.03):
+            p = np.array(proj, np.float32)
+            p.reshape(-1)[0] *= np.float32(squeeze)
+            rp = sphx.render_params(view, p, particle_size=size, color_mode=0, width=image[0],
+                                    height=image[1])
+            got, want = ctx.render_image(rp), port.render_image(rp, pos, vel, None)
+            assert np.array_equal(got, want)
+    ctx.close()
