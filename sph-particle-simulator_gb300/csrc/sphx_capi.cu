@@ -342,6 +342,11 @@ int enter(sphx_ctx* c) {
     return SPHX_OK;
 }
 
+// Largest set whose download a kernel stores straight into pinned memory: one launch instead of
+// two, two events and six copies.  All five fields: 4k particles 15 us against 29, 22k 29
+// against 34, 47k 45 against 40; one field 11 to 14 against 16.
+constexpr size_t kDirectMax = 1 << 15;
+
 int run_phases(sphx_ctx* c, float dt, bool integrate) {
     fill_step_const(c);
     sphx_ctx::ProfSlot* slot = nullptr;
@@ -1164,6 +1169,23 @@ int sphx_download(sphx_ctx* c, float* pos, float* vel, float* rho, float* pressu
     if (rc) return rc;
     const size_t n = c->n;
     if (n == 0) return sync_status(c);
+    if (n <= kDirectMax && !(pos && c->b.cell4) &&
+        (c->have_fields || !(rho || pressure || acc))) {
+        // a small set into pinned memory: one kernel stores it there
+        float* const out[] = {pos, vel, rho, pressure, acc};
+        float* dev[5] = {};
+        bool all = true;
+        for (int k = 0; k < 5 && all; ++k)
+            if (out[k]) all = (dev[k] = const_cast<float*>(mapped(out[k]))) != nullptr;
+        int* const status = all ? const_cast<int*>(mapped(c->h_status)) : nullptr;
+        if (status) {
+            launch_unpack_direct(c->L, (int)n, c->b, c->ds, dev[0], dev[1], dev[2], dev[3], dev[4],
+                                 status);
+            SPHX_CUDA(cudaGetLastError());
+            SPHX_CUDA(cudaStreamSynchronize(c->stream));
+            return *c->h_status;  // a failed step's outputs are not to be used
+        }
+    }
     // outputs go through device staging and the copy engines (on Grace + Blackwell the
     // copy engines write host memory faster than kernel stores over the C2C link do); the
     // copies are split over two streams so that two copy engines run at once

@@ -362,9 +362,44 @@ void launch_unpack_sorted(const LaunchCtx& L, int n, const uint32_t* id_s, const
                                                                      rho, pressure, acc3);
 }
 
-}  // namespace sphx
+// Any of the download's fields straight to pinned host memory, and the status word with them.
+__global__ void k_unpack_direct(int n, const Buffers b, const DevState* ds, float* pos3,
+                                float* vel3, float* rho, float* pressure, float* acc3,
+                                int* status) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) *status = ds->status;
+    if (k >= n) return;
+    if (pos3) {
+        const float4 p = b.pos4[k];
+        pos3[3 * k] = p.x;
+        pos3[3 * k + 1] = p.y;
+        pos3[3 * k + 2] = p.z;
+    }
+    if (vel3) {
+        const float4 v = b.vel4[k];
+        vel3[3 * k] = v.x;
+        vel3[3 * k + 1] = v.y;
+        vel3[3 * k + 2] = v.z;
+    }
+    if (!rho && !pressure && !acc3) return;
+    const uint32_t id = b.id_s[k];
+    const float4 a = b.aux4_s[k];
+    if (rho) rho[id] = a.x;
+    if (pressure) pressure[id] = a.y;
+    if (acc3) {
+        const float4 g = b.acc4_s[k];
+        acc3[3 * id] = g.x;
+        acc3[3 * id + 1] = g.y;
+        acc3[3 * id + 2] = g.z;
+    }
+}
 
-namespace sphx {
+void launch_unpack_direct(const LaunchCtx& L, int n, const Buffers& b, const DevState* ds,
+                          float* pos3, float* vel3, float* rho, float* pressure, float* acc3,
+                          int* status) {
+    k_unpack_direct<<<(n + 127) / 128, 128, 0, L.stream>>>(n, b, ds, pos3, vel3, rho, pressure,
+                                                           acc3, status);
+}
 
 // Absolute position (double) -> integer cell + offset in [0, cs); non-finite -> w = 1.
 __device__ __forceinline__ void to_cell(double X, double cs, int fp16, int& c, float& o) {

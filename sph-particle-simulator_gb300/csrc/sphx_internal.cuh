@@ -667,6 +667,9 @@ void launch_pack(const LaunchCtx& L, int n, const float* pos3, const float* vel3
                  const float* mass, float4* pos4, float4* vel4);
 void launch_unpack_state(const LaunchCtx& L, int n, const float4* pos4, const float4* vel4,
                          float* pos3, float* vel3);
+void launch_unpack_direct(const LaunchCtx& L, int n, const Buffers& b, const DevState* ds,
+                          float* pos3, float* vel3, float* rho, float* pressure, float* acc3,
+                          int* status);
 void launch_unpack_sorted(const LaunchCtx& L, int n, const uint32_t* id_s,
                           const float4* aux4_s, const float4* acc4_s, float* rho,
                           float* pressure, float* acc3);

@@ -69,6 +69,8 @@ class ParticleSystem {
     auto end() const { return particles_.cend(); }
 
     void add_particle(const Particle& particle);
+    // add_particles of particles made from arrays (3 n, 3 n or null, n floats)
+    void add_arrays(size_t n, const float* pos, const float* vel, const float* mass);
     void add_particles(const std::vector<Particle>& new_particles);
 
     void remove_particle(size_t index);

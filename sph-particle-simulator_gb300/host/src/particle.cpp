@@ -35,6 +35,19 @@ void ParticleSystem::add_particles(const std::vector<Particle>& new_particles) {
     for (const Particle& p : new_particles) add_particle(p);
 }
 
+void ParticleSystem::add_arrays(size_t n, const float* pos, const float* vel, const float* mass) {
+    for (size_t i = 0; i < n; ++i) {
+        if (particles_.size() >= capacity_) {
+            std::cerr << "Warning: Particle capacity exceeded\n";
+            continue;
+        }
+        particles_.emplace_back(glm::vec3(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]), mass[i]);
+        Particle& p = particles_.back();
+        if (vel) p.velocity = glm::vec3(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2]);
+        p.id = static_cast<int>(particles_.size() - 1);
+    }
+}
+
 void ParticleSystem::remove_particle(size_t index) {
     if (index >= particles_.size()) return;
     particles_.erase(particles_.begin() + static_cast<std::ptrdiff_t>(index));

@@ -116,7 +116,7 @@ void SPHEngine::initialize_granular_flow() {
 
 // the initialize_* scenes: the host set replaced by `ps`
 void SPHEngine::replace_particles(const std::vector<Particle>& ps) {
-    host_will_change();
+    host_will_clear();
     particles_.clear();
     staged_ = 0;
     particles_.add_particles(ps);
@@ -130,9 +130,28 @@ void SPHEngine::add_particles(const std::vector<Particle>& particles) {
     stage_append(old);
 }
 
+void SPHEngine::add_arrays(size_t n, const float* pos, const float* vel, const float* mass) {
+    host_will_change();
+    const size_t old = particles_.size();
+    particles_.add_arrays(n, pos, vel, mass);
+    float* buf = stage();
+    if (!buf || staged_ != old || particles_.size() != old + n) {
+        stage_append(old);
+        return;
+    }
+    // the upload region takes the arrays as they are
+    const size_t C = std::max<size_t>(particles_.capacity(), 1);
+    std::copy(pos, pos + 3 * n, buf + 3 * old);
+    if (vel) std::copy(vel, vel + 3 * n, buf + 3 * C + 3 * old);
+    else std::fill_n(buf + 3 * C + 3 * old, 3 * n, 0.0f);
+    std::copy(mass, mass + n, buf + 6 * C + old);
+    staged_ = old + n;
+    stage_current_ = true;
+}
+
 // SPHEngine::clear_particles (src/sph_engine.cpp:87-91)
 void SPHEngine::clear_particles() {
-    host_will_change();
+    host_will_clear();
     particles_.clear();
     staged_ = 0;
     step_count_ = 0;
@@ -170,6 +189,23 @@ void SPHEngine::stage_append(size_t from) {
 
 void SPHEngine::host_will_change() {
     sync_to_host();
+    device_dirty_ = true;
+}
+
+// As host_will_change, ahead of dropping every particle: of a newer device state only the
+// density and pressure vectors outlive the particles.
+void SPHEngine::host_will_clear() {
+    float* buf = host_stale_ ? stage() : nullptr;
+    if (!buf) {
+        host_will_change();
+        return;
+    }
+    const size_t n = particles_.size(), C = std::max<size_t>(particles_.capacity(), 1);
+    const float *rho = buf + 7 * C, *P = buf + 8 * C;
+    check(sphx_download(gpu_, nullptr, nullptr, buf + 7 * C, buf + 8 * C, nullptr), "sphx_download");
+    std::copy(rho, rho + std::min(n, densities_.size()), densities_.begin());
+    std::copy(P, P + std::min(n, pressures_.size()), pressures_.begin());
+    host_stale_ = false;
     device_dirty_ = true;
 }
 

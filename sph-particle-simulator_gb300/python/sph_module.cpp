@@ -176,15 +176,7 @@ PYBIND11_MODULE(sph, m) {
                      v = vel.cast<py::array_t<float, py::array::c_style | py::array::forcecast>>();
                      if (static_cast<size_t>(v.size()) != 3 * n) throw std::invalid_argument("vel is (n, 3)");
                  }
-                 std::vector<sph::Particle> ps(n);
-                 const float* p = pos.data();
-                 const float* mm = mass.data();
-                 for (size_t i = 0; i < n; ++i) {
-                     ps[i] = sph::Particle(glm::vec3(p[3 * i], p[3 * i + 1], p[3 * i + 2]), mm[i]);
-                     if (!vel.is_none())
-                         ps[i].velocity = glm::vec3(v.data()[3 * i], v.data()[3 * i + 1], v.data()[3 * i + 2]);
-                 }
-                 e.add_particles(ps);
+                 e.add_arrays(n, pos.data(), vel.is_none() ? nullptr : v.data(), mass.data());
              },
              py::arg("pos"), py::arg("vel") = py::none(), py::arg("mass"))
         .def("clear_particles", &sph::SPHEngine::clear_particles)

@@ -200,3 +200,26 @@ def test_render_quad_sizes_match_the_oracle(built, port, size, image):
             got, want = ctx.render_image(rp), port.render_image(rp, pos, vel, None)
             assert np.array_equal(got, want)
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 127, 32768, 32769])
+@pytest.mark.parametrize("fields", ["all", "pos", "rho", "acc"])
+def test_download_into_pinned_memory(built, n, fields):
+    """Fields stored into pinned memory by one kernel (small sets) equal the staged copies."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    pos = (0.4 * rng.random((n, 3))).astype(np.float32)
+    ctx = sphx.Context(n)
+    ctx.set_params(I.params16(gas_constant=2e-3))
+    ctx.upload(pos, np.zeros_like(pos), np.full(n, 1e-3, np.float32))
+    ctx.step(1e-4)
+    names = ("pos", "vel", "rho", "pressure", "acc")
+    want = ctx.download()
+    out = {k: torch.full((3 * n if k in ("pos", "vel", "acc") else n,), 7.0).pin_memory()
+           for k in names}
+    ctx.download_ptr(*[out[k].data_ptr() if fields in ("all", k) else 0 for k in names])
+    for k in names:
+        w = want[k].reshape(-1) if fields in ("all", k) else np.full(out[k].shape[0], 7, np.float32)
+        assert O.bits_equal(out[k].numpy(), w), k
+    ctx.close()
