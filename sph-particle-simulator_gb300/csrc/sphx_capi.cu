@@ -346,6 +346,7 @@ int enter(sphx_ctx* c) {
 // two, two events and six copies.  All five fields: 4k particles 15 us against 29, 22k 29
 // against 34, 47k 45 against 40; one field 11 to 14 against 16.
 constexpr size_t kDirectMax = 1 << 15;
+constexpr size_t kManyParticles = 1 << 19;  // some ten tiles for every resident warp
 
 int run_phases(sphx_ctx* c, float dt, bool integrate) {
     fill_step_const(c);
@@ -699,15 +700,16 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
          (rc = dmalloc(&b.spread_tiles, C))))
         return fail(rc);
     if ((rc = dmalloc(&b.tgt, C))) return fail(rc);
-    // Record pool (Buffers::records): 4 records (128 B each) per particle of capacity.  The
-    // lattice and uniform states need about 2 per particle in exact mode (32-particle tiles,
-    // the candidates their boxes keep) and 1 in the precision mode; the rest is room for
-    // denser states and for the uneven split of tiles over the warps.  The small sets' lists
-    // (270 neighbours of 4 bytes a particle) take 8.5, so up to that size 12 are held.  Without the pool (or
-    // where a warp's region runs out) the force pass walks the candidates itself.
+    // Record pool (Buffers::records), in records (128 B) per particle of capacity: 3, or 4 where
+    // few warps share it.  The lattice and uniform states need about 2 in exact mode
+    // (32-particle tiles, the candidates their boxes keep) and 1 in the precision mode; the rest
+    // is room for denser states and for the uneven split of tiles over the warps.  The small
+    // sets' lists (270 neighbours of 4 bytes a particle) take 8.5, so up to that size 12 are
+    // held.  Without the pool (or where a warp's region runs out) the force pass walks the
+    // candidates itself.
     if (dmalloc(&b.tile_list, C) == SPHX_OK) {
         unsigned long long cap = std::max<unsigned long long>(
-            4ull * C, c->tuning.mode != SPHX_MODE_EXACT
+            (C > kManyParticles ? 3ull : 4ull) * C, c->tuning.mode != SPHX_MODE_EXACT
                           ? 0ull : 12ull * std::min<unsigned long long>(C, kTeamMax));
         if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
         if (dmalloc(&b.records, (size_t)cap * 32) == SPHX_OK) {

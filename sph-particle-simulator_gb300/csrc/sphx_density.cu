@@ -30,6 +30,21 @@ struct DensitySmem {
 };
 static_assert(sizeof(DensitySmem) % 16 == 0, "per-warp regions stay 16-byte aligned");
 
+// If `on`: a candidate's coordinates and mass into the ring arrays and, if there is `room`, its
+// position j into the tile's records (a streaming store: the records must not evict the
+// candidates from L2).  Predicated stores; the compiler branches around them.
+__device__ __forceinline__ void keep_candidate(uint32_t on, uint32_t slot, const float4& p,
+                                               bool room, uint32_t* rec, uint32_t j) {
+    constexpr int kArray = kDensityRing * 32 * 4;  // bytes
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %0, 0;\n\tsetp.ne.and.u32 q, %6, 0, p;\n\t"
+        "@p st.shared.f32 [%1], %2;\n\t@p st.shared.f32 [%1+%9], %3;\n\t"
+        "@p st.shared.f32 [%1+%10], %4;\n\t@p st.shared.f32 [%1+%11], %5;\n\t"
+        "@q st.global.cs.u32 [%7], %8;\n\t}"
+        ::"r"(on), "r"(slot), "f"(p.x), "f"(p.y), "f"(p.z), "f"(p.w), "r"((uint32_t)room), "l"(rec),
+        "r"(j), "n"(kArray), "n"(2 * kArray), "n"(3 * kArray) : "memory");
+}
+
 // kNZ: the pair forms' divisions are in range (StepConst::div_nz)
 template <bool kBatch, int kKern, bool kNZ>
 __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Buffers b,
@@ -77,16 +92,9 @@ __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Bu
                 const int m = st.count(), s = st.s;
                 const uint32_t surv =
                     __ballot_sync(kFull, lane < m && box_near(B, pl, r2m));
-                if ((surv >> lane) & 1u) {
-                    const int a = kept + __popc(surv & lt);
-                    const int slot = ring_slot<kDensityRing>(a);
-                    S->cx[slot] = pl.x;
-                    S->cy[slot] = pl.y;
-                    S->cz[slot] = pl.z;
-                    S->cm[slot] = pl.w;
-                    // streaming stores: the records must not evict the candidates from L2
-                    if ((a >> 5) < room) __stcs(rec + (a >> 5) * 64 + (a & 31), (uint32_t)(s + lane));
-                }
+                const int a = kept + __popc(surv & lt);
+                keep_candidate((surv >> lane) & 1u, smem_u32(&S->cx[ring_slot<kDensityRing>(a)]), pl,
+                               (a >> 5) < room, rec + (a >> 5) * 64 + (a & 31), (uint32_t)(s + lane));
                 if ((unsigned)(i - s) < (unsigned)m) self = kept + __popc(surv & ((1u << (i - s)) - 1u));
                 st.next();
                 if (st.more() && lane < st.count()) pl = b.pos4_s[st.s + lane];

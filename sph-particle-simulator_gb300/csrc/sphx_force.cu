@@ -13,18 +13,18 @@ namespace sphx {
 // ---------------------------------------------------------------------------------------
 // Per warp: the candidate ring -- positions and mass, velocities and density, the two
 // per-candidate factors -- the lanes' masks and the tile's row segments.  40 bytes a candidate:
-// 12 chunks leave room for 12 warps per SM; 8 chunks (16 warps) took 9% longer on the 1M dam
-// break, 10 (14 warps) 8%, 16 (8 warps) 17%.
+// 13 chunks are what 12 warps per SM leave room for; on the 1M dam break 12 chunks took 4%
+// longer, 8 (16 warps) 13%, 10 (14 warps) 12%, 16 (8 warps) 21%.
 //
 // Bound: instruction issue (64% of the slots with 3 warps per scheduler) and the FP32 pipe
 // (58%; a packed instruction holds it two cycles): about 1,200 warp instructions per particle
 // in 5.7 turns, each finishing one pair of neighbours per lane and starting the next.  1M dam
-// break, force + leapfrog: 1.52 ms; walking and culling the candidates again instead of
-// reading the density pass's list 1.71 ms; with hit lists, terms passed through shared memory and
+// break, force + leapfrog: 1.44 ms (1.53 with 12 chunks and a branch at each new mask); walking
+// and culling the candidates again instead of reading the density pass's list 1.71 ms; with hit lists, terms passed through shared memory and
 // in-order folds by their lanes (2,479 instructions) 2.60 ms; one neighbour per turn with the
 // compiler's division and square root 2.72 ms, pairs 2.08, staged by asynchronous copies 1.83,
 // the two halves of a turn overlapped 1.73.
-constexpr int kForceRing = 12;
+constexpr int kForceRing = 13;
 struct ForceSmem {
     float4 pos[kForceRing * 32];  // x, y, z, m
     float4 vel[kForceRing * 32];  // vx, vy, vz, rho
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
             if (nz) {
                 // starts `next` and adds `done`; false when no lane needs a chunk before `until`
                 auto turn = [&](PairStart& next, const PairStart& done) -> bool {
-                    at.advance(S->mask, ready, lane);
+                    at.advance_flat(S->mask, ready, lane);
                     at.take2(next.qa, next.qb, next.ha, next.hb);
                     next.start(lit, xi, S->pos[next.qa], S->pos[next.qb]);
                     add_pair<kKern>(lit, c.pair, vi0, Pi, done, S->vel[done.qa], S->vel[done.qb],
