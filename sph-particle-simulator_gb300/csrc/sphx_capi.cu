@@ -63,6 +63,7 @@ struct sphx_ctx {
     uchar4* r_rgba = nullptr;
     size_t r_pix_cap = 0;
     int* h_status = nullptr;  // pinned host word: the device status, read with the results
+    int* d_status = nullptr;  // the same word as the device sees it, if it does
     // second stream for device-to-host copies that can run beside the main stream's
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev_unpacked = nullptr, ev_copied = nullptr;
@@ -342,10 +343,6 @@ int enter(sphx_ctx* c) {
     return SPHX_OK;
 }
 
-// Largest set whose download a kernel stores straight into pinned memory: one launch instead of
-// two, two events and six copies.  All five fields: 4k particles 15 us against 29, 22k 29
-// against 34, 47k 45 against 40; one field 11 to 14 against 16.
-constexpr size_t kDirectMax = 1 << 15;
 constexpr size_t kManyParticles = 1 << 19;  // some ten tiles for every resident warp
 
 int run_phases(sphx_ctx* c, float dt, bool integrate) {
@@ -699,7 +696,8 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
         ((rc = dmalloc(&b.cell4, C)) || (rc = dmalloc(&b.cell4_s, C)) ||
          (rc = dmalloc(&b.spread_tiles, C))))
         return fail(rc);
-    if ((rc = dmalloc(&b.tgt, C))) return fail(rc);
+    if ((rc = dmalloc(&b.tgt, 2 * C))) return fail(rc);
+    b.rank = b.tgt + C;
     // Record pool (Buffers::records), in records (128 B) per particle of capacity: 3, or 4 where
     // few warps share it.  The lattice and uniform states need about 2 in exact mode
     // (32-particle tiles, the candidates their boxes keep) and 1 in the precision mode; the rest
@@ -735,6 +733,7 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
         return fail(SPHX_ERR_OOM);
     }
     *c->h_status = 0;
+    c->d_status = mapped(c->h_status);
     if (cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_unpacked, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_copied, cudaEventDisableTiming) != cudaSuccess)
@@ -1171,26 +1170,30 @@ int sphx_download(sphx_ctx* c, float* pos, float* vel, float* rho, float* pressu
     if (rc) return rc;
     const size_t n = c->n;
     if (n == 0) return sync_status(c);
-    if (n <= kDirectMax && !(pos && c->b.cell4) &&
-        (c->have_fields || !(rho || pressure || acc))) {
-        // a small set into pinned memory: one kernel stores it there
+    if (c->have_fields || !(rho || pressure || acc)) {
+        // into pinned memory: one kernel stores everything there, instead of two unpack kernels,
+        // two events and six copies (all five fields end to end, us: 4k particles 15 against 29,
+        // 79k lattice 21 less, 1M 42 less)
         float* const out[] = {pos, vel, rho, pressure, acc};
         float* dev[5] = {};
         bool all = true;
         for (int k = 0; k < 5 && all; ++k)
-            if (out[k]) all = (dev[k] = const_cast<float*>(mapped(out[k]))) != nullptr;
-        int* const status = all ? const_cast<int*>(mapped(c->h_status)) : nullptr;
+            if (out[k]) {
+                const size_t last = (k == 2 || k == 3 ? 1 : 3) * n - 1;  // pinned as a whole
+                all = (dev[k] = mapped(out[k])) && mapped(out[k] + last) == dev[k] + last;
+            }
+        int* const status = all ? c->d_status : nullptr;
         if (status) {
-            launch_unpack_direct(c->L, (int)n, c->b, c->ds, dev[0], dev[1], dev[2], dev[3], dev[4],
-                                 status);
+            if (pos && c->b.cell4) fill_step_const(c);
+            launch_unpack_direct(c->L, (int)n, c->b, c->ds, c->sc.cs_d, dev[0], dev[1], dev[2],
+                                 dev[3], dev[4], status);
             SPHX_CUDA(cudaGetLastError());
             SPHX_CUDA(cudaStreamSynchronize(c->stream));
             return *c->h_status;  // a failed step's outputs are not to be used
         }
     }
-    // outputs go through device staging and the copy engines (on Grace + Blackwell the
-    // copy engines write host memory faster than kernel stores over the C2C link do); the
-    // copies are split over two streams so that two copy engines run at once
+    // into pageable memory (or zeros, where no step has made fields yet): through device staging
+    // and the copy engines, split over two streams so that two copy engines run at once
     float* s0 = c->stage;
     float* s1 = c->stage + 3 * c->capacity;
     float* s_rho = c->stage + 6 * c->capacity;

@@ -192,6 +192,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
         const float4 pos = b.pos4[it.y];
         b.key_s[at] = it.x;
         b.id_s[at] = it.y;
+        if (b.rank) b.rank[it.y] = (uint32_t)at;
         b.pos4_s[at] = pos;
         b.vel4_s[at] = b.vel4[it.y];
         if (kCells) b.cell4_s[at] = b.cell4[it.y];

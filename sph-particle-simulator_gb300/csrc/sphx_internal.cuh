@@ -161,6 +161,7 @@ struct Buffers {
     uint32_t* val[2];
     uint32_t* key_s;  // sorted cell keys
     uint32_t* id_s;   // sorted position -> insertion index
+    uint32_t* rank = nullptr;  // insertion index -> sorted position (a context's steps)
     uint32_t* off;    // dense cell grid: first sorted position of each cell (max_cells + 2)
     uint2* tiles;     // warp work items: first target position and number of targets
     // Target order: the particle of target position k is sorted position tgt[k]; null: k.
@@ -668,7 +669,7 @@ void launch_pack(const LaunchCtx& L, int n, const float* pos3, const float* vel3
 void launch_unpack_state(const LaunchCtx& L, int n, const float4* pos4, const float4* vel4,
                          float* pos3, float* vel3);
 void launch_unpack_direct(const LaunchCtx& L, int n, const Buffers& b, const DevState* ds,
-                          float* pos3, float* vel3, float* rho, float* pressure, float* acc3,
+                          double cs, float* pos3, float* vel3, float* rho, float* pressure, float* acc3,
                           int* status);
 void launch_unpack_sorted(const LaunchCtx& L, int n, const uint32_t* id_s,
                           const float4* aux4_s, const float4* acc4_s, float* rho,
