@@ -701,14 +701,18 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     // Record pool (Buffers::records), in records (128 B) per particle of capacity: 3, or 4 where
     // few warps share it.  The lattice and uniform states need about 2 in exact mode
     // (32-particle tiles, the candidates their boxes keep) and 1 in the precision mode; the rest
-    // is room for denser states and for the uneven split of tiles over the warps.  The small
-    // sets' lists (270 neighbours of 4 bytes a particle) take 8.5, so up to that size 12 are
-    // held.  Without the pool (or where a warp's region runs out) the force pass walks the
-    // candidates itself.
+    // is room for denser states and for the uneven split of tiles over the warps.  Small sets
+    // hold more (up to 0.5 GB), since their collapsed states are common and a warp's share of
+    // the pool has to hold whole tiles: lists of 4 bytes a neighbour, 8.5 records a particle on
+    // the lattice, 47 at 1,500 neighbours.  Force pass with 12, 24 and 64 of them, us: collapsed
+    // 8k 56, 26 and 26, 14k 114, 113 and 45, 24k 184, 181 and 83, 30k 236, 229 and 110; lattice
+    // 17k (two tiles a warp) 70, 42 and 42.  Without the pool (or where a warp's share runs out)
+    // the force pass walks the candidates itself.
     if (dmalloc(&b.tile_list, C) == SPHX_OK) {
         unsigned long long cap = std::max<unsigned long long>(
-            (C > kManyParticles ? 3ull : 4ull) * C, c->tuning.mode != SPHX_MODE_EXACT
-                          ? 0ull : 12ull * std::min<unsigned long long>(C, kTeamMax));
+            (C > kManyParticles ? 3ull : 4ull) * C,
+            (c->tuning.mode == SPHX_MODE_EXACT ? 64ull : 0ull) *
+                std::min<unsigned long long>(C, kTeamMax));
         if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
         if (dmalloc(&b.records, (size_t)cap * 32) == SPHX_OK) {
             b.record_cap = cap;
