@@ -37,3 +37,31 @@ def test_pinned_and_pageable_downloads_agree(built, n, mode, offset):
                 got = np.concatenate([got[:offset], got[offset + w * n:]])
             assert (got == 7.0).all(), k  # nothing else written
     ctx.close()
+
+
+@pytest.mark.parametrize("mode", [sphx.MODE_EXACT, sphx.MODE_PRECISE, sphx.MODE_PRECISE_FP16])
+@pytest.mark.parametrize("pinned", [("pos",), ("vel", "mass"), ("pos", "vel", "mass")])
+@pytest.mark.parametrize("with_vel", [True, False])
+def test_fp64_uploads_from_pinned_memory_agree(built, mode, pinned, with_vel):
+    """Positions in FP64 from pinned memory (read in place), pageable memory (staged) and mixtures
+    of both: the same state."""
+    n = 5001
+    rng = np.random.default_rng(n)
+    src = {"pos": 1000.0 + 0.2 * rng.random((n, 3)),
+           "vel": rng.standard_normal((n, 3)).astype(np.float32),
+           "mass": np.full(n, 1e-3, np.float32) * (1 + np.arange(n, dtype=np.float32) % 3)}
+    held = {k: torch.from_numpy(v).pin_memory() for k, v in src.items() if k in pinned}
+
+    def state(arrays):
+        ctx = sphx.Context(n, mode=mode)
+        ctx.set_params(I.params16(xmin=0.0, xmax=2e3, ymin=0.0, ymax=2e3, zmin=0.0, zmax=2e3))
+        ctx.upload_f64(arrays["pos"], arrays["vel"] if with_vel else None, arrays["mass"])
+        ctx.step(1e-4)
+        out = ctx.download()
+        ctx.close()
+        return out
+
+    want = state(src)
+    got = state({k: held[k].numpy() if k in held else v for k, v in src.items()})
+    for k in want:
+        assert got[k].tobytes() == want[k].tobytes(), k
