@@ -30,6 +30,7 @@ struct sphx_ctx {
     int kernel = SPHX_KERNEL_CUBIC_SPLINE;
     DevState* ds = nullptr;
     float* stage = nullptr;    // 11 * capacity floats (FP64 positions; all download fields)
+    unsigned char* arena = nullptr;  // the buffers of fixed size (sphx_create)
     float4* snap_pos = nullptr;
     float4* snap_vel = nullptr;
     int4* snap_cell = nullptr;
@@ -264,12 +265,8 @@ __global__ void k_f32_to_f64(int n3, const float* __restrict__ in, double* __res
 
 void free_all(sphx_ctx* c) {
     Buffers& b = c->b;
-    void* ptrs[] = {b.pos4, b.vel4,   b.pos4_s, b.vel4_s,     b.aux4_s,    b.acc4_s,
-                    b.key[0], b.key[1], b.val[0], b.val[1],   b.key_s,     b.id_s,
-                    b.off,  b.tiles, b.tgt, b.sync, b.diag_part, c->ds,
-                    c->stage, c->snap_pos, c->snap_vel, c->snap_cell, b.cell4, b.cell4_s,
-                    b.spread_tiles,
-                    b.scene_of, b.scene_s, b.scenes, b.records, b.tile_list,
+    void* ptrs[] = {c->arena, b.records, c->snap_pos, c->snap_vel, c->snap_cell,
+                    b.scene_of, b.scene_s, b.scenes,
                     c->r_colors, c->r_inst, c->r_keys, c->r_rgba};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -690,21 +687,32 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     const size_t C = capacity;
     b.diag_blocks = c->L.num_sms * 2;
     b.num_sms = c->L.num_sms;
-    if ((rc = dmalloc(&b.pos4, C)) || (rc = dmalloc(&b.vel4, C)) || (rc = dmalloc(&b.pos4_s, C)) ||
-        (rc = dmalloc(&b.vel4_s, C)) || (rc = dmalloc(&b.aux4_s, C)) ||
-        (rc = dmalloc(&b.acc4_s, C)) || (rc = dmalloc(&b.key[0], C)) ||
-        (rc = dmalloc(&b.key[1], C)) || (rc = dmalloc(&b.val[0], C)) ||
-        (rc = dmalloc(&b.val[1], C)) || (rc = dmalloc(&b.key_s, C)) ||
-        (rc = dmalloc(&b.id_s, C)) || (rc = dmalloc(&b.off, (size_t)max_cells + 2)) ||
-        (rc = dmalloc(&b.tiles, C)) ||         (rc = dmalloc(&b.diag_part, (size_t)b.diag_blocks * kDiagSums)) ||
-        (rc = dmalloc(&c->ds, 1)) || (rc = dmalloc(&c->stage, 11 * C)))
-        return fail(rc);
-    if (c->tuning.mode != SPHX_MODE_EXACT &&
-        ((rc = dmalloc(&b.cell4, C)) || (rc = dmalloc(&b.cell4_s, C)) ||
-         (rc = dmalloc(&b.spread_tiles, C))))
-        return fail(rc);
-    if ((rc = dmalloc(&b.tgt, 2 * C))) return fail(rc);
-    b.rank = b.tgt + C;
+    // everything but the pool in one allocation: with one each, making a context of 1M particles
+    // and uploading them took 2.8 ms, 0.7 of it for the pool; now as long as without a pool
+    std::vector<std::pair<void**, size_t>> parts;
+    size_t arena_bytes = 0;
+    auto part = [&](auto** p, size_t count) {
+        parts.emplace_back(reinterpret_cast<void**>(p), arena_bytes);
+        arena_bytes += (count * sizeof(**p) + 511) / 512 * 512;
+    };
+    unsigned char* scratch = nullptr;
+    for (float4** p : {&b.pos4, &b.vel4, &b.pos4_s, &b.vel4_s, &b.aux4_s, &b.acc4_s}) part(p, C);
+    for (uint32_t** p : {&b.key[0], &b.key[1], &b.val[0], &b.val[1], &b.key_s, &b.id_s, &b.tgt, &b.rank})
+        part(p, C);
+    part(&b.tiles, C);
+    part(&b.tile_list, C);
+    part(&b.off, (size_t)max_cells + 2);
+    part(&b.diag_part, (size_t)b.diag_blocks * kDiagSums);
+    part(&c->ds, 1);
+    part(&c->stage, 11 * C);
+    part(&scratch, grid_scratch_bytes(C));
+    if (c->tuning.mode != SPHX_MODE_EXACT) {
+        part(&b.cell4, C);
+        part(&b.cell4_s, C);
+        part(&b.spread_tiles, C);
+    }
+    if ((rc = dmalloc(&c->arena, arena_bytes))) return fail(rc);
+    for (const auto& [p, at] : parts) *p = c->arena + at;
     // Record pool (Buffers::records), in records (128 B) per particle of capacity: 3, or 4 where
     // few warps share it.  The lattice and uniform states need about 2 in exact mode
     // (32-particle tiles, the candidates their boxes keep) and 1 in the precision mode; the rest
@@ -715,25 +723,13 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     // 8k 56, 26 and 26, 14k 114, 113 and 45, 24k 184, 181 and 83, 30k 236, 229 and 110; lattice
     // 17k (two tiles a warp) 70, 42 and 42.  Without the pool (or where a warp's share runs out)
     // the force pass walks the candidates itself.
-    if (dmalloc(&b.tile_list, C) == SPHX_OK) {
-        unsigned long long cap = std::max<unsigned long long>(
-            (C > kManyParticles ? 3ull : 4ull) * C,
-            (c->tuning.mode == SPHX_MODE_EXACT ? 64ull : 0ull) *
-                std::min<unsigned long long>(C, kTeamMax));
-        if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
-        if (dmalloc(&b.records, (size_t)cap * 32) == SPHX_OK) {
-            b.record_cap = cap;
-        } else {
-            cudaGetLastError();
-            cudaFree(b.tile_list);
-            b.tile_list = nullptr;
-        }
-    } else {
-        cudaGetLastError();
-    }
+    unsigned long long cap = std::max<unsigned long long>(
+        (C > kManyParticles ? 3ull : 4ull) * C,
+        (c->tuning.mode == SPHX_MODE_EXACT ? 64ull : 0ull) * std::min<unsigned long long>(C, kTeamMax));
+    if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
+    if (dmalloc(&b.records, (size_t)cap * 32) == SPHX_OK) b.record_cap = cap;
+    else cudaGetLastError();
     // (look-back words of an absent epoch: an epoch is at least kMaxPasses)
-    unsigned char* scratch = nullptr;
-    if ((rc = dmalloc(&scratch, grid_scratch_bytes(C)))) return fail(rc);
     set_grid_scratch(b, scratch);
     if (cudaMemset(c->ds, 0, sizeof(DevState)) != cudaSuccess ||
         cudaMemset(scratch, 0, grid_scratch_bytes(C)) != cudaSuccess)
