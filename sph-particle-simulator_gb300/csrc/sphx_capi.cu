@@ -689,10 +689,14 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     b.num_sms = c->L.num_sms;
     // everything but the pool in one allocation: with one each, making a context of 1M particles
     // and uploading them took 2.8 ms, 0.7 of it for the pool; now as long as without a pool
-    std::vector<std::pair<void**, size_t>> parts;
+    struct {
+        void** p;
+        size_t at;
+    } parts[32];
     size_t arena_bytes = 0;
+    int nparts = 0;
     auto part = [&](auto** p, size_t count) {
-        parts.emplace_back(reinterpret_cast<void**>(p), arena_bytes);
+        parts[nparts++] = {reinterpret_cast<void**>(p), arena_bytes};
         arena_bytes += (count * sizeof(**p) + 511) / 512 * 512;
     };
     unsigned char* scratch = nullptr;
@@ -712,7 +716,7 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
         part(&b.spread_tiles, C);
     }
     if ((rc = dmalloc(&c->arena, arena_bytes))) return fail(rc);
-    for (const auto& [p, at] : parts) *p = c->arena + at;
+    for (int k = 0; k < nparts; ++k) *parts[k].p = c->arena + parts[k].at;
     // Record pool (Buffers::records), in records (128 B) per particle of capacity: 3, or 4 where
     // few warps share it.  The lattice and uniform states need about 2 in exact mode
     // (32-particle tiles, the candidates their boxes keep) and 1 in the precision mode; the rest

@@ -16,8 +16,8 @@ namespace sphx {
 // 16 take 0.97, 20 (16 warps) 1.05.
 //
 // Bound: instruction issue (72% of the slots) and the FP32 pipe (56%; a packed instruction
-// holds it two cycles).  Of 841 warp instructions per particle about 210 are distance tests
-// (900 kept candidates per tile, 29 chunks), 80 the walk and box cull, 500 the pair terms
+// holds it two cycles).  Of 882 warp instructions per particle about 220 are distance tests
+// (900 kept candidates per tile, 29 chunks), 110 the walk, box cull and lists, 500 the pair terms
 // (5 turns of two neighbours per lane and particle).  1M dam break: 0.96 ms; with hit lists
 // worked through by the whole warp and folded back lane by lane (1,502 instructions, of which
 // the lists and folds were half) 1.45 ms.

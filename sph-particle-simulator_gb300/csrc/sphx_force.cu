@@ -17,7 +17,7 @@ namespace sphx {
 // longer, 8 (16 warps) 13%, 10 (14 warps) 12%, 16 (8 warps) 21%.
 //
 // Bound: instruction issue (64% of the slots with 3 warps per scheduler) and the FP32 pipe
-// (58%; a packed instruction holds it two cycles): about 1,200 warp instructions per particle
+// (58%; a packed instruction holds it two cycles): about 1,130 warp instructions per particle
 // in 5.7 turns, each finishing one pair of neighbours per lane and starting the next.  1M dam
 // break, force + leapfrog: 1.44 ms (1.53 with 12 chunks and a branch at each new mask); walking
 // and culling the candidates again instead of reading the density pass's list 1.71 ms; with hit lists, terms passed through shared memory and
