@@ -69,12 +69,12 @@ DENSITY_BYTES_PER_PARTICLE = 24  # read x,m (16 B); write rho,P (8 B)
 # integer cell (12 B) plus an FP32 offset (12 B): force reads x (24), v, rho, P, m (24) and
 # writes x, v, a (48); density reads x, m (28) and writes rho, P (8).
 PASSES = {
-    "exact": {"force": "k_force<1,0,0,1,0,0> (force + leapfrog + clamp)",
-              "density": "k_density<0,0,1,0>", "force_bytes": FORCE_BYTES_PER_PARTICLE,
+    "exact": {"force": "k_force<1,0,0,1> (force + leapfrog + clamp)",
+              "density": "k_density<0,0,1>", "force_bytes": FORCE_BYTES_PER_PARTICLE,
               "density_bytes": DENSITY_BYTES_PER_PARTICLE, "issue_force": "k_force",
               "issue_density": "k_density", "traffic": "force"},
     "precise": {"force": "k_force_sweep<1,0,0> (force + leapfrog + clamp, tile sweep)",
-                "density": "k_density_sweep<0>", "force_bytes": 96, "density_bytes": 36,
+                "density": "k_density_sweep<0,0>", "force_bytes": 96, "density_bytes": 36,
                 "issue_force": "k_force_sweep", "issue_density": "k_density_sweep",
                 "traffic": "force_sweep"},
 }
@@ -122,7 +122,7 @@ def ncu_traffic(key: str, n: int):
     """Per-launch DRAM bytes of a force kernel ("force": exact mode, "force_sweep":
     precision mode) from the committed ncu summary (measured per particle on the 4.1M
     lattice, whose arrays exceed L2), scaled to this workload's particle count; returns
-    (total, hit-mask records part) or (None, None)."""
+    (total, candidate lists' part) or (None, None)."""
     p = REPO / "profiles" / "ncu_traffic.json"
     if not p.exists():
         return None, None
@@ -819,12 +819,12 @@ def bench_ours(args, world, rank, local):
                      "frac": achieved / peak, "traffic": traffic,
                      "traffic_hit_masks": traffic_masks,
                      "traffic_note": ("DRAM bytes per launch = the particle data (%.1fx the "
-                                      "%d B/particle algorithmic bytes) + the hit-mask records "
+                                      "%d B/particle algorithmic bytes) + the candidate lists "
                                       "the density pass wrote for this pass (read once)"
                                       % ((traffic - traffic_masks) / (ps["force_bytes"] * w.n),
                                          ps["force_bytes"])) if traffic and traffic_masks else
                                      ("DRAM bytes per launch = %.1fx the %d B/particle "
-                                      "algorithmic bytes (no hit-mask records in this mode)"
+                                      "algorithmic bytes, candidate lists included"
                                       % (traffic / (ps["force_bytes"] * w.n), ps["force_bytes"])
                                       if traffic else None),
                      "kernel": ps["force"],
