@@ -727,9 +727,15 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     // 8k 56, 26 and 26, 14k 114, 113 and 45, 24k 184, 181 and 83, 30k 236, 229 and 110; lattice
     // 17k (two tiles a warp) 70, 42 and 42.  Without the pool (or where a warp's share runs out)
     // the force pass walks the candidates itself.
-    unsigned long long cap = std::max<unsigned long long>(
-        (C > kManyParticles ? 3ull : 4ull) * C,
-        (c->tuning.mode == SPHX_MODE_EXACT ? 64ull : 0ull) * std::min<unsigned long long>(C, kTeamMax));
+    unsigned long long cap = (C > kManyParticles ? 3ull : 4ull) * C;
+    if (c->tuning.mode == SPHX_MODE_EXACT && C <= 4 * (size_t)kTeamMax) {
+        // at most 1/256 of the memory that is free, so that many contexts leave each other room
+        size_t free_bytes = 0, all_bytes = 0;
+        if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess) cudaGetLastError();
+        cap = std::max<unsigned long long>(
+            cap, std::min<unsigned long long>(64ull * std::min<size_t>(C, kTeamMax),
+                                              free_bytes / 256 / (32 * sizeof(uint32_t))));
+    }
     if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
     if (dmalloc(&b.records, (size_t)cap * 32) == SPHX_OK) b.record_cap = cap;
     else cudaGetLastError();
