@@ -187,7 +187,9 @@ int sphx_download(sphx_ctx* ctx, float* pos_xyz, float* vel_xyz, float* rho, flo
 /* Replaces the particle set from FP64 positions (host memory).  In the precision modes
  * the cell + offset split is taken in FP64, so positions keep their bits far from the
  * origin; in SPHX_MODE_EXACT positions are rounded to float.  Parameters must be set
- * first (the cell size is the search radius). */
+ * first (the cell size is the search radius).  Pinned arrays are read in place (see
+ * sphx_upload: in the precision modes keep them unchanged until the stream has reached the
+ * call; SPHX_MODE_EXACT has consumed them when the call returns). */
 int sphx_upload_f64(sphx_ctx* ctx, size_t n, const double* pos_xyz, const float* vel_xyz,
                     const float* mass);
 /* Current positions in FP64 (cell * cell_size + offset in the precision modes). */
@@ -235,7 +237,7 @@ int sphx_autotune(sphx_ctx* ctx, float dt, int* warps_per_block, int* blocks_per
 int sphx_get_tuning(sphx_ctx* ctx, sphx_tuning* out);
 
 /* Page-locked host memory for a caller's transfer buffers: sphx_upload reads such buffers in
- * place over the CPU-GPU link and sphx_download fills them with the copy engines at full
+ * place over the CPU-GPU link and sphx_download stores straight into them at the link's
  * speed (pageable buffers go through staging copies).  The drop-in SPHEngine keeps its
  * host mirror's transfer buffers here.  *out = NULL and SPHX_ERR_OOM when the allocation
  * fails.  No counterpart in the reference (its particle set never leaves the host). */

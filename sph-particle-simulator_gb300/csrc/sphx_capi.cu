@@ -922,14 +922,15 @@ int sphx_upload_f64(sphx_ctx* c, size_t n, const double* pos, const float* vel,
                               c->b.pos4, c->b.vel4);
         } else {
             k_f64_to_f32<<<c->L.num_sms * 4, 256, 0, c->stream>>>((int)(3 * n), src, s_posf);
-            // velocities staged after the conversion, in the place of the positions
-            float* s_vel2 = reinterpret_cast<float*>(s_pos);
-            SPHX_CUDA(cudaStreamSynchronize(c->stream));
             if (vel && !src_vel) {
+                // staged after the conversion, in the place of the positions
+                float* s_vel2 = reinterpret_cast<float*>(s_pos);
+                SPHX_CUDA(cudaStreamSynchronize(c->stream));
                 SPHX_CUDA(cudaMemcpyAsync(s_vel2, vel, 3 * n * sizeof(float), cudaMemcpyHostToDevice, c->stream));
                 src_vel = s_vel2;
             }
             launch_pack(c->L, (int)n, s_posf, src_vel, src_mass, c->b.pos4, c->b.vel4);
+            SPHX_CUDA(cudaStreamSynchronize(c->stream));  // the caller's arrays are consumed
         }
         SPHX_CUDA(cudaGetLastError());
     }
