@@ -286,7 +286,8 @@ int sphx_debug_pairs_subset(sphx_ctx* ctx, size_t nsel, const int64_t* sel, int6
  * sphx_grid_query returns, for every query point p, the indices j with
  * dot(p - x_j, p - x_j) <= radius_squared in the reference's order (stencil cells
  * (dx,dy,dz) in [-cr,cr]^3 lexicographically, cr = ceil(sqrt(r2) * inv_cell) + 1, then
- * insertion order), like SpatialHash::query_squared (src/spatial_hash.cpp:31-57). */
+ * insertion order), like SpatialHash::query_squared (src/spatial_hash.cpp:31-57).  Several
+ * host threads may query one built grid at the same time; a build needs it to itself. */
 typedef struct sphx_grid sphx_grid;
 int sphx_grid_create(sphx_grid** out, size_t capacity);
 void sphx_grid_destroy(sphx_grid* grid);

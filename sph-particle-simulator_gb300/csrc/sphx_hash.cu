@@ -8,11 +8,19 @@
 // lexicographic order -- and each cell's particles in insertion order, keeping those with
 // dot(p - x_j, p - x_j) <= r2: the reference's list, element for element.
 #include <cmath>
+#include <mutex>
+#include <utility>
 #include <vector>
 
 #include "sphx_internal.cuh"
 
 using namespace sphx;
+
+// Device blocks of one query, grown as needed.
+struct QueryWork {
+    void* p[4] = {};         // query points, counts, list offsets, lists
+    size_t bytes[4] = {};
+};
 
 struct sphx_grid {
     int device = 0;
@@ -27,14 +35,15 @@ struct sphx_grid {
     float* stage = nullptr;  // 4 * capacity floats
     LaunchCtx L{};
     DevState host{};         // copy of the device state after the last build
-    // Query workspace, grown as needed and kept for the next query (each allocation and release
-    // of the result array synchronises and takes 0.1 ms); a block above kKeepBytes is given
-    // back when the call returns.
-    void* work[4] = {};      // query points, counts, list offsets, lists
-    size_t work_bytes[4] = {};
+    // The query workspace of the last call, for the next one (each allocation and release of the
+    // result array synchronises and takes 0.1 ms).  A call takes it out of the grid for as long
+    // as it runs, so that calls from several threads never share a block: those that find it
+    // gone allocate their own.
+    QueryWork kept;
+    std::mutex kept_mutex;
 };
 
-constexpr size_t kKeepBytes = (size_t)256 << 20;
+constexpr size_t kKeepBytes = (size_t)256 << 20;  // of each block: a larger one is given back
 
 namespace {
 
@@ -159,34 +168,55 @@ int galloc(T** p, size_t count) {
     return SPHX_OK;
 }
 
-// the workspace block k with room for count elements
+// block k with room for count elements
 template <class T>
-int workspace(sphx_grid* g, int k, size_t count, T** p) {
+int workspace(QueryWork& w, int k, size_t count, T** p) {
     const size_t bytes = (count ? count : 1) * sizeof(T);
-    if (bytes > g->work_bytes[k]) {
-        if (g->work[k]) cudaFree(g->work[k]);
-        g->work[k] = nullptr;
-        g->work_bytes[k] = 0;
+    if (bytes > w.bytes[k]) {
+        if (w.p[k]) cudaFree(w.p[k]);
+        w.p[k] = nullptr;
+        w.bytes[k] = 0;
         unsigned char* q = nullptr;
         const int rc = galloc(&q, bytes);
         if (rc) return rc;
-        g->work[k] = q;
-        g->work_bytes[k] = bytes;
+        w.p[k] = q;
+        w.bytes[k] = bytes;
     }
-    *p = static_cast<T*>(g->work[k]);
+    *p = static_cast<T*>(w.p[k]);
     return SPHX_OK;
 }
-void trim_workspace(sphx_grid* g, size_t keep) {
+// gives back the blocks of more than `keep` bytes
+void trim(QueryWork& w, size_t keep) {
     for (int k = 0; k < 4; ++k)
-        if (g->work[k] && g->work_bytes[k] > keep) {
-            cudaFree(g->work[k]);
-            g->work[k] = nullptr;
-            g->work_bytes[k] = 0;
+        if (w.p[k] && w.bytes[k] > keep) {
+            cudaFree(w.p[k]);
+            w.p[k] = nullptr;
+            w.bytes[k] = 0;
         }
 }
 
+// The grid's workspace for the duration of a call.
+struct QueryWorkLease {
+    sphx_grid* g;
+    QueryWork w;
+    explicit QueryWorkLease(sphx_grid* grid) : g(grid) {
+        std::lock_guard<std::mutex> lock(g->kept_mutex);
+        std::swap(w, g->kept);
+    }
+    ~QueryWorkLease() {
+        trim(w, kKeepBytes);
+        {
+            std::lock_guard<std::mutex> lock(g->kept_mutex);
+            std::swap(w, g->kept);
+        }
+        trim(w, 0);  // another call's, given back in the meantime
+    }
+    QueryWorkLease(const QueryWorkLease&) = delete;
+    QueryWorkLease& operator=(const QueryWorkLease&) = delete;
+};
+
 void grid_free(sphx_grid* g) {
-    trim_workspace(g, 0);
+    trim(g->kept, 0);
     Buffers& b = g->b;
     void* ptrs[] = {b.pos4, b.vel4, b.pos4_s, b.vel4_s, b.key[0], b.key[1], b.val[0], b.val[1],
                     b.key_s, b.id_s, b.off, b.tiles, b.sync, g->ds, g->stage};
@@ -304,11 +334,9 @@ int sphx_grid_query(sphx_grid* g, size_t nq, const float* q_xyz, float radius_sq
     uint64_t* d_off = nullptr;
     int64_t* d_out = nullptr;
     int rc = SPHX_OK;
-    auto cleanup = [&]() { trim_workspace(g, kKeepBytes); };
-    if ((rc = workspace(g, 0, 3 * nq, &d_q)) || (rc = workspace(g, 1, nq, &d_cnt))) {
-        cleanup();
-        return rc;
-    }
+    QueryWorkLease lease(g);
+    QueryWork& work = lease.w;
+    if ((rc = workspace(work, 0, 3 * nq, &d_q)) || (rc = workspace(work, 1, nq, &d_cnt))) return rc;
     QueryArgs qa{d_q, (int)nq, radius_squared, cr, g->sc.inv_cell, g->cell_size};
     const int threads = 128, blocks = (int)((nq + threads / 32 - 1) / (threads / 32));
     std::vector<uint32_t> h_cnt(nq);
@@ -320,10 +348,7 @@ int sphx_grid_query(sphx_grid* g, size_t nq, const float* q_xyz, float radius_sq
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h_cnt.data(), d_cnt, nq * sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    if (e != cudaSuccess) {
-        cleanup();
-        return cuda_err(e);
-    }
+    if (e != cudaSuccess) return cuda_err(e);
     std::vector<uint64_t> off(nq);
     uint64_t total = 0;
     for (size_t i = 0; i < nq; ++i) {
@@ -332,18 +357,9 @@ int sphx_grid_query(sphx_grid* g, size_t nq, const float* q_xyz, float radius_sq
         total += h_cnt[i];
     }
     *total_inout = (size_t)total;
-    if (!idx || total == 0) {
-        cleanup();
-        return SPHX_OK;
-    }
-    if (cap < total) {
-        cleanup();
-        return SPHX_ERR_OVERFLOW;
-    }
-    if ((rc = workspace(g, 2, nq, &d_off)) || (rc = workspace(g, 3, total, &d_out))) {
-        cleanup();
-        return rc;
-    }
+    if (!idx || total == 0) return SPHX_OK;
+    if (cap < total) return SPHX_ERR_OVERFLOW;
+    if ((rc = workspace(work, 2, nq, &d_off)) || (rc = workspace(work, 3, total, &d_out))) return rc;
     e = cudaMemcpyAsync(d_off, off.data(), nq * sizeof(uint64_t), cudaMemcpyHostToDevice, g->stream);
     if (e == cudaSuccess) {
         k_grid_query<true><<<blocks, threads, 0, g->stream>>>(qa, g->b, g->ds, nullptr, d_off, d_out);
@@ -352,7 +368,6 @@ int sphx_grid_query(sphx_grid* g, size_t nq, const float* q_xyz, float radius_sq
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(idx, d_out, total * sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    cleanup();
     return e == cudaSuccess ? SPHX_OK : cuda_err(e);
 }
 
