@@ -187,9 +187,10 @@ int sphx_download(sphx_ctx* ctx, float* pos_xyz, float* vel_xyz, float* rho, flo
 /* Replaces the particle set from FP64 positions (host memory).  In the precision modes
  * the cell + offset split is taken in FP64, so positions keep their bits far from the
  * origin; in SPHX_MODE_EXACT positions are rounded to float.  Parameters must be set
- * first (the cell size is the search radius).  Pinned arrays are read in place (see
- * sphx_upload: in the precision modes keep them unchanged until the stream has reached the
- * call; SPHX_MODE_EXACT has consumed them when the call returns). */
+ * first (the cell size is the search radius).  Pinned arrays that are aligned to their
+ * elements are read in place (see sphx_upload: in the precision modes keep them unchanged
+ * until the stream has reached the call; SPHX_MODE_EXACT has consumed them when the call
+ * returns). */
 int sphx_upload_f64(sphx_ctx* ctx, size_t n, const double* pos_xyz, const float* vel_xyz,
                     const float* mass);
 /* Current positions in FP64 (cell * cell_size + offset in the precision modes). */

@@ -429,10 +429,12 @@ int run_step_graph(sphx_ctx* c, float dt) {
 
 // Device address of a host buffer the GPU can access in place (pinned: cudaHostAlloc or
 // cudaHostRegister), or null (pageable memory: the caller's data go through staging).
-// On Grace + Blackwell the kernels then read and write it over the coherent C2C link.
+// On Grace + Blackwell the kernels then read and write it over the coherent C2C link.  An array
+// that is not aligned to its elements goes through staging, too: the copies take any address,
+// the kernels' loads and stores do not.
 template <class T>
 T* mapped(T* h) {
-    if (!h) return nullptr;
+    if (!h || reinterpret_cast<uintptr_t>(h) % alignof(T) != 0) return nullptr;
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, h) != cudaSuccess) {
         cudaGetLastError();
