@@ -80,7 +80,9 @@ namespace {
 
 constexpr int kDefaultWarpsPerBlock = 4;
 
+// (the runtime's record of the error is cleared: it is this call's to report, not the next one's)
 int cuda_fail(cudaError_t e) {
+    cudaGetLastError();
     if (e == cudaErrorMemoryAllocation) return SPHX_ERR_OOM;
     return SPHX_ERR_CUDA;
 }

@@ -150,7 +150,11 @@ __global__ void __launch_bounds__(128) k_grid_query(const QueryArgs a, const Buf
     if (!kFill && lane == 0) counts[qi] = found;
 }
 
-int cuda_err(cudaError_t e) { return e == cudaErrorMemoryAllocation ? SPHX_ERR_OOM : SPHX_ERR_CUDA; }
+// (the runtime's record of the error is cleared: it is this call's to report, not the next one's)
+int cuda_err(cudaError_t e) {
+    cudaGetLastError();
+    return e == cudaErrorMemoryAllocation ? SPHX_ERR_OOM : SPHX_ERR_CUDA;
+}
 
 #define GRID_CUDA(call)                             \
     do {                                            \
@@ -162,6 +166,7 @@ template <class T>
 int galloc(T** p, size_t count) {
     *p = nullptr;
     if (cudaMalloc(reinterpret_cast<void**>(p), (count ? count : 1) * sizeof(T)) != cudaSuccess) {
+        cudaGetLastError();
         *p = nullptr;
         return SPHX_ERR_OOM;
     }
