@@ -10,6 +10,8 @@
 #include <utility>
 #include <vector>
 
+#include <cuda.h>
+
 #include "sphx_internal.cuh"
 
 using namespace sphx;
@@ -446,11 +448,46 @@ T* mapped(T* h) {
                                                              : nullptr;
 }
 
-// The same for an array of which every element is pinned.
+// The pinned range (one cudaHostAlloc or cudaHostRegister) that holds address p; false: none.
+bool pinned_range(const void* p, uintptr_t* first, size_t* bytes) {
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = []() -> Query {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault,
+                                             &found) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(f) : nullptr;
+    }();
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    CUdeviceptr start = 0;
+    *bytes = 0;
+    void* into[] = {&start, bytes};
+    if (!query || query(2, what, into, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return false;
+    *first = static_cast<uintptr_t>(start);
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    return *bytes && at >= *first && at - *first < *bytes;
+}
+
+// The same for an array of which every byte is pinned (an array may lie in several ranges that
+// follow one another; two with pageable memory between them do not do).
 template <class T>
 T* mapped(T* h, size_t count) {
-    T* d = mapped(h);
-    return d && mapped(h + (count - 1)) == d + (count - 1) ? d : nullptr;
+    T* const d = mapped(h);
+    if (!d) return nullptr;
+    const uintptr_t begin = reinterpret_cast<uintptr_t>(h), end = begin + count * sizeof(T);
+    for (uintptr_t at = begin; at < end;) {
+        const char* p = reinterpret_cast<const char*>(at);
+        if (at > begin && mapped(p) != reinterpret_cast<const char*>(d) + (at - begin)) return nullptr;
+        uintptr_t first = 0;
+        size_t bytes = 0;
+        if (!pinned_range(p, &first, &bytes)) return nullptr;
+        at = first + bytes;
+    }
+    return d;
 }
 
 // ---- headless rendering helpers ----------------------------------------------------------

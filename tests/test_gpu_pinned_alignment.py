@@ -92,3 +92,49 @@ def test_floats_at_odd_addresses(built, n, shift):
             assert got[shift:shift + len(w)] == w, k
             assert not any(got[:shift]) and not any(got[shift + len(w):]), k
     ctx.close()
+
+
+def register(cudart, a, first, bytes_):
+    assert int(cudart.cudaHostRegister(a.ctypes.data + first, bytes_, 0)) == 0
+
+
+@pytest.mark.parametrize("gap", [False, True])
+def test_arrays_across_two_registrations(built, gap):
+    """Two registered ranges that follow one another are pinned memory throughout; with pageable
+    memory between them an array is neither one nor the other, which the copies refuse."""
+    import torch
+
+    n, page = 60_000, 65536
+    pos, vel, mass = particles(n)
+    ctx = context(n, sphx.MODE_EXACT)
+    ctx.upload_f64(pos, vel, mass)
+    want = state_after_step(ctx)
+    raw = np.zeros(25 * page, np.uint8)
+    block = raw[-raw.ctypes.data % page:][:24 * page]  # whole pages
+    cudart = torch.cuda.cudart()
+    first = 4 * page
+    register(cudart, block, 0, first)
+    second = first + (page if gap else 0)
+    register(cudart, block, second, 24 * page - second)
+    try:
+        put(block, 0, pos)
+        assert first < pos.nbytes < 24 * page and second < 3 * 4 * n
+        f = ctx._lib.sphx_upload_f64
+        rc = f(ctx._h, n, block.ctypes.data, vel.ctypes.data, mass.ctypes.data)
+        assert (rc != sphx.OK) == gap
+        if not gap:
+            ctx.set_time(0.0)
+            same(state_after_step(ctx), want)
+        block[:] = 0
+        ctx.upload_f64(pos, vel, mass)
+        ctx.set_time(0.0)
+        ctx.step(1e-4)
+        rc = ctx._lib.sphx_download(ctx._h, block.ctypes.data, None, None, None, None)
+        assert (rc != sphx.OK) == gap
+        got = block[:want["pos"].nbytes].tobytes()
+        assert got == (b"\0" * len(got) if gap else want["pos"].tobytes())
+        same(ctx.download(), {k: v for k, v in want.items() if k != "pos64"})
+    finally:
+        ctx.close()
+        for at in (0, second):
+            cudart.cudaHostUnregister(block.ctypes.data + at)
