@@ -20,6 +20,12 @@ namespace cg = cooperative_groups;
 constexpr int kSmallCtas = 16, kSmallThreads = 1024, kSmallWarps = kSmallThreads / 32;
 constexpr int kSmallPer = kSmallMax / kSmallCtas;  // particles of a CTA at most
 static_assert(kSmallPer % kSmallThreads == 0, "whole rounds");
+// Runs of empty cells (their offsets are all the same): up to kShortRun are written by the thread
+// of the particle behind them, longer ones by its warp, and those above 1/kMaxRuns of the grid
+// (and kLongRun) by the whole cluster.  16 million cells, us for the density and force passes and
+// the build with a thread for each run, whatever its length, and now: 4k particles spread evenly
+// 2,190 and 319, 33k 961 and 254, 64k 818 and 322; two clumps far apart 69,000 and 120 to 410.
+constexpr uint32_t kShortRun = 8, kLongRun = 1 << 16, kMaxRuns = 256;
 
 struct SmallSmem {
     uint2 item[2][kSmallPer];  // (key, insertion index): the sort's two buffers
@@ -29,6 +35,8 @@ struct SmallSmem {
     uint32_t scan[kSmallWarps];
     uint32_t flags[kSmallPer / 32 + 1], flags_before[kSmallPer / 32];
     uint32_t occ, max_occ, base;
+    uint32_t runs;  // for the cluster: first cell, last cell + 1, offset (the same in every CTA)
+    uint3 run[kMaxRuns];
     PrepPart part;
     DevState ds;                               // the step's grid
     alignas(4) uint8_t lev[kSmallPer + 2 * kZOrderMax];  // z levels, with those of the neighbours' ends
@@ -54,6 +62,16 @@ __device__ __forceinline__ uint32_t scan_block(uint32_t x, uint32_t* warp_sums, 
     return before + inc - x;
 }
 
+// off[from .. to) = value, by `workers` (at least 4) threads; off is 16-byte aligned
+__device__ __forceinline__ void fill_cells(uint32_t* off, uint32_t from, uint32_t to, uint32_t value,
+                                           uint32_t worker, uint32_t workers) {
+    const uint32_t a = min((from + 3u) & ~3u, to), e = max(a, to & ~3u);
+    if (worker < a - from) off[from + worker] = value;
+    if (worker < to - e) off[e + worker] = value;
+    for (uint32_t q = a + 4u * worker; q < e; q += 4u * workers)
+        *reinterpret_cast<uint4*>(off + q) = make_uint4(value, value, value, value);
+}
+
 template <bool kCells, bool kVmax>
 __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads, 1)
     k_grid_small(const StepConst c, const Buffers b, DevState* ds, int how, float host_dt, int per) {
@@ -70,7 +88,10 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
     PrepPart p = prep_empty();
     for (int i = tid; i < mine; i += kSmallThreads) prep_add<kCells, kVmax>(p, c, b, lo + i);
     p = merge_block<kSmallThreads>(p);
-    if (tid == 0) S.part = p;
+    if (tid == 0) {
+        S.part = p;
+        S.runs = 0;
+    }
     cluster.sync();
     if (warp == 0) {
         p = prep_empty();
@@ -180,25 +201,54 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
     // gather, sorted keys and permutation, cell offsets (see k_reorder), z levels
     const uint2* sorted = S.item[passes & 1];
     const float levels = 16.0f / c.cs;
-    for (int k = tid; k < mine; k += kSmallThreads) {
-        const uint2 it = sorted[k];
-        const int at = lo + k;
-        uint32_t prev = 0xffffffffu;  // + 1 = 0
-        if (k > 0) prev = sorted[k - 1].x;
-        else if (rank > 0) prev = remote(rank - 1)->item[passes & 1][per - 1].x;
-        for (uint32_t q = prev + 1u; q <= it.x; ++q) b.off[q] = (uint32_t)at;
-        if (at == n - 1)
-            for (uint32_t q = it.x + 1u; q <= nc + 1u; ++q) b.off[q] = (uint32_t)n;
-        const float4 pos = b.pos4[it.y];
-        b.key_s[at] = it.x;
-        b.id_s[at] = it.y;
-        if (b.rank) b.rank[it.y] = (uint32_t)at;
-        b.pos4_s[at] = pos;
-        b.vel4_s[at] = b.vel4[it.y];
-        if (kCells) b.cell4_s[at] = b.cell4[it.y];
-        S.lev[kZOrderMax + k] = z_level_of(pos.z, kCells, c.inv_cell, levels);
+    const uint32_t long_run = max(kLongRun, nc / kMaxRuns);  // at most kMaxRuns are longer
+    // the lanes' runs: off[from .. to) = value
+    auto put_runs = [&](uint32_t from, uint32_t to, uint32_t value) {
+        const bool by_warp = to - from > kShortRun;
+        if (!by_warp)
+            for (uint32_t q = from; q < to; ++q) b.off[q] = value;
+        for (uint32_t todo = __ballot_sync(0xffffffffu, by_warp); todo; todo &= todo - 1u) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t f = __shfl_sync(0xffffffffu, from, src),
+                           t = __shfl_sync(0xffffffffu, to, src),
+                           v = __shfl_sync(0xffffffffu, value, src);
+            if (t - f <= long_run) {
+                fill_cells(b.off, f, t, v, (uint32_t)lane, 32u);
+            } else if (lane < kSmallCtas) {
+                SmallSmem* R = remote(lane);
+                const uint32_t slot = atomicAdd(&R->runs, 1u);
+                if (slot < kMaxRuns) R->run[slot] = make_uint3(f, t, v);  // always
+            }
+        }
+    };
+    for (int k0 = warp * 32; k0 < mine; k0 += kSmallThreads) {
+        const int k = k0 + lane, at = lo + k;
+        uint32_t from = 0, to = 0;
+        if (k < mine) {
+            const uint2 it = sorted[k];
+            const float4 pos = b.pos4[it.y];
+            to = it.x + 1u;
+            if (k > 0) from = sorted[k - 1].x + 1u;
+            else if (rank > 0) from = remote(rank - 1)->item[passes & 1][per - 1].x + 1u;
+            b.key_s[at] = it.x;
+            b.id_s[at] = it.y;
+            if (b.rank) b.rank[it.y] = (uint32_t)at;
+            b.pos4_s[at] = pos;
+            b.vel4_s[at] = b.vel4[it.y];
+            if (kCells) b.cell4_s[at] = b.cell4[it.y];
+            S.lev[kZOrderMax + k] = z_level_of(pos.z, kCells, c.inv_cell, levels);
+        }
+        put_runs(from, to, (uint32_t)at);
+        if (lo + k0 + 32 >= n)  // the cells after the last particle's
+            put_runs(at == n - 1 ? to : 0u, at == n - 1 ? nc + 2u : 0u, (uint32_t)n);
     }
     cluster.sync();
+    if (S.runs) {
+        for (uint32_t r = 0; r < min(S.runs, kMaxRuns); ++r)
+            fill_cells(b.off, S.run[r].x, S.run[r].y, S.run[r].z, (uint32_t)(rank * kSmallThreads + tid),
+                       (uint32_t)(kSmallCtas * kSmallThreads));
+        cluster.sync();
+    }
 
     // in-cell order and tiles (see k_order_tiles)
     const bool folded_cells = !kCells && S.ds.wrap[2];
