@@ -597,7 +597,8 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep(const StepConst c, const
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
     const float kg = sweep_kg(c);
-    const F2 kappa = f2(sweep_kappa(c));
+    const float visc = sweep_kappa(c);
+    const F2 kappa = f2(visc);
     const TileQueue queue(&ds->work[1], b.num_sms);
     for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
@@ -644,8 +645,10 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep(const StepConst c, const
             S->pf[lane] = pf;
             S->cf[lane] = pf * d.a.y;
             __syncwarp();
-            // a non-finite velocity or factor is not cancelled by a zero factor
-            return kCut || __any_sync(kFull, !isfinite(d.v.x + d.v.y + d.v.z + d.a.y + pf));
+            // a non-finite velocity or factor (the pressure's, the viscosity's) is not cancelled
+            // by a zero shape
+            return kCut || __any_sync(kFull, !isfinite(d.v.x + d.v.y + d.v.z + d.a.y +
+                                                       pf * d.a.y + pf * visc));
         };
         auto sweep = [&](bool masked, int left) {
             F2 Fx = f2(0.0f), Fy = Fx, Fz = Fx;

@@ -1,0 +1,38 @@
+"""The precision mode's force sweep over the density sweep's candidate lists."""
+import numpy as np
+import pytest
+
+import sphx
+import sphx_inputs as I
+
+pytestmark = pytest.mark.gpu
+
+
+def evaluate(pos, vel, mass, prm, capacity=0, kernel=0, mode=sphx.MODE_PRECISE):
+    ctx = sphx.Context(max(capacity, len(pos)), mode=mode)
+    ctx.set_params(prm)
+    ctx.set_kernel(kernel)
+    ctx.upload(pos, vel, mass)
+    ctx.eval()
+    out = ctx.download()
+    ctx.close()
+    return out
+
+
+@pytest.mark.parametrize("kernel", [sphx.KERNEL_CUBIC_SPLINE, sphx.KERNEL_WENDLAND_C2])
+def test_an_overflowing_viscosity_factor_reaches_neighbours_only(built, kernel):
+    """A particle whose viscosity factor overflows beside a clump whose factors do not: the
+    clump's particles out of its reach feel nothing of it.  The velocities are zero, so that
+    they get what they get without viscosity."""
+    rng = np.random.default_rng(1)
+    u = rng.standard_normal((200, 3))
+    clump = 0.5 + 0.004 * u / np.linalg.norm(u, axis=1)[:, None]
+    pos = np.concatenate([clump, [[0.54, 0.5, 0.5]]]).astype(np.float32)
+    vel, mass = np.zeros_like(pos), np.full(len(pos), 1e-3, np.float32)
+    # (m / rho) mu kl: 1.5 mu / h^2 and 5 mu / h^2 on its own, 1/200 of that in the clump
+    want = evaluate(pos, vel, mass, I.params16(gas_constant=2e-3, viscosity=0.0), kernel=kernel)
+    got = evaluate(pos, vel, mass, I.params16(gas_constant=2e-3, viscosity=2e35), kernel=kernel)
+    away = np.linalg.norm(pos.astype(np.float64) - pos[-1], axis=1) > 0.0401
+    assert 20 < away.sum() < 180
+    assert got["acc"][away].tobytes() == want["acc"][away].tobytes()
+    assert got["rho"].tobytes() == want["rho"].tobytes()
