@@ -424,9 +424,9 @@ __host__ __device__ __forceinline__ float sweep_kl(const StepConst& c) {
 }
 
 // The viscosity factor kl (m_j / rho_j) mu is the pressure factor kg m_j / (2 rho_j) times
-// this constant.
+// this constant (kl mu on its own could overflow where no particle's factor does).
 __host__ __device__ __forceinline__ float sweep_kappa(const StepConst& c) {
-    return 2.0f * sweep_kl(c) * c.visc / sweep_kg(c);
+    return 2.0f * sweep_kl(c) / sweep_kg(c) * c.visc;
 }
 
 // (|r|/h)^2 of a pair is formed with kCoincident added: far below the rounding of any other pair
