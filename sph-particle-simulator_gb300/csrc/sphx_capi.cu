@@ -204,11 +204,12 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
     s.rcp_hsq = 1.0f / s.h_sq;
     s.fast_div_h = verify_fixed_divisor(h) ? 1 : 0;
     s.fast_div_hsq = verify_fixed_divisor(s.h_sq) ? 1 : 0;
-    // the cubic passes' untested divisions: |r| of a hit is at most r (1 + 2^-23) and the
+    // the pair forms' untested divisions: |r| of a hit is at most r (1 + 2^-23) and the
     // Laplacian's numerator at most 2 sigma; both divisors verified (so h, h^2 in
-    // [2^-20, 2^20] and sigma = 1/(pi h^3) within [2^-62, 2^59])
+    // [2^-20, 2^20] and sigma = 1/(pi h^3) within [2^-62, 2^59]); their square root takes
+    // |r|^2 of up to 2^86 (sqrt2_exact)
     s.div_nz = s.fast_div_h && s.fast_div_hsq && p.neighbor_search_radius > 0.0f &&
-                       p.neighbor_search_radius <= 0x1p99f
+                       p.neighbor_search_radius <= 0x1p43f
                    ? 1 : 0;
     // the force pass's divisions by |r| or |r| h through one reciprocal, and of the cubic
     // spline's gradient components by h: with |x_t - x_j| per axis 0 or at least 2^-68, the
