@@ -36,3 +36,16 @@ def test_an_overflowing_viscosity_factor_reaches_neighbours_only(built, kernel):
     assert 20 < away.sum() < 180
     assert got["acc"][away].tobytes() == want["acc"][away].tobytes()
     assert got["rho"].tobytes() == want["rho"].tobytes()
+
+
+@pytest.mark.parametrize("kernel", [sphx.KERNEL_CUBIC_SPLINE, sphx.KERNEL_WENDLAND_C2,
+                                    sphx.KERNEL_GAUSSIAN])
+@pytest.mark.parametrize("h", [7e11, 1e12])
+def test_lengths_whose_kernel_gradient_underflows(built, kernel, h):
+    """Kernel gradients below the smallest float give no force: gravity is what remains."""
+    rng = np.random.default_rng(2)
+    pos = (4 * h * rng.random((300, 3))).astype(np.float32)
+    vel = rng.standard_normal(pos.shape).astype(np.float32)
+    prm = I.params16(smoothing_length=h, neighbor_search_radius=2 * h)
+    acc = evaluate(pos, vel, np.full(len(pos), 2.0 ** 120, np.float32), prm, kernel=kernel)["acc"]
+    assert np.array_equal(acc, np.tile(np.float32([0.0, prm[6], 0.0]), (300, 1)))
