@@ -770,13 +770,23 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     // 17k (two tiles a warp) 70, 42 and 42.  Without the pool (or where a warp's share runs out)
     // the force pass walks the candidates itself.
     unsigned long long cap = (C > kManyParticles ? 3ull : 4ull) * C;
-    if (c->tuning.mode == SPHX_MODE_EXACT && C <= 4 * (size_t)kTeamMax) {
-        // at most 1/256 of the memory that is free, so that many contexts leave each other room
+    const bool exact = c->tuning.mode == SPHX_MODE_EXACT;
+    if (!exact || C <= 4 * (size_t)kTeamMax) {
         size_t free_bytes = 0, all_bytes = 0;
         if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess) cudaGetLastError();
-        cap = std::max<unsigned long long>(
-            cap, std::min<unsigned long long>(64ull * std::min<size_t>(C, kTeamMax),
-                                              free_bytes / 256 / (32 * sizeof(uint32_t))));
+        constexpr size_t kRecord = 32 * sizeof(uint32_t);
+        if (exact) {
+            // at most 1/256 of the memory that is free, so that many contexts leave each other room
+            cap = std::max<unsigned long long>(
+                cap, std::min<unsigned long long>(64ull * std::min<size_t>(C, kTeamMax),
+                                                  free_bytes / 256 / kRecord));
+        } else {
+            // at most half of what a snapshot leaves free: the precision mode runs without a pool,
+            // and a set that fills the memory keeps room for what its program allocates later
+            const size_t snap = C * (2 * sizeof(float4) + sizeof(int4));
+            cap = std::min<unsigned long long>(
+                cap, (free_bytes > snap ? free_bytes - snap : 0) / 2 / kRecord);
+        }
     }
     if (cap > 0xffff0000ull) cap = 0xffff0000ull;  // record indices are 32-bit
     if (dmalloc(&b.records, (size_t)cap * 32) == SPHX_OK) b.record_cap = cap;
