@@ -417,12 +417,20 @@ __host__ __device__ __forceinline__ float sweep_kg(const StepConst& c) {
     if (c.kern == SPHX_KERNEL_WENDLAND_C2) return 5.0f * c.wnorm * c.rcp_h;
     return -0.5f * c.sigma * c.rcp_h;
 }
+__host__ __device__ __forceinline__ float sweep_kl(const StepConst& c) {
+    if (c.kern == SPHX_KERNEL_GAUSSIAN) return c.gl;
+    if (c.kern == SPHX_KERNEL_WENDLAND_C2) return c.wl;
+    return c.sigma * c.rcp_hsq;
+}
+
 // The viscosity factor kl (m_j / rho_j) mu is the pressure factor kg m_j / (2 rho_j) times
-// 2 kl / kg mu, whose quotient is a multiple of 1/h for every kernel (formed from kl and kg it
-// would be 0 / 0 where they underflow, for h above some 1e11).
+// this constant (kl mu on its own could overflow where no particle's factor does).  Where kl or
+// kg underflows (h above some 1e9) the quotient is written as the multiple of 1/h that it is.
 __host__ __device__ __forceinline__ float sweep_kappa(const StepConst& c) {
+    const float kl = sweep_kl(c), kg = sweep_kg(c);
     const float k = c.kern == SPHX_KERNEL_CUBIC_SPLINE ? -4.0f : 2.0f;
-    return k * c.rcp_h * c.visc;
+    const bool normal = fminf(fabsf(kl), fabsf(kg)) >= 0x1p-126f;
+    return (normal ? 2.0f * kl / kg : k * c.rcp_h) * c.visc;
 }
 
 // (|r|/h)^2 of a pair is formed with kCoincident added: far below the rounding of any other pair
