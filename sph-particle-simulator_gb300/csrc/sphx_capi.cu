@@ -45,7 +45,7 @@ struct sphx_ctx {
     // or the stats are requested, so profiling adds no per-step host sync
     // batched scenes
     uint32_t nscenes = 0;
-    bool scenes_div_nz = false, scenes_force_nz = false;  // StepConst's flags hold for every scene
+    int scenes_div_nz = 0, scenes_force_nz = 0;  // the least of StepConst's over the scenes
     uint32_t scene_cap = 0;
     std::vector<sphx_params> scene_params;
     std::vector<uint64_t> scene_start;
@@ -214,12 +214,13 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
     // the force pass's divisions by |r| or |r| h through one reciprocal, and of the cubic
     // spline's gradient components by h: with |x_t - x_j| per axis 0 or at least 2^-68, the
     // smallest nonzero component is at least gmin 2^-68 / r, gmin the smallest nonzero
-    // gradient factor -- sigma 2^-47 for 2 - q >= 2^-23, 0.49 sigma q for q >= 1e-6 / h
+    // gradient factor -- sigma 2^-47 for 2 - q >= 2^-23, 0.49 sigma q for q >= 1e-6 / h.  Where
+    // that is too small (h above 0.045 for r = 2h) the pass asks each pair (kCheck)
     s.force_nz = 0;
     if (s.div_nz && p.neighbor_search_radius <= 0x1p20f) {
         const double r = p.neighbor_search_radius, q1 = 0.49 * std::min(1e-6 / h, 1.0);
         const double gmin = (double)s.sigma * std::min(0x1p-47, q1);
-        s.force_nz = kernel == SPHX_KERNEL_WENDLAND_C2 || gmin * 0x1p-68 / r >= 0x1p-99;
+        s.force_nz = kernel == SPHX_KERNEL_WENDLAND_C2 || gmin * 0x1p-68 / r >= 0x1p-99 ? 2 : 1;
     }
     s.precise = mode != SPHX_MODE_EXACT;
     s.fp16 = mode == SPHX_MODE_PRECISE_FP16;
@@ -360,8 +361,8 @@ int run_phases(sphx_ctx* c, float dt, bool integrate) {
     const bool batch = c->b.nscenes > 0;
     if (c->tile_auto) c->b.tile_n = pass_tile((int)c->n, c->sc.precise && !batch);
     if (batch) {  // the passes' kernels serve all scenes
-        c->sc.div_nz = c->scenes_div_nz ? 1 : 0;
-        c->sc.force_nz = c->scenes_force_nz ? 1 : 0;
+        c->sc.div_nz = c->scenes_div_nz;
+        c->sc.force_nz = c->scenes_force_nz;
     }
     int k = 0;
     const int how = !integrate ? kNoStep : (dt <= 0.0f ? kCflDt : kHostDt);
@@ -877,11 +878,12 @@ int sphx_set_kernel(sphx_ctx* c, int kernel) {
             std::vector<SceneInfo> info(c->nscenes);
             SPHX_CUDA(cudaMemcpy(info.data(), c->b.scenes, c->nscenes * sizeof(SceneInfo),
                                  cudaMemcpyDeviceToHost));
-            c->scenes_div_nz = c->scenes_force_nz = true;
+            c->scenes_div_nz = 1;
+            c->scenes_force_nz = 2;
             for (uint32_t s = 0; s < c->nscenes; ++s) {
                 fill_step_const_from(c, c->scene_params[s], info[s].count, info[s].c);
-                c->scenes_div_nz = c->scenes_div_nz && info[s].c.div_nz;
-                c->scenes_force_nz = c->scenes_force_nz && info[s].c.force_nz;
+                c->scenes_div_nz = std::min(c->scenes_div_nz, info[s].c.div_nz);
+                c->scenes_force_nz = std::min(c->scenes_force_nz, info[s].c.force_nz);
             }
             SPHX_CUDA(cudaMemcpy(c->b.scenes, info.data(), c->nscenes * sizeof(SceneInfo),
                                  cudaMemcpyHostToDevice));
@@ -1057,10 +1059,10 @@ int sphx_set_scenes(sphx_ctx* c, uint32_t nscenes, const uint64_t* scene_start,
         fill_step_const_from(c, params[s], si.count, si.c);
         for (uint64_t i = scene_start[s]; i < scene_start[s + 1]; ++i) owner[i] = s;
     }
-    bool div_nz = true, force_nz = true;
+    int div_nz = 1, force_nz = 2;
     for (const SceneInfo& si : info) {
-        div_nz = div_nz && si.c.div_nz;
-        force_nz = force_nz && si.c.force_nz;
+        div_nz = std::min(div_nz, si.c.div_nz);
+        force_nz = std::min(force_nz, si.c.force_nz);
     }
     SPHX_CUDA(cudaStreamSynchronize(c->stream));
     SPHX_CUDA(cudaMemcpy(b.scenes, info.data(), nscenes * sizeof(SceneInfo), cudaMemcpyHostToDevice));

@@ -151,11 +151,11 @@ __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Bu
             // the per-candidate factors of the force pass's pair terms, each formed once here
             // with the rounding the reference applies per pair: (rho, P, (m / rho) mu, 1 / 2 rho)
             const float mr = xdiv(xi.w, rho);
-            b.aux4_s[i] = make_float4(rho, P, xmul(mr, c.visc), __frcp_rn(xmul(2.0f, rho)));
-            // outside these ranges the force pass divides by 2 rho in the general way
-            if (!(rho >= 0x1p-30f && rho <= 0x1p40f) ||
-                !(P == 0.0f || (fabsf(P) >= 0x1p-40f && fabsf(P) <= 0x1p60f)))
-                ds->general = 1;
+            // (0: the force pass takes the particle's pairs in the general form)
+            const bool in = pair_range(rho, P);
+            b.aux4_s[i] = make_float4(rho, P, xmul(mr, c.visc),
+                                      in ? __frcp_rn(xmul(2.0f, rho)) : 0.0f);
+            if (!in) ds->general = 1;
             b.vel4_s[i].w = rho;  // read with the candidate's velocity by the force pass
             my_max = max(my_max, nn);
         }

@@ -56,16 +56,22 @@ __device__ __noinline__ ForceSums add_term_general(const StepConst& c, float4 xt
     return F;
 }
 
-// pair_terms of `p`, added to the sums in order (a if ha, b if hb)
+// add_term_general of the candidate in ring slot q
 template <int K>
-__device__ __forceinline__ void add_pair(const PairLits& k, const PairConst& c, const float4& vt,
-                                         float Pt, const PairStart& p, const float4& va,
-                                         const float4& vb, const float2& fa, const float2& fb,
-                                         ForceSums& F) {
-    const PairTerms t = pair_terms<K>(k, c, vt, Pt, p, va, vb, fa, fb);
+__device__ __forceinline__ void add_slot_general(const StepConst& c, const ForceSmem* S, int q,
+                                                 const float4& xt, const float4& vt, float Pt,
+                                                 ForceSums& F) {
+    const float4 vj = S->vel[q];
+    const float Pj = xmul(c.gas, xsub(vj.w, c.rest));
+    F = add_term_general<K>(c, xt, vt, Pt, S->pos[q], vj,
+                            make_float4(vj.w, Pj, xmul(2.0f, vj.w), S->fac[q].x), F);
+}
+
+// the terms added to the sums in order (a if ha, b if hb)
+__device__ __forceinline__ void add_terms(const PairTerms& t, bool ha, bool hb, ForceSums& F) {
     const float2 ax = upk2(t.px.v), ay = upk2(t.py.v), az = upk2(t.pz.v);
     const float2 bx = upk2(t.wx.v), by = upk2(t.wy.v), bz = upk2(t.wz.v);
-    if (p.ha) {
+    if (ha) {
         F.px = xadd(F.px, ax.x);
         F.py = xadd(F.py, ay.x);
         F.pz = xadd(F.pz, az.x);
@@ -73,7 +79,7 @@ __device__ __forceinline__ void add_pair(const PairLits& k, const PairConst& c, 
         F.vy = xadd(F.vy, by.x);
         F.vz = xadd(F.vz, bz.x);
     }
-    if (p.hb) {
+    if (hb) {
         F.px = xadd(F.px, ax.y);
         F.py = xadd(F.py, ay.y);
         F.pz = xadd(F.pz, az.y);
@@ -83,9 +89,58 @@ __device__ __forceinline__ void add_pair(const PairLits& k, const PairConst& c, 
     }
 }
 
+// pair_terms of `p`, added to the sums
+template <int K>
+__device__ __forceinline__ void add_pair(const PairLits& k, const PairConst& c, const float4& vt,
+                                         float Pt, const PairStart& p, const float4& va,
+                                         const float4& vb, const float2& fa, const float2& fb,
+                                         ForceSums& F) {
+    add_terms(pair_terms<K>(k, c, vt, Pt, p, va, vb, fa, fb), p.ha, p.hb, F);
+}
+
+// pair_terms of two neighbours with the answer whether they are in range, added to the sums: in
+// the general form where one of the two, or the lane's own particle (`out`), is not.
+template <int K>
+__device__ __forceinline__ void add_pair_checked(const PairLits& k, const StepConst& c,
+                                                 const ForceSmem* S, const float4& xt,
+                                                 const float4& vt, float Pt, bool out,
+                                                 const PairStart& p, ForceSums& F) {
+    const PairTerms t = pair_terms<K, true>(k, c.pair, vt, Pt, p, S->vel[p.qa], S->vel[p.qb],
+                                            S->fac[p.qa], S->fac[p.qb]);
+    if (((out || !t.oka) && p.ha) || ((out || !t.okb) && p.hb)) {
+        if (p.ha) add_slot_general<K>(c, S, p.qa, xt, vt, Pt, F);
+        if (p.hb) add_slot_general<K>(c, S, p.qb, xt, vt, Pt, F);
+    } else {
+        add_terms(t, p.ha, p.hb, F);
+    }
+}
+// the same as a call
+template <int K>
+__device__ __noinline__ ForceSums add_slots_checked(const PairLits& k, const StepConst& c,
+                                                    const ForceSmem* S, float4 xt, float4 vt,
+                                                    float Pt, bool out, int qa, int qb, bool hb,
+                                                    ForceSums F) {
+    PairStart p;
+    p.qa = qa;
+    p.qb = qb;
+    p.ha = true;
+    p.hb = hb;
+    p.start(k, xt, S->pos[qa], S->pos[qb]);
+    add_pair_checked<K>(k, c, S, xt, vt, Pt, out, p, F);
+    return F;
+}
+
+// The forms of the pair terms that a kernel takes, by StepConst::force_nz: 0 the general one; 1
+// the packed one with a range check for every pair (the cubic spline's, for h above 0.045); 2 the
+// packed one as it is, and where a particle is out of range (DevState::general) the checked one
+// as a call, so that it takes no registers from the first.  1M dam break, ms, with the general
+// form and now: at h = 0.05 4.32 and 1.53, with one coordinate of 1e-20 4.40 and 2.06.  The
+// Wendland kernel keeps the general one there (2.90, with the checked one 1.94, but then the
+// first loop takes 1.304 instead of 1.287); both loops in one kernel cost it 8%.
+//
 // Candidates go from global to shared memory by asynchronous copies (cp.async), a round of the
 // ring ahead of their use.
-template <bool kIntegrate, bool kBatch, int kKern, bool kNZ>
+template <bool kIntegrate, bool kBatch, int kKern, int kForm>
 __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buffers b,
                                                   DevState* ds) {
     if (ds->status) return;
@@ -95,7 +150,7 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
     const uint32_t ntiles = ds->n_tiles;
     const uint32_t lt = (1u << lane) - 1u;
     const PairLits& lit = cp.lit;
-    const bool nz = kNZ && !ds->general;
+    const bool nz = kForm == 2 && !ds->general;
     const TileQueue queue(&ds->work[1], b.num_sms);
     for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         const uint2 tile = b.tiles[t];
@@ -109,6 +164,8 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
         tile_setup(c, b, g, tile, lane, T, i, xi, valid);
         const float4 vi0 = valid ? b.vel4_s[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float Pi = valid ? b.aux4_s[i].y : 0.0f;
+        // (see pair_range)
+        const bool out = (kForm == 1 || (kForm == 2 && !nz)) && valid && b.aux4_s[i].w == 0.0f;
         // the density pass's records of this tile: its kept candidates and the lanes' masks
         const uint2 list = b.records ? b.tile_list[t] : make_uint2(kNoSlot, 0u);
         const bool listed = list.x != kNoSlot;
@@ -174,14 +231,15 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
             }
             const bool all = !st.more() && staged * 32 >= nlist && ready == staged;
             const int until = all ? ready : min(head + 1, ready);
-            if (nz) {
+            if (kForm == 1 || nz) {
                 // starts `next` and adds `done`; false when no lane needs a chunk before `until`
                 auto turn = [&](PairStart& next, const PairStart& done) -> bool {
                     at.advance_flat(S->mask, ready, lane);
                     at.take2(next.qa, next.qb, next.ha, next.hb);
                     next.start(lit, xi, S->pos[next.qa], S->pos[next.qb]);
-                    add_pair<kKern>(lit, c.pair, vi0, Pi, done, S->vel[done.qa], S->vel[done.qb],
-                                    S->fac[done.qa], S->fac[done.qb], F);
+                    if (kForm == 1) add_pair_checked<kKern>(lit, c, S, xi, vi0, Pi, out, done, F);
+                    else add_pair<kKern>(lit, c.pair, vi0, Pi, done, S->vel[done.qa], S->vel[done.qb],
+                                         S->fac[done.qa], S->fac[done.qb], F);
                     need = at.next - (next.ha ? 1 : 0);
                     return __any_sync(kFull, need < until);
                 };
@@ -201,13 +259,13 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
                     int q[2];
                     bool h[2];
                     at.take2(q[0], q[1], h[0], h[1]);
-                    for (int k = 0; k < 2; ++k) {
-                        if (!h[k]) continue;
-                        const float4 vj = S->vel[q[k]];
-                        const float Pj = xmul(c.gas, xsub(vj.w, c.rest));
-                        F = add_term_general<kKern>(
-                            c, xi, vi0, Pi, S->pos[q[k]], vj,
-                            make_float4(vj.w, Pj, xmul(2.0f, vj.w), S->fac[q[k]].x), F);
+                    if constexpr (kForm == 2 && kKern == SPHX_KERNEL_CUBIC_SPLINE) {
+                        if (h[0])
+                            F = add_slots_checked<kKern>(lit, c, S, xi, vi0, Pi, out, q[0], q[1],
+                                                         h[1], F);
+                    } else {
+                        for (int k = 0; k < 2; ++k)
+                            if (h[k]) add_slot_general<kKern>(c, S, q[k], xi, vi0, Pi, F);
                     }
                 }
             }
@@ -243,27 +301,27 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
     }
 }
 
-template <bool kIntegrate, bool kBatch, int kKern, bool kNZ>
+template <bool kIntegrate, bool kBatch, int kKern, int kForm>
 static void launch_force_t(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                            DevState* ds) {
     const int threads = 32 * L.warps_per_block;
     const size_t sm = (size_t)L.warps_per_block * sizeof(ForceSmem);
     static LaunchShapeCache cache;
     const int nb = cached_resident_blocks(
-        cache, L, k_force<kIntegrate, kBatch, kKern, kNZ>, threads, sm);
-    k_force<kIntegrate, kBatch, kKern, kNZ><<<nb, threads, sm, L.stream>>>(c, b, ds);
+        cache, L, k_force<kIntegrate, kBatch, kKern, kForm>, threads, sm);
+    k_force<kIntegrate, kBatch, kKern, kForm><<<nb, threads, sm, L.stream>>>(c, b, ds);
 }
 
-template <int kKern, bool kNZ>
+template <int kKern, int kForm>
 static void launch_force_n(const LaunchCtx& L, const StepConst& c, const Buffers& b,
                            DevState* ds, int integrate) {
     const bool batch = b.nscenes > 0;
     if (integrate) {
-        if (batch) launch_force_t<true, true, kKern, kNZ>(L, c, b, ds);
-        else launch_force_t<true, false, kKern, kNZ>(L, c, b, ds);
+        if (batch) launch_force_t<true, true, kKern, kForm>(L, c, b, ds);
+        else launch_force_t<true, false, kKern, kForm>(L, c, b, ds);
     } else {
-        if (batch) launch_force_t<false, true, kKern, kNZ>(L, c, b, ds);
-        else launch_force_t<false, false, kKern, kNZ>(L, c, b, ds);
+        if (batch) launch_force_t<false, true, kKern, kForm>(L, c, b, ds);
+        else launch_force_t<false, false, kKern, kForm>(L, c, b, ds);
     }
 }
 
@@ -273,15 +331,19 @@ int launch_force(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevSt
                  int integrate) {
     if (c.precise && b.nscenes == 0) return launch_force_sweep(L, c, b, ds, integrate);
     if (b.tile_n <= kTeamTile) return launch_force_team(L, c, b, ds, integrate);
-    if (c.kern == SPHX_KERNEL_WENDLAND_C2) {
-        if (c.force_nz) launch_force_n<SPHX_KERNEL_WENDLAND_C2, true>(L, c, b, ds, integrate);
-        else launch_force_n<SPHX_KERNEL_WENDLAND_C2, false>(L, c, b, ds, integrate);
-    } else if (c.kern == SPHX_KERNEL_GAUSSIAN) {
-        launch_force_n<SPHX_KERNEL_GAUSSIAN, false>(L, c, b, ds, integrate);
-    } else if (c.force_nz) {
-        launch_force_n<SPHX_KERNEL_CUBIC_SPLINE, true>(L, c, b, ds, integrate);
+    constexpr int kCubic = SPHX_KERNEL_CUBIC_SPLINE, kWendland = SPHX_KERNEL_WENDLAND_C2,
+                  kGaussian = SPHX_KERNEL_GAUSSIAN;
+    if (c.kern == kWendland) {
+        if (c.force_nz == 2) launch_force_n<kWendland, 2>(L, c, b, ds, integrate);
+        else launch_force_n<kWendland, 0>(L, c, b, ds, integrate);
+    } else if (c.kern == kGaussian) {
+        launch_force_n<kGaussian, 0>(L, c, b, ds, integrate);
+    } else if (c.force_nz == 2) {
+        launch_force_n<kCubic, 2>(L, c, b, ds, integrate);
+    } else if (c.force_nz == 1) {
+        launch_force_n<kCubic, 1>(L, c, b, ds, integrate);
     } else {
-        launch_force_n<SPHX_KERNEL_CUBIC_SPLINE, false>(L, c, b, ds, integrate);
+        launch_force_n<kCubic, 0>(L, c, b, ds, integrate);
     }
     return 1;
 }

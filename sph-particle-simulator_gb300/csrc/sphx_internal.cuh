@@ -28,9 +28,9 @@ constexpr int kPrepThreads = 256, kMaxPrepBlocks = 608;   // first kernel of a s
 constexpr int kDiagThreads = 256;
 constexpr int kDiagSums = 8;
 constexpr float kCoincident = 1e-30f;  // see sweep_d2
-// A nonzero coordinate below this (in magnitude) sends a step's exact passes to the general
-// pair forms (DevState::general): the others rely on x_i - x_j being 0 or at least 2^-68.
-constexpr float kTiny = 0x1p-45f;
+// A nonzero coordinate below kTiny (in magnitude) sets DevState::general: without one x_i - x_j
+// is 0 or at least kLeastStep, on which the pair forms rely.
+constexpr float kTiny = 0x1p-45f, kLeastStep = 0x1p-68f;
 constexpr int kCellClamp = 1 << 30;    // |cell coordinate| clamp for finite positions
 
 // Operands of the packed pair arithmetic (F2), both halves equal: read as 64-bit operands from
@@ -80,8 +80,8 @@ struct StepConst {
     float gl;     // Gaussian 2 sigma_sq_inv_ norm_
     float g2s;    // Gaussian 2 sigma_sq_inv_
     // 1: the pair forms' divisions by h and h^2 (div_fixed2) are in range: |r| of a hit is +0
-    // or in [2^-74.5, r (1 + 2^-23)] (div_nz); the gradient's and the Laplacian's dividends of
-    // pairs without tiny coordinates are, too (force_nz)
+    // or in [2^-74.5, r (1 + 2^-23)] (div_nz); the Laplacian's dividends are, too (force_nz = 1),
+    // and the gradient's of all pairs without tiny coordinates (2)
     int div_nz, force_nz;
 };
 
@@ -106,7 +106,7 @@ struct DevState {
     double dt64, time64;        // precision mode: dt and current time in FP64
     uint32_t n_spread;          // precision mode: spread tiles listed this step
     uint32_t spread_work[2];    // precision mode: tile counters of the spread-tile kernels
-    uint32_t general;           // exact mode: 1 if a value lies outside the pair forms' ranges
+    uint32_t general;           // exact mode: 1 if a particle lies outside the pair forms' ranges
 };
 
 // What blocks of one grid-build kernel tell each other; not part of the step's state (never
@@ -474,6 +474,13 @@ __device__ __forceinline__ int cell_coord(float x, float inv_cell) {
     float f = floorf(xmul(x, inv_cell));
     f = fminf(fmaxf(f, -(float)kCellClamp), (float)(kCellClamp - 1));
     return (int)f;
+}
+
+// Density and pressure in the ranges of the force pass's pair forms (pair_terms): P_i + P_j is
+// then 0 or in [2^-74, 2^61] and its quotient by 2 rho_j in [2^-115, 2^120].
+__device__ __forceinline__ bool pair_range(float rho, float P) {
+    return rho >= 0x1p-60f && rho <= 0x1p40f &&
+           (P == 0.0f || (fabsf(P) >= 0x1p-50f && fabsf(P) <= 0x1p60f));
 }
 
 // a nonzero coordinate below kTiny in magnitude

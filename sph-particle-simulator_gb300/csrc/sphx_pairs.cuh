@@ -78,10 +78,13 @@ __device__ __forceinline__ void force_term(const StepConst& c, const float4& xt,
 // pressure-force contributions (every sum then only adds), wx, wy, wz the viscosity ones.  The
 // three divisions by |r| (cubic spline) or |r| h (Wendland)
 // share one reciprocal, the division by 2 rho_j has its reciprocal with the candidate, and
-// those by h and h^2 need no range tests.  Valid where StepConst::force_nz holds and
+// those by h and h^2 need no range tests.  Valid where StepConst::force_nz is 2 and
 // DevState::general is 0: a component of x_t - x_j is then 0 or in [2^-68, r], P_t + P_j 0 or
-// in [2^-64, 2^61] and rho in [2^-30, 2^40], and every dividend below stays in the range its
-// division needs.  The signs of zero terms are not kept: the sums start at +0 and so never
+// in [2^-74, 2^61] and rho in [2^-60, 2^40], and every dividend below stays in the range its
+// division needs.  Where force_nz is 1 or a particle left those ranges (kCheck), the terms come
+// with the answer whether this pair is in range: its components, the dividends of the division
+// by h, and the candidate, whose factor 1 / (2 rho_j) is 0 if its density or pressure is out of
+// range.  The signs of zero terms are not kept: the sums start at +0 and so never
 // become -0, and adding a zero of either sign leaves any other value unchanged.  A pair with
 // |r| < 1e-6, whose pressure term the reference skips, gets m_j pt = 0 and with it zero terms
 // (what it multiplies is finite there).
@@ -106,8 +109,14 @@ struct PairStart {
 };
 struct PairTerms {
     F2 px, py, pz, wx, wy, wz;
+    bool oka, okb;  // (kCheck)
 };
-template <int K>
+// three numbers 0 or at least `least` in magnitude
+__device__ __forceinline__ bool zero_or_above(float x, float y, float z, float least) {
+    auto order = [](float v) { return 2u * __float_as_uint(v) - 1u; };  // (0 becomes the largest)
+    return min(min(order(x), order(y)), order(z)) >= order(least);
+}
+template <int K, bool kCheck = false>
 __device__ __forceinline__ PairTerms pair_terms(const PairLits& k, const PairConst& c,
                                                 const float4& vt, float Pt, const PairStart& p,
                                                 const float4& va, const float4& vb,
@@ -123,6 +132,12 @@ __device__ __forceinline__ PairTerms pair_terms(const PairLits& k, const PairCon
     const F2 sp = select2(la, lb, p.m * npt, zero);  // -m_j pt
     const F2 y1 = p.hr * F2{k.p2p21};               // ~ 1/|r|
     F2 px, py, pz, lap;
+    bool oka = true, okb = true;
+    if (kCheck) {
+        const float2 x = upk2(dx.v), y = upk2(dy.v), z = upk2(dz.v);
+        oka = fa.y != 0.0f && zero_or_above(x.x, y.x, z.x, kLeastStep);
+        okb = fb.y != 0.0f && zero_or_above(x.y, y.y, z.y, kLeastStep);
+    }
     // beyond the support q = 2 the clamped 2 - q (1 - q/2) makes the terms the zeros that the
     // reference returns there
     if (K == SPHX_KERNEL_WENDLAND_C2) {
@@ -143,16 +158,24 @@ __device__ __forceinline__ PairTerms pair_terms(const PairLits& k, const PairCon
         const F2 g2 = F2{c.neg_sigma} * (F2{k.half} * t * t);
         const F2 gf = select2(ia, ib, g1, g2);
         const F2 y = rcp2_exact(k, ns, y1);
-        px = sp * div_fixed2(gf * div_rcp2(dx, ns, y), F2{c.neg_h}, F2{c.rcp_h});
-        py = sp * div_fixed2(gf * div_rcp2(dy, ns, y), F2{c.neg_h}, F2{c.rcp_h});
-        pz = sp * div_fixed2(gf * div_rcp2(dz, ns, y), F2{c.neg_h}, F2{c.rcp_h});
+        const F2 ux = gf * div_rcp2(dx, ns, y), uy = gf * div_rcp2(dy, ns, y),
+                 uz = gf * div_rcp2(dz, ns, y);
+        if (kCheck) {
+            const float2 a = upk2(ux.v), e = upk2(uy.v), f = upk2(uz.v);
+            oka = oka && zero_or_above(a.x, e.x, f.x, 0x1p-100f);
+            okb = okb && zero_or_above(a.y, e.y, f.y, 0x1p-100f);
+        }
+        px = sp * div_fixed2(ux, F2{c.neg_h}, F2{c.rcp_h});
+        py = sp * div_fixed2(uy, F2{c.neg_h}, F2{c.rcp_h});
+        pz = sp * div_fixed2(uz, F2{c.neg_h}, F2{c.rcp_h});
         // Laplacian (kernels.cpp:130-138)
         const F2 l = select2(ia, ib, F2{k.neg2} + pmul(F2{k.three}, q, neg0), t);
         lap = div_fixed2(F2{c.sigma} * l, F2{c.neg_hsq}, F2{c.rcp_hsq});
     }
     const F2 mv = f2(fa.x, fb.x);  // (m_j / rho_j) mu, formed by the density pass
     return {px, py, pz, mv * (f2(va.x, vb.x) - f2(vt.x)) * lap,
-            mv * (f2(va.y, vb.y) - f2(vt.y)) * lap, mv * (f2(va.z, vb.z) - f2(vt.z)) * lap};
+            mv * (f2(va.y, vb.y) - f2(vt.y)) * lap, mv * (f2(va.z, vb.z) - f2(vt.z)) * lap,
+            oka, okb};
 }
 
 }  // namespace sphx

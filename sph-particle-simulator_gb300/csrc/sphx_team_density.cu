@@ -109,10 +109,10 @@ __global__ void __launch_bounds__(32 * kDensityWarps, 1) k_density_team(const St
                 const float P = xmul(c.gas, xsub(rho, c.rest));
                 // see k_density
                 const float mr = xdiv(xi.w, rho);
-                b.aux4_s[i] = make_float4(rho, P, xmul(mr, c.visc), __frcp_rn(xmul(2.0f, rho)));
-                if (!(rho >= 0x1p-30f && rho <= 0x1p40f) ||
-                    !(P == 0.0f || (fabsf(P) >= 0x1p-40f && fabsf(P) <= 0x1p60f)))
-                    ds->general = 1;
+                const bool in = pair_range(rho, P);
+                b.aux4_s[i] = make_float4(rho, P, xmul(mr, c.visc),
+                                          in ? __frcp_rn(xmul(2.0f, rho)) : 0.0f);
+                if (!in) ds->general = 1;
                 b.vel4_s[i].w = rho;
             }
         }

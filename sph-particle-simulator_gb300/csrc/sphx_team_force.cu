@@ -217,7 +217,7 @@ template <int kKern>
 static void launch_team_k(const LaunchCtx& L, const StepConst& c, const Buffers& b, DevState* ds,
                           int integrate) {
     constexpr bool kPairs = kKern != SPHX_KERNEL_GAUSSIAN;
-    const bool nz = kPairs && c.force_nz;
+    const bool nz = kPairs && c.force_nz == 2;
     if (b.nscenes > 0) {
         if (nz) launch_team_t<true, kKern, kPairs>(L, c, b, ds, integrate);
         else launch_team_t<true, kKern, false>(L, c, b, ds, integrate);
