@@ -122,11 +122,12 @@ float host_cubic_w(float sigma, float q) {
 
 // Verifies the one-correction division sequence of xdiv_fixed for divisor b against IEEE
 // float division, for every dividend significand of the binade [1, 2) (about 8 ms).
-// Results are cached per divisor; only b in [2^-20, 2^20] qualifies.
+// Results are cached per divisor; only b in [2^-48, 2^40] qualifies (h from 60 nm to 1,000 km
+// and its square).
 bool verify_fixed_divisor(float b) {
     static std::mutex mu;
     static std::vector<std::pair<uint32_t, bool>> cache;
-    if (!(b >= 0x1p-20f && b <= 0x1p20f)) return false;
+    if (!(b >= 0x1p-48f && b <= 0x1p40f)) return false;
     uint32_t bits;
     std::memcpy(&bits, &b, 4);
     {
@@ -205,9 +206,9 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
     s.fast_div_h = verify_fixed_divisor(h) ? 1 : 0;
     s.fast_div_hsq = verify_fixed_divisor(s.h_sq) ? 1 : 0;
     // the pair forms' untested divisions: |r| of a hit is at most r (1 + 2^-23) and the
-    // Laplacian's numerator at most 2 sigma; both divisors verified (so h, h^2 in
-    // [2^-20, 2^20] and sigma = 1/(pi h^3) within [2^-62, 2^59]); their square root takes
-    // |r|^2 of up to 2^86 (sqrt2_exact)
+    // Laplacian's numerator 0 or in [2^-24 sigma, 2 sigma]; both divisors verified (so h in
+    // [2^-24, 2^20], sigma = 1/(pi h^3) in [2^-61.7, 2^70.4] and the Laplacian in [2^-125.7,
+    // 2^119.4]); their square root takes |r|^2 of up to 2^86 (sqrt2_exact)
     s.div_nz = s.fast_div_h && s.fast_div_hsq && p.neighbor_search_radius > 0.0f &&
                        p.neighbor_search_radius <= 0x1p43f
                    ? 1 : 0;
@@ -217,7 +218,7 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
     // gradient factor -- sigma 2^-47 for 2 - q >= 2^-23, 0.49 sigma q for q >= 1e-6 / h.  Where
     // that is too small (h above 0.045 for r = 2h) the pass asks each pair (kCheck)
     s.force_nz = 0;
-    if (s.div_nz && p.neighbor_search_radius <= 0x1p20f) {
+    if (s.div_nz && p.neighbor_search_radius <= 0x1p21f) {
         const double r = p.neighbor_search_radius, q1 = 0.49 * std::min(1e-6 / h, 1.0);
         const double gmin = (double)s.sigma * std::min(0x1p-47, q1);
         s.force_nz = kernel == SPHX_KERNEL_WENDLAND_C2 || gmin * 0x1p-68 / r >= 0x1p-99 ? 2 : 1;

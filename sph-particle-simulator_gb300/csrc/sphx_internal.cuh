@@ -263,7 +263,7 @@ __device__ __forceinline__ float xsqrt(float a) { return __fsqrt_rn(a); }
 // when the divisor is known in advance", IEEE TC 53(8), 2004).  The host verifies the
 // sequence for the divisor against IEEE division over every dividend significand of one
 // binade (`verified`); the sequence commutes with power-of-two scaling while every
-// intermediate stays normal, which |a| in [2^-60, 2^60] and b in [2^-20, 2^20] ensure.
+// intermediate stays normal, which |a| in [2^-60, 2^60] and b in [2^-48, 2^40] ensure.
 // Anything else (zero, subnormal, huge, NaN/inf dividend, unverified divisor) takes the
 // IEEE division.
 __device__ __forceinline__ float xdiv_fixed(float a, float b, float y, int verified) {
@@ -341,8 +341,8 @@ __device__ __forceinline__ F2 max0(F2 a) {
 }
 
 // xdiv_fixed of both halves without the range test, nb = -b, y = RN(1/b), for dividends known
-// to be +-0 or of magnitude in [2^-100, 2^100] with a verified divisor b in [2^-20, 2^20].  In
-// that range q0 and the quotient are normal and the residual r is exact (a multiple of
+// to be +-0 or of magnitude in [2^-100, 2^100], with a verified divisor b in [2^-48, 2^40] and
+// a normal quotient.  Then q0 is normal, too, and the residual r is exact (a multiple of
 // 2^(e_a - 46) >= 2^-146, at most about 2^-22 |a|), so the sequence scales exactly with powers
 // of two of a and the verification on one binade covers every binade.  A zero dividend gives
 // a zero whose sign is not kept.

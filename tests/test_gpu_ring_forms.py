@@ -53,6 +53,19 @@ def test_smoothing_lengths(port, scale, kernel, tile):
 
 
 @pytest.mark.parametrize("kernel", KERNELS)
+@pytest.mark.parametrize("scale", [5.9e-8, 6.1e-8, 1e-7, 1.04e6, 1.06e6])
+@pytest.mark.parametrize("tile", [0, 32])
+def test_edges_of_the_smoothing_lengths(port, scale, kernel, tile):
+    """Lengths on both sides of the ends of the range of the pair forms."""
+    pos, vel, _, _ = block(12, 34)
+    s = scale / 0.02
+    pos[20:40] = pos[60:80]
+    prm = I.params16(smoothing_length=scale, neighbor_search_radius=2 * scale)
+    check(port, (pos * s).astype(np.float32), vel, np.full(len(pos), 1e-3 * s ** 3, np.float32), prm,
+          kernel, tile=tile)
+
+
+@pytest.mark.parametrize("kernel", KERNELS)
 @pytest.mark.parametrize("h", [0.02, 0.1])
 @pytest.mark.parametrize("odd", ["light", "massless", "heavy", "tiny", "far_tiny", "fast", "negative"])
 def test_a_few_particles_out_of_range(port, odd, h, kernel):
@@ -121,7 +134,7 @@ def test_tiles_without_room_for_their_candidates(port, kernel, h):
     check(port, pos, vel, mass, prm, kernel, capacity=300_000, tile=0)
 
 
-@pytest.mark.parametrize("state_of", ["length", "tiny"])
+@pytest.mark.parametrize("state_of", ["length", "half_millimetre", "tiny"])
 def test_out_of_range_states_take_no_multiple_of_the_time(built, state_of):
     """The force pass of 103,823 particles at another smoothing length, or with one coordinate of
     1e-20, against the ordinary set: 1.1 and 1.5 times as long, 3 in the general form."""
@@ -142,5 +155,6 @@ def test_out_of_range_states_take_no_multiple_of_the_time(built, state_of):
         return np.median(times[2:])
 
     plain = force_time(0.02, False)
-    other = force_time(0.1, False) if state_of == "length" else force_time(0.02, True)
+    h = {"length": 0.1, "half_millimetre": 5e-4, "tiny": 0.02}[state_of]
+    other = force_time(h, state_of == "tiny")
     assert 0 < other < 2 * plain
