@@ -238,11 +238,26 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
                      both(-3.0f), both(kCoincident)};
     s.pair = PairConst{both(-h), both(h), both(s.rcp_h), both(-s.h_sq), both(s.rcp_hsq),
                        both(s.sigma), both(-s.sigma), both(s.gas), both(s.rest), both(s.wnorm),
-                       both(s.wl)};
+                       both(s.wl), 0};
     s.sw_cs = s.cs * s.rcp_h;  // 2 exactly for r_search = 2h
     s.sw_r2 = s.r2 * s.rcp_hsq;
     s.sw_r2m = s.sw_r2 * 1.0001f;
     s.sw_skip2 = 1e-12f * s.rcp_hsq;
+    float kl = s.sigma * s.rcp_hsq;
+    s.sw_kg = -0.5f * s.sigma * s.rcp_h;
+    if (kernel == SPHX_KERNEL_GAUSSIAN) {
+        kl = s.gl;
+        s.sw_kg = -s.gg * s.h;  // (the gradient shape times r_vec in units of h)
+    } else if (kernel == SPHX_KERNEL_WENDLAND_C2) {
+        kl = s.wl;
+        s.sw_kg = 5.0f * s.wnorm * s.rcp_h;
+    }
+    // 2 kl / kg mu (kl mu on its own could overflow where no particle's factor does); where kl or
+    // kg underflows, h above some 1e9, the quotient is written as the multiple of 1/h that it is
+    const float multiple = kernel == SPHX_KERNEL_CUBIC_SPLINE ? -4.0f : 2.0f;
+    const bool normal = std::min(std::fabs(kl), std::fabs(s.sw_kg)) >= 0x1p-126f;
+    s.sw_kappa = (normal ? 2.0f * kl / s.sw_kg : multiple * s.rcp_h) * s.visc;
+    s.pair.kappa = both(s.sw_kappa);
 }
 
 }  // namespace sphx

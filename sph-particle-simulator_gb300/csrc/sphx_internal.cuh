@@ -43,6 +43,7 @@ struct PairLits {  // numbers
 };
 struct PairConst {  // of the step's parameters
     f32x2 neg_h, h, rcp_h, neg_hsq, rcp_hsq, sigma, neg_sigma, gas, rest, wnorm, wl;
+    f32x2 kappa;  // StepConst::sw_kappa
 };
 
 // Constants of one step, computed on the host in float exactly as the reference does
@@ -68,6 +69,7 @@ struct StepConst {
     // rather than held in registers: cs / h, r^2 / h^2, the same with the box cull's margin,
     // (1e-6 m / h)^2
     float sw_cs, sw_r2, sw_r2m, sw_skip2;
+    float sw_kg, sw_kappa;  // force factors, see sphx_sweep.cu
     int fast_div_h, fast_div_hsq;  // 1: the one-correction sequence is verified for it
     // smoothing kernel (SPHX_KERNEL_*) and the constants its constructor computes in float
     PairLits lit;

@@ -411,27 +411,8 @@ struct SweepForceSpreadSmem {
 // Pressure and viscosity factors of the kernel: the force on particle t from candidate j is
 //   kg (m_j / (2 rho_j)) (P_t + P_j) G' r_vec  +  kl (m_j / rho_j) mu L' (v_j - v_t)
 // with G' and L' the kernel's gradient and Laplacian shapes below: grad W_tj = -kg G' r_vec
-// and laplacian W_tj = kl L' (r_vec = x_t - x_j, in units of h).
-__host__ __device__ __forceinline__ float sweep_kg(const StepConst& c) {
-    if (c.kern == SPHX_KERNEL_GAUSSIAN) return -c.gg * c.h;  // G' r_vec in h units
-    if (c.kern == SPHX_KERNEL_WENDLAND_C2) return 5.0f * c.wnorm * c.rcp_h;
-    return -0.5f * c.sigma * c.rcp_h;
-}
-__host__ __device__ __forceinline__ float sweep_kl(const StepConst& c) {
-    if (c.kern == SPHX_KERNEL_GAUSSIAN) return c.gl;
-    if (c.kern == SPHX_KERNEL_WENDLAND_C2) return c.wl;
-    return c.sigma * c.rcp_hsq;
-}
-
-// The viscosity factor kl (m_j / rho_j) mu is the pressure factor kg m_j / (2 rho_j) times
-// this constant (kl mu on its own could overflow where no particle's factor does).  Where kl or
-// kg underflows (h above some 1e9) the quotient is written as the multiple of 1/h that it is.
-__host__ __device__ __forceinline__ float sweep_kappa(const StepConst& c) {
-    const float kl = sweep_kl(c), kg = sweep_kg(c);
-    const float k = c.kern == SPHX_KERNEL_CUBIC_SPLINE ? -4.0f : 2.0f;
-    const bool normal = fminf(fabsf(kl), fabsf(kg)) >= 0x1p-126f;
-    return (normal ? 2.0f * kl / kg : k * c.rcp_h) * c.visc;
-}
+// and laplacian W_tj = kl L' (r_vec = x_t - x_j, in units of h).  The host forms kg and the
+// constant kappa = 2 kl / kg mu between the two factors (StepConst::sw_kg, sw_kappa).
 
 // (|r|/h)^2 of a pair is formed with kCoincident added: far below the rounding of any other pair
 __device__ __forceinline__ F2 sweep_d2(const PairLits& k, F2 dx, F2 dy, F2 dz) {
@@ -600,9 +581,8 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep(const StepConst c, const
     const uint32_t ntiles = ds->n_tiles;
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
-    const float kg = sweep_kg(c);
-    const float visc = sweep_kappa(c);
-    const F2 kappa = f2(visc);
+    const float kg = c.sw_kg;
+    const F2 kappa{c.pair.kappa};
     const TileQueue queue(&ds->work[1], b.num_sms);
     for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
@@ -652,7 +632,7 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep(const StepConst c, const
             // a non-finite velocity or factor (the pressure's, the viscosity's) is not cancelled
             // by a zero shape
             return kCut || __any_sync(kFull, !isfinite(d.v.x + d.v.y + d.v.z + d.a.y +
-                                                       pf * d.a.y + pf * visc));
+                                                       pf * d.a.y + pf * c.sw_kappa));
         };
         auto sweep = [&](bool masked, int left) {
             F2 Fx = f2(0.0f), Fy = Fx, Fz = Fx;
@@ -710,8 +690,8 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep_spread(const StepConst c
     const uint32_t ntiles = ds->n_spread;
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
-    const float kg = sweep_kg(c);
-    const F2 kappa = f2(sweep_kappa(c));
+    const float kg = c.sw_kg;
+    const F2 kappa{c.pair.kappa};
     const TileQueue queue(&ds->spread_work[1], b.num_sms);
     for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
