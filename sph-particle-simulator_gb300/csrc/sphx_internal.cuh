@@ -186,7 +186,8 @@ struct Buffers {
     // sorted positions of the kept candidates that are a neighbour of some lane.  Every warp of the density grid
     // owns an equal region of the pool and stores its tiles one after another; tile_list[t] =
     // first record and candidates (or rows), or kNoSlot when the tile did not fit in what was left of
-    // the region (the force pass then walks and tests that tile itself).
+    // the region (the force pass then walks and tests that tile itself); an exact tile of more
+    // than 8 whose particles have no neighbour leaves no candidates.
     uint32_t* records = nullptr;
     uint2* tile_list = nullptr;
     unsigned long long record_cap = 0;

@@ -158,3 +158,36 @@ def test_out_of_range_states_take_no_multiple_of_the_time(built, state_of):
     h = {"length": 0.1, "half_millimetre": 5e-4, "tiny": 0.02}[state_of]
     other = force_time(h, state_of == "tiny")
     assert 0 < other < 2 * plain
+
+
+@pytest.mark.parametrize("kernel", KERNELS + [sphx.KERNEL_GAUSSIAN])
+@pytest.mark.parametrize("count", [70_000, 300_000])
+def test_lone_particles(port, kernel, count):
+    """Particles without a neighbour, and a few pairs among them: no forces but in the pairs, and
+    a force pass that takes no longer than the density pass."""
+    rng = np.random.default_rng(71)
+    k = np.arange(count)
+    pos = np.stack([k % 100, k // 100 % 100, k // 10_000], -1) * 0.1 + 0.02 * rng.random((count, 3))
+    pos = pos.astype(np.float32)
+    pos[1:2000:100] = pos[0:2000:100] + np.float32([0.01, 0.0, 0.0])
+    vel = rng.standard_normal(pos.shape).astype(np.float32)
+    mass = np.full(count, 1e-3, np.float32)
+    prm = I.params16(gas_constant=2e-3)
+    ctx = sphx.Context(count, profile=True)
+    ctx.set_params(prm)
+    ctx.set_kernel(kernel)
+    ctx.upload(pos, vel, mass)
+    times = []
+    for _ in range(7):
+        ctx.reset_stats()
+        ctx.eval()
+        st = ctx.stats()
+        times.append(st["force_computation_time"] / st["density_computation_time"])
+    out = ctx.download()
+    ctx.close()
+    paired = np.any(out["acc"] != np.float32([0.0, prm[6], 0.0]), axis=1)
+    assert np.array_equal(np.flatnonzero(paired), np.flatnonzero((k < 2000) & (k % 100 < 2)))
+    if kernel != sphx.KERNEL_GAUSSIAN:
+        for got, want in zip((out["rho"], out["acc"]), port.fields(pos, vel, mass, prm, kernel=kernel)[::2]):
+            assert O.bits_equal(got, want)
+    assert np.median(times) < 1.1
