@@ -1491,6 +1491,7 @@ int sphx_debug_pairs(sphx_ctx* c, int64_t* counts, int64_t* idx, size_t* total_i
     Buffers bq = c->b;
     bq.columns = 0;
     bq.tgt = nullptr;
+    if (c->tile_auto) bq.tile_n = kTile;  // (a lane per particle)
     launch_grid(c->L, c->sc, bq, c->ds, kNoStep, 0.0f);
     uint32_t* d_cnt = nullptr;
     if ((rc = dmalloc(&d_cnt, n))) return rc;
@@ -1553,6 +1554,7 @@ int sphx_debug_pairs_subset(sphx_ctx* c, size_t nsel, const int64_t* sel, int64_
     Buffers bq = c->b;
     bq.columns = 0;
     bq.tgt = nullptr;
+    if (c->tile_auto) bq.tile_n = kTile;  // (a lane per particle)
     launch_grid(c->L, c->sc, bq, c->ds, kNoStep, 0.0f);
     uint32_t* d_cnt = nullptr;
     if ((rc = dmalloc(&d_cnt, n))) return rc;
