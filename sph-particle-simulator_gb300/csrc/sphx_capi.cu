@@ -993,9 +993,8 @@ int sphx_upload_f64(sphx_ctx* c, size_t n, const double* pos, const float* vel,
         } else {
             k_f64_to_f32<<<c->L.num_sms * 4, 256, 0, c->stream>>>((int)(3 * n), src, s_posf);
             if (vel && !src_vel) {
-                // staged after the conversion, in the place of the positions
+                // staged after the conversion (the stream's order), in the place of the positions
                 float* s_vel2 = reinterpret_cast<float*>(s_pos);
-                SPHX_CUDA(cudaStreamSynchronize(c->stream));
                 SPHX_CUDA(cudaMemcpyAsync(s_vel2, vel, 3 * n * sizeof(float), cudaMemcpyHostToDevice, c->stream));
                 src_vel = s_vel2;
             }
