@@ -228,9 +228,10 @@ int sphx_get_scene_stats(sphx_ctx* ctx, uint32_t scene, sphx_scene_stats* out);
 
 /* Picks the neighbour passes' launch shape for the loaded workload: times two steps of
  * dt for each candidate -- warps per CTA x resident CTAs per SM, then the tile size
- * (particles per warp work item) at the best of those -- restores the particles, times
- * and scene records after every trial, and keeps the fastest in the context.  Returns
- * the launch choice and its time per step (sphx_get_tuning gives all of it).
+ * (particles per warp work item: 32, 24, 16, the present one, and where tile_particles was 0
+ * the set's own choice, which is still reported as 32) at the best of those -- restores the
+ * particles, times and scene records after every trial, and keeps the fastest in the context.
+ * Returns the launch choice and its time per step (sphx_get_tuning gives all of it).
  * Synchronises.  No counterpart in the reference (its loops are OpenMP over particles). */
 int sphx_autotune(sphx_ctx* ctx, float dt, int* warps_per_block, int* blocks_per_sm,
                   float* best_ms);

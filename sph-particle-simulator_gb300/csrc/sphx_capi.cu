@@ -1133,6 +1133,8 @@ int sphx_autotune(sphx_ctx* c, float dt, int* warps_per_block, int* blocks_per_s
     const int cand[][2] = {{4, 0}, {2, 0}, {4, 4}, {4, 2}, {2, 4}, {1, 0}};
     float best = 0.0f;
     int bw = c->L.warps_per_block, bb = c->L.blocks_per_sm;
+    const bool exact = c->tuning.mode == SPHX_MODE_EXACT, was_auto = c->tile_auto;
+    const int own = c->tuning.tile_particles;  // 32 where the choice is the set's
     auto reset = [&]() -> int {
         SPHX_CUDA(cudaMemcpyAsync(c->ds, &ds_save, sizeof(DevState), cudaMemcpyHostToDevice, c->stream));
         if (c->nscenes)
@@ -1140,51 +1142,65 @@ int sphx_autotune(sphx_ctx* c, float dt, int* warps_per_block, int* blocks_per_s
         SPHX_CUDA(cudaStreamSynchronize(c->stream));
         return sphx_restore(c);
     };
-    for (const auto& cd : cand) {
-        c->L.warps_per_block = cd[0];
-        c->L.blocks_per_sm = cd[1];
-        if ((rc = reset()) || (rc = run_phases(c, dt, true))) break;  // warm-up
-        if ((rc = reset())) break;
+    // two steps on the saved state, after a warm-up; the faster of them and the best so far
+    auto faster = [&](bool* is_best) -> int {
+        int r;
+        if ((r = reset()) || (r = run_phases(c, dt, true))) return r;  // warm-up
+        if ((r = reset())) return r;
         SPHX_CUDA(cudaEventRecord(e0, c->stream));
-        if ((rc = run_phases(c, dt, true))) break;
-        if ((rc = reset())) break;  // identical work for the second timed step
-        if ((rc = run_phases(c, dt, true))) break;
+        if ((r = run_phases(c, dt, true))) return r;
+        if ((r = reset())) return r;  // identical work for the second timed step
+        if ((r = run_phases(c, dt, true))) return r;
         SPHX_CUDA(cudaEventRecord(e1, c->stream));
         SPHX_CUDA(cudaEventSynchronize(e1));
         float ms = 0.0f;
         SPHX_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if (best == 0.0f || ms < best) {
-            best = ms;
-            bw = cd[0];
-            bb = cd[1];
+        *is_best = best == 0.0f || ms < best;
+        if (*is_best) best = ms;
+        return SPHX_OK;
+    };
+    // the launch shapes, of the passes they apply to: those on tiles of up to 8 take one CTA per
+    // SM whatever the shape, so that the shape is chosen with tiles of 32 where the set's own
+    // choice is 8, and not at all where the caller's is
+    bool is_best = false;
+    c->tile_auto = false;
+    c->b.tile_n = own;
+    if (exact && own <= kTeamTile) {
+        rc = faster(&is_best);
+    } else {
+        for (const auto& cd : cand) {
+            c->L.warps_per_block = cd[0];
+            c->L.blocks_per_sm = cd[1];
+            if ((rc = faster(&is_best))) break;
+            if (is_best) {
+                bw = cd[0];
+                bb = cd[1];
+            }
         }
     }
-    // then the tile size at the chosen launch shape
+    // then the tile size at the chosen launch shape, the set's own choice (0) among them
     c->L.warps_per_block = bw;
     c->L.blocks_per_sm = bb;
-    int bt = c->tuning.tile_particles;
-    const bool was_auto = c->tile_auto;
-    const int tiles[] = {16, 24};
+    const bool own_choice = was_auto && pass_tile((int)c->n, !exact) != own;
+    bool keeps_auto = was_auto && !own_choice;
+    int bt = own;
+    const int tiles[] = {own_choice ? 0 : own, 16, 24, 32};
     for (const int tn : tiles) {
         if (rc) break;
-        c->tile_auto = false;
-        c->b.tile_n = tn;
-        if ((rc = reset()) || (rc = run_phases(c, dt, true))) break;  // warm-up
-        if ((rc = reset())) break;
-        SPHX_CUDA(cudaEventRecord(e0, c->stream));
-        if ((rc = run_phases(c, dt, true))) break;
-        if ((rc = reset())) break;
-        if ((rc = run_phases(c, dt, true))) break;
-        SPHX_CUDA(cudaEventRecord(e1, c->stream));
-        SPHX_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.0f;
-        SPHX_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best) {
-            best = ms;
-            bt = tn;
+        if (tn == own) continue;  // timed above
+        c->tile_auto = tn == 0;
+        if (tn) c->b.tile_n = tn;
+        if ((rc = faster(&is_best))) break;
+        if (is_best) {
+            keeps_auto = tn == 0;
+            bt = tn ? tn : own;
         }
     }
-    c->tile_auto = was_auto && bt == c->tuning.tile_particles;
+    if (rc) {
+        keeps_auto = was_auto;
+        bt = own;
+    }
+    c->tile_auto = keeps_auto;
     c->b.tile_n = bt;
     c->tuning.tile_particles = bt;
     cudaEventDestroy(e0);

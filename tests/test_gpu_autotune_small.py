@@ -1,0 +1,43 @@
+"""The autotuner on small sets, whose own tile size is 8: it is compared with the tiles of 16 to 32
+of the passes with a lane per particle, and the best of them all is kept."""
+import numpy as np
+import pytest
+
+import sphx
+import sphx_inputs as I
+
+pytestmark = pytest.mark.gpu
+
+
+def tuned(pos, tile):
+    """The tuned context, its time per step as the tuner found it and as a step takes it."""
+    ctx = sphx.Context(len(pos), tile_particles=tile, profile=True)
+    ctx.set_params(I.params16(gas_constant=2e-3, gravity=0.0))
+    ctx.upload(pos, np.zeros_like(pos), np.full(len(pos), 1e-3, np.float32))
+    _, _, ms = ctx.autotune(1e-9)
+    assert ctx.tuning()["tile_particles"] in (16, 24, 32)
+    times = []
+    for _ in range(9):
+        ctx.reset_stats()
+        ctx.eval()
+        st = ctx.stats()
+        times.append(st["density_computation_time"] + st["force_computation_time"])
+    ctx.close()
+    return ms, np.median(times)
+
+
+def test_crowded_set_takes_tiles_of_32(built):
+    rng = np.random.default_rng(1)
+    centre = 0.2 * np.stack(np.meshgrid(*[np.arange(3)] * 3, indexing="ij"), -1).reshape(-1, 1, 3)
+    pos = (centre[:9] + 0.015 * rng.random((9, 5000, 3))).astype(np.float32).reshape(-1, 3)
+    ms, step = tuned(pos, 0)
+    ms32, step32 = tuned(pos, 32)
+    # (the own tiles of 8 take 1.27 times as long)
+    assert ms < 1.12 * ms32 and step < 1.12 * step32
+
+
+def test_lattice_keeps_its_own_tiles(built):
+    pos = I.lattice(20, 20, 20, seed=3, origin=(0.1,) * 3)
+    _, step = tuned(pos, 0)
+    _, step32 = tuned(pos, 32)
+    assert step < 0.8 * step32  # 0.4
