@@ -787,11 +787,12 @@ int sphx_create(sphx_ctx** out, size_t capacity, const sphx_tuning* tuning) {
     // 17k (two tiles a warp) 70, 42 and 42.  Without the pool (or where a warp's share runs out)
     // the force pass walks the candidates itself.
     unsigned long long cap = (C > kManyParticles ? 3ull : 4ull) * C;
+    constexpr size_t kRecord = 32 * sizeof(uint32_t);
     const bool exact = c->tuning.mode == SPHX_MODE_EXACT;
-    if (!exact || C <= 4 * (size_t)kTeamMax) {
+    // (asking for the free memory takes 30 us; a precision pool of up to 64 MB matters to nobody)
+    if (exact ? C <= 4 * (size_t)kTeamMax : cap * kRecord > (64u << 20)) {
         size_t free_bytes = 0, all_bytes = 0;
         if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess) cudaGetLastError();
-        constexpr size_t kRecord = 32 * sizeof(uint32_t);
         if (exact) {
             // at most 1/256 of the memory that is free, so that many contexts leave each other room
             cap = std::max<unsigned long long>(
