@@ -180,9 +180,11 @@ __device__ __forceinline__ void for_each_row(const Buffers& b, const Geom& g, co
     // z range of every row: [z0, z1] plus, when z wraps past the end, [0, z2]
     int z0 = T.cz + T.lo[2], z1 = T.cz + T.hi[2], z2 = -1;
     int zp = -1, zq = -2;  // a wrapped piece at the front (dz < 0 past 0)
-    if (w2 && z1 - z0 + 1 >= d2) {  // the range covers the folded axis: each cell once
+    if (w2 && z1 - z0 + 1 >= d2) {  // it covers the folded axis: each cell once
+        zp = z0 < 0 ? z0 + d2 : z0;
+        zq = d2 - 1;
         z0 = 0;
-        z1 = d2 - 1;
+        z1 = zp - 1;
     } else if (w2) {
         if (z0 < 0) {
             zp = z0 + d2;
@@ -233,9 +235,11 @@ __device__ __forceinline__ int build_segments(const Buffers& b, const Geom& g, c
     const int d0 = g.dim[0], d1 = g.dim[1], d2 = g.dim[2];
     int z0 = T.cz + T.lo[2], z1 = T.cz + T.hi[2], z2 = -1;
     int zp = -1, zq = -2;
-    if (g.wrap[2] && z1 - z0 + 1 >= d2) {  // the range covers the folded axis: each cell once
+    if (g.wrap[2] && z1 - z0 + 1 >= d2) {  // it covers the folded axis: each cell once
+        zp = z0 < 0 ? z0 + d2 : z0;
+        zq = d2 - 1;
         z0 = 0;
-        z1 = d2 - 1;
+        z1 = zp - 1;
     } else if (g.wrap[2]) {
         if (z0 < 0) {
             zp = z0 + d2;
