@@ -6,7 +6,7 @@ namespace sphx {
 
 // Grid extent.  The occupied-cell box is laid out densely when it has at most max_cells
 // cells.  Otherwise (particles spread over a huge box) every axis longer than F =
-// floor(cbrt(max_cells)) >= 256 cells is folded: its cell index is taken modulo F.  Cells
+// floor(cbrt(max_cells)) >= 5 cells is folded: its cell index is taken modulo F.  Cells
 // that fold onto each other are at least F - 2 cells apart, so a candidate from a folded
 // neighbour fails the distance test; sets and visiting order are unchanged, only the
 // number of candidates grows.
@@ -229,6 +229,8 @@ __device__ __forceinline__ ColumnInfo column_info(const Buffers& b, const DevSta
 __device__ __forceinline__ bool tile_starts(const Buffers& b, const ColumnInfo& g, uint32_t nc,
                                             int k, uint32_t key, uint32_t prev, bool new_cell) {
     const uint32_t tn = (uint32_t)b.tile_n;
+    // (the group of particles without a cell is all scenes'; a tile has the constants of one)
+    if (key >= nc && b.nscenes && k > 0 && b.scene_s[k] != b.scene_s[k - 1]) return true;
     if (key >= nc || g.each_cell) return ((uint32_t)k - b.off[key]) % tn == 0;
     const uint32_t z = (key - g.base) % g.d2, cb = key - z;
     if (((uint32_t)k - b.off[cb]) % tn == 0) return true;
