@@ -20,7 +20,8 @@ namespace sphx {
 // (900 kept candidates per tile, 29 chunks), 110 the walk, box cull and lists, 500 the pair terms
 // (5 turns of two neighbours per lane and particle).  1M dam break: 0.96 ms; with hit lists
 // worked through by the whole warp and folded back lane by lane (1,502 instructions, of which
-// the lists and folds were half) 1.45 ms.
+// the lists and folds were half) 1.45 ms.  Five CTAs per SM leave 96 registers, at which 8 bytes
+// spill; four without spill 1.00 ms.
 constexpr int kDensityRing = 16;
 struct DensitySmem {
     float cx[kDensityRing * 32], cy[kDensityRing * 32], cz[kDensityRing * 32];

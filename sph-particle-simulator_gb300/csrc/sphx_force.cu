@@ -19,7 +19,7 @@ namespace sphx {
 // Bound: instruction issue (64% of the slots with 3 warps per scheduler) and the FP32 pipe
 // (58%; a packed instruction holds it two cycles): about 1,130 warp instructions per particle
 // in 5.7 turns, each finishing one pair of neighbours per lane and starting the next.  1M dam
-// break, force + leapfrog: 1.44 ms (1.53 with 12 chunks and a branch at each new mask); walking
+// break, force + leapfrog: 1.41 ms (1.53 with 12 chunks and a branch at each new mask); walking
 // and culling the candidates again instead of reading the density pass's list 1.71 ms; with hit lists, terms passed through shared memory and
 // in-order folds by their lanes (2,479 instructions) 2.60 ms; one neighbour per turn with the
 // compiler's division and square root 2.72 ms, pairs 2.08, staged by asynchronous copies 1.83,

@@ -155,7 +155,8 @@ struct Buffers {
     float4* vel4;     // insertion order: vx, vy, vz, 0
     float4* pos4_s;   // cell-sorted copies
     float4* vel4_s;
-    float4* aux4_s;   // cell-sorted: rho, P, (m/rho) mu, 1/(2 rho); precision mode: see density_out
+    float4* aux4_s;   // cell-sorted: rho, P, (m/rho) mu, 1/(2 rho) or 0 (pair_range);
+                      // precision mode: rho, P, m/(2 rho)
     float4* acc4_s;   // cell-sorted accelerations of the last step/eval
     int4* cell4;      // precision mode, insertion order: cell (x, y, z), w = 1 if not finite
     int4* cell4_s;    // precision mode, cell-sorted copy

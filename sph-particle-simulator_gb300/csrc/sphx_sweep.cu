@@ -198,13 +198,13 @@ __device__ __forceinline__ void sweep_density_spread(const StepConst& c, const B
 }
 
 // The density epilogue of the lane's particle: rho, P and the force sweep's per-candidate
-// factors (rho, P, m / (2 rho), (m / rho) mu).
+// factor m / (2 rho) (the viscosity's is a multiple of it: StepConst::sw_kappa).
 __device__ __forceinline__ void density_out(const StepConst& c, const Buffers& b, int i,
                                             bool cells, float mi, const KSum& rk) {
     const float rho = cells ? rk.value() * sweep_w_scale(c) : xmul(mi, c.w0);
     const float P = xmul(c.gas, xsub(rho, c.rest));
     const float mr = xdiv(mi, rho);
-    b.aux4_s[i] = make_float4(rho, P, 0.5f * mr, mr * c.visc);
+    b.aux4_s[i] = make_float4(rho, P, 0.5f * mr, 0.0f);
 }
 
 // A tile with a particle more than kSpreadCells cells from its frame (listed for the
@@ -253,7 +253,8 @@ __device__ __forceinline__ uint32_t sweep_density_chunk(const StepConst& c, cons
 // particle, of which 415 are the chunks (27.7 per pair of candidates, 29 chunks a tile) and
 // most of the rest the walk of 55 chunks of 32, its conversion to the tile's frame and its box
 // cull.  1M dam break: 0.74 ms (0.76 with a sweep of each culled chunk on its own, without the
-// list for the force pass).
+// list for the force pass).  Six CTAs per SM leave 80 registers, at which up to 12 bytes spill;
+// five without spill take as long.
 template <int kKern, bool kCut>
 __global__ void __launch_bounds__(128, 6) k_density_sweep(const StepConst c, const Buffers b,
                                                           DevState* ds) {
@@ -568,9 +569,10 @@ __device__ __forceinline__ void force_out(const StepConst& c, const Buffers& b, 
 }
 
 // Bound: the FP32 pipe (27 packed instructions of two cycles per pair of candidates, 374 pairs
-// a tile and lane).  1M dam break: 0.82 ms; walking and culling the candidates again instead
+// a tile and lane).  1M dam break: 0.78 ms; walking and culling the candidates again instead
 // of reading the density pass's list (1.8 times the instructions) 1.14 ms, sweeping all kept
-// candidates 1.20 ms.
+// candidates 1.20 ms.  Four CTAs per SM leave 128 registers, at which up to 28 bytes spill in
+// some forms; three without spill 0.84 ms.
 template <bool kIntegrate, int kKern, bool kCut>
 __global__ void __launch_bounds__(128, 4) k_force_sweep(const StepConst c, const Buffers b,
                                                         DevState* ds) {
