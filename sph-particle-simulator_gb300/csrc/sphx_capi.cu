@@ -238,7 +238,7 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
                      both(-3.0f), both(kCoincident)};
     s.pair = PairConst{both(-h), both(h), both(s.rcp_h), both(-s.h_sq), both(s.rcp_hsq),
                        both(s.sigma), both(-s.sigma), both(s.gas), both(s.rest), both(s.wnorm),
-                       both(s.wl), 0};
+                       both(s.wl)};
     s.sw_cs = s.cs * s.rcp_h;  // 2 exactly for r_search = 2h
     s.sw_r2 = s.r2 * s.rcp_hsq;
     s.sw_r2m = s.sw_r2 * 1.0001f;
@@ -257,7 +257,7 @@ void step_const_from_params(const sphx_params& p, size_t n, int kernel, int mode
     const float multiple = kernel == SPHX_KERNEL_CUBIC_SPLINE ? -4.0f : 2.0f;
     const bool normal = std::min(std::fabs(kl), std::fabs(s.sw_kg)) >= 0x1p-126f;
     s.sw_kappa = (normal ? 2.0f * kl / s.sw_kg : multiple * s.rcp_h) * s.visc;
-    s.pair.kappa = both(s.sw_kappa);
+    s.sw_kappa2 = both(s.sw_kappa);
 }
 
 }  // namespace sphx

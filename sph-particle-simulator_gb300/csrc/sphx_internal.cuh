@@ -43,7 +43,6 @@ struct PairLits {  // numbers
 };
 struct PairConst {  // of the step's parameters
     f32x2 neg_h, h, rcp_h, neg_hsq, rcp_hsq, sigma, neg_sigma, gas, rest, wnorm, wl;
-    f32x2 kappa;  // StepConst::sw_kappa
 };
 
 // Constants of one step, computed on the host in float exactly as the reference does
@@ -69,7 +68,6 @@ struct StepConst {
     // rather than held in registers: cs / h, r^2 / h^2, the same with the box cull's margin,
     // (1e-6 m / h)^2
     float sw_cs, sw_r2, sw_r2m, sw_skip2;
-    float sw_kg, sw_kappa;  // force factors, see sphx_sweep.cu
     int fast_div_h, fast_div_hsq;  // 1: the one-correction sequence is verified for it
     // smoothing kernel (SPHX_KERNEL_*) and the constants its constructor computes in float
     PairLits lit;
@@ -85,6 +83,9 @@ struct StepConst {
     // or in [2^-74.5, r (1 + 2^-23)] (div_nz); the Laplacian's dividends are, too (force_nz = 1),
     // and the gradient's of all pairs without tiny coordinates (2)
     int div_nz, force_nz;
+    // the precision force sweep's factors (sphx_sweep.cu); sw_kappa also as a packed operand
+    float sw_kg, sw_kappa;
+    f32x2 sw_kappa2;
 };
 
 // Device-resident scalars written and read by the kernels of a step.
@@ -187,8 +188,7 @@ struct Buffers {
     // sorted positions of the kept candidates that are a neighbour of some lane.  Every warp of the density grid
     // owns an equal region of the pool and stores its tiles one after another; tile_list[t] =
     // first record and candidates (or rows), or kNoSlot when the tile did not fit in what was left of
-    // the region (the force pass then walks and tests that tile itself); an exact tile of more
-    // than 8 whose particles have no neighbour leaves no candidates.
+    // the region (the force pass then walks and tests that tile itself).
     uint32_t* records = nullptr;
     uint2* tile_list = nullptr;
     unsigned long long record_cap = 0;

@@ -569,7 +569,7 @@ __device__ __forceinline__ void force_out(const StepConst& c, const Buffers& b, 
 }
 
 // Bound: the FP32 pipe (27 packed instructions of two cycles per pair of candidates, 374 pairs
-// a tile and lane).  1M dam break: 0.78 ms; walking and culling the candidates again instead
+// a tile and lane).  1M dam break: 0.81 ms; walking and culling the candidates again instead
 // of reading the density pass's list (1.8 times the instructions) 1.14 ms, sweeping all kept
 // candidates 1.20 ms.  Four CTAs per SM leave 128 registers, at which up to 28 bytes spill in
 // some forms; three without spill 0.84 ms.
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep(const StepConst c, const
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
     const float kg = c.sw_kg;
-    const F2 kappa{c.pair.kappa};
+    const F2 kappa{c.sw_kappa2};
     const TileQueue queue(&ds->work[1], b.num_sms);
     for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(128, 4) k_force_sweep_spread(const StepConst c
     const Geom g = grid_geom(ds);
     const SweepUnits U = sweep_units(c);
     const float kg = c.sw_kg;
-    const F2 kappa{c.pair.kappa};
+    const F2 kappa{c.sw_kappa2};
     const TileQueue queue(&ds->spread_work[1], b.num_sms);
     for (uint32_t t = queue.start(); t < ntiles; t = queue.next(lane)) {
         Tile T;
