@@ -143,12 +143,9 @@ __global__ void __launch_bounds__(128, 5) k_density(const StepConst cp, const Bu
             head = __reduce_min_sync(kFull, at.need());
         }
         if (b.records) {
-            // (particles without a neighbour leave an empty list)
-            const bool alone = !__any_sync(kFull, nn > (self >= 0 ? 1u : 0u));
-            const bool fits = alone || tested <= room;
-            if (lane == 0)
-                b.tile_list[t] = make_uint2(fits ? region.cur : kNoSlot, alone ? 0u : (uint32_t)kept);
-            if (fits && !alone) region.cur += 2u * (uint32_t)tested;
+            const bool fits = tested <= room;
+            if (lane == 0) b.tile_list[t] = make_uint2(fits ? region.cur : kNoSlot, (uint32_t)kept);
+            if (fits) region.cur += 2u * (uint32_t)tested;
         }
         if (valid) {
             const float P = xmul(c.gas, xsub(rho, c.rest));

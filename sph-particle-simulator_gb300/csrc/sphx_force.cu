@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
         const uint2 list = b.records ? b.tile_list[t] : make_uint2(kNoSlot, 0u);
         const bool listed = list.x != kNoSlot;
         const uint32_t* rec = b.records + (size_t)list.x * 32 + lane;
-        const int nlist = listed ? (int)list.y : 0;  // candidates
+        // candidates; a single one is a lone particle's own
+        const int nlist = listed && list.y > 1 ? (int)list.y : 0;
         uint32_t ahead = lane < nlist ? __ldcs(rec) : 0u;  // the next chunk's, read ahead
         TileBox B;
         int nseg = 0;
@@ -188,9 +189,9 @@ __global__ void __launch_bounds__(128, 3) k_force(const StepConst cp, const Buff
         pair.qa = pair.qb = 0;
         pair.start(lit, xi, xi, xi);
         int need = 0;  // first chunk the lane still needs
-        // A tile without neighbours has an empty list and no turns (1M lone particles 1.51 ms, with
-        // one round of turns over their own candidates 2.13).  The Wendland kernel takes one turn
-        // even so (1.68 ms): with the test its loop is 1.5% slower wherever there are neighbours.
+        // A lone particle takes no turns (1M lone particles 1.56 ms, with a round of turns over its
+        // own candidate 2.15).  The Wendland kernel takes one even so (1.82 ms): with the test its
+        // loop is 1.5% slower wherever there are neighbours.
         while (kKern == SPHX_KERNEL_WENDLAND_C2 || !listed || nlist > 0) {
             cp_async_wait_all();
             __syncwarp();  // staged chunks are in place, every lane is done with those before head
