@@ -85,8 +85,7 @@ typedef struct sphx_tuning {
     int tile_particles;    /* particles of one cell column per warp work item (tile), 1..32;
                               0 = chosen by the set's size (8 up to 65,536 particles in exact
                               mode, else 32; reported as 32) */
-    int bulk_copy;         /* accepted and reported back; the force pass stages its candidates
-                              by asynchronous copies whatever its value */
+    int bulk_copy;         /* accepted and reported back, without effect */
 } sphx_tuning;
 
 /* PerformanceStats (src/sph_engine.h:51-59) plus GPU-side diagnostics. */

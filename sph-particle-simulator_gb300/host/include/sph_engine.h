@@ -138,8 +138,8 @@ class SPHEngine {
     void push_params();
     void sync_to_host() const;   // device -> host mirror, when the device is newer
     void sync_to_device();       // host mirror -> device, when the host changed
-    void host_will_change();
-    void host_will_clear();     // call before mutating the host mirror
+    void host_will_change();     // call before mutating the host mirror
+    void host_will_clear();      // the same before dropping every particle of it
     void replace_particles(const std::vector<Particle>& ps);
     void stage_append(size_t from);  // mirror particles [from, size) -> upload region
     void copy_field(int field, float* out) const;

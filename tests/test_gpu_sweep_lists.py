@@ -49,3 +49,21 @@ def test_lengths_whose_kernel_gradient_underflows(built, kernel, h):
     prm = I.params16(smoothing_length=h, neighbor_search_radius=2 * h)
     acc = evaluate(pos, vel, np.full(len(pos), 2.0 ** 120, np.float32), prm, kernel=kernel)["acc"]
     assert np.array_equal(acc, np.tile(np.float32([0.0, prm[6], 0.0]), (300, 1)))
+
+
+@pytest.mark.parametrize("kernel", [sphx.KERNEL_CUBIC_SPLINE, sphx.KERNEL_WENDLAND_C2])
+def test_tiles_without_room_for_their_list(built, kernel):
+    """Six clumps of 16,000 particles within reach of each other: 3,000 tiles that need 500
+    records each.  A pool of four records a particle of a capacity of 300,000 has 400 for each,
+    the one of a larger context enough; the two passes sum the same terms in other chunks."""
+    rng = np.random.default_rng(3)
+    centre = 0.3 * np.arange(6)[:, None, None] * np.ones(3)
+    pos = (centre + 0.014 * rng.random((6, 16_000, 3))).astype(np.float32).reshape(-1, 3)
+    vel = (0.1 * rng.standard_normal(pos.shape)).astype(np.float32)
+    mass = np.full(len(pos), 1e-3, np.float32)
+    prm = I.params16(gas_constant=2e-3, xmax=3, ymax=3, zmax=3)
+    a, b = (evaluate(pos, vel, mass, prm, capacity=c, kernel=kernel) for c in (300_000, 3_000_000))
+    assert a["rho"].tobytes() == b["rho"].tobytes()
+    # 16,000 terms of a few ulp (2^-23) each, of at most the largest acceleration's size in sum
+    scale = np.abs(b["acc"]).max()
+    assert np.abs(a["acc"].astype(np.float64) - b["acc"]).max() < 16 * 2.0 ** -23 * scale
